@@ -678,6 +678,9 @@ def attention(q: torch.Tensor, pages: torch.Tensor, meta, ctx, out: torch.Tensor
                                       grid_context=min(layout, max(1, ctx.max_context)))
         else:
             attention_prefill(q, pages, meta.block_tables, ctx.pre_tiles, out, nh, nkv, hd, scale, window)
+    if not pre_ok and attention_rows_tile_takes(q, pages, hd, hd, ctx):
+        attention_rows_tile(q, pages, meta.block_tables, ctx.pre_tiles, out, nh, nkv, hd, hd, pages.shape[3], scale, window)
+        pre_ok = True
     if not dec_ok and not pre_ok:
         return attention_rows(q, pages, meta.block_tables, ctx.token_seg, ctx.positions, out, nh, nkv, hd, scale, window)
     if ctx.num_pre and not pre_ok:
@@ -833,6 +836,35 @@ def attention_rows_biased(q: torch.Tensor, cache_layer: torch.Tensor, block_tabl
                                           nkv, hd, vd, page_size, block_tables.shape[1], ctypes.c_float(scale), window, _p(dist_bias),
                                           0 if dist_bias is None else dist_bias.shape[0], int(v_in_key), int(v_share), out_ld, _p(gate), gate_ld, _dt(q), _stream()),
            "attention_rows_biased")
+    return out
+
+
+def attention_rows_tile_takes(q: torch.Tensor, cache_layer: torch.Tensor, hd: int, vd: int, ctx) -> bool:
+    """Whether a batch's prompt portions take attention_rows_tile: float32, heads and values of multiples of four up to 128, rows that start on
+    16 bytes."""
+    return (q.dtype == torch.float32 and bool(ctx.num_pre) and ctx.pre_tiles is not None and q.data_ptr() % 16 == 0 and cache_layer.data_ptr() % 16 == 0
+            and bool(lib().vk_attention_rows_tile_takes(hd, vd)))
+
+
+def attention_rows_tile(q: torch.Tensor, cache_layer: torch.Tensor, block_tables: torch.Tensor, tiles: torch.Tensor, out: torch.Tensor, nh: int, nkv: int,
+                        hd: int, vd: int, page_size: int, scale: float, window: int = 0, dist_bias: Optional[torch.Tensor] = None, v_in_key: bool = False,
+                        v_share: int = 1, gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """attention_rows_biased of the tokens of prompt portions in float32, bit for bit, 32 neighbouring tokens a block.  tiles int32 [n, 4]: first
+    token, rows (1..64), position of the first token, segment."""
+    _req(q, "q", torch.float32, 2); _req(cache_layer, "cache_layer", torch.float32); _req(block_tables, "block_tables", torch.int32, 2)
+    _req(tiles, "tiles", torch.int32, 2)
+    T = q.shape[0]
+    out_ld = _out_rows(out, q.dtype, T, nh * vd, "attention_rows_tile")
+    gate_ld = _gate_rows(gate, T, nh, "attention_rows_tile")
+    if q.shape[1] != nh * hd or _page_size_of(cache_layer, nkv, hd, 0 if v_in_key else vd, v_share) != page_size or tiles.shape[1] != 4:
+        raise KernelError("attention_rows_tile: shapes do not fit the head counts")
+    if dist_bias is not None:
+        _req(dist_bias, "dist_bias", torch.float32, 2)
+        if dist_bias.shape[1] != nh:
+            raise KernelError("attention_rows_tile: the bias table is not [distances, heads]")
+    _check(lib().vk_attention_rows_tile(_p(q), _p(cache_layer), _p(block_tables), _p(tiles), _p(out), tiles.shape[0], nh, nkv, hd, vd, page_size,
+                                        block_tables.shape[1], ctypes.c_float(scale), window, _p(dist_bias), 0 if dist_bias is None else dist_bias.shape[0],
+                                        int(v_in_key), int(v_share), out_ld, _p(gate), gate_ld, _stream()), "attention_rows_tile")
     return out
 
 
@@ -1000,6 +1032,9 @@ def attention_biased(q: torch.Tensor, pages: torch.Tensor, meta, ctx, out: torch
     if pre_ok:
         attention_prefill_biased(q, pages, meta.block_tables, ctx.pre_tiles, out, nh, nkv, hd, vd, page_size, scale, window, dist_bias, v_in_key, v_share,
                                  gate)
+    if not pre_ok and attention_rows_tile_takes(q, pages, hd, vd, ctx):
+        attention_rows_tile(q, pages, meta.block_tables, ctx.pre_tiles, out, nh, nkv, hd, vd, page_size, scale, window, dist_bias, v_in_key, v_share, gate)
+        pre_ok = True
     if not dec_ok and not pre_ok:
         return rows(None)
     if ctx.num_pre and not pre_ok:
@@ -1791,6 +1826,9 @@ def attention_mixed(q: torch.Tensor, pages: torch.Tensor, meta, ctx, out: torch.
                               cap, mix, vfreq, window, ctx.dec_tokens)
     if pre_ok:
         attention_mixed_prefill(q, pages, meta.block_tables, ctx.pre_tiles, out, nh, nkv, hd, vd, page_size, scale, cap, mix, vfreq)
+    if not pre_ok and attention_rows_tile_takes(q, pages, hd, vd, ctx):
+        attention_rows_tile(q, pages, meta.block_tables, ctx.pre_tiles, out, nh, nkv, hd, vd, page_size, scale, window, dist_bias, v_in_key, v_share, gate)
+        pre_ok = True
     if not dec_ok and not pre_ok:
         return rows(None)
     if ctx.num_pre and not pre_ok:
