@@ -1826,9 +1826,6 @@ def attention_mixed(q: torch.Tensor, pages: torch.Tensor, meta, ctx, out: torch.
                               cap, mix, vfreq, window, ctx.dec_tokens)
     if pre_ok:
         attention_mixed_prefill(q, pages, meta.block_tables, ctx.pre_tiles, out, nh, nkv, hd, vd, page_size, scale, cap, mix, vfreq)
-    if not pre_ok and attention_rows_tile_takes(q, pages, hd, vd, ctx):
-        attention_rows_tile(q, pages, meta.block_tables, ctx.pre_tiles, out, nh, nkv, hd, vd, page_size, scale, window, dist_bias, v_in_key, v_share, gate)
-        pre_ok = True
     if not dec_ok and not pre_ok:
         return rows(None)
     if ctx.num_pre and not pre_ok:
