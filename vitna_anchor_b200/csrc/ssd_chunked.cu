@@ -16,6 +16,7 @@
 // to three blocks a multiprocessor; a tile of tcgen05 (128 rows) would be half empty.
 //
 // Which chunk a block has is worked out from the segments' starts on the device, so the launches depend on the step's counts alone.
+#include "chunks.cuh"
 #include "delta_common.cuh"
 
 namespace vk {
@@ -45,39 +46,6 @@ __device__ __forceinline__ uint32_t sc_pack(float lo, float hi) {
 // the parts that rounding (a, b) to bfloat16 leaves over, again in bfloat16
 __device__ __forceinline__ uint32_t sc_pack_rest(float a, float b, uint32_t hi) {
     return sc_pack(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
-}
-
-struct SscChunk { int seg, first, rows; };      // segment (-1: this block has no chunk), first token, rows
-
-// The chunk with number n: segments have ceil(length / 64) chunks each, numbered one after another.
-__device__ __forceinline__ SscChunk ssc_find(int n, const int32_t* __restrict__ seg_starts, int segments, int* sh) {
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        int base = 0, found = 0;
-        for (int s0 = 0; s0 < segments && !found; s0 += 32) {
-            const int s = s0 + lane;
-            const int a = s < segments ? seg_starts[s] : 0, b = s < segments ? seg_starts[s + 1] : 0;
-            const int mine = (b - a + SC_Q - 1) / SC_Q;
-            int upto = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, upto, o);
-                if (lane >= o) upto += v;
-            }
-            const int lo = base + upto - mine;
-            const bool here = n >= lo && n < lo + mine;
-            if (here) {
-                sh[0] = s;
-                sh[1] = a + (n - lo) * SC_Q;
-                sh[2] = min(SC_Q, b - sh[1]);
-            }
-            found = __any_sync(0xffffffffu, here);
-            base += __shfl_sync(0xffffffffu, upto, 31);
-        }
-        if (!found && lane == 0) sh[0] = -1;
-    }
-    __syncthreads();
-    return SscChunk{sh[0], sh[1], sh[2]};
 }
 
 // rows x cols bfloat16 from src (rows ld apart) into dst (rows COLS + 8 apart), zeros up to ROWS x COLS (COLS a multiple of 8)
@@ -134,12 +102,12 @@ __global__ void __launch_bounds__(SC_THREADS) ssd_chunk_state_kernel(const __nv_
                                                                      float* __restrict__ whole, int C, int H, int G, int N, int P) {
     extern __shared__ __align__(16) unsigned char ss_raw[];
     __shared__ float L[SC_Q], dt[SC_Q];
-    __shared__ int find[3];
+    __shared__ int find[4];
     constexpr int LDB = NP + 8;
     __nv_bfloat16* sb = reinterpret_cast<__nv_bfloat16*>(ss_raw);       // [64][LDB]
     __nv_bfloat16* sx = sb + SC_Q * LDB;                                // [64][SC_LD] high parts of w x (first: x itself)
     __nv_bfloat16* sl = sx + SC_Q * SC_LD;                              // [64][SC_LD] low parts
-    const SscChunk ch = ssc_find(blockIdx.x, seg_starts, segments, find);
+    const Chunk ch = find_chunk<SC_Q>(blockIdx.x, seg_starts, segments, find);
     if (ch.seg < 0) return;
     const int h = blockIdx.y, p0 = blockIdx.z * SC_P, pc = min(SC_P, P - p0), g = h / (H / G);
     const __nv_bfloat16* base = xbc + (size_t)ch.first * C;
@@ -212,11 +180,8 @@ __global__ void __launch_bounds__(256) ssd_chunk_scan_kernel(const float* __rest
                                                              __nv_bfloat16* __restrict__ lo, int H, int NPe) {
     __shared__ int base_sh;
     const int seg = blockIdx.z, h = blockIdx.y;
-    if (threadIdx.x < 32) {                                             // chunks of the segments before this one
-        int n = 0;
-        for (int s = threadIdx.x; s < seg; s += 32) n += (seg_starts[s + 1] - seg_starts[s] + SC_Q - 1) / SC_Q;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    if (threadIdx.x < 32) {
+        const int n = first_chunk_of<SC_Q>(seg, seg_starts);
         if (threadIdx.x == 0) base_sh = n;
     }
     __syncthreads();
@@ -270,14 +235,14 @@ __global__ void __launch_bounds__(SC_THREADS) ssd_chunk_out_kernel(const __nv_bf
                                                                    float* __restrict__ y, int C, int H, int G, int N, int P) {
     extern __shared__ __align__(16) unsigned char so_raw[];
     __shared__ float L[SC_Q], dt[SC_Q];
-    __shared__ int find[3];
+    __shared__ int find[4];
     constexpr int LDB = NP + 8;
     __nv_bfloat16* sc = reinterpret_cast<__nv_bfloat16*>(so_raw);       // [64][LDB]
     __nv_bfloat16* sb = sc + SC_Q * LDB;                                // [64][LDB]
     __nv_bfloat16* sx = sb + SC_Q * LDB;                                // [64][SC_LD]
     __nv_bfloat16* sh = sx + SC_Q * SC_LD;                              // [NP][SC_LD] the state before the chunk, high parts
     __nv_bfloat16* sl = sh + NP * SC_LD;                                // [NP][SC_LD] low parts
-    const SscChunk ch = ssc_find(blockIdx.x, seg_starts, segments, find);
+    const Chunk ch = find_chunk<SC_Q>(blockIdx.x, seg_starts, segments, find);
     if (ch.seg < 0) return;
     const int h = blockIdx.y, p0 = blockIdx.z * SC_P, pc = min(SC_P, P - p0), g = h / (H / G);
     const __nv_bfloat16* base = xbc + (size_t)ch.first * C;

@@ -9,8 +9,9 @@ With H heads, keys and queries of size dim and values of size vdim:
 
 The five projections q, k, v, g and W_a1 x are ONE product with float32 results; the wide half of the decays' projection, the
 decays (through their logarithm), the state and the output's norm are float32.  A request's state lives in its state slot and is
-carried from step to step; the recurrence runs token after token in both dtypes, so the result does not depend on how a prompt is
-cut.  All launches depend on the step's counts and device arrays alone.
+carried from step to step.  A prompt's step in bfloat16 runs the recurrence in chunks on the tensor cores (float32 operands in parts, float32
+sums); short steps, float32 and heads the chunks do not take run it token after token.  All launches depend on the step's counts and
+device arrays alone.
 """
 from __future__ import annotations
 
@@ -22,6 +23,8 @@ from .base import Mixer, StepContext
 
 
 class GatedLinearAttention(Mixer):
+    CHUNKED_FROM = 64       # bfloat16 steps of more tokens than this run the recurrence in chunks
+
     def __init__(self, hidden: int, num_heads: int, dim: int, vdim: int, tau: float, w_in: torch.Tensor, w_a2: torch.Tensor, a_bias: torch.Tensor,
                  norm_weight: torch.Tensor, w_out: torch.Tensor, eps: float):
         """w_in: W_q | W_k | W_v | W_g | W_a1 stacked by rows ([2 H dim + 2 H vdim + rank, hidden], compute dtype); w_a2 [H dim, rank] and
@@ -56,7 +59,11 @@ class GatedLinearAttention(Mixer):
             raise ValueError("a recurrent mixer has no cache that another run could read")
         T, ws, HV = ctx.num_tokens, ctx.workspace, self.H * self.vdim
         proj = ops.linear(xn, self.w_in, ws.rows("gla.proj", T, self.w_in.shape[0], torch.float32), ops.LINEAR_F32)
+        scratch = None
+        if T > self.CHUNKED_FROM and ctx.dtype == torch.bfloat16 and not ctx.decode_only and ops.memory_chunked_takes(proj.shape[1], self.dim, self.vdim):
+            scratch = ws.flat(f"gla.chunks/{self.H}/{self.dim}/{self.vdim}",
+                              ops.gla_chunked_scratch_bytes(ws.max_tokens, ws.max_segments, self.H, self.dim, self.vdim), torch.uint8)
         out = ops.gla(proj, self.a_off, self.a2t, self.a_bias, self.tau, self.norm_weight, self.eps, ctx, cache.state,
                       ws.rows("gla.decay", T, self.H * self.dim, torch.float32), ws.rows("gla.o", T, HV, torch.float32),
-                      ws.rows("gla.out", T, HV, ctx.dtype), self.H, self.dim, self.vdim, self.gate_off)
+                      ws.rows("gla.out", T, HV, ctx.dtype), self.H, self.dim, self.vdim, self.gate_off, chunk_scratch=scratch)
         ops.linear(out, self.w_out, residual, ops.LINEAR_ACC_F32)

@@ -9,8 +9,9 @@ With H heads, keys and queries of size dim and values of size vdim:
     out = W_o (o / rms(o) per head * w_norm * sigmoid(W_g x))                                  w_norm over all heads' values
 
 The six projections are ONE product with float32 results; gates, the running maximum, the state and the output's norm are float32.
-A request's state lives in its state slot and is carried from step to step; the recurrence runs token after token in both dtypes, so
-the result does not depend on how a prompt is cut.  All launches depend on the step's counts and device arrays alone.
+A request's state lives in its state slot and is carried from step to step.  A prompt's step in bfloat16 runs the recurrence in chunks on the
+tensor cores (float32 operands in parts, float32 sums); short steps, float32 and heads the chunks do not take run it token after token.  All
+launches depend on the step's counts and device arrays alone.
 """
 from __future__ import annotations
 
@@ -22,6 +23,8 @@ from .base import Mixer, StepContext
 
 
 class MatrixLSTM(Mixer):
+    CHUNKED_FROM = 64       # bfloat16 steps of more tokens than this run the recurrence in chunks
+
     def __init__(self, hidden: int, num_heads: int, dim: int, vdim: int, gate_cap: float, w_in: torch.Tensor, gate_bias: torch.Tensor,
                  norm_weight: torch.Tensor, w_out: torch.Tensor, eps: float):
         """w_in: W_q | W_k | W_v | W_g | W_i | W_f stacked by rows ([2 H dim + 2 H vdim + 2 H, hidden], compute dtype); gate_bias: b_i | b_f."""
@@ -51,6 +54,10 @@ class MatrixLSTM(Mixer):
             raise ValueError("a recurrent mixer has no cache that another run could read")
         T, ws, HV = ctx.num_tokens, ctx.workspace, self.H * self.vdim
         proj = ops.linear(xn, self.w_in, ws.rows("mlstm.proj", T, self.w_in.shape[0], torch.float32), ops.LINEAR_F32)
+        scratch = None
+        if T > self.CHUNKED_FROM and ctx.dtype == torch.bfloat16 and not ctx.decode_only and ops.memory_chunked_takes(proj.shape[1], self.dim, self.vdim):
+            scratch = ws.flat(f"mlstm.chunks/{self.H}/{self.dim}/{self.vdim}",
+                              ops.mlstm_chunked_scratch_bytes(ws.max_tokens, ws.max_segments, self.H, self.dim, self.vdim), torch.uint8)
         out = ops.mlstm(proj, self.gate_bias, self.cap, self.norm_weight, self.eps, ctx, cache.state, ws.rows("mlstm.o", T, self.H * (self.vdim + 2), torch.float32),
-                        ws.rows("mlstm.out", T, HV, ctx.dtype), self.H, self.dim, self.vdim)
+                        ws.rows("mlstm.out", T, HV, ctx.dtype), self.H, self.dim, self.vdim, chunk_scratch=scratch)
         ops.linear(out, self.w_out, residual, ops.LINEAR_ACC_F32)
