@@ -59,6 +59,32 @@ struct TcExtra {
     int tok_ld, tok_off, tok_vocab;
 };
 
+// A warp's 32 x 32 float32 sums, a row a thread, into rows row0 .. of the matrix out [M, N] at column col: through `box`, 4 KB of shared memory of the warp's own
+// (16-byte pieces, turned by the row so that neither side meets a bank twice), so that an instruction writes whole rows' 128 bytes.  A thread that
+// stored its own row touched 32 lines an instruction, and where N is not a multiple of four it did so four bytes at a time: 38 us of a
+// 2,048 x 1,746 x 576 product whose operands and results are 7 us of traffic.
+__device__ __forceinline__ void store_rows_f32(float* box, const uint32_t* r, float* __restrict__ out, int row0, int col, int M, int N, int lane) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) *reinterpret_cast<uint4*>(box + lane * 32 + ((j ^ (lane & 7)) << 2)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+    __syncwarp();
+    if (N % 4 == 0) {                                   // (columns come in whole pieces of four)
+        const int piece = lane & 7;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int row = 4 * i + (lane >> 3);
+            const float4 v = *reinterpret_cast<const float4*>(box + row * 32 + ((piece ^ (row & 7)) << 2));
+            if (row0 + row < M && col + 4 * piece < N) *reinterpret_cast<float4*>(out + (size_t)(row0 + row) * N + col + 4 * piece) = v;
+        }
+    } else {
+#pragma unroll 8
+        for (int row = 0; row < 32; row++) {
+            const float v = box[row * 32 + ((((lane >> 2) ^ (row & 7)) << 2) | (lane & 3))];
+            if (row0 + row < M && col + lane < N) out[(size_t)(row0 + row) * N + col + lane] = v;
+        }
+    }
+    __syncwarp();
+}
+
 template <int BN, int EPI>
 __global__ void __launch_bounds__(TC_THREADS) linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                     const __grid_constant__ CUtensorMap map_w,
@@ -311,7 +337,9 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tcgen05_kernel(const __grid
                 tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + c, r);
                 const int col = n0 + c;
                 const bool whole = col + 32 <= N;
-                if (row >= M || col >= N) {
+                if (EPI == TC_F32) {               // (the stages are free: every product has read them)
+                    store_rows_f32(reinterpret_cast<float*>(smem + quarter * 4096), r, reinterpret_cast<float*>(out), m0 + quarter * 32, col, M, N, lane);
+                } else if (row >= M || col >= N) {
                     // nothing of this thread's to store
                 } else if (EPI == TC_TOKEN) {
                     int id = ex.tok_ids[row];
@@ -408,6 +436,8 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tcgen05_kernel(const __grid
 // the wider tile would be mostly empty.
 constexpr int TW_BN = 256, TW_STAGES = 4, TW_THREADS = 320;      // warps 0 and 1 feed and issue; eight warps drain the accumulators
 
+__host__ __device__ constexpr uint32_t wide_boxes(int epi) { return epi == TC_ACC || epi == TC_F32 ? 8 * 4096 : 0; }
+
 template <int EPI, int HD = 0, int BNW = TW_BN>
 __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                          const __grid_constant__ CUtensorMap map_w,
@@ -417,7 +447,8 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
     constexpr uint32_t TM_COLS = 2 * BNW <= 256 ? 256 : 512;      // the two accumulators; tensor memory comes in powers of two
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + TW_STAGES * STAGE_BYTES);
+    uint8_t* boxes = smem + TW_STAGES * STAGE_BYTES;             // 4 KB an epilogue warp, where the epilogue goes through shared memory
+    uint64_t* full = reinterpret_cast<uint64_t*>(boxes + wide_boxes(EPI));
     uint64_t* empty = full + TW_STAGES;
     uint64_t* acc_full = empty + TW_STAGES;       // [2]
     uint64_t* acc_empty = acc_full + 2;           // [2]
@@ -501,41 +532,36 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
             const int b = j & 1;
             const int row = (t % tiles_m) * TC_BM + quarter * 32 + lane, n0 = (t / tiles_m) * tile_cols;
             if (ok && !__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (j >> 1) & 1, wc.cycles))) { if (lane == 0) give_up(wc.error, &failed, 34); ok = false; }
-            // The block's last tile of a residual sum goes out by TMA reductions from shared memory (see the narrow kernel): its
-            // epilogue hides behind no further tile, and every stage is free by now.  The eight epilogue warps meet for it,
-            // so they go on together or not at all.
-            const bool by_tma = EPI == TC_ACC && ex.tma_out && t + (int)gridDim.x >= num_tiles;
-            if (by_tma) {
-                asm volatile("bar.sync 2, 256;" ::: "memory");
-                if (*reinterpret_cast<volatile int*>(&failed)) ok = false;
-            }
-            if (ok && by_tma) {
+            // A residual sum goes out by TMA reductions from shared memory (see the narrow kernel), a box of 32 rows x 32 columns a warp: from the warp's
+            // own box, or, for the block's last tile, whose epilogue hides behind no further tile, from the stages, which are free by now.
+            if (ok && EPI == TC_ACC && ex.tma_out) {
                 tc_fence_after();
                 const uint32_t acc = lane_base + b * BNW;
-                const int r_loc = quarter * 32 + lane;
+                const bool last = t + (int)gridDim.x >= num_tiles;
+                const int row0 = (t % tiles_m) * TC_BM + quarter * 32;
 #pragma unroll 1
                 for (int c = half * (BNW / 2); c < (half + 1) * (BNW / 2); c += 32) {
                     uint32_t r[32];
                     tmem_ld32(acc + c, r);
                     tmem_loaded(r);
-                    uint8_t* box = smem + (c / 32) * (TC_BM * 128) + r_loc * 128;
+                    uint8_t* box = last ? smem + (c / 32) * (TC_BM * 128) + quarter * 4096 : boxes + (warp - 2) * 4096;
+                    if (!last) {                        // the box before this one has been read
+                        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                        __syncwarp();
+                    }
 #pragma unroll
                     for (int q = 0; q < 8; q++)
-                        *reinterpret_cast<uint4*>(box + ((q ^ (r_loc & 7)) << 4)) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                tc_fence_before();
-                asm volatile("bar.sync 2, 256;" ::: "memory");
-                if (warp == 2 && lane == 0) {
-                    const int m0 = (t % tiles_m) * TC_BM;
-                    for (int c = 0; c < BNW; c += 32) {
-                        if (n0 + c < N)
+                        *reinterpret_cast<uint4*>(box + lane * 128 + ((q ^ (lane & 7)) << 4)) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (n0 + c < N && row0 < M)
                             asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
-                                         ::"l"(&map_out), "r"(smem_u32(smem + (c / 32) * (TC_BM * 128))), "r"(n0 + c), "r"(m0) : "memory");
+                                         ::"l"(&map_out), "r"(smem_u32(box)), "r"(n0 + c), "r"(row0) : "memory");
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     }
-                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
                 }
+                tc_fence_before();
             } else if (ok) {
                 tc_fence_after();
                 const uint32_t acc = lane_base + b * BNW;
@@ -640,6 +666,12 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                         tmem_ld32(acc + c, r);
                         tmem_loaded(r);
                         const int col = n0 + c;
+                        if (EPI == TC_F32) {
+                            if (col < N)
+                                store_rows_f32(reinterpret_cast<float*>(boxes + (warp - 2) * 4096), r, reinterpret_cast<float*>(out),
+                                               (t % tiles_m) * TC_BM + quarter * 32, col, M, N, lane);
+                            continue;
+                        }
                         if (row >= M || col >= N) continue;
                         const bool whole = col + 32 <= N;
                         if (EPI == TC_SAME) {
@@ -692,6 +724,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
             __syncwarp();
             if (lane == 0) mbar_arrive_plain(&acc_empty[b]);      // kept even after a failed wait: nobody waits for this warp without a limit
         }
+        if (EPI == TC_ACC && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // the boxes outlive their reductions
     }
     tc_fence_before();
     __syncthreads();
@@ -714,13 +747,13 @@ static bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// out [rows, cols] float32, dense: added into in boxes of 128 rows x 32 columns, 128-byte swizzle.
-static bool make_out_map(CUtensorMap* map, void* base, int rows, int cols) {
+// out [rows, cols] float32, dense: added into in boxes of box_rows x 32 columns, 128-byte swizzle.
+static bool make_out_map(CUtensorMap* map, void* base, int rows, int cols, int box_rows) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return false;
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)cols * 4};
-    cuuint32_t box[2] = {32u, (cuuint32_t)TC_BM};
+    cuuint32_t box[2] = {32u, (cuuint32_t)box_rows};
     cuuint32_t elem[2] = {1, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -734,7 +767,7 @@ static int launch_tc(const CUtensorMap& mx, const CUtensorMap& mw, void* out, in
     TcExtra exx = ex;
     CUtensorMap mo = mx;                               // (a valid map for the epilogues that do not use it)
     exx.tma_out = 0;
-    if (EPI == TC_ACC && N % 4 == 0 && ((uintptr_t)out % 16 == 0) && make_out_map(&mo, out, M, N)) exx.tma_out = 1;
+    if (EPI == TC_ACC && N % 4 == 0 && ((uintptr_t)out % 16 == 0) && make_out_map(&mo, out, M, N, TC_BM)) exx.tma_out = 1;
     auto kern = linear_tcgen05_kernel<BN, EPI>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
@@ -775,11 +808,11 @@ template <int EPI, int HD = 0, int BNW = TW_BN>
 static int launch_wide(const CUtensorMap& mx, const CUtensorMap& mw, void* out, int M, int N, int K, int* error, cudaStream_t stream,
                        const TcExtra& ex = TcExtra{}) {
     const WaitCtl wc = wait_ctl(error, WAIT_FAMILY_LINEAR_WIDE);
-    const size_t smem = (size_t)TW_STAGES * (TC_BM * TC_BK * 2 + BNW * TC_BK * 2) + 1024 + 128;
+    const size_t smem = (size_t)TW_STAGES * (TC_BM * TC_BK * 2 + BNW * TC_BK * 2) + wide_boxes(EPI) + 1024 + 128;
     TcExtra exx = ex;
     CUtensorMap mo = mx;                               // (a valid map for the epilogues that do not use it)
     exx.tma_out = 0;
-    if (EPI == TC_ACC && N % 4 == 0 && ((uintptr_t)out % 16 == 0) && make_out_map(&mo, out, M, N)) exx.tma_out = 1;
+    if (EPI == TC_ACC && N % 4 == 0 && ((uintptr_t)out % 16 == 0) && make_out_map(&mo, out, M, N, 32)) exx.tma_out = 1;
     auto kern = linear_tcgen05_wide_kernel<EPI, HD, BNW>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
