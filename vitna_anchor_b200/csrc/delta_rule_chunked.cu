@@ -1,472 +1,659 @@
-// The gated delta rule over a prompt's portion in chunks: what can be worked out without the state is worked out for all
-// chunks at once, and only a short pass per chunk runs in order.
+// The gated delta rule over a prompt's portion in chunks of 64 tokens: what can be worked out without the state is worked out for all
+// chunks at once, only a short pass per chunk runs in order, and the outputs follow for all chunks at once again.
 //
-// For a chunk of C tokens with the state S before it, L_t = ln(g_1 .. g_t) (the decays up to t, inside the chunk):
+// For a chunk with the state S before it, L_t = ln(g_1 .. g_t) (the decays up to t, inside the chunk):
 //     A[t][i] = beta_t e^(L_t - L_i) (k_t . k_i)   (i < t)          the updates u_t solve  (I + A) U = diag(beta) V - diag(beta e^L) K S
 //     so with  U' = (I + A)^-1 diag(beta) V   and   W = (I + A)^-1 diag(beta e^L) K :     U = U' - W S
 //     P[t][i] = e^(L_t - L_i) (q_t . k_i)          (i <= t)         O = diag(e^L) Q S + P U
-//     S <- e^(L_C) S + (diag(e^(L_C - L)) K)^T U
-// Kernel 1 (a block per chunk and head, all chunks of the step side by side): L, A, P, the triangular solve for U' and W by
-// forward substitution, and the scaled copies of Q and K; everything goes to a scratch.  Kernel 2 (a block per request, head
-// and slice of the state's columns) walks the request's chunks in order with the state slice in shared memory: three small
-// products a chunk.  All float32 on CUDA cores: the decays, beta, the unit vectors and the state are 32-bit quantities of this
-// mixer, and the sums are of float32 values.  The results equal the token-by-token recurrence up to the order of sums.
-// A chunk that reaches past its segment's end is filled with tokens that do nothing.  Inputs are the rows `delta_prepare`
-// writes (q | k | v | log decay | beta).
+//     S <- e^(L_64) S + (diag(e^(L_64 - L)) K)^T U
 //
-// The form with a decay per head AND key channel (template flag CH; inputs are the rows `cdelta_prepare` writes, q | k | v | log
-// decay [H][dk] | beta [H] | ..): L_t is a vector over the key channels, and the decays no longer leave the sums over dk:
-//     A[t][i] = beta_t sum_d k_t[d] k_i[d] e^(L_t[d] - L_i[d]),     P[t][i] = sum_d q_t[d] k_i[d] e^(L_t[d] - L_i[d])
-// (an exponential per pair and channel; for 4 x 4 pieces below the diagonal it is split as e^(L_t - r) e^(r - L_i) with r = L of the
-// piece's last column token, both factors at most 1, which makes eight exponentials a channel for a piece instead of sixteen; a piece's
-// channels are shared out over two to eight threads),
-// W and Qg carry e^(L_t[d]), KgT carries e^(L_C[d] - L_i[d]), and the state's rows decay by the vector e^(L_C[d]), which follows
-// U' in the scratch.  Everything else, the triangular solve and the scan included, is the same code.
+//  delta_chunk_prepare   a block a chunk and head, all chunks side by side: A, P, T = (I + A)^-1 (the four 16 x 16 blocks on the diagonal by substitution, the
+//                        others from them), W and U' as products with T, and the scaled Q and K.
+//  delta_chunk_scan      a block a request, head and 8 or 16 columns of the state walks the request's chunks in order: two small products a chunk, the state's
+//                        slice in registers and, as an operand, in shared memory; leaves U and the state before every chunk.  Chunks' operands arrive by cp.async two
+//                        chunks ahead.
+//  delta_chunk_out       a block a chunk, head and 64 columns, all chunks side by side: O.
+//
+// The decays, beta, the unit vectors and the state are 32-bit quantities of this mixer: products take them as two tf32 parts (tf32.cuh), every other operation is
+// float32.  The results equal the token-by-token recurrence up to the order of sums.  A chunk that reaches past its segment's end is filled
+// with tokens that do nothing.  Inputs are the rows `delta_prepare` writes (q | k | v | log decay | beta).
+//
+// The form with a decay per head AND key channel (template flag CH; inputs are the rows `cdelta_prepare` writes, q | k | v | log decay [H][dk] | beta [H] | ..): L_t is a
+// vector over the key channels, and the decays no longer leave the sums over dk: A[t][i] = beta_t sum_d k_t[d] k_i[d] e^(L_t[d] - L_i[d]), P likewise.  Pairs inside 16
+// tokens are taken one by one; between different sixteens the exponential is split into what the row's sixteen leaves up to its token, what whole
+// sixteens between leave, and what the column's sixteen leaves behind its token, each at most 1.  The state's rows decay by the vector e^(L_64[d]).
+//
+// What bounds it: the scan is a chain of 2 products, 2 barriers a chunk; the other two kernels the tensor cores' rate for three tf32 products.
+#include "chunks.cuh"
 #include "common.cuh"
+#include "tf32.cuh"
 
 namespace vk {
 
-constexpr int DC_THREADS = 256;
+constexpr int DC_C = 64;                    // tokens of a chunk
 constexpr int DC_MAX_TAPS = 16;
-constexpr int DC_MAX_DK = 128;
+constexpr int DC_LDA = DC_C + 8;            // a padded row of a 64 x 64 matrix
 
-__device__ __forceinline__ void dc_cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+// Floats of scratch for one (chunk, head):  W [64][dk] | Kg [64][dk] | Qg [64][dk] | P [64][64] | U', then U [64][dv] | S before the chunk [dv][dk] | e^(L_64)
+// (one, or one a channel), padded to a multiple of four.
+__host__ __device__ __forceinline__ size_t dc_stride(int dk, int dv, bool ch) {
+    return (size_t)DC_C * (3 * dk + DC_C + dv) + (size_t)dk * dv + (ch ? (dk + 3) / 4 * 4 : 4);
 }
 
-// Which segment and which of its chunks the step's chunk number `b` is; false when the step has fewer chunks.
-template <int C>
-__device__ __forceinline__ bool find_chunk(const int32_t* seg_starts, int segments, int b, int& seg, int& c0) {
-    int acc = 0;
-    for (int s = 0; s < segments; s++) {
-        const int n = seg_starts[s + 1] - seg_starts[s];
-        const int nc = (n + C - 1) / C;
-        if (b < acc + nc) { seg = s; c0 = (b - acc) * C; return true; }
-        acc += nc;
-    }
-    return false;
-}
+struct DcArgs {
+    const float* prep;
+    int P;                                  // floats of a row of prep
+    const int32_t* seg_starts;
+    const int32_t* seg_slots;
+    int segments;
+    float* scratch;
+    int G, H, dk, dv;
+};
 
-// Floats of scratch for one (chunk, head):  W [C][dk] | Qg [C][dk] | KgT [dk][C] | P [C][C] | U' [C][dv] | e^(L_C) and padding [4]
-// (with a decay per channel: e^(L_C[d]) for every d, padded to a multiple of four)
-__host__ __device__ __forceinline__ size_t dc_stride(int C, int dk, int dv, bool ch = false) {
-    return (size_t)C * (3 * dk + C + dv) + (ch ? (dk + 3) / 4 * 4 : 4);
-}
+__host__ __device__ __forceinline__ int dc_ldv(int dv) { return (dv + 15) / 16 * 16 + 4; }
 
-// grid (chunks of the step, H); 256 threads = a 16 x 16 arrangement for the products.
-template <int C, bool CH>
-__global__ void __launch_bounds__(DC_THREADS) delta_chunk_prepare_kernel(const float* __restrict__ prep, int P, const int32_t* __restrict__ seg_starts,
-                                                                         const int32_t* __restrict__ seg_slots, int segments,
-                                                                         float* __restrict__ scratch, int G, int H, int dk, int dv) {
-    extern __shared__ __align__(16) float sm[];
-    __shared__ float L[C], beta[C];
-    __shared__ int where[2];
-    const int tid = threadIdx.x, h = blockIdx.y;
-    if (tid == 0) {
-        int seg = -1, c0 = 0;
-        if (!find_chunk<C>(seg_starts, segments, blockIdx.x, seg, c0) || seg_slots[seg] < 0) seg = -1;
-        where[0] = seg;
-        where[1] = c0;
-    }
-    __syncthreads();
-    const int seg = where[0], c0 = where[1];
-    if (seg < 0) return;
-    const int start = seg_starts[seg], n = seg_starts[seg + 1] - start;
-    const int cn = n - c0 < C ? n - c0 : C;
-    const int Cq = 2 * G * dk + H * dv, g = h / (H / G);
-    const int ldk = dk + 1, ldc = C + 1, nr = dv + dk;
-    float* k_s = sm;                       // [C][dk+1]
-    float* q_s = k_s + C * ldk;            // [C][dk+1]
-    float* A_s = q_s + C * ldk;            // [C][C+1]
-    float* P_s = A_s + C * ldc;            // [C][C+1]
-    float* x_s = P_s + C * ldc;            // [C][dv + dk]: the right sides, then the solutions
-    float* Lv = x_s + C * nr;              // CH: [C][dk+1], the decays' logarithms of every channel, then their running sums
+template <int DKP, bool CH>
+__host__ __device__ constexpr int dc_prepare_floats_fixed() { return DC_C * (DKP + 8) * (CH ? 3 : 2) + 2 * DC_C * DC_LDA + (CH ? 4 * DKP : 0); }
 
-    if (tid < C) {
-        const bool on = tid < cn;
-        if (!CH) L[tid] = on ? prep[(size_t)(start + c0 + tid) * P + Cq + h] : 0.0f;
-        beta[tid] = on ? prep[(size_t)(start + c0 + tid) * P + Cq + (CH ? H * dk : H) + h] : 0.0f;
+// grid (chunks, H)
+template <int DKP, bool CH>
+__global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p) {
+    constexpr int LDQ = DKP + 8;
+    extern __shared__ __align__(16) float dp_smem[];
+    __shared__ float L[DC_C], beta[DC_C];
+    __shared__ int find[4];
+    const int LDV = dc_ldv(p.dv);
+    float* sq = dp_smem;                            // [64][LDQ]
+    float* sk = sq + DC_C * LDQ;                    // [64][LDQ]
+    float* sA = sk + DC_C * LDQ;                    // [64][DC_LDA]
+    float* sT = sA + DC_C * DC_LDA;                 // [64][DC_LDA]
+    float* sl = sT + DC_C * DC_LDA;                 // CH: [64][LDQ] the decays' logarithms, then k times what its sixteen leaves behind it
+    float* vec = sl + (CH ? DC_C * LDQ : 0);        // CH: [4][DKP] what whole sixteens leave
+    float* sv = vec + (CH ? 4 * DKP : 0);           // [64][LDV]
+    const Chunk ch = find_chunk<DC_C>(blockIdx.x, p.seg_starts, p.segments, find);
+    if (ch.seg < 0 || p.seg_slots[ch.seg] < 0) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, wm = warp & 1, wn = warp >> 1;
+    const int h = blockIdx.y, dk = p.dk, dv = p.dv, rows = ch.rows, kh = h / (p.H / p.G), Cq = 2 * p.G * dk + p.H * dv;
+    const float* row0 = p.prep + (size_t)ch.first * p.P;
+    for (int e = tid; e < DC_C * (DKP / 4); e += 256) {
+        const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
+        const bool on = r < rows && d < dk;
+        const float* row = row0 + (size_t)(on ? r : 0) * p.P + (on ? d : 0);
+        tf_cp16(sq + r * LDQ + d, row + kh * dk, on);
+        tf_cp16(sk + r * LDQ + d, row + (p.G + kh) * dk, on);
+        if (CH) tf_cp16(sl + r * LDQ + d, row + Cq + h * dk, on);
     }
-    if (CH) {
-        for (int e = tid; e < C * dk; e += DC_THREADS) {
-            const int t = e / dk, d = e - t * dk;
-            Lv[t * ldk + d] = t < cn ? prep[(size_t)(start + c0 + t) * P + Cq + (size_t)h * dk + d] : 0.0f;
-        }
+    const int vp = (LDV - 4) / 4;
+    for (int e = tid; e < DC_C * vp; e += 256) {
+        const int r = e / vp, c = 4 * (e - r * vp);
+        const bool on = r < rows && c < dv;
+        tf_cp16(sv + r * LDV + c, row0 + (size_t)(on ? r : 0) * p.P + 2 * p.G * dk + h * dv + (on ? c : 0), on);
     }
-    for (int e = tid; e < C * dk; e += DC_THREADS) {
-        const int t = e / dk, d = e - t * dk;
-        const float* row = prep + (size_t)(start + c0 + t) * P;
-        k_s[t * ldk + d] = t < cn ? row[(size_t)(G + g) * dk + d] : 0.0f;
-        q_s[t * ldk + d] = t < cn ? row[(size_t)g * dk + d] : 0.0f;
-    }
-    __syncthreads();
-    if (CH) {                               // the decays' logarithms summed up to each token, a channel a thread
-        for (int d = tid; d < dk; d += DC_THREADS) {
-            float acc = 0.0f;
-            for (int t = 0; t < C; t++) { acc += Lv[t * ldk + d]; Lv[t * ldk + d] = acc; }
-        }
-    } else if (tid == 0) {
-        float acc = 0.0f;
-        for (int t = 0; t < C; t++) { acc += L[t]; L[t] = acc; }
-    }
-    __syncthreads();
-    for (int e = tid; e < C * nr; e += DC_THREADS) {
-        const int t = e / nr, c = e - t * nr;
-        float v = 0.0f;
-        if (t < cn) v = c < dv ? beta[t] * prep[(size_t)(start + c0 + t) * P + 2 * G * dk + (size_t)h * dv + c]
-                               : beta[t] * expf(CH ? Lv[t * ldk + (c - dv)] : L[t]) * k_s[t * ldk + (c - dv)];
-        x_s[e] = v;
-    }
-    if (CH) {
-        // k k^T and q k^T with the pairs' decays, in 4 x 4 pieces.  The exponentials make a piece expensive, so the channels of a
-        // piece are shared out: the threads that would have a piece above the diagonal take half of the channels of the piece
-        // mirrored below it, and with C = 32 (a quarter as many pieces as threads) every piece's channels are cut in four again.
-        // The parts of a piece are added in a fixed order, one barrier a part.
-        constexpr int NB = C / 4, NPC = NB * NB, S = DC_THREADS / NPC;
-        for (int e = tid; e < C * ldc; e += DC_THREADS) { A_s[e] = 0.0f; P_s[e] = 0.0f; }
-        const int piece = tid % NPC, dsplit = tid / NPC;
-        int ty = piece / NB, tx = piece % NB;
-        const bool mirror = tx > ty;
-        if (mirror) { const int z = ty; ty = tx; tx = z; }
-        const bool diag = tx == ty;
-        const int parts = diag ? S : 2 * S, part = diag ? dsplit : dsplit * 2 + (mirror ? 1 : 0);
-        float kk[4][4], qk[4][4];
+    tf_commit();
+    if (tid < 32) {                                 // beta, and the sums of the decays' logarithms
+        float carry = 0.0f;
 #pragma unroll
-        for (int a = 0; a < 4; a++)
+        for (int u = 0; u < 2; u++) {
+            const int r = 32 * u + tid;
+            const float* row = row0 + (size_t)(r < rows ? r : 0) * p.P + Cq;
+            beta[r] = r < rows ? row[(CH ? p.H * dk : p.H) + h] : 0.0f;
+            if (!CH) {
+                float s = r < rows ? row[h] : 0.0f;
 #pragma unroll
-            for (int b = 0; b < 4; b++) kk[a][b] = qk[a][b] = 0.0f;
-        for (int d = part * dk / parts; d < (part + 1) * dk / parts; d++) {
-            float kt[4], qt[4], ki[4], lt[4], li[4];
-#pragma unroll
-            for (int a = 0; a < 4; a++) {
-                kt[a] = k_s[(ty * 4 + a) * ldk + d];
-                qt[a] = q_s[(ty * 4 + a) * ldk + d];
-                ki[a] = k_s[(tx * 4 + a) * ldk + d];
-                lt[a] = Lv[(ty * 4 + a) * ldk + d];
-                li[a] = Lv[(tx * 4 + a) * ldk + d];
-            }
-            if (diag) {                     // the exponent of every pair by itself: six below the diagonal, none on or above it
-#pragma unroll
-                for (int a = 0; a < 4; a++)
-#pragma unroll
-                    for (int b = 0; b <= a; b++) {
-                        const float w = b < a ? expf(lt[a] - lt[b]) * ki[b] : ki[b];
-                        kk[a][b] = fmaf(kt[a], w, kk[a][b]);
-                        qk[a][b] = fmaf(qt[a], w, qk[a][b]);
-                    }
-            } else {                        // every row token comes after every column token: e^(L_t - r) e^(r - L_i), r = L of the last
-                const float ref = li[3];    // column token, both factors at most 1
-#pragma unroll
-                for (int a = 0; a < 4; a++) {
-                    const float et = expf(lt[a] - ref);
-                    kt[a] *= et;
-                    qt[a] *= et;
-                    ki[a] *= expf(ref - li[a]);
+                for (int o = 1; o < 32; o <<= 1) {
+                    const float v = __shfl_up_sync(0xffffffffu, s, o);
+                    if (tid >= o) s += v;
                 }
-#pragma unroll
-                for (int a = 0; a < 4; a++)
-#pragma unroll
-                    for (int b = 0; b < 4; b++) {
-                        kk[a][b] = fmaf(kt[a], ki[b], kk[a][b]);
-                        qk[a][b] = fmaf(qt[a], ki[b], qk[a][b]);
-                    }
+                L[r] = carry + s;
+                carry += __shfl_sync(0xffffffffu, s, 31);
             }
-        }
-        for (int ph = 0; ph < 2 * S; ph++) {
-            __syncthreads();
-            if (part == ph) {
-#pragma unroll
-                for (int a = 0; a < 4; a++)
-#pragma unroll
-                    for (int b = 0; b < 4; b++) {
-                        const int t = ty * 4 + a, i = tx * 4 + b;
-                        if (i < t) A_s[t * ldc + i] += beta[t] * kk[a][b];
-                        if (i <= t) P_s[t * ldc + i] += qk[a][b];
-                    }
-            }
-        }
-    } else
-    // k k^T and q k^T in 4 x 4 pieces: thread (ty, tx) has rows ty*4.., columns tx*4.. (C = 64: one piece a thread; C = 32: a quarter idle)
-    {
-        const int ty = tid / 16, tx = tid % 16;
-        if (ty * 4 < C && tx * 4 < C) {
-            float kk[4][4], qk[4][4];
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) kk[a][b] = qk[a][b] = 0.0f;
-            if (tx <= ty) {                 // pieces above the diagonal are never read
-                for (int d = 0; d < dk; d++) {
-                    float kt[4], qt[4], ki[4];
-#pragma unroll
-                    for (int a = 0; a < 4; a++) {
-                        kt[a] = k_s[(ty * 4 + a) * ldk + d];
-                        qt[a] = q_s[(ty * 4 + a) * ldk + d];
-                        ki[a] = k_s[(tx * 4 + a) * ldk + d];
-                    }
-#pragma unroll
-                    for (int a = 0; a < 4; a++)
-#pragma unroll
-                        for (int b = 0; b < 4; b++) {
-                            kk[a][b] = fmaf(kt[a], ki[b], kk[a][b]);
-                            qk[a][b] = fmaf(qt[a], ki[b], qk[a][b]);
-                        }
-                }
-            }
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) {
-                    const int t = ty * 4 + a, i = tx * 4 + b;
-                    const float ratio = i <= t ? expf(L[t] - L[i]) : 0.0f;
-                    A_s[t * ldc + i] = i < t ? beta[t] * ratio * kk[a][b] : 0.0f;
-                    P_s[t * ldc + i] = ratio * qk[a][b];
-                }
         }
     }
+    tf_wait<0>();
     __syncthreads();
-    // (I + A) X = right sides, a column a thread, rows in order
-    for (int c = tid; c < nr; c += DC_THREADS) {
-        for (int t = 1; t < C; t++) {
-            float a0 = x_s[t * nr + c], a1 = 0.0f;
-            int i = 0;
-            for (; i + 1 < t; i += 2) {
-                a0 = fmaf(-A_s[t * ldc + i], x_s[i * nr + c], a0);
-                a1 = fmaf(-A_s[t * ldc + i + 1], x_s[(i + 1) * nr + c], a1);
-            }
-            if (i < t) a0 = fmaf(-A_s[t * ldc + i], x_s[i * nr + c], a0);
-            x_s[t * nr + c] = a0 + a1;
-        }
-    }
-    __syncthreads();
-    float* out = scratch + ((size_t)blockIdx.x * H + h) * dc_stride(C, dk, dv, CH);
+
+    float* out = p.scratch + ((size_t)blockIdx.x * p.H + h) * dc_stride(dk, dv, CH);
     float* W_g = out;
-    float* Q_g = W_g + C * dk;
-    float* K_g = Q_g + C * dk;             // transposed: [dk][C]
-    float* P_g = K_g + C * dk;
-    float* U_g = P_g + C * C;
-    const float LC = CH ? 0.0f : L[C - 1];
-    for (int e = tid; e < C * dk; e += DC_THREADS) {
-        const int t = e / dk, d = e - t * dk;
-        W_g[e] = x_s[t * nr + dv + d];
-        Q_g[e] = expf(CH ? Lv[t * ldk + d] : L[t]) * q_s[t * ldk + d];
-    }
-    for (int e = tid; e < dk * C; e += DC_THREADS) {
-        const int d = e / C, i = e - d * C;
-        K_g[e] = expf(CH ? Lv[(C - 1) * ldk + d] - Lv[i * ldk + d] : LC - L[i]) * k_s[i * ldk + d];
-    }
-    for (int e = tid; e < C * C; e += DC_THREADS) P_g[e] = P_s[(e / C) * ldc + e % C];
-    for (int e = tid; e < C * dv; e += DC_THREADS) U_g[e] = x_s[(e / dv) * nr + e % dv];
+    float* K_g = W_g + DC_C * dk;
+    float* Q_g = K_g + DC_C * dk;
+    float* P_g = Q_g + DC_C * dk;
+    float* U_g = P_g + DC_C * DC_C;
+    float* E_g = U_g + DC_C * dv + (size_t)dk * dv;
+
+    // k k^T and q k^T: a warp has the 16 x 16 pieces (rows 32 wm + 16 m .., columns 16 wn ..), m = 0, 1
+    float kk[2][2][4], qk[2][2][4];
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) kk[m][n][e] = qk[m][n][e] = 0.0f;
     if (CH) {
-        for (int d = tid; d < dk; d += DC_THREADS) U_g[C * dv + d] = expf(Lv[(C - 1) * ldk + d]);
-    } else if (tid == 0) U_g[C * dv] = expf(LC);
-}
-
-// grid (segments, H, column slices); 256 threads; COLS columns of the state a block.  A chunk's operands arrive by cp.async in one of
-// two buffers, a chunk ahead.
-template <int C, int COLS, bool CH>
-__global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __restrict__ scratch, const float* __restrict__ proj, int N,
-                                                               const int32_t* __restrict__ seg_starts, const int32_t* __restrict__ seg_slots,
-                                                               float* __restrict__ state, size_t state_stride, size_t conv_off,
-                                                               float* __restrict__ o, int G, int H, int dk, int dv, int taps) {
-    extern __shared__ __align__(16) float sm[];
-    constexpr int T = 256, RG = T / COLS;                   // row groups: a thread has column tid % COLS and rows tid / COLS + RG * j
-    const int seg = blockIdx.x, h = blockIdx.y, part = blockIdx.z, tid = threadIdx.x;
-    const int slot = seg_slots[seg];
-    if (slot < 0) return;
-    const int start = seg_starts[seg], n = seg_starts[seg + 1] - start;
-    int base = 0;                                            // the step's chunk number of this segment's first chunk
-    for (int s = 0; s < seg; s++) base += (seg_starts[s + 1] - seg_starts[s] + C - 1) / C;
-    const int Cq = 2 * G * dk + H * dv;                     // N: floats of a row of proj
-    const size_t stride = dc_stride(C, dk, dv, CH);
-    const int c = tid % COLS, r0 = tid / COLS, col = part * COLS + c;
-    const bool live = col < dv;
-    float* row = state + (size_t)slot * state_stride;
-
-    const int opnd = C * (3 * dk + C);      // floats of a chunk's W, Qg, KgT and P, which lie in this order
-    const int lds = dk + 4, ldu = C + 4;    // the state's and the updates' slices are kept transposed: a column's values lie together,
-    float* S_s = sm;                        // [COLS][dk + 4]        so that every load below is 16 bytes
-    float* U_s = S_s + COLS * lds;          // [COLS][C + 4]
-    float* bufs = U_s + COLS * ldu;         // two buffers of `opnd` floats
-    for (int e = tid; e < dk * COLS; e += T) {
-        const int cc = e / dk, d = e - cc * dk, gc = part * COLS + cc;
-        S_s[cc * lds + d] = gc < dv ? row[((size_t)h * dv + gc) * dk + d] : 0.0f;
-    }
-    for (int e = tid; e < opnd / 4; e += T) dc_cp_async16(bufs + e * 4, scratch + ((size_t)base * H + h) * stride + e * 4);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    int turn = 0;
-    for (int c0 = 0, b = base; c0 < n; c0 += C, b++, turn ^= 1) {
-        const float* in = scratch + ((size_t)b * H + h) * stride;
-        const int cn = n - c0 < C ? n - c0 : C;
-        __syncthreads();                                     // the other buffer is free, the state slice is written
-        if (c0 + C < n) {
-            const float* nxt = in + (size_t)H * stride;
-            for (int e = tid; e < opnd / 4; e += T) dc_cp_async16(bufs + (turn ^ 1) * opnd + e * 4, nxt + e * 4);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        const float* W_s = bufs + turn * opnd;  // [C][dk]
-        const float* Q_s = W_s + C * dk;        // [C][dk]
-        const float* K_s = Q_s + C * dk;        // [dk][C]
-        const float* P_s = K_s + C * dk;        // [C][C]
-        const float* U_g = in + (size_t)opnd;
-        float up[C / RG];                                    // U' of this thread's places
+        // pairs inside sixteen tokens: four threads a row, a quarter of the channels each, walk back from the row's token with the sum of the logarithms so far
+        const int r = tid >> 2, p0 = r & ~15;
+        float pk[16], pq[16];
 #pragma unroll
-        for (int j = 0; j < C / RG; j++) up[j] = live ? U_g[(size_t)(r0 + RG * j) * dv + col] : 0.0f;
-        const float gC = CH ? 0.0f : U_g[(size_t)C * dv];
-        float gv[DC_MAX_DK / RG];                            // CH: the chunk's decay of each of this thread's rows of the state
-        if (CH) {
+        for (int j = 0; j < 16; j++) pk[j] = pq[j] = 0.0f;
+        for (int d = tid & 3; d < DKP; d += 4) {
+            float sum = 0.0f;
+            const float qv = sq[r * LDQ + d], kv = sk[r * LDQ + d];
 #pragma unroll
-            for (int j = 0; j < DC_MAX_DK / RG; j++) gv[j] = r0 + RG * j < dk ? U_g[(size_t)C * dv + r0 + RG * j] : 0.0f;
-        }
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();
-        // W S and Qg S together: the state's values are loaded once for both
-        float ws[C / RG], qs[C / RG];
-#pragma unroll
-        for (int j = 0; j < C / RG; j++) ws[j] = qs[j] = 0.0f;
-        const float* sc = S_s + c * lds;
-        for (int d = 0; d < dk; d += 4) {
-            const float4 sv = *reinterpret_cast<const float4*>(sc + d);
-#pragma unroll
-            for (int j = 0; j < C / RG; j++) {
-                const float4 w = *reinterpret_cast<const float4*>(W_s + (r0 + RG * j) * dk + d);
-                const float4 q = *reinterpret_cast<const float4*>(Q_s + (r0 + RG * j) * dk + d);
-                ws[j] = fmaf(w.x, sv.x, fmaf(w.y, sv.y, fmaf(w.z, sv.z, fmaf(w.w, sv.w, ws[j]))));
-                qs[j] = fmaf(q.x, sv.x, fmaf(q.y, sv.y, fmaf(q.z, sv.z, fmaf(q.w, sv.w, qs[j]))));
-            }
-        }
-        float* uc = U_s + c * ldu;
-#pragma unroll
-        for (int j = 0; j < C / RG; j++) uc[r0 + RG * j] = up[j] - ws[j];          // U = U' - W S
-        __syncthreads();
-        // O = Qg S + P U
-        for (int i = 0; i < C; i += 4) {
-            const float4 uv = *reinterpret_cast<const float4*>(uc + i);
-#pragma unroll
-            for (int j = 0; j < C / RG; j++) {
-                const float4 w = *reinterpret_cast<const float4*>(P_s + (r0 + RG * j) * C + i);
-                qs[j] = fmaf(w.x, uv.x, fmaf(w.y, uv.y, fmaf(w.z, uv.z, fmaf(w.w, uv.w, qs[j]))));
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < C / RG; j++) {
-            const int t = r0 + RG * j;
-            if (live && t < cn) o[((size_t)(start + c0 + t) * H + h) * dv + col] = qs[j];
-        }
-        // S <- e^(L_C) S + KgT U: a thread has rows r0 + RG * j of its column; the new values wait in registers until every
-        // thread has read the old state
-        float s_new[DC_MAX_DK / RG];
-#pragma unroll
-        for (int j = 0; j < DC_MAX_DK / RG; j++) s_new[j] = 0.0f;
-        for (int i = 0; i < C; i += 4) {
-            const float4 uv = *reinterpret_cast<const float4*>(uc + i);
-#pragma unroll
-            for (int j = 0; j < DC_MAX_DK / RG; j++) {
-                const int d = r0 + RG * j;
-                if (d < dk) {
-                    const float4 w = *reinterpret_cast<const float4*>(K_s + d * C + i);
-                    s_new[j] = fmaf(w.x, uv.x, fmaf(w.y, uv.y, fmaf(w.z, uv.z, fmaf(w.w, uv.w, s_new[j]))));
+            for (int j = 15; j >= 0; j--)
+                if (p0 + j <= r) {
+                    const float x = sk[(p0 + j) * LDQ + d] * expf(sum);
+                    pk[j] = fmaf(kv, x, pk[j]);
+                    pq[j] = fmaf(qv, x, pq[j]);
+                    sum += sl[(p0 + j) * LDQ + d];
                 }
-            }
+        }
+        float* tk = sA;                             // (sA and sT are free until the pieces are collected)
+        float* tq = sT;
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            pk[j] += __shfl_xor_sync(0xffffffffu, pk[j], 1);
+            pk[j] += __shfl_xor_sync(0xffffffffu, pk[j], 2);
+            pq[j] += __shfl_xor_sync(0xffffffffu, pq[j], 1);
+            pq[j] += __shfl_xor_sync(0xffffffffu, pq[j], 2);
+            if ((tid & 3) == (j & 3)) { tk[r * 17 + j] = pk[j]; tq[r * 17 + j] = pq[j]; }
         }
         __syncthreads();
 #pragma unroll
-        for (int j = 0; j < DC_MAX_DK / RG; j++) {
-            const int d = r0 + RG * j;
-            if (d < dk) S_s[c * lds + d] = fmaf(CH ? gv[j] : gC, S_s[c * lds + d], s_new[j]);
+        for (int m = 0; m < 2; m++)
+            if (2 * wm + m == wn) {
+#pragma unroll
+                for (int n = 0; n < 2; n++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int at = (16 * wn + g + (e >> 1) * 8) * 17 + n * 8 + 2 * t4 + (e & 1);
+                        kk[m][n][e] = tk[at];
+                        qk[m][n][e] = tq[at];
+                    }
+            }
+        for (int e = tid; e < 4 * DKP; e += 256) {  // a channel of a sixteen a thread
+            const int s = e / DKP, d = e % DKP;
+            float l[16], k[16], sum = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 16; j++) { l[j] = sl[(16 * s + j) * LDQ + d]; k[j] = sk[(16 * s + j) * LDQ + d]; }
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                sum += l[j];
+                const float f = expf(sum);
+                sq[(16 * s + j) * LDQ + d] *= f;
+                sk[(16 * s + j) * LDQ + d] = k[j] * f;
+            }
+            vec[e] = expf(sum);
+            sum = 0.0f;
+#pragma unroll
+            for (int j = 15; j >= 0; j--) {
+                sl[(16 * s + j) * LDQ + d] = k[j] * expf(sum);
+                sum += l[j];
+            }
+        }
+        __syncthreads();
+    }
+    {
+        const float* right = CH ? sl : sk;
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            const int I = 2 * wm + m;
+            if (CH ? wn >= I : wn > I) continue;
+#pragma unroll 2
+            for (int ks = 0; ks < DKP / 8; ks++) {
+                const int d = ks * 8 + 2 * t4;
+                float2 x[4] = {*reinterpret_cast<const float2*>(sk + (16 * I + g) * LDQ + d), *reinterpret_cast<const float2*>(sk + (16 * I + g + 8) * LDQ + d),
+                               *reinterpret_cast<const float2*>(sq + (16 * I + g) * LDQ + d), *reinterpret_cast<const float2*>(sq + (16 * I + g + 8) * LDQ + d)};
+                if (CH) {
+                    float f0 = 1.0f, f1 = 1.0f;
+                    for (int u = wn + 1; u < I; u++) { f0 *= vec[u * DKP + d]; f1 *= vec[u * DKP + d + 1]; }
+#pragma unroll
+                    for (int i = 0; i < 4; i++) { x[i].x *= f0; x[i].y *= f1; }
+                }
+                const Tf a[2][4] = {{tf_split(x[0].x), tf_split(x[1].x), tf_split(x[0].y), tf_split(x[1].y)},
+                                    {tf_split(x[2].x), tf_split(x[3].x), tf_split(x[2].y), tf_split(x[3].y)}};
+                Tf b[2][2];
+#pragma unroll
+                for (int n = 0; n < 2; n++) {
+                    const float2 kb = *reinterpret_cast<const float2*>(right + (16 * wn + n * 8 + g) * LDQ + d);
+                    b[n][0] = tf_split(kb.x);
+                    b[n][1] = tf_split(kb.y);
+                }
+                float* const d_[2][2] = {{kk[m][0], kk[m][1]}, {qk[m][0], qk[m][1]}};
+                tf_mma3(d_, a, b);
+            }
+        }
+    }
+    if (CH) __syncthreads();                        // (the pieces that lay in sA and sT have been collected)
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int r = 32 * wm + 16 * m + g + 8 * u, i = 16 * wn + n * 8 + 2 * t4;
+                float a[2], w[2];
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const float ratio = i + e <= r ? (CH ? 1.0f : expf(L[r] - L[i + e])) : 0.0f;
+                    a[e] = i + e < r ? beta[r] * ratio * kk[m][n][2 * u + e] : 0.0f;
+                    w[e] = i + e <= r ? ratio * qk[m][n][2 * u + e] : 0.0f;
+                }
+                *reinterpret_cast<float2*>(sA + r * DC_LDA + i) = make_float2(a[0], a[1]);
+                *reinterpret_cast<float2*>(P_g + r * DC_C + i) = make_float2(w[0], w[1]);
+            }
+    // the scaled q and k; with a decay a channel k times e^L takes k's place
+    for (int e = tid; e < DC_C * (DKP / 4); e += 256) {
+        const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
+        if (d >= dk) continue;
+        float4 kq, kb;
+        if (CH) {
+            kq = *reinterpret_cast<const float4*>(sq + r * LDQ + d);
+            kb = *reinterpret_cast<const float4*>(sl + r * LDQ + d);
+            float4 kw = *reinterpret_cast<const float4*>(sk + r * LDQ + d);
+            for (int u = 0; u < r / 16; u++) {
+                const float4 f = *reinterpret_cast<const float4*>(vec + u * DKP + d);
+                kq.x *= f.x; kq.y *= f.y; kq.z *= f.z; kq.w *= f.w;
+                kw.x *= f.x; kw.y *= f.y; kw.z *= f.z; kw.w *= f.w;
+            }
+            for (int u = r / 16 + 1; u < 4; u++) {
+                const float4 f = *reinterpret_cast<const float4*>(vec + u * DKP + d);
+                kb.x *= f.x; kb.y *= f.y; kb.z *= f.z; kb.w *= f.w;
+            }
+            *reinterpret_cast<float4*>(sk + r * LDQ + d) = kw;
+        } else {
+            const float fq = expf(L[r]), fk = expf(L[DC_C - 1] - L[r]);
+            kq = *reinterpret_cast<const float4*>(sq + r * LDQ + d);
+            kb = *reinterpret_cast<const float4*>(sk + r * LDQ + d);
+            kq.x *= fq; kq.y *= fq; kq.z *= fq; kq.w *= fq;
+            kb.x *= fk; kb.y *= fk; kb.z *= fk; kb.w *= fk;
+        }
+        *reinterpret_cast<float4*>(Q_g + r * dk + d) = kq;
+        *reinterpret_cast<float4*>(K_g + r * dk + d) = kb;
+    }
+    if (CH) {
+        for (int d = tid; d < dk; d += 256) E_g[d] = (vec[d] * vec[DKP + d]) * (vec[2 * DKP + d] * vec[3 * DKP + d]);
+    } else if (tid == 0) E_g[0] = expf(L[DC_C - 1]);
+    __syncthreads();
+
+    // T = (I + A)^-1.  The blocks on the diagonal, a column a thread ..
+    if (tid < DC_C) {
+        const int b = tid >> 4, j = tid & 15;
+        const float* a = sA + 16 * b * DC_LDA + 16 * b;
+        float x[16];
+#pragma unroll
+        for (int r = 0; r < 16; r++) {
+            float s = 0.0f;
+#pragma unroll
+            for (int i = 0; i < r; i++) s = fmaf(a[r * DC_LDA + i], x[i], s);
+            x[r] = r < j ? 0.0f : r == j ? 1.0f : -s;
+            sT[(16 * b + r) * DC_LDA + 16 * b + j] = x[r];
         }
     }
     __syncthreads();
-    for (int e = tid; e < dk * COLS; e += T) {
-        const int cc = e / dk, d = e - cc * dk, gc = part * COLS + cc;
-        if (gc < dv) row[((size_t)h * dv + gc) * dk + d] = S_s[cc * lds + d];
+    // .. and T_ij = -T_ii sum_k A_ik T_kj below it, one step from the diagonal after the other (the sum waits in the block mirrored above the diagonal)
+    {
+        const int r = tid >> 4, c = tid & 15;
+        for (int step = 1; step < 4; step++) {
+            for (int j = 0; j + step < 4; j++) {
+                const int i = j + step;
+                float s0 = 0.0f, s1 = 0.0f;
+                for (int k = 16 * j; k < 16 * i; k += 2) {
+                    s0 = fmaf(sA[(16 * i + r) * DC_LDA + k], sT[k * DC_LDA + 16 * j + c], s0);
+                    s1 = fmaf(sA[(16 * i + r) * DC_LDA + k + 1], sT[(k + 1) * DC_LDA + 16 * j + c], s1);
+                }
+                sT[(16 * j + r) * DC_LDA + 16 * i + c] = s0 + s1;
+            }
+            __syncthreads();
+            for (int j = 0; j + step < 4; j++) {
+                const int i = j + step;
+                float s = 0.0f;
+#pragma unroll
+                for (int u = 0; u < 16; u++) s = fmaf(sT[(16 * i + r) * DC_LDA + 16 * i + u], sT[(16 * j + u) * DC_LDA + 16 * i + c], s);
+                sT[(16 * i + r) * DC_LDA + 16 * j + c] = -s;
+            }
+            __syncthreads();
+        }
+    }
+    // W = T diag(beta e^L) K and U' = T diag(beta) V, eight columns a warp at a time
+    if (tid < DC_C) L[tid] = CH ? beta[tid] : beta[tid] * expf(L[tid]);         // (the factor of k's rows from here on)
+    __syncthreads();
+    const int nw = (dk + 7) / 8, nv = (dv + 7) / 8;
+    for (int n = warp; n < nw + nv; n += 8) {
+        const bool is_w = n < nw;
+        const int c0 = (is_w ? n : n - nw) * 8, ld = is_w ? LDQ : LDV;
+        const float* src = (is_w ? sk : sv) + c0 + g;
+        const float* fac = is_w ? L : beta;
+        float acc[4][4];
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[m][e] = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < 8; ks++) {
+            const int k = ks * 8 + 2 * t4;
+            const Tf b[1][2] = {{tf_split(fac[k] * src[k * ld]), tf_split(fac[k + 1] * src[(k + 1) * ld])}};
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                if (m < ks / 2) continue;           // T is lower triangular
+                const float2 x = *reinterpret_cast<const float2*>(sT + (16 * m + g) * DC_LDA + k), y = *reinterpret_cast<const float2*>(sT + (16 * m + g + 8) * DC_LDA + k);
+                const Tf a[1][4] = {{tf_split(x.x), tf_split(y.x), tf_split(x.y), tf_split(y.y)}};
+                float* const d_[1][1] = {{acc[m]}};
+                tf_mma3(d_, a, b);
+            }
+        }
+        float* dst = is_w ? W_g : U_g;
+        const int width = is_w ? dk : dv, c = c0 + 2 * t4;
+        if (c < width) {
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                *reinterpret_cast<float2*>(dst + (size_t)(16 * m + g) * width + c) = make_float2(acc[m][0], acc[m][1]);
+                *reinterpret_cast<float2*>(dst + (size_t)(16 * m + g + 8) * width + c) = make_float2(acc[m][2], acc[m][3]);
+            }
+        }
+    }
+}
+
+// grid (segments, H, slices of COLS columns); DKP / 16 warps: warp w has rows 16 w .. of the state's slice, and in the first product rows 16 (w & 3) .. of U and, with
+// 16 columns, the 8 columns w >> 2.
+constexpr int DC_STAGES = 3;
+
+template <int DKP, int COLS, bool CH>
+__global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs p, const float* __restrict__ proj, int N, float* __restrict__ state,
+                                                                   size_t state_stride, size_t conv_off, int taps) {
+    constexpr int NTH = DKP * 2, LDQ = DKP + 8, LDS = DKP + 4, LDU = DC_C + 4, NT = COLS / 8, STAGE = 2 * DC_C * LDQ;
+    static_assert(NT == DKP / 64, "the warps of the first product");
+    extern __shared__ __align__(16) float ds_smem[];
+    __shared__ int base_sh;
+    float* ring = ds_smem;
+    float* sS = ring + DC_STAGES * STAGE;           // [COLS][LDS]
+    float* sU = sS + COLS * LDS;                    // [COLS][LDU]
+    const int seg = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    const int slot = p.seg_slots[seg], start = p.seg_starts[seg], n = p.seg_starts[seg + 1] - start;
+    if (slot < 0 || n <= 0) return;
+    if (warp == 0) {
+        const int b = first_chunk_of<DC_C>(seg, p.seg_starts);
+        if (lane == 0) base_sh = b;
+    }
+    const int dk = p.dk, dv = p.dv, H = p.H, c0 = blockIdx.z * COLS, chunks = (n + DC_C - 1) / DC_C;
+    float* row = state + (size_t)slot * state_stride;
+    for (int e = tid; e < COLS * DKP; e += NTH) {
+        const int c = e / DKP, d = e % DKP;
+        sS[c * LDS + d] = (c0 + c < dv && d < dk) ? row[((size_t)h * dv + c0 + c) * dk + d] : 0.0f;
+    }
+    __syncthreads();
+    const size_t stride = dc_stride(dk, dv, CH);
+    float* mine = p.scratch + ((size_t)base_sh * H + h) * stride;
+    const size_t u_off = (size_t)DC_C * (3 * dk + DC_C), s_off = u_off + (size_t)DC_C * dv, e_off = s_off + (size_t)dk * dv;
+    auto issue = [&](int c) {
+        if (c < chunks) {
+            const float* in = mine + (size_t)c * H * stride;
+            float* st = ring + (c % DC_STAGES) * STAGE;
+            for (int e = tid; e < 2 * DC_C * (DKP / 4); e += NTH) {
+                const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));           // rows of W, then of Kg
+                tf_cp16(st + r * LDQ + d, in + (d < dk ? (size_t)r * dk + d : 0), d < dk);
+            }
+        }
+        tf_commit();
+    };
+    float s[NT][4];                                 // this warp's rows of the state: rows d, d + 8, columns 8 i + 2 t4, + 1
+    const int d = 16 * warp + g;
+#pragma unroll
+    for (int i = 0; i < NT; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) s[i][e] = sS[(8 * i + 2 * t4 + (e & 1)) * LDS + d + 8 * (e >> 1)];
+    const int ur = 16 * (warp & 3) + g, uc = 8 * (warp >> 2) + 2 * t4;          // this thread's places in U: rows ur, ur + 8, columns uc, + 1
+    float2 up[2];
+    float dec[2];
+    auto fetch = [&](int c) {                       // U' and the decays of chunk c
+        const float* in = mine + (size_t)(c < chunks ? c : 0) * H * stride;
+        const bool on = c < chunks && c0 + uc < dv;
+        up[0] = on ? *reinterpret_cast<const float2*>(in + u_off + (size_t)ur * dv + c0 + uc) : make_float2(0.0f, 0.0f);
+        up[1] = on ? *reinterpret_cast<const float2*>(in + u_off + (size_t)(ur + 8) * dv + c0 + uc) : make_float2(0.0f, 0.0f);
+        dec[0] = CH ? (d < dk ? in[e_off + d] : 0.0f) : in[e_off];
+        dec[1] = CH ? (d + 8 < dk ? in[e_off + d + 8] : 0.0f) : dec[0];
+    };
+    issue(0);
+    issue(1);
+    fetch(0);
+    for (int c = 0; c < chunks; c++) {
+        tf_wait<1>();
+        __syncthreads();                            // the chunk's operands are there, the state's slice is written, and everybody has left the chunk before
+        issue(c + 2);
+        float* in = mine + (size_t)c * H * stride;
+        const float* sW = ring + (c % DC_STAGES) * STAGE;
+        const float* sK = sW + DC_C * LDQ;
+        for (int e = tid; e < COLS * (DKP / 4); e += NTH) {                     // the state before the chunk
+            const int cc = e / (DKP / 4), dd = 4 * (e % (DKP / 4));
+            if (c0 + cc < dv && dd < dk) *reinterpret_cast<float4*>(in + s_off + (size_t)(c0 + cc) * dk + dd) = *reinterpret_cast<const float4*>(sS + cc * LDS + dd);
+        }
+        float x[3][4];
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) x[i][e] = 0.0f;
+        const float* wa = sW + ur * LDQ + 2 * t4;
+        const float* sb = sS + (8 * (warp >> 2) + g) * LDS + 2 * t4;
+#pragma unroll 4
+        for (int ks = 0; ks < DKP / 8; ks++) {
+            const float2 a0 = *reinterpret_cast<const float2*>(wa + ks * 8), a1 = *reinterpret_cast<const float2*>(wa + 8 * LDQ + ks * 8);
+            const float2 b0 = *reinterpret_cast<const float2*>(sb + ks * 8);
+            const Tf a[4] = {tf_split(a0.x), tf_split(a1.x), tf_split(a0.y), tf_split(a1.y)}, b[2] = {tf_split(b0.x), tf_split(b0.y)};
+            tf_mma(x[0], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
+            tf_mma(x[1], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
+            tf_mma(x[2], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
+        }
+        float2 u[2];
+        u[0] = make_float2(up[0].x - ((x[0][0] + x[1][0]) + x[2][0]), up[0].y - ((x[0][1] + x[1][1]) + x[2][1]));
+        u[1] = make_float2(up[1].x - ((x[0][2] + x[1][2]) + x[2][2]), up[1].y - ((x[0][3] + x[1][3]) + x[2][3]));
+        sU[uc * LDU + ur] = u[0].x;
+        sU[(uc + 1) * LDU + ur] = u[0].y;
+        sU[uc * LDU + ur + 8] = u[1].x;
+        sU[(uc + 1) * LDU + ur + 8] = u[1].y;
+        if (c0 + uc < dv) {
+            *reinterpret_cast<float2*>(in + u_off + (size_t)ur * dv + c0 + uc) = u[0];
+            *reinterpret_cast<float2*>(in + u_off + (size_t)(ur + 8) * dv + c0 + uc) = u[1];
+        }
+        const float da = dec[0], db = dec[1];
+        fetch(c + 1);
+        __syncthreads();                            // U is there, and nobody reads the old state any more
+        float y[NT][3][4];
+#pragma unroll
+        for (int i = 0; i < NT; i++)
+#pragma unroll
+            for (int j = 0; j < 3; j++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) y[i][j][e] = 0.0f;
+#pragma unroll 4
+        for (int ks = 0; ks < DC_C / 8; ks++) {
+            const float* ka = sK + (ks * 8 + t4) * LDQ + d;
+            const Tf a[4] = {tf_split(ka[0]), tf_split(ka[8]), tf_split(ka[4 * LDQ]), tf_split(ka[4 * LDQ + 8])};
+#pragma unroll
+            for (int i = 0; i < NT; i++) {
+                const float* ub = sU + (8 * i + g) * LDU + ks * 8 + t4;
+                const Tf b[2] = {tf_split(ub[0]), tf_split(ub[4])};
+                tf_mma(y[i][0], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
+                tf_mma(y[i][1], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
+                tf_mma(y[i][2], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NT; i++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                s[i][e] = fmaf(e < 2 ? da : db, s[i][e], (y[i][0][e] + y[i][1][e]) + y[i][2][e]);
+                sS[(8 * i + 2 * t4 + (e & 1)) * LDS + d + 8 * (e >> 1)] = s[i][e];
+            }
+    }
+    __syncthreads();
+    for (int e = tid; e < COLS * DKP; e += NTH) {
+        const int c = e / DKP, dd = e % DKP;
+        if (c0 + c < dv && dd < dk) row[((size_t)h * dv + c0 + c) * dk + dd] = sS[c * LDS + dd];
     }
     // the convolution's memory: the last taps-1 inputs of the request, this step's tokens included
     if (taps > 1) {
+        const int Cq = 2 * p.G * dk + H * dv;
         float* cs = row + conv_off;
-        const int nb = gridDim.y * gridDim.z, bi = h * gridDim.z + part;
-        for (int ch = bi * T + tid; ch < Cq; ch += nb * T) {
+        const int nb = gridDim.y * gridDim.z, bi = h * gridDim.z + blockIdx.z;
+        for (int chn = bi * NTH + tid; chn < Cq; chn += nb * NTH) {
             float keep[DC_MAX_TAPS];
 #pragma unroll
             for (int rr = 0; rr < DC_MAX_TAPS; rr++)
                 if (rr < taps - 1) {
                     const int src = n - (taps - 1) + rr;
-                    keep[rr] = src >= 0 ? proj[(size_t)(start + src) * N + ch] : cs[(size_t)(rr + n) * Cq + ch];
+                    keep[rr] = src >= 0 ? proj[(size_t)(start + src) * N + chn] : cs[(size_t)(rr + n) * Cq + chn];
                 }
 #pragma unroll
             for (int rr = 0; rr < DC_MAX_TAPS; rr++)
-                if (rr < taps - 1) cs[(size_t)rr * Cq + ch] = keep[rr];
+                if (rr < taps - 1) cs[(size_t)rr * Cq + chn] = keep[rr];
         }
     }
+}
+
+// grid (chunks, H, slices of 64 columns); 256 threads: warp w has rows 16 (w & 3) .. and columns 32 (w >> 2) .. of the slice
+template <int DKP>
+__global__ void __launch_bounds__(256) delta_chunk_out_kernel(const DcArgs p, bool ch_decay, float* __restrict__ o) {
+    constexpr int LDQ = DKP + 8, LDU = 64 + 4;
+    extern __shared__ __align__(16) float do_smem[];
+    __shared__ int find[4];
+    float* sQ = do_smem;                            // [64][LDQ]
+    float* sS = sQ + DC_C * LDQ;                    // [64 columns][LDQ]
+    float* sP = sS + 64 * LDQ;                      // [64][DC_LDA]
+    float* sU = sP + DC_C * DC_LDA;                 // [64][LDU]
+    const Chunk ch = find_chunk<DC_C>(blockIdx.x, p.seg_starts, p.segments, find);
+    if (ch.seg < 0 || p.seg_slots[ch.seg] < 0) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, m = warp & 3, cw = 32 * (warp >> 2);
+    const int h = blockIdx.y, c0 = blockIdx.z * 64, dk = p.dk, dv = p.dv;
+    const float* in = p.scratch + ((size_t)blockIdx.x * p.H + h) * dc_stride(dk, dv, ch_decay);
+    const float* Q_g = in + 2 * (size_t)DC_C * dk;
+    const float* P_g = Q_g + (size_t)DC_C * dk;
+    const float* U_g = P_g + DC_C * DC_C;
+    const float* S_g = U_g + (size_t)DC_C * dv;
+    for (int e = tid; e < DC_C * (DKP / 4); e += 256) {
+        const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
+        const bool on = d < dk, ons = on && c0 + r < dv;
+        tf_cp16(sQ + r * LDQ + d, Q_g + (on ? (size_t)r * dk + d : 0), on);
+        tf_cp16(sS + r * LDQ + d, S_g + (ons ? (size_t)(c0 + r) * dk + d : 0), ons);
+    }
+    for (int e = tid; e < DC_C * 16; e += 256) {
+        const int r = e / 16, c = 4 * (e % 16);
+        const bool on = c0 + c < dv;
+        tf_cp16(sP + r * DC_LDA + c, P_g + r * DC_C + c, true);
+        tf_cp16(sU + r * LDU + c, U_g + (on ? (size_t)r * dv + c0 + c : 0), on);
+    }
+    tf_commit();
+    tf_wait<0>();
+    __syncthreads();
+    if (16 * m >= ch.rows) return;
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[i][e] = 0.0f;
+    float* const d_[1][4] = {{acc[0], acc[1], acc[2], acc[3]}};
+#pragma unroll 4
+    for (int ks = 0; ks < DKP / 8; ks++) {
+        const int k = ks * 8 + 2 * t4;
+        const float2 x = *reinterpret_cast<const float2*>(sQ + (16 * m + g) * LDQ + k), y = *reinterpret_cast<const float2*>(sQ + (16 * m + g + 8) * LDQ + k);
+        const Tf a[1][4] = {{tf_split(x.x), tf_split(y.x), tf_split(x.y), tf_split(y.y)}};
+        Tf b[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 v = *reinterpret_cast<const float2*>(sS + (cw + 8 * i + g) * LDQ + k);
+            b[i][0] = tf_split(v.x);
+            b[i][1] = tf_split(v.y);
+        }
+        tf_mma3(d_, a, b);
+    }
+#pragma unroll 2
+    for (int ks = 0; ks < 2 * (m + 1); ks++) {      // (P is lower triangular)
+        const int k = ks * 8 + 2 * t4;
+        const float2 x = *reinterpret_cast<const float2*>(sP + (16 * m + g) * DC_LDA + k), y = *reinterpret_cast<const float2*>(sP + (16 * m + g + 8) * DC_LDA + k);
+        const Tf a[1][4] = {{tf_split(x.x), tf_split(y.x), tf_split(x.y), tf_split(y.y)}};
+        Tf b[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float* ub = sU + k * LDU + cw + 8 * i + g;
+            b[i][0] = tf_split(ub[0]);
+            b[i][1] = tf_split(ub[LDU]);
+        }
+        tf_mma3(d_, a, b);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int r = 16 * m + g + 8 * u, c = c0 + cw + 8 * i + 2 * t4;
+            if (r < ch.rows && c < dv) *reinterpret_cast<float2*>(o + ((size_t)(ch.first + r) * p.H + h) * dv + c) = make_float2(acc[i][2 * u], acc[i][2 * u + 1]);
+        }
 }
 
 }  // namespace vk
 
 using namespace vk;
 
-static int dc_chunk(int dk) { return dk <= 64 ? 64 : 32; }
+static int dc_chunks(int tokens, int segments) { return tokens / DC_C + (segments < tokens ? segments : tokens); }
 
 // Whether the chunked kernels take these sizes (else the token-by-token kernel does the work).
 VK_API int vk_delta_chunked_takes(int G, int H, int dk, int dv, int taps) {
-    const int C = dc_chunk(dk);
-    return G > 0 && H > 0 && H % G == 0 && dk % 4 == 0 && dk >= 8 && dk <= 128 && dv > 0 && dv % 4 == 0 && dv <= 256 && taps >= 1 &&
-           taps <= DC_MAX_TAPS;
+    return G > 0 && H > 0 && H % G == 0 && dk % 4 == 0 && dk >= 8 && dk <= 128 && dv > 0 && dv % 4 == 0 && dv <= 256 && taps >= 1 && taps <= DC_MAX_TAPS;
 }
 
 // Bytes of scratch for a step of `tokens` tokens in `segments` segments.
 VK_API size_t vk_delta_chunked_scratch_bytes(int tokens, int segments, int H, int dk, int dv) {
-    const int C = dc_chunk(dk);
-    return ((size_t)tokens / C + segments + 1) * H * dc_stride(C, dk, dv) * sizeof(float);
+    return (size_t)dc_chunks(tokens, segments) * H * dc_stride(dk, dv, false) * sizeof(float);
+}
+
+template <int DKP, bool CH>
+static int delta_chunked_launch(const DcArgs& p, const float* proj, int proj_width, float* state, size_t state_stride, float* o, int tokens, int taps,
+                                cudaStream_t stream) {
+    constexpr int COLS = DKP / 8;
+    const int chunks = dc_chunks(tokens, p.segments);
+    const int smem1 = (dc_prepare_floats_fixed<DKP, CH>() + DC_C * dc_ldv(p.dv)) * (int)sizeof(float);
+    const int smem2 = (DC_STAGES * 2 * DC_C * (DKP + 8) + COLS * (DKP + 4) + COLS * (DC_C + 4)) * (int)sizeof(float);
+    const int smem3 = (2 * DC_C * (DKP + 8) + DC_C * DC_LDA + DC_C * 68) * (int)sizeof(float);
+    auto k1 = delta_chunk_prepare_kernel<DKP, CH>;
+    auto k2 = delta_chunk_scan_kernel<DKP, COLS, CH>;
+    auto k3 = delta_chunk_out_kernel<DKP>;
+    cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, smem3);
+    if (e != cudaSuccess) return (int)e;
+    int rc = launch_plain(k1, dim3(chunks, p.H), dim3(256), smem1, stream, p);
+    if (rc != VK_OK) return rc;
+    rc = launch_plain(k2, dim3(p.segments, p.H, (p.dv + COLS - 1) / COLS), dim3(DKP * 2), smem2, stream, p, proj, proj_width, state, state_stride,
+                      (size_t)p.H * p.dv * p.dk, taps);
+    if (rc != VK_OK) return rc;
+    return launch_plain(k3, dim3(chunks, p.H, (p.dv + 63) / 64), dim3(256), smem3, stream, p, CH, o);
 }
 
 template <bool CH>
-static int delta_chunked_launch(const float* prep, int prep_width, const float* proj, int proj_width, const int32_t* seg_starts,
-                                const int32_t* seg_slots, float* state, size_t state_stride, float* o, float* scratch, int segments, int tokens,
-                                int G, int H, int dk, int dv, int taps, cudaStream_t stream) {
+static int delta_chunked(const float* prep, int prep_width, const float* proj, int proj_width, const int32_t* seg_starts, const int32_t* seg_slots, float* state,
+                         size_t state_stride, float* o, float* scratch, int segments, int tokens, int G, int H, int dk, int dv, int taps, cudaStream_t stream) {
     if (segments <= 0 || tokens <= 0) return VK_OK;
-    if (!vk_delta_chunked_takes(G, H, dk, dv, taps)) return VK_BAD_SHAPE;
-    if (((uintptr_t)scratch % 16) || H > 65535) return VK_BAD_ALIGNMENT;
-    const int C = dc_chunk(dk);
-    const int chunks = tokens / C + segments;
-    const size_t smem1 = (size_t)(2 * C * (dk + 1) + 2 * C * (C + 1) + C * (dv + dk) + (CH ? C * (dk + 1) : 0)) * sizeof(float);
-    constexpr int COLS = 16;
-    const size_t smem2 = (size_t)(COLS * (dk + 4) + COLS * (C + 4) + 2 * C * (3 * dk + C)) * sizeof(float);
-    const int parts = (dv + COLS - 1) / COLS;
-    if (smem1 > 200 * 1024 || smem2 > 200 * 1024) return VK_TOO_LARGE;
-#define GO(CC)                                                                                                                             \
-    {                                                                                                                                      \
-        auto k1 = delta_chunk_prepare_kernel<CC, CH>;                                                                                      \
-        auto k2 = delta_chunk_scan_kernel<CC, COLS, CH>;                                                                                   \
-        cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);                                                 \
-        cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);                                                 \
-        int rc = launch_plain(k1, dim3(chunks, H), dim3(DC_THREADS), smem1, stream, prep, prep_width, seg_starts, seg_slots, segments,    \
-                              scratch, G, H, dk, dv);                                                                                      \
-        if (rc != 0) return rc;                                                                                                            \
-        return launch_plain(k2, dim3(segments, H, parts), dim3(256), smem2, stream, (const float*)scratch, proj, proj_width, seg_starts,  \
-                            seg_slots, state, state_stride, (size_t)H * dv * dk, o, G, H, dk, dv, taps);                                   \
-    }
-    if (C == 64) GO(64) else GO(32)
-#undef GO
+    if (!vk_delta_chunked_takes(G, H, dk, dv, taps) || prep_width % 4) return VK_BAD_SHAPE;
+    if ((uintptr_t)scratch % 16 || (uintptr_t)prep % 16 || (uintptr_t)o % 8) return VK_BAD_ALIGNMENT;
+    if (H > 65535) return VK_TOO_LARGE;
+    const DcArgs p = {prep, prep_width, seg_starts, seg_slots, segments, scratch, G, H, dk, dv};
+    return dk <= 64 ? delta_chunked_launch<64, CH>(p, proj, proj_width, state, state_stride, o, tokens, taps, stream)
+                    : delta_chunked_launch<128, CH>(p, proj, proj_width, state, state_stride, o, tokens, taps, stream);
 }
 
-// prep [tokens][prep width] as delta_prepare leaves it; proj as for the token-by-token kernel; o [tokens][H*dv] float32.
+// prep [tokens][prep width] as delta_prepare leaves it; proj as for the token-by-token kernel; o [tokens][H*dv] float32; three kernels.
 VK_API int vk_delta_chunked(const float* prep, int prep_width, const float* proj, const int32_t* seg_starts, const int32_t* seg_slots, float* state,
                             size_t state_stride, float* o, float* scratch, int segments, int tokens, int G, int H, int dk, int dv, int taps,
                             cudaStream_t stream) {
-    return delta_chunked_launch<false>(prep, prep_width, proj, 2 * G * dk + 2 * H * dv + 2 * H, seg_starts, seg_slots, state, state_stride, o,
-                                       scratch, segments, tokens, G, H, dk, dv, taps, stream);
+    return delta_chunked<false>(prep, prep_width, proj, 2 * G * dk + 2 * H * dv + 2 * H, seg_starts, seg_slots, state, state_stride, o, scratch, segments,
+                                tokens, G, H, dk, dv, taps, stream);
 }
 
 // The form with a decay per head and key channel: prep as cdelta_prepare leaves it, proj rows of proj_width floats (the
 // convolution's inputs first).  The sizes are those vk_delta_chunked_takes.
 VK_API size_t vk_cdelta_chunked_scratch_bytes(int tokens, int segments, int H, int dk, int dv) {
-    const int C = dc_chunk(dk);
-    return ((size_t)tokens / C + segments + 1) * H * dc_stride(C, dk, dv, true) * sizeof(float);
+    return (size_t)dc_chunks(tokens, segments) * H * dc_stride(dk, dv, true) * sizeof(float);
 }
 
 VK_API int vk_cdelta_chunked(const float* prep, int prep_width, const float* proj, int proj_width, const int32_t* seg_starts,
                              const int32_t* seg_slots, float* state, size_t state_stride, float* o, float* scratch, int segments, int tokens,
                              int G, int H, int dk, int dv, int taps, cudaStream_t stream) {
-    return delta_chunked_launch<true>(prep, prep_width, proj, proj_width, seg_starts, seg_slots, state, state_stride, o, scratch, segments,
-                                      tokens, G, H, dk, dv, taps, stream);
+    return delta_chunked<true>(prep, prep_width, proj, proj_width, seg_starts, seg_slots, state, state_stride, o, scratch, segments, tokens, G, H, dk, dv, taps,
+                               stream);
 }

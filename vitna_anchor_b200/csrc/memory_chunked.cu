@@ -17,9 +17,7 @@
 //
 // Why chunks: token after token the recurrence is a chain of 2,048 steps of 0.24 us in at most 136 blocks.  Every exponent here is at most 0.
 //
-// Products take float32 operands as two tf32 parts (x = high + low, 11 bits each; high high + high low + low high, float32 sums), so a product is as exact as
-// a float32 one to 2^-22; the tensor cores do 159 such multiply-adds a cycle and multiprocessor where the float32 units do 124 and would need
-// every operand from shared memory again for every 4 x 4 outputs.  Two bfloat16 parts would be twice as fast and lose a float32 state's last 7 bits.
+// Products take float32 operands as two tf32 parts (tf32.cuh).
 //
 // Measured, a whole mixer with its two products: mLSTM, one request of 2,048 tokens, 8 heads of 128 x 256: 599 us token after token, 208 us here (gates 11,
 // cm_add 26, cm_scan 10, cm_out 55: the tensor cores' rate for three tf32 products is 23 us of it on the multiprocessors that have two of its blocks);
@@ -27,6 +25,7 @@
 // whose blocks walked the chunks in order with their tile of the state in the accumulators took 2.9 us a chunk, 90 us for cm_add's and cm_scan's work.
 #include "chunks.cuh"
 #include "common.cuh"
+#include "tf32.cuh"
 
 namespace vk {
 
@@ -34,47 +33,7 @@ constexpr int CM_Q = 64;                    // tokens of a chunk
 constexpr int CM_LOCAL = 16;                // tokens over which a channel's logarithms are added up (gated linear attention)
 constexpr int CM_T = 64, CM_LD = CM_T + 8;   // the tile of the state that a block of cm_add works out, and a padded row of one of its operands
 
-__device__ __forceinline__ void cm_cp16(float* dst, const float* src, bool there) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cm_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int LEFT> __device__ __forceinline__ void cm_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
-
-__device__ __forceinline__ float cm_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ float cm_log_sigmoid(float z) { return fminf(z, 0.0f) - log1pf(expf(-fabsf(z))); }
-
-// a float32 operand as two tf32 parts: its 11 leading bits rounded to the nearest, and the 11 leading bits (the tensor core does not read the others)
-// of what that leaves, rounded likewise
-struct Tf { uint32_t hi, lo; };
-__device__ __forceinline__ Tf cm_split(float x) {
-    const uint32_t hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    return Tf{hi, __float_as_uint(x - __uint_as_float(hi)) + 0x1000u};
-}
-__device__ __forceinline__ void cm_mma(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// d[m][n] += a[m] b[n] in three products, the small ones first; products of one sum stand M N instructions apart
-template <int M, int N>
-__device__ __forceinline__ void cm_mma3(float* const (&d)[M][N], const Tf (&a)[M][4], const Tf (&b)[N][2]) {
-#pragma unroll
-    for (int m = 0; m < M; m++)
-#pragma unroll
-        for (int n = 0; n < N; n++) cm_mma(d[m][n], a[m][0].lo, a[m][1].lo, a[m][2].lo, a[m][3].lo, b[n][0].hi, b[n][1].hi);
-#pragma unroll
-    for (int m = 0; m < M; m++)
-#pragma unroll
-        for (int n = 0; n < N; n++) cm_mma(d[m][n], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[n][0].lo, b[n][1].lo);
-#pragma unroll
-    for (int m = 0; m < M; m++)
-#pragma unroll
-        for (int n = 0; n < N; n++) cm_mma(d[m][n], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[n][0].hi, b[n][1].hi);
-}
 
 struct CmArgs {
     const float* proj;              // [tokens][N]: q | k | v | ..
@@ -238,13 +197,13 @@ __global__ void __launch_bounds__(128) cm_add_kernel(const CmArgs p, int col_til
         const int r = e / (CM_T / 4), c = 4 * (e % (CM_T / 4));
         const bool onk = r < rows && d0 + c < dk, onv = r < rows && v0 + c < dv;
         const float* row = p.proj + (size_t)(ch.first + (r < rows ? r : 0)) * p.N;
-        cm_cp16(sk + r * CM_LD + c, onk ? row + H * dk + h * dk + d0 + c : p.proj, onk);
-        cm_cp16(sv + r * CM_LD + c, onv ? row + 2 * H * dk + h * dv + v0 + c : p.proj, onv);
-        if (!MLSTM) cm_cp16(sl + r * CM_LD + c, onk ? p.logs + (size_t)(ch.first + r) * H * dk + h * dk + d0 + c : p.proj, onk);
+        tf_cp16(sk + r * CM_LD + c, onk ? row + H * dk + h * dk + d0 + c : p.proj, onk);
+        tf_cp16(sv + r * CM_LD + c, onv ? row + 2 * H * dk + h * dv + v0 + c : p.proj, onv);
+        if (!MLSTM) tf_cp16(sl + r * CM_LD + c, onk ? p.logs + (size_t)(ch.first + r) * H * dk + h * dk + d0 + c : p.proj, onk);
     }
-    cm_commit();
+    tf_commit();
     if (MLSTM && tid < CM_Q) wt[tid] = tid < rows ? p.weight[(size_t)(ch.first + tid) * H + h] : 0.0f;
-    cm_wait<0>();
+    tf_wait<0>();
     __syncthreads();
     const size_t at = (size_t)blockIdx.x * H + h;
     if (!MLSTM) {
@@ -256,7 +215,7 @@ __global__ void __launch_bounds__(128) cm_add_kernel(const CmArgs p, int col_til
             total[s] = 0.0f;
 #pragma unroll
             for (int r = 0; r < CM_LOCAL; r++) total[s] += sl[(s * CM_LOCAL + r) * CM_LD + d];
-            total[s] = cm_exp2(total[s]);
+            total[s] = tf_exp2(total[s]);
         }
         if (part == 0 && v0 == 0 && d0 + d < dk) p.decay[at * dk + d0 + d] = total[0] * total[1] * total[2] * total[3];
 #pragma unroll
@@ -268,7 +227,7 @@ __global__ void __launch_bounds__(128) cm_add_kernel(const CmArgs p, int col_til
 #pragma unroll
             for (int r = CM_LOCAL - 1; r >= 0; r--) {
                 float* k = sk + (s * CM_LOCAL + r) * CM_LD + d;
-                *k *= cm_exp2(sum) * after;
+                *k *= tf_exp2(sum) * after;
                 sum += sl[(s * CM_LOCAL + r) * CM_LD + d];
             }
         }
@@ -289,16 +248,16 @@ __global__ void __launch_bounds__(128) cm_add_kernel(const CmArgs p, int col_til
 #pragma unroll
         for (int m = 0; m < 2; m++) {
             const float* ka = sk + (ks * 8 + t4) * CM_LD + wd + 16 * m + g;
-            a[m][0] = cm_split(ka[0]); a[m][1] = cm_split(ka[8]); a[m][2] = cm_split(ka[4 * CM_LD]); a[m][3] = cm_split(ka[4 * CM_LD + 8]);
+            a[m][0] = tf_split(ka[0]); a[m][1] = tf_split(ka[8]); a[m][2] = tf_split(ka[4 * CM_LD]); a[m][3] = tf_split(ka[4 * CM_LD + 8]);
         }
         const float w0 = MLSTM ? wt[ks * 8 + t4] : 1.0f, w1 = MLSTM ? wt[ks * 8 + t4 + 4] : 1.0f;
 #pragma unroll
         for (int n = 0; n < 4; n++) {
             const float* vb = sv + (ks * 8 + t4) * CM_LD + wv + n * 8 + g;
-            b[n][0] = cm_split(MLSTM ? w0 * vb[0] : vb[0]);
-            b[n][1] = cm_split(MLSTM ? w1 * vb[4 * CM_LD] : vb[4 * CM_LD]);
+            b[n][0] = tf_split(MLSTM ? w0 * vb[0] : vb[0]);
+            b[n][1] = tf_split(MLSTM ? w1 * vb[4 * CM_LD] : vb[4 * CM_LD]);
         }
-        cm_mma3(d_, a, b);
+        tf_mma3(d_, a, b);
     }
     float* out = p.before + at * dk * dv;
 #pragma unroll
@@ -417,12 +376,12 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
         const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
         const bool on = r < rows && d < dk;
         const float* src = p.proj + (size_t)(ch.first + (on ? r : 0)) * p.N + h * dk + (on ? d : 0);
-        cm_cp16(sq + r * LDQ + d, src, on);
-        cm_cp16(sk + r * LDQ + d, src + H * dk, on);
+        tf_cp16(sq + r * LDQ + d, src, on);
+        tf_cp16(sk + r * LDQ + d, src + H * dk, on);
         // the decays' logarithms lie in the first slot until the weights of the chunk are known
-        if (!MLSTM) cm_cp16(ring + r * LDQ + d, p.logs + (size_t)(ch.first + (on ? r : 0)) * H * dk + h * dk + (on ? d : 0), on);
+        if (!MLSTM) tf_cp16(ring + r * LDQ + d, p.logs + (size_t)(ch.first + (on ? r : 0)) * H * dk + h * dk + (on ? d : 0), on);
     }
-    cm_commit();
+    tf_commit();
     auto issue = [&](int s) {                           // slice s: 32 rows of the state, then of v
         if (s < KS + 2) {
             float* dst = ring + (s & 1) * L::SLOT;
@@ -430,10 +389,10 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
                 const int r = e / (DVP / 4), v = 4 * (e % (DVP / 4)), row = (s < KS ? s : s - KS) * 32 + r;
                 const bool on = v < dv && row < (s < KS ? dk : rows);
                 const float* src = s < KS ? p.before + (at * dk + row) * dv + v : p.proj + (size_t)(ch.first + row) * p.N + 2 * H * dk + h * dv + v;
-                cm_cp16(dst + r * LDB + v, on ? src : p.proj, on);
+                tf_cp16(dst + r * LDB + v, on ? src : p.proj, on);
             }
         }
-        cm_commit();
+        tf_commit();
     };
     if (MLSTM) {
         issue(0);
@@ -447,9 +406,9 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
             row_n[tid] = expf(-(float)(p.F[i] + Nt));   // e^-m
         }
         for (int d = tid; d < DKP; d += 256) vec[d] = d < dk ? p.n_before[at * dk + d] : 0.0f;
-        cm_wait<1>();
+        tf_wait<1>();
     } else {
-        cm_wait<0>();
+        tf_wait<0>();
     }
     __syncthreads();
 
@@ -476,7 +435,7 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
 #pragma unroll
             for (int j = CM_LOCAL - 1; j >= 0; j--)
                 if (p0 + j <= r) {
-                    pw[j] = fmaf(qv * sk[(p0 + j) * LDQ + d], cm_exp2(sum), pw[j]);
+                    pw[j] = fmaf(qv * sk[(p0 + j) * LDQ + d], tf_exp2(sum), pw[j]);
                     sum += sl[(p0 + j) * LDQ + d];
                 }
         }
@@ -502,12 +461,12 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
 #pragma unroll
             for (int j = 0; j < CM_LOCAL; j++) {
                 before += sl[(16 * s + j) * LDQ + d];
-                sq[(16 * s + j) * LDQ + d] *= cm_exp2(before);
+                sq[(16 * s + j) * LDQ + d] *= tf_exp2(before);
             }
-            vec[e] = cm_exp2(before);
+            vec[e] = tf_exp2(before);
 #pragma unroll
             for (int j = CM_LOCAL - 1; j >= 0; j--) {
-                sk[(16 * s + j) * LDQ + d] *= cm_exp2(behind);
+                sk[(16 * s + j) * LDQ + d] *= tf_exp2(behind);
                 behind += sl[(16 * s + j) * LDQ + d];
             }
         }
@@ -529,16 +488,16 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
                 for (int u = wn + 1; u < I; u++) { f0 *= vec[u * DKP + d]; f1 *= vec[u * DKP + d + 1]; }
                 x.x *= f0; x.y *= f1; y.x *= f0; y.y *= f1;
             }
-            const Tf a[1][4] = {{cm_split(x.x), cm_split(y.x), cm_split(x.y), cm_split(y.y)}};
+            const Tf a[1][4] = {{tf_split(x.x), tf_split(y.x), tf_split(x.y), tf_split(y.y)}};
             Tf b[2][2];
 #pragma unroll
             for (int n = 0; n < 2; n++) {
                 const float2 kb = *reinterpret_cast<const float2*>(sk + (16 * wn + n * 8 + g) * LDQ + d);
-                b[n][0] = cm_split(kb.x);
-                b[n][1] = cm_split(kb.y);
+                b[n][0] = tf_split(kb.x);
+                b[n][1] = tf_split(kb.y);
             }
             float* const d_[1][2] = {{w[m][0], w[m][1]}};
-            cm_mma3(d_, a, b);
+            tf_mma3(d_, a, b);
         }
     }
     if (MLSTM) {
@@ -587,7 +546,7 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
     const int col0 = wn * (DVP / 4);
 #pragma unroll 1
     for (int s = 0; s < KS + 2; s++) {
-        cm_wait<1>();
+        tf_wait<1>();
         __syncthreads();                                // slice s is there
         if (s == KS) {                                  // q with the state is done: the weights take q's place
 #pragma unroll
@@ -625,7 +584,7 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
                         for (int u = 0; u < 2 * wm + m; u++) { f0 *= vec[u * DKP + d]; f1 *= vec[u * DKP + d + 1]; }
                         x.x *= f0; x.y *= f1; y.x *= f0; y.y *= f1;
                     }
-                    a[m][0] = cm_split(x.x); a[m][1] = cm_split(y.x); a[m][2] = cm_split(x.y); a[m][3] = cm_split(y.y);
+                    a[m][0] = tf_split(x.x); a[m][1] = tf_split(y.x); a[m][2] = tf_split(x.y); a[m][3] = tf_split(y.y);
                 }
 #pragma unroll
                 for (int n = 0; n < NT; n += 2) {
@@ -633,11 +592,11 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         const float* vb = sb + (ks * 8 + 2 * t4) * LDB + (n + u) * 8;
-                        b[u][0] = cm_split(vb[0]);
-                        b[u][1] = cm_split(vb[LDB]);
+                        b[u][0] = tf_split(vb[0]);
+                        b[u][1] = tf_split(vb[LDB]);
                     }
                     float* const d_[2][2] = {{o[0][n], o[0][n + 1]}, {o[1][n], o[1][n + 1]}};
-                    cm_mma3(d_, a, b);
+                    tf_mma3(d_, a, b);
                 }
             }
         }

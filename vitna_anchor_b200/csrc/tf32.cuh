@@ -1,0 +1,52 @@
+// Products of float32 operands on the tensor cores with float32's precision, for the chunked recurrences.
+//
+// Products take float32 operands as two tf32 parts (x = high + low, 11 bits each; high high + high low + low high, float32 sums), so a product is as exact as
+// a float32 one to 2^-22; the tensor cores do 159 such multiply-adds a cycle and multiprocessor where the float32 units do 124 and would need
+// every operand from shared memory again for every 4 x 4 outputs.  Two bfloat16 parts would be twice as fast and lose a float32 state's last 7 bits.
+#pragma once
+
+#include <stdint.h>
+
+namespace vk {
+
+__device__ __forceinline__ void tf_cp16(float* dst, const float* src, bool there) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void tf_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void tf_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+__device__ __forceinline__ float tf_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// a float32 operand as two tf32 parts: its 11 leading bits rounded to the nearest, and the 11 leading bits (the tensor core does not read the others)
+// of what that leaves, rounded likewise
+struct Tf { uint32_t hi, lo; };
+__device__ __forceinline__ Tf tf_split(float x) {
+    const uint32_t hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+    return Tf{hi, __float_as_uint(x - __uint_as_float(hi)) + 0x1000u};
+}
+__device__ __forceinline__ void tf_mma(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// d[m][n] += a[m] b[n] in three products, the small ones first; products of one sum stand M N instructions apart
+template <int M, int N>
+__device__ __forceinline__ void tf_mma3(float* const (&d)[M][N], const Tf (&a)[M][4], const Tf (&b)[N][2]) {
+#pragma unroll
+    for (int m = 0; m < M; m++)
+#pragma unroll
+        for (int n = 0; n < N; n++) tf_mma(d[m][n], a[m][0].lo, a[m][1].lo, a[m][2].lo, a[m][3].lo, b[n][0].hi, b[n][1].hi);
+#pragma unroll
+    for (int m = 0; m < M; m++)
+#pragma unroll
+        for (int n = 0; n < N; n++) tf_mma(d[m][n], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[n][0].lo, b[n][1].lo);
+#pragma unroll
+    for (int m = 0; m < M; m++)
+#pragma unroll
+        for (int n = 0; n < N; n++) tf_mma(d[m][n], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[n][0].hi, b[n][1].hi);
+}
+
+}  // namespace vk

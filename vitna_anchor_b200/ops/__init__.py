@@ -908,8 +908,8 @@ def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt
     proj float32 [T, 2 G dk + 2 H dv + 2 H] = q | k | v | gate | b | a;  conv_w float32 [2 G dk + H dv, taps];  a_log, dt_bias [H];
     norm_w [dv];  state float32 [slots, delta_state_floats];  prep [T, delta_prep_width] and o [T, H dv] float32 scratch;
     out [T, H dv] in the compute dtype.  Three launches: prepare, recurrence (which also writes the state), gate.  With
-    chunk_scratch (float32, delta_chunked_scratch_floats(T, segments, ...)) the recurrence runs in its chunked form, two launches:
-    what does not need the state for all chunks side by side, then the chunks of every request in order.  With single_tokens
+    chunk_scratch (float32, delta_chunked_scratch_floats(T, segments, ...)) the recurrence runs in its chunked form, three launches:
+    what does not need the state for all chunks side by side, then the chunks of every request in order, then the outputs side by side.  With single_tokens
     (every segment is one token; sizes that delta_decode_takes) everything is ONE launch."""
     C = 2 * G * dk + H * dv
     _req(proj, "proj", torch.float32, 2); _req(conv_w, "conv_w", torch.float32, 2); _req(a_log, "a_log", torch.float32, 1)
@@ -934,8 +934,7 @@ def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt
             raise KernelError("delta_rule: the scratch of the chunked form is too small")
         _check(lib().vk_delta_chunked(_p(prep), prep.shape[1], _p(proj), _p(seg_starts), _p(seg_slots), _p(state), stride, _p(o),
                                       _p(chunk_scratch), S, T, G, H, dk, dv, taps, _stream()), "delta_chunked")
-        global _launches
-        _launches += 1                              # two kernels
+        add_launches(2)                             # three kernels
     else:
         _check(lib().vk_delta_recurrence(_p(prep), _p(proj), _p(seg_starts), _p(seg_slots), _p(state), stride, _p(o), S, T, G, H, dk, dv, taps,
                                          _stream()), "delta_recurrence")
@@ -1219,17 +1218,17 @@ def channel_delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Te
         return out
     _check(lib().vk_cdelta_prepare(_p(proj), _p(conv_w), _p(a_log), _p(dt_bias), _p(a2t), _p(g2t), _p(token_seg), _p(seg_starts), _p(seg_slots),
                                    _p(state), stride, _p(prep), T, G, H, dk, dv, taps, ra, rg, _stream()), "cdelta_prepare")
-    global _launches
     if chunk_scratch is not None:
         _req(chunk_scratch, "chunk_scratch", torch.float32, 1)
         if chunk_scratch.numel() < channel_delta_chunked_scratch_floats(T, S, H, dk, dv):
             raise KernelError("channel_delta_rule: the scratch of the chunked form is too small")
         _check(lib().vk_cdelta_chunked(_p(prep), prep.shape[1], _p(proj), proj.shape[1], _p(seg_starts), _p(seg_slots), _p(state), stride, _p(o),
                                        _p(chunk_scratch), S, T, G, H, dk, dv, taps, _stream()), "cdelta_chunked")
+        add_launches(2)                             # three kernels
     else:
         _check(lib().vk_cdelta_recurrence(_p(prep), _p(proj), proj.shape[1], _p(token_seg), _p(seg_starts), _p(seg_slots), _p(state), stride,
                                           _p(groups), _p(o), S, T, G, H, dk, dv, taps, _stream()), "cdelta_recurrence")
-    _launches += 1                                  # two kernels either way
+        add_launches(1)                             # two kernels
     _check(lib().vk_cdelta_gate(_p(o), _p(prep), _p(norm_w), ctypes.c_float(eps), _p(out), T, G, H, dk, dv, _dt(out), _stream()), "cdelta_gate")
     return out
 
