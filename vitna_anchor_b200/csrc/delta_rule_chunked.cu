@@ -10,9 +10,11 @@
 //  delta_chunk_prepare   a block a chunk and head, all chunks side by side: A, P, T = (I + A)^-1 (the four 16 x 16 blocks on the diagonal by substitution, the
 //                        others from them), W and U' as products with T, and the scaled Q and K.
 //  delta_chunk_scan      a block a request, head and 8 or 16 columns of the state walks the request's chunks in order: two small products a chunk, the state's
-//                        slice in registers and, as an operand, in shared memory; leaves U and the state before every chunk.  Chunks' operands arrive by cp.async two
-//                        chunks ahead.
-//  delta_chunk_out       a block a chunk, head and 64 columns, all chunks side by side: O.
+//                        slice in registers and, as an operand, in shared memory; leaves U and the state before every chunk.  A chunk's two operands are one bulk
+//                        copy into a ring of three stages, two chunks ahead (asked for piece by piece with cp.async they cost the block 890 of a chunk's 2,900 cycles);
+//                        every wait for one is bounded.
+//  delta_chunk_out       a block a chunk, head and 64 or 128 columns, all chunks side by side: O, and where a head's values are in one block and the decay is one
+//                        a head, its norm and gate.
 //
 // The decays, beta, the unit vectors and the state are 32-bit quantities of this mixer: products take them as two tf32 parts (tf32.cuh), every other operation is
 // float32.  The results equal the token-by-token recurrence up to the order of sums.  A chunk that reaches past its segment's end is filled
@@ -26,6 +28,7 @@
 // What bounds it: the scan is a chain of 2 products, 2 barriers a chunk; the other two kernels the tensor cores' rate for three tf32 products.
 #include "chunks.cuh"
 #include "common.cuh"
+#include "tcgen05_common.cuh"
 #include "tf32.cuh"
 
 namespace vk {
@@ -34,11 +37,15 @@ constexpr int DC_C = 64;                    // tokens of a chunk
 constexpr int DC_MAX_TAPS = 16;
 constexpr int DC_LDA = DC_C + 8;            // a padded row of a 64 x 64 matrix
 
-// Floats of scratch for one (chunk, head):  W [64][dk] | Kg [64][dk] | Qg [64][dk] | P [64][64] | U', then U [64][dv] | S before the chunk [dv][dk] | e^(L_64)
-// (one, or one a channel), padded to a multiple of four.
-__host__ __device__ __forceinline__ size_t dc_stride(int dk, int dv, bool ch) {
-    return (size_t)DC_C * (3 * dk + DC_C + dv) + (size_t)dk * dv + (ch ? (dk + 3) / 4 * 4 : 4);
-}
+// Floats of scratch for one (chunk, head):  W [64][LDQ] | Kg [64][LDQ] (rows as they lie in shared memory, dk of DKP = 64 or 128 columns used, LDQ = DKP + 8) |
+// Qg [64][dk] | P [64][64] | U', then U [64][dv] | S before the chunk [dv][dk] | e^(L_64) (one, or one a channel), padded to a multiple of four.
+__host__ __device__ __forceinline__ int dc_ldq(int dk) { return dk <= 64 ? 72 : 136; }
+__host__ __device__ __forceinline__ size_t dc_q_off(int dk) { return (size_t)2 * DC_C * dc_ldq(dk); }
+__host__ __device__ __forceinline__ size_t dc_p_off(int dk) { return dc_q_off(dk) + (size_t)DC_C * dk; }
+__host__ __device__ __forceinline__ size_t dc_u_off(int dk) { return dc_p_off(dk) + DC_C * DC_C; }
+__host__ __device__ __forceinline__ size_t dc_s_off(int dk, int dv) { return dc_u_off(dk) + (size_t)DC_C * dv; }
+__host__ __device__ __forceinline__ size_t dc_e_off(int dk, int dv) { return dc_s_off(dk, dv) + (size_t)dk * dv; }
+__host__ __device__ __forceinline__ size_t dc_stride(int dk, int dv, bool ch) { return dc_e_off(dk, dv) + (ch ? (dk + 3) / 4 * 4 : 4); }
 
 struct DcArgs {
     const float* prep;
@@ -114,11 +121,11 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
 
     float* out = p.scratch + ((size_t)blockIdx.x * p.H + h) * dc_stride(dk, dv, CH);
     float* W_g = out;
-    float* K_g = W_g + DC_C * dk;
-    float* Q_g = K_g + DC_C * dk;
-    float* P_g = Q_g + DC_C * dk;
-    float* U_g = P_g + DC_C * DC_C;
-    float* E_g = U_g + DC_C * dv + (size_t)dk * dv;
+    float* K_g = W_g + DC_C * LDQ;
+    float* Q_g = out + dc_q_off(dk);
+    float* P_g = out + dc_p_off(dk);
+    float* U_g = out + dc_u_off(dk);
+    float* E_g = out + dc_e_off(dk, dv);
 
     // k k^T and q k^T: a warp has the 16 x 16 pieces (rows 32 wm + 16 m .., columns 16 wn ..), m = 0, 1
     float kk[2][2][4], qk[2][2][4];
@@ -242,8 +249,7 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
             }
     // the scaled q and k; with a decay a channel k times e^L takes k's place
     for (int e = tid; e < DC_C * (DKP / 4); e += 256) {
-        const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
-        if (d >= dk) continue;
+        const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));      // (q and k are zero from dk on, and the scan reads Kg to DKP)
         float4 kq, kb;
         if (CH) {
             kq = *reinterpret_cast<const float4*>(sq + r * LDQ + d);
@@ -266,8 +272,8 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
             kq.x *= fq; kq.y *= fq; kq.z *= fq; kq.w *= fq;
             kb.x *= fk; kb.y *= fk; kb.z *= fk; kb.w *= fk;
         }
-        *reinterpret_cast<float4*>(Q_g + r * dk + d) = kq;
-        *reinterpret_cast<float4*>(K_g + r * dk + d) = kb;
+        if (d < dk) *reinterpret_cast<float4*>(Q_g + r * dk + d) = kq;
+        *reinterpret_cast<float4*>(K_g + r * LDQ + d) = kb;
     }
     if (CH) {
         for (int d = tid; d < dk; d += 256) E_g[d] = (vec[d] * vec[DKP + d]) * (vec[2 * DKP + d] * vec[3 * DKP + d]);
@@ -316,7 +322,8 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
     // W = T diag(beta e^L) K and U' = T diag(beta) V, eight columns a warp at a time
     if (tid < DC_C) L[tid] = CH ? beta[tid] : beta[tid] * expf(L[tid]);         // (the factor of k's rows from here on)
     __syncthreads();
-    const int nw = (dk + 7) / 8, nv = (dv + 7) / 8;
+    constexpr int nw = DKP / 8;
+    const int nv = (dv + 7) / 8;
     for (int n = warp; n < nw + nv; n += 8) {
         const bool is_w = n < nw;
         const int c0 = (is_w ? n : n - nw) * 8, ld = is_w ? LDQ : LDV;
@@ -330,19 +337,23 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
 #pragma unroll
         for (int ks = 0; ks < 8; ks++) {
             const int k = ks * 8 + 2 * t4;
-            const Tf b[1][2] = {{tf_split(fac[k] * src[k * ld]), tf_split(fac[k + 1] * src[(k + 1) * ld])}};
+            const Tf b[2] = {tf_split(fac[k] * src[k * ld]), tf_split(fac[k + 1] * src[(k + 1) * ld])};
+            Tf a[4][4];
 #pragma unroll
-            for (int m = 0; m < 4; m++) {
-                if (m < ks / 2) continue;           // T is lower triangular
+            for (int m = ks / 2; m < 4; m++) {      // T is lower triangular
                 const float2 x = *reinterpret_cast<const float2*>(sT + (16 * m + g) * DC_LDA + k), y = *reinterpret_cast<const float2*>(sT + (16 * m + g + 8) * DC_LDA + k);
-                const Tf a[1][4] = {{tf_split(x.x), tf_split(y.x), tf_split(x.y), tf_split(y.y)}};
-                float* const d_[1][1] = {{acc[m]}};
-                tf_mma3(d_, a, b);
+                a[m][0] = tf_split(x.x); a[m][1] = tf_split(y.x); a[m][2] = tf_split(x.y); a[m][3] = tf_split(y.y);
             }
+#pragma unroll
+            for (int m = ks / 2; m < 4; m++) tf_mma(acc[m], a[m][0].lo, a[m][1].lo, a[m][2].lo, a[m][3].lo, b[0].hi, b[1].hi);
+#pragma unroll
+            for (int m = ks / 2; m < 4; m++) tf_mma(acc[m], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[0].lo, b[1].lo);
+#pragma unroll
+            for (int m = ks / 2; m < 4; m++) tf_mma(acc[m], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[0].hi, b[1].hi);
         }
         float* dst = is_w ? W_g : U_g;
-        const int width = is_w ? dk : dv, c = c0 + 2 * t4;
-        if (c < width) {
+        const int width = is_w ? LDQ : dv, c = c0 + 2 * t4;
+        if (is_w || c < dv) {
 #pragma unroll
             for (int m = 0; m < 4; m++) {
                 *reinterpret_cast<float2*>(dst + (size_t)(16 * m + g) * width + c) = make_float2(acc[m][0], acc[m][1]);
@@ -358,11 +369,12 @@ constexpr int DC_STAGES = 3;
 
 template <int DKP, int COLS, bool CH>
 __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs p, const float* __restrict__ proj, int N, float* __restrict__ state,
-                                                                   size_t state_stride, size_t conv_off, int taps) {
+                                                                   size_t state_stride, size_t conv_off, int taps, const WaitCtl wc) {
     constexpr int NTH = DKP * 2, LDQ = DKP + 8, LDS = DKP + 4, LDU = DC_C + 4, NT = COLS / 8, STAGE = 2 * DC_C * LDQ;
     static_assert(NT == DKP / 64, "the warps of the first product");
-    extern __shared__ __align__(16) float ds_smem[];
-    __shared__ int base_sh;
+    extern __shared__ __align__(128) float ds_smem[];
+    __shared__ __align__(8) uint64_t full[DC_STAGES];
+    __shared__ int base_sh, failed;
     float* ring = ds_smem;
     float* sS = ring + DC_STAGES * STAGE;           // [COLS][LDS]
     float* sU = sS + COLS * LDS;                    // [COLS][LDU]
@@ -371,7 +383,13 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
     if (slot < 0 || n <= 0) return;
     if (warp == 0) {
         const int b = first_chunk_of<DC_C>(seg, p.seg_starts);
-        if (lane == 0) base_sh = b;
+        if (lane == 0) {
+            base_sh = b;
+            failed = 0;
+            for (int i = 0; i < DC_STAGES; i++) mbar_init(&full[i], 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
     }
     const int dk = p.dk, dv = p.dv, H = p.H, c0 = blockIdx.z * COLS, chunks = (n + DC_C - 1) / DC_C;
     float* row = state + (size_t)slot * state_stride;
@@ -382,17 +400,13 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
     __syncthreads();
     const size_t stride = dc_stride(dk, dv, CH);
     float* mine = p.scratch + ((size_t)base_sh * H + h) * stride;
-    const size_t u_off = (size_t)DC_C * (3 * dk + DC_C), s_off = u_off + (size_t)DC_C * dv, e_off = s_off + (size_t)dk * dv;
-    auto issue = [&](int c) {
-        if (c < chunks) {
-            const float* in = mine + (size_t)c * H * stride;
-            float* st = ring + (c % DC_STAGES) * STAGE;
-            for (int e = tid; e < 2 * DC_C * (DKP / 4); e += NTH) {
-                const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));           // rows of W, then of Kg
-                tf_cp16(st + r * LDQ + d, in + (d < dk ? (size_t)r * dk + d : 0), d < dk);
-            }
-        }
-        tf_commit();
+    const size_t u_off = dc_u_off(dk), s_off = dc_s_off(dk, dv), e_off = dc_e_off(dk, dv);
+    auto issue = [&](int c) {                       // thread 0: chunk c's W and Kg, one copy
+        if (c >= chunks || c == wc.skip_stage) return;          // (a chunk named by wc.skip_stage is left out: a test of the give-up path)
+        uint64_t* bar = &full[c % DC_STAGES];
+        mbar_expect_tx(bar, STAGE * 4);
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(smem_u32(ring + (c % DC_STAGES) * STAGE)), "l"(mine + (size_t)c * H * stride), "r"(STAGE * 4), "r"(smem_u32(bar)) : "memory");
     };
     float s[NT][4];                                 // this warp's rows of the state: rows d, d + 8, columns 8 i + 2 t4, + 1
     const int d = 16 * warp + g;
@@ -411,13 +425,19 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
         dec[0] = CH ? (d < dk ? in[e_off + d] : 0.0f) : in[e_off];
         dec[1] = CH ? (d + 8 < dk ? in[e_off + d + 8] : 0.0f) : dec[0];
     };
-    issue(0);
-    issue(1);
+    if (tid == 0) {
+        issue(0);
+        issue(1);
+    }
     fetch(0);
     for (int c = 0; c < chunks; c++) {
-        tf_wait<1>();
+        if (!mbar_wait(&full[c % DC_STAGES], (c / DC_STAGES) & 1, wc.cycles)) give_up(wc.error, &failed, 61);
         __syncthreads();                            // the chunk's operands are there, the state's slice is written, and everybody has left the chunk before
-        issue(c + 2);
+        if (*reinterpret_cast<volatile int*>(&failed)) {        // the same for every thread: all have written it before the barrier or nobody has
+            __nanosleep(200000);                    // let copies in flight land
+            return;
+        }
+        if (tid == 0) issue(c + 2);
         float* in = mine + (size_t)c * H * stride;
         const float* sW = ring + (c % DC_STAGES) * STAGE;
         const float* sK = sW + DC_C * LDQ;
@@ -425,25 +445,33 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
             const int cc = e / (DKP / 4), dd = 4 * (e % (DKP / 4));
             if (c0 + cc < dv && dd < dk) *reinterpret_cast<float4*>(in + s_off + (size_t)(c0 + cc) * dk + dd) = *reinterpret_cast<const float4*>(sS + cc * LDS + dd);
         }
-        float x[3][4];
+        // (a product of one sum waits some 70 cycles for the one before it: the steps take turns on four sets of sums)
+        float x[4][3][4];
 #pragma unroll
-        for (int i = 0; i < 3; i++)
+        for (int j = 0; j < 4; j++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) x[i][e] = 0.0f;
+            for (int i = 0; i < 3; i++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) x[j][i][e] = 0.0f;
         const float* wa = sW + ur * LDQ + 2 * t4;
         const float* sb = sS + (8 * (warp >> 2) + g) * LDS + 2 * t4;
-#pragma unroll 4
+#pragma unroll
         for (int ks = 0; ks < DKP / 8; ks++) {
             const float2 a0 = *reinterpret_cast<const float2*>(wa + ks * 8), a1 = *reinterpret_cast<const float2*>(wa + 8 * LDQ + ks * 8);
             const float2 b0 = *reinterpret_cast<const float2*>(sb + ks * 8);
             const Tf a[4] = {tf_split(a0.x), tf_split(a1.x), tf_split(a0.y), tf_split(a1.y)}, b[2] = {tf_split(b0.x), tf_split(b0.y)};
-            tf_mma(x[0], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
-            tf_mma(x[1], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
-            tf_mma(x[2], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
+            tf_mma(x[ks & 3][0], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
+            tf_mma(x[ks & 3][1], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
+            tf_mma(x[ks & 3][2], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
         }
-        float2 u[2];
-        u[0] = make_float2(up[0].x - ((x[0][0] + x[1][0]) + x[2][0]), up[0].y - ((x[0][1] + x[1][1]) + x[2][1]));
-        u[1] = make_float2(up[1].x - ((x[0][2] + x[1][2]) + x[2][2]), up[1].y - ((x[0][3] + x[1][3]) + x[2][3]));
+        float ws[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            ws[e] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 3; i++) ws[e] += (x[0][i][e] + x[1][i][e]) + (x[2][i][e] + x[3][i][e]);
+        }
+        const float2 u[2] = {make_float2(up[0].x - ws[0], up[0].y - ws[1]), make_float2(up[1].x - ws[2], up[1].y - ws[3])};
         sU[uc * LDU + ur] = u[0].x;
         sU[(uc + 1) * LDU + ur] = u[0].y;
         sU[uc * LDU + ur + 8] = u[1].x;
@@ -455,14 +483,17 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
         const float da = dec[0], db = dec[1];
         fetch(c + 1);
         __syncthreads();                            // U is there, and nobody reads the old state any more
-        float y[NT][3][4];
+        constexpr int SETS = 4 / NT;
+        float y[NT][SETS][3][4];
 #pragma unroll
         for (int i = 0; i < NT; i++)
 #pragma unroll
-            for (int j = 0; j < 3; j++)
+            for (int q = 0; q < SETS; q++)
 #pragma unroll
-                for (int e = 0; e < 4; e++) y[i][j][e] = 0.0f;
-#pragma unroll 4
+                for (int j = 0; j < 3; j++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) y[i][q][j][e] = 0.0f;
+#pragma unroll
         for (int ks = 0; ks < DC_C / 8; ks++) {
             const float* ka = sK + (ks * 8 + t4) * LDQ + d;
             const Tf a[4] = {tf_split(ka[0]), tf_split(ka[8]), tf_split(ka[4 * LDQ]), tf_split(ka[4 * LDQ + 8])};
@@ -470,16 +501,22 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
             for (int i = 0; i < NT; i++) {
                 const float* ub = sU + (8 * i + g) * LDU + ks * 8 + t4;
                 const Tf b[2] = {tf_split(ub[0]), tf_split(ub[4])};
-                tf_mma(y[i][0], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
-                tf_mma(y[i][1], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
-                tf_mma(y[i][2], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
+                float (*z)[4] = y[i][ks % SETS];
+                tf_mma(z[0], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
+                tf_mma(z[1], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
+                tf_mma(z[2], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
             }
         }
 #pragma unroll
         for (int i = 0; i < NT; i++)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                s[i][e] = fmaf(e < 2 ? da : db, s[i][e], (y[i][0][e] + y[i][1][e]) + y[i][2][e]);
+                float add = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 3; j++)
+#pragma unroll
+                    for (int q = 0; q < SETS; q++) add += y[i][q][j][e];
+                s[i][e] = fmaf(e < 2 ? da : db, s[i][e], add);
                 sS[(8 * i + 2 * t4 + (e & 1)) * LDS + d + 8 * (e >> 1)] = s[i][e];
             }
     }
@@ -508,82 +545,122 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
     }
 }
 
-// grid (chunks, H, slices of 64 columns); 256 threads: warp w has rows 16 (w & 3) .. and columns 32 (w >> 2) .. of the slice
-template <int DKP>
-__global__ void __launch_bounds__(256) delta_chunk_out_kernel(const DcArgs p, bool ch_decay, float* __restrict__ o) {
-    constexpr int LDQ = DKP + 8, LDU = 64 + 4;
+// grid (chunks, H, slices of COLS columns); 256 threads: warp w has rows 16 (w & 3) .. and half of the slice's columns, w >> 2.  norm_w (null: o [tokens][H dv] gets the
+// outputs as they are): out [tokens][H dv] in T gets o / rms(o) over the head's dv <= COLS values * norm_w * silu(gate), the gate at gate_off of proj's rows.
+template <int DKP, int COLS, typename T>
+__global__ void __launch_bounds__(256) delta_chunk_out_kernel(const DcArgs p, bool ch_decay, float* __restrict__ o, const float* __restrict__ proj, int N, int gate_off,
+                                                              const float* __restrict__ norm_w, float eps, T* __restrict__ out) {
+    constexpr int LDQ = DKP + 8, LDU = COLS + 4, NT = COLS / 16;
     extern __shared__ __align__(16) float do_smem[];
     __shared__ int find[4];
+    __shared__ float squares[2][DC_C];
     float* sQ = do_smem;                            // [64][LDQ]
-    float* sS = sQ + DC_C * LDQ;                    // [64 columns][LDQ]
-    float* sP = sS + 64 * LDQ;                      // [64][DC_LDA]
+    float* sS = sQ + DC_C * LDQ;                    // [COLS columns][LDQ]
+    float* sP = sS + COLS * LDQ;                    // [64][DC_LDA]
     float* sU = sP + DC_C * DC_LDA;                 // [64][LDU]
     const Chunk ch = find_chunk<DC_C>(blockIdx.x, p.seg_starts, p.segments, find);
     if (ch.seg < 0 || p.seg_slots[ch.seg] < 0) return;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, m = warp & 3, cw = 32 * (warp >> 2);
-    const int h = blockIdx.y, c0 = blockIdx.z * 64, dk = p.dk, dv = p.dv;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, m = warp & 3, half = warp >> 2, cw = (COLS / 2) * half;
+    const int h = blockIdx.y, c0 = blockIdx.z * COLS, dk = p.dk, dv = p.dv;
     const float* in = p.scratch + ((size_t)blockIdx.x * p.H + h) * dc_stride(dk, dv, ch_decay);
-    const float* Q_g = in + 2 * (size_t)DC_C * dk;
-    const float* P_g = Q_g + (size_t)DC_C * dk;
-    const float* U_g = P_g + DC_C * DC_C;
-    const float* S_g = U_g + (size_t)DC_C * dv;
     for (int e = tid; e < DC_C * (DKP / 4); e += 256) {
         const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
-        const bool on = d < dk, ons = on && c0 + r < dv;
-        tf_cp16(sQ + r * LDQ + d, Q_g + (on ? (size_t)r * dk + d : 0), on);
-        tf_cp16(sS + r * LDQ + d, S_g + (ons ? (size_t)(c0 + r) * dk + d : 0), ons);
+        tf_cp16(sQ + r * LDQ + d, in + dc_q_off(dk) + (d < dk ? (size_t)r * dk + d : 0), d < dk);
+    }
+    for (int e = tid; e < COLS * (DKP / 4); e += 256) {
+        const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
+        const bool on = d < dk && c0 + r < dv;
+        tf_cp16(sS + r * LDQ + d, in + dc_s_off(dk, dv) + (on ? (size_t)(c0 + r) * dk + d : 0), on);
     }
     for (int e = tid; e < DC_C * 16; e += 256) {
         const int r = e / 16, c = 4 * (e % 16);
+        tf_cp16(sP + r * DC_LDA + c, in + dc_p_off(dk) + r * DC_C + c, true);
+    }
+    for (int e = tid; e < DC_C * (COLS / 4); e += 256) {
+        const int r = e / (COLS / 4), c = 4 * (e % (COLS / 4));
         const bool on = c0 + c < dv;
-        tf_cp16(sP + r * DC_LDA + c, P_g + r * DC_C + c, true);
-        tf_cp16(sU + r * LDU + c, U_g + (on ? (size_t)r * dv + c0 + c : 0), on);
+        tf_cp16(sU + r * LDU + c, in + dc_u_off(dk) + (on ? (size_t)r * dv + c0 + c : 0), on);
     }
     tf_commit();
     tf_wait<0>();
     __syncthreads();
-    if (16 * m >= ch.rows) return;
-    float acc[4][4];
+    float acc[NT][4];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < NT; i++)
 #pragma unroll
         for (int e = 0; e < 4; e++) acc[i][e] = 0.0f;
-    float* const d_[1][4] = {{acc[0], acc[1], acc[2], acc[3]}};
-#pragma unroll 4
-    for (int ks = 0; ks < DKP / 8; ks++) {
-        const int k = ks * 8 + 2 * t4;
-        const float2 x = *reinterpret_cast<const float2*>(sQ + (16 * m + g) * LDQ + k), y = *reinterpret_cast<const float2*>(sQ + (16 * m + g + 8) * LDQ + k);
+    auto step = [&](const float* pa, int lda, auto&& right) {
+        const float2 x = *reinterpret_cast<const float2*>(pa), y = *reinterpret_cast<const float2*>(pa + 8 * lda);
         const Tf a[1][4] = {{tf_split(x.x), tf_split(y.x), tf_split(x.y), tf_split(y.y)}};
-        Tf b[4][2];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float2 v = *reinterpret_cast<const float2*>(sS + (cw + 8 * i + g) * LDQ + k);
-            b[i][0] = tf_split(v.x);
-            b[i][1] = tf_split(v.y);
+        for (int i0 = 0; i0 < NT; i0 += 4) {
+            Tf b[4][2];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 v = right(i0 + i);
+                b[i][0] = tf_split(v.x);
+                b[i][1] = tf_split(v.y);
+            }
+            float* const d_[1][4] = {{acc[i0], acc[i0 + 1], acc[i0 + 2], acc[i0 + 3]}};
+            tf_mma3(d_, a, b);
         }
-        tf_mma3(d_, a, b);
-    }
+    };
+    if (16 * m < ch.rows) {
 #pragma unroll 2
-    for (int ks = 0; ks < 2 * (m + 1); ks++) {      // (P is lower triangular)
-        const int k = ks * 8 + 2 * t4;
-        const float2 x = *reinterpret_cast<const float2*>(sP + (16 * m + g) * DC_LDA + k), y = *reinterpret_cast<const float2*>(sP + (16 * m + g + 8) * DC_LDA + k);
-        const Tf a[1][4] = {{tf_split(x.x), tf_split(y.x), tf_split(x.y), tf_split(y.y)}};
-        Tf b[4][2];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float* ub = sU + k * LDU + cw + 8 * i + g;
-            b[i][0] = tf_split(ub[0]);
-            b[i][1] = tf_split(ub[LDU]);
+        for (int ks = 0; ks < DKP / 8; ks++) {
+            const int k = ks * 8 + 2 * t4;
+            step(sQ + (16 * m + g) * LDQ + k, LDQ, [&](int i) { return *reinterpret_cast<const float2*>(sS + (cw + 8 * i + g) * LDQ + k); });
         }
-        tf_mma3(d_, a, b);
+#pragma unroll 2
+        for (int ks = 0; ks < 2 * (m + 1); ks++) {  // (P is lower triangular)
+            const int k = ks * 8 + 2 * t4;
+            step(sP + (16 * m + g) * DC_LDA + k, DC_LDA, [&](int i) { const float* ub = sU + k * LDU + cw + 8 * i + g; return make_float2(ub[0], ub[LDU]); });
+        }
+    }
+    if (!norm_w) {
+#pragma unroll
+        for (int i = 0; i < NT; i++)
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int r = 16 * m + g + 8 * u, c = c0 + cw + 8 * i + 2 * t4;
+                if (r < ch.rows && c < dv) *reinterpret_cast<float2*>(o + ((size_t)(ch.first + r) * p.H + h) * dv + c) = make_float2(acc[i][2 * u], acc[i][2 * u + 1]);
+            }
+        return;
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int u = 0; u < 2; u++) {
+        float ss = 0.0f;
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int r = 16 * m + g + 8 * u, c = c0 + cw + 8 * i + 2 * t4;
-            if (r < ch.rows && c < dv) *reinterpret_cast<float2*>(o + ((size_t)(ch.first + r) * p.H + h) * dv + c) = make_float2(acc[i][2 * u], acc[i][2 * u + 1]);
+        for (int i = 0; i < NT; i++) {
+            ss = fmaf(acc[i][2 * u], acc[i][2 * u], ss);
+            ss = fmaf(acc[i][2 * u + 1], acc[i][2 * u + 1], ss);
         }
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+        if (t4 == 0) squares[half][16 * m + g + 8 * u] = ss;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int r = 16 * m + g + 8 * u;
+        if (r >= ch.rows) continue;
+        const float inv = 1.0f / sqrtf((squares[0][r] + squares[1][r]) / (float)dv + eps);
+        const float* gate = proj + (size_t)(ch.first + r) * N + gate_off + (size_t)h * dv;
+        T* orow = out + ((size_t)(ch.first + r) * p.H + h) * dv;
+#pragma unroll
+        for (int i = 0; i < NT; i++) {
+            const int c = cw + 8 * i + 2 * t4;
+            if (c >= dv) continue;
+            float v[2];
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const float gt = gate[c + e];
+                v[e] = ((acc[i][2 * u + e] * inv) * norm_w[c + e]) * (gt / (1.0f + expf(-gt)));
+            }
+            if (sizeof(T) == 2) *reinterpret_cast<__nv_bfloat162*>(orow + c) = __floats2bfloat162_rn(v[0], v[1]);
+            else { orow[c] = from_f32<T>(v[0]); orow[c + 1] = from_f32<T>(v[1]); }
+        }
+    }
 }
 
 }  // namespace vk
@@ -602,47 +679,72 @@ VK_API size_t vk_delta_chunked_scratch_bytes(int tokens, int segments, int H, in
     return (size_t)dc_chunks(tokens, segments) * H * dc_stride(dk, dv, false) * sizeof(float);
 }
 
+// Whether delta_chunk_out norms and gates the outputs itself (else the gate kernel follows): a head's values lie in one of its blocks.
+VK_API int vk_delta_chunked_gates(int dv) { return dv <= 128; }
+
+struct DcOut {
+    float* o;
+    const float* proj;
+    int N, gate_off;
+    const float* norm_w;                    // null: o
+    float eps;
+    void* out;
+    int dtype;
+};
+
+template <int DKP, int COLS, typename T>
+static int delta_out_launch(const DcArgs& p, bool ch, const DcOut& f, int chunks, cudaStream_t stream) {
+    auto kern = delta_chunk_out_kernel<DKP, COLS, T>;
+    const int smem = (DC_C * (DKP + 8) + COLS * (DKP + 8) + DC_C * DC_LDA + DC_C * (COLS + 4)) * (int)sizeof(float);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    return launch_plain(kern, dim3(chunks, p.H, (p.dv + COLS - 1) / COLS), dim3(256), smem, stream, p, ch, f.o, f.proj, f.N, f.gate_off, f.norm_w, f.eps, (T*)f.out);
+}
+
 template <int DKP, bool CH>
-static int delta_chunked_launch(const DcArgs& p, const float* proj, int proj_width, float* state, size_t state_stride, float* o, int tokens, int taps,
-                                cudaStream_t stream) {
+static int delta_chunked_launch(const DcArgs& p, const float* proj, int proj_width, float* state, size_t state_stride, const DcOut& f, int tokens, int taps,
+                                int* error, cudaStream_t stream) {
     constexpr int COLS = DKP / 8;
     const int chunks = dc_chunks(tokens, p.segments);
     const int smem1 = (dc_prepare_floats_fixed<DKP, CH>() + DC_C * dc_ldv(p.dv)) * (int)sizeof(float);
     const int smem2 = (DC_STAGES * 2 * DC_C * (DKP + 8) + COLS * (DKP + 4) + COLS * (DC_C + 4)) * (int)sizeof(float);
-    const int smem3 = (2 * DC_C * (DKP + 8) + DC_C * DC_LDA + DC_C * 68) * (int)sizeof(float);
     auto k1 = delta_chunk_prepare_kernel<DKP, CH>;
     auto k2 = delta_chunk_scan_kernel<DKP, COLS, CH>;
-    auto k3 = delta_chunk_out_kernel<DKP>;
     cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, smem3);
     if (e != cudaSuccess) return (int)e;
     int rc = launch_plain(k1, dim3(chunks, p.H), dim3(256), smem1, stream, p);
     if (rc != VK_OK) return rc;
     rc = launch_plain(k2, dim3(p.segments, p.H, (p.dv + COLS - 1) / COLS), dim3(DKP * 2), smem2, stream, p, proj, proj_width, state, state_stride,
-                      (size_t)p.H * p.dv * p.dk, taps);
+                      (size_t)p.H * p.dv * p.dk, taps, wait_ctl(error, WAIT_FAMILY_DELTA));
     if (rc != VK_OK) return rc;
-    return launch_plain(k3, dim3(chunks, p.H, (p.dv + 63) / 64), dim3(256), smem3, stream, p, CH, o);
+    // slices of 128 columns only where a head's outputs are normed here: the smaller block's two a multiprocessor are otherwise the better
+    if (f.norm_w && p.dv > 64)
+        return f.dtype == 0 ? delta_out_launch<DKP, 128, float>(p, CH, f, chunks, stream) : delta_out_launch<DKP, 128, __nv_bfloat16>(p, CH, f, chunks, stream);
+    return f.dtype == 0 ? delta_out_launch<DKP, 64, float>(p, CH, f, chunks, stream) : delta_out_launch<DKP, 64, __nv_bfloat16>(p, CH, f, chunks, stream);
 }
 
 template <bool CH>
 static int delta_chunked(const float* prep, int prep_width, const float* proj, int proj_width, const int32_t* seg_starts, const int32_t* seg_slots, float* state,
-                         size_t state_stride, float* o, float* scratch, int segments, int tokens, int G, int H, int dk, int dv, int taps, cudaStream_t stream) {
+                         size_t state_stride, const DcOut& f, float* scratch, int segments, int tokens, int G, int H, int dk, int dv, int taps, int* error,
+                         cudaStream_t stream) {
     if (segments <= 0 || tokens <= 0) return VK_OK;
-    if (!vk_delta_chunked_takes(G, H, dk, dv, taps) || prep_width % 4) return VK_BAD_SHAPE;
-    if ((uintptr_t)scratch % 16 || (uintptr_t)prep % 16 || (uintptr_t)o % 8) return VK_BAD_ALIGNMENT;
+    if (!vk_delta_chunked_takes(G, H, dk, dv, taps) || prep_width % 4 || !error || (f.norm_w && !vk_delta_chunked_gates(dv))) return VK_BAD_SHAPE;
+    if ((uintptr_t)scratch % 16 || (uintptr_t)prep % 16 || (uintptr_t)f.o % 8 || (f.norm_w && (uintptr_t)f.out % 4)) return VK_BAD_ALIGNMENT;
     if (H > 65535) return VK_TOO_LARGE;
     const DcArgs p = {prep, prep_width, seg_starts, seg_slots, segments, scratch, G, H, dk, dv};
-    return dk <= 64 ? delta_chunked_launch<64, CH>(p, proj, proj_width, state, state_stride, o, tokens, taps, stream)
-                    : delta_chunked_launch<128, CH>(p, proj, proj_width, state, state_stride, o, tokens, taps, stream);
+    return dk <= 64 ? delta_chunked_launch<64, CH>(p, proj, proj_width, state, state_stride, f, tokens, taps, error, stream)
+                    : delta_chunked_launch<128, CH>(p, proj, proj_width, state, state_stride, f, tokens, taps, error, stream);
 }
 
-// prep [tokens][prep width] as delta_prepare leaves it; proj as for the token-by-token kernel; o [tokens][H*dv] float32; three kernels.
+// prep [tokens][prep width] as delta_prepare leaves it; proj as for the token-by-token kernel; three kernels.  norm_w null: o [tokens][H*dv] float32 gets the outputs.
+// Else (sizes that vk_delta_chunked_gates) out [tokens][H*dv] in dtype gets them as vk_delta_gate makes them.  error: as for vk_linear_tcgen05.
 VK_API int vk_delta_chunked(const float* prep, int prep_width, const float* proj, const int32_t* seg_starts, const int32_t* seg_slots, float* state,
-                            size_t state_stride, float* o, float* scratch, int segments, int tokens, int G, int H, int dk, int dv, int taps,
-                            cudaStream_t stream) {
-    return delta_chunked<false>(prep, prep_width, proj, 2 * G * dk + 2 * H * dv + 2 * H, seg_starts, seg_slots, state, state_stride, o, scratch, segments,
-                                tokens, G, H, dk, dv, taps, stream);
+                            size_t state_stride, float* o, float* scratch, const float* norm_w, float eps, void* out, int dtype, int segments, int tokens, int G,
+                            int H, int dk, int dv, int taps, int* error, cudaStream_t stream) {
+    const int N = 2 * G * dk + 2 * H * dv + 2 * H;
+    const DcOut f = {o, proj, N, 2 * G * dk + H * dv, norm_w, eps, out, dtype};
+    return delta_chunked<false>(prep, prep_width, proj, N, seg_starts, seg_slots, state, state_stride, f, scratch, segments, tokens, G, H, dk, dv, taps, error, stream);
 }
 
 // The form with a decay per head and key channel: prep as cdelta_prepare leaves it, proj rows of proj_width floats (the
@@ -653,7 +755,8 @@ VK_API size_t vk_cdelta_chunked_scratch_bytes(int tokens, int segments, int H, i
 
 VK_API int vk_cdelta_chunked(const float* prep, int prep_width, const float* proj, int proj_width, const int32_t* seg_starts,
                              const int32_t* seg_slots, float* state, size_t state_stride, float* o, float* scratch, int segments, int tokens,
-                             int G, int H, int dk, int dv, int taps, cudaStream_t stream) {
-    return delta_chunked<true>(prep, prep_width, proj, proj_width, seg_starts, seg_slots, state, state_stride, o, scratch, segments, tokens, G, H, dk, dv, taps,
-                               stream);
+                             int G, int H, int dk, int dv, int taps, int* error, cudaStream_t stream) {
+    const DcOut f = {o, nullptr, 0, 0, nullptr, 0.0f, nullptr, 0};
+    return delta_chunked<true>(prep, prep_width, proj, proj_width, seg_starts, seg_slots, state, state_stride, f, scratch, segments, tokens, G, H, dk, dv, taps,
+                               error, stream);
 }

@@ -392,7 +392,7 @@ def set_wait_limit_ms(ms: float) -> None:
         raise KernelError(f"set_wait_limit_ms: CUDA error {status}")
 
 
-WAIT_FAMILIES = {"linear_tcgen05": 1, "linear_tcgen05_wide": 2, "attention_prefill_tcgen05": 3, "attention_decode_tma": 4}
+WAIT_FAMILIES = {"linear_tcgen05": 1, "linear_tcgen05_wide": 2, "attention_prefill_tcgen05": 3, "attention_decode_tma": 4, "delta_chunked": 5}
 
 
 def skip_stage_once(family: str, stage: int) -> None:
@@ -909,7 +909,8 @@ def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt
     norm_w [dv];  state float32 [slots, delta_state_floats];  prep [T, delta_prep_width] and o [T, H dv] float32 scratch;
     out [T, H dv] in the compute dtype.  Three launches: prepare, recurrence (which also writes the state), gate.  With
     chunk_scratch (float32, delta_chunked_scratch_floats(T, segments, ...)) the recurrence runs in its chunked form, three launches:
-    what does not need the state for all chunks side by side, then the chunks of every request in order, then the outputs side by side.  With single_tokens
+    what does not need the state for all chunks side by side, then the chunks of every request in order, then the outputs side by side
+    (normed and gated there where vk_delta_chunked_gates(dv); o is then not used).  With single_tokens
     (every segment is one token; sizes that delta_decode_takes) everything is ONE launch."""
     C = 2 * G * dk + H * dv
     _req(proj, "proj", torch.float32, 2); _req(conv_w, "conv_w", torch.float32, 2); _req(a_log, "a_log", torch.float32, 1)
@@ -932,9 +933,13 @@ def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt
         _req(chunk_scratch, "chunk_scratch", torch.float32, 1)
         if chunk_scratch.numel() < delta_chunked_scratch_floats(T, S, H, dk, dv):
             raise KernelError("delta_rule: the scratch of the chunked form is too small")
-        _check(lib().vk_delta_chunked(_p(prep), prep.shape[1], _p(proj), _p(seg_starts), _p(seg_slots), _p(state), stride, _p(o),
-                                      _p(chunk_scratch), S, T, G, H, dk, dv, taps, _stream()), "delta_chunked")
+        gated_here = bool(lib().vk_delta_chunked_gates(dv))
+        _check(lib().vk_delta_chunked(_p(prep), prep.shape[1], _p(proj), _p(seg_starts), _p(seg_slots), _p(state), stride, _p(o), _p(chunk_scratch),
+                                      _p(norm_w if gated_here else None), ctypes.c_float(eps), _p(out), _dt(out), S, T, G, H, dk, dv, taps, _p(error_word()),
+                                      _stream()), "delta_chunked")
         add_launches(2)                             # three kernels
+        if gated_here:
+            return out
     else:
         _check(lib().vk_delta_recurrence(_p(prep), _p(proj), _p(seg_starts), _p(seg_slots), _p(state), stride, _p(o), S, T, G, H, dk, dv, taps,
                                          _stream()), "delta_recurrence")
@@ -1223,7 +1228,7 @@ def channel_delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Te
         if chunk_scratch.numel() < channel_delta_chunked_scratch_floats(T, S, H, dk, dv):
             raise KernelError("channel_delta_rule: the scratch of the chunked form is too small")
         _check(lib().vk_cdelta_chunked(_p(prep), prep.shape[1], _p(proj), proj.shape[1], _p(seg_starts), _p(seg_slots), _p(state), stride, _p(o),
-                                       _p(chunk_scratch), S, T, G, H, dk, dv, taps, _stream()), "cdelta_chunked")
+                                       _p(chunk_scratch), S, T, G, H, dk, dv, taps, _p(error_word()), _stream()), "cdelta_chunked")
         add_launches(2)                             # three kernels
     else:
         _check(lib().vk_cdelta_recurrence(_p(prep), _p(proj), proj.shape[1], _p(token_seg), _p(seg_starts), _p(seg_slots), _p(state), stride,
