@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(1024) delta_prepare_kernel(
 // once for each; the same operations in the same order, so the same bits.  2,048 tokens of 1,152 channels: 23.6 us a block a token, FIG_PREP.  smem: act [DP_TOKENS][2 G dk].
 constexpr int DP_TOKENS = 8, DP_TAPS = 4;
 
-__global__ void __launch_bounds__(512) delta_prepare_tokens_kernel(
+__global__ void __launch_bounds__(256, 4) delta_prepare_tokens_kernel(
     const float* __restrict__ proj, const float* __restrict__ conv_w, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
     const int32_t* __restrict__ token_seg, const int32_t* __restrict__ seg_starts, const int32_t* __restrict__ seg_slots,
     const float* __restrict__ state, size_t state_stride, size_t conv_off, float* __restrict__ prep, int P, int G, int H, int dk, int dv,
@@ -541,7 +541,7 @@ VK_API int vk_delta_prepare(const float* proj, const float* conv_w, const float*
     // from 148 blocks on: below, a block a token has the shorter way
     const size_t smem8 = (size_t)DP_TOKENS * 2 * G * dk * sizeof(float);
     if (taps <= DP_TAPS && tokens >= 148 * DP_TOKENS && smem8 <= 48 * 1024)
-        return launch_plain(delta_prepare_tokens_kernel, dim3((tokens + DP_TOKENS - 1) / DP_TOKENS), dim3(512), smem8, stream, proj, conv_w, a_log, dt_bias, token_seg,
+        return launch_plain(delta_prepare_tokens_kernel, dim3((tokens + DP_TOKENS - 1) / DP_TOKENS), dim3(256), smem8, stream, proj, conv_w, a_log, dt_bias, token_seg,
                             seg_starts, seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps, tokens);
     return launch_plain(delta_prepare_kernel, dim3(tokens), dim3(256), smem, stream, proj, conv_w, a_log, dt_bias, token_seg, seg_starts,
                         seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps);

@@ -582,6 +582,20 @@ __global__ void __launch_bounds__(256) delta_chunk_out_kernel(const DcArgs p, bo
         tf_cp16(sU + r * LDU + c, in + dc_u_off(dk) + (on ? (size_t)r * dv + c0 + c : 0), on);
     }
     tf_commit();
+    // the gate's values are asked for with the operands
+    float2 gt[2][NT];
+    if (norm_w) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int r = 16 * m + g + 8 * u;
+            const float* gate = proj + (size_t)(ch.first + (r < ch.rows ? r : 0)) * N + gate_off + (size_t)h * dv;
+#pragma unroll
+            for (int i = 0; i < NT; i++) {
+                const int c = cw + 8 * i + 2 * t4;
+                gt[u][i] = c < dv ? make_float2(gate[c], gate[c + 1]) : make_float2(0.0f, 0.0f);
+            }
+        }
+    }
     tf_wait<0>();
     __syncthreads();
     float acc[NT][4];
@@ -645,7 +659,6 @@ __global__ void __launch_bounds__(256) delta_chunk_out_kernel(const DcArgs p, bo
         const int r = 16 * m + g + 8 * u;
         if (r >= ch.rows) continue;
         const float inv = 1.0f / sqrtf((squares[0][r] + squares[1][r]) / (float)dv + eps);
-        const float* gate = proj + (size_t)(ch.first + r) * N + gate_off + (size_t)h * dv;
         T* orow = out + ((size_t)(ch.first + r) * p.H + h) * dv;
 #pragma unroll
         for (int i = 0; i < NT; i++) {
@@ -654,8 +667,8 @@ __global__ void __launch_bounds__(256) delta_chunk_out_kernel(const DcArgs p, bo
             float v[2];
 #pragma unroll
             for (int e = 0; e < 2; e++) {
-                const float gt = gate[c + e];
-                v[e] = ((acc[i][2 * u + e] * inv) * norm_w[c + e]) * (gt / (1.0f + expf(-gt)));
+                const float x = e ? gt[u][i].y : gt[u][i].x;
+                v[e] = ((acc[i][2 * u + e] * inv) * norm_w[c + e]) * (x / (1.0f + expf(-x)));
             }
             if (sizeof(T) == 2) *reinterpret_cast<__nv_bfloat162*>(orow + c) = __floats2bfloat162_rn(v[0], v[1]);
             else { orow[c] = from_f32<T>(v[0]); orow[c + 1] = from_f32<T>(v[1]); }

@@ -62,8 +62,6 @@ constexpr int MG_THREADS = 512, MG_BATCH = 128;     // chunks whose maxima meet 
 __global__ void __launch_bounds__(MG_THREADS) mlstm_chunk_gates_kernel(const CmArgs p, const float* __restrict__ gate_bias, float cap) {
     __shared__ double sF[MG_BATCH], sG[MG_BATCH], sM[MG_BATCH];
     __shared__ int base_sh;
-    dependency_wait();
-    let_dependents_start();
     const int h = blockIdx.x, seg = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = p.H;
     const int first = p.seg_starts[seg], end = p.seg_starts[seg + 1], slot = p.seg_slots[seg];
     if (first >= end) return;
@@ -149,8 +147,6 @@ __global__ void __launch_bounds__(GD_THREADS) gla_chunk_decays_kernel(const CmAr
                                                                       const float* __restrict__ bias, float inv_tau) {
     extern __shared__ float gd_sh[];                    // [rank][16]
     __shared__ int find[4];
-    dependency_wait();
-    let_dependents_start();
     const Chunk ch = find_chunk<CM_Q>(blockIdx.x / 4, p.seg_starts, p.segments, find);
     const int r0 = (blockIdx.x & 3) * CM_LOCAL, cnt = ch.seg < 0 ? 0 : min(CM_LOCAL, ch.rows - r0);
     if (cnt <= 0) return;
@@ -186,8 +182,6 @@ __global__ void __launch_bounds__(128) cm_add_kernel(const CmArgs p, int col_til
     float* sk = ca_smem;                            // [64][CM_LD] k
     float* sv = sk + CM_Q * CM_LD;                  // [64][CM_LD] v
     float* sl = sv + CM_Q * CM_LD;                  // [64][CM_LD] the decays' logarithms (gated linear attention)
-    dependency_wait();
-    let_dependents_start();
     const Chunk ch = find_chunk<CM_Q>(blockIdx.x, p.seg_starts, p.segments, find);
     if (ch.seg < 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, wd = (warp & 1) * 32, wv = (warp >> 1) * 32;
@@ -286,8 +280,6 @@ __global__ void __launch_bounds__(128) cm_add_kernel(const CmArgs p, int col_til
 template <bool MLSTM>
 __global__ void __launch_bounds__(256) cm_scan_kernel(const CmArgs p) {
     __shared__ int base_sh;
-    dependency_wait();
-    let_dependents_start();
     const int seg = blockIdx.z, h = blockIdx.y, H = p.H, dk = p.dk, dv = p.dv;
     const int first = p.seg_starts[seg], end = p.seg_starts[seg + 1], slot = p.seg_slots[seg];
     if (first >= end) return;
@@ -365,8 +357,6 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
     float* sq = co_smem;
     float* ring = co_smem + CM_Q * LDQ;
     float* sk = ring + L::SLOT;                         // k waits in the second slot
-    dependency_wait();
-    let_dependents_start();
     const Chunk ch = find_chunk<CM_Q>(blockIdx.x, p.seg_starts, p.segments, find);
     if (ch.seg < 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, wm = warp & 1, wn = warp >> 1;
@@ -671,7 +661,7 @@ static int cm_launch_out(const CmArgs& p, int tokens, int gate_off, const float*
     const int smem = CmOut<DK, DV>::FLOATS * (int)sizeof(float);
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
-    return launch_dependent(kern, dim3(cm_chunks(tokens, p.segments), p.H), dim3(256), smem, stream, p, gate_off, norm_w, eps, (T*)out);
+    return launch_plain(kern, dim3(cm_chunks(tokens, p.segments), p.H), dim3(256), smem, stream, p, gate_off, norm_w, eps, (T*)out);
 }
 
 template <bool MLSTM>
@@ -681,9 +671,9 @@ static int cm_launch(const CmArgs& p, int tokens, int gate_off, const float* nor
     const cudaError_t e = cudaFuncSetAttribute(add, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     const int col_tiles = (p.dv + CM_T - 1) / CM_T, row_tiles = (p.dk + CM_T - 1) / CM_T;
-    int s = launch_dependent(add, dim3(cm_chunks(tokens, p.segments), p.H, row_tiles * col_tiles), dim3(128), smem, stream, p, col_tiles);
+    int s = launch_plain(add, dim3(cm_chunks(tokens, p.segments), p.H, row_tiles * col_tiles), dim3(128), smem, stream, p, col_tiles);
     if (s != VK_OK) return s;
-    s = launch_dependent(cm_scan_kernel<MLSTM>, dim3((p.dk * p.dv + 1023) / 1024 + (MLSTM ? 1 : 0), p.H, p.segments), dim3(256), 0, stream, p);
+    s = launch_plain(cm_scan_kernel<MLSTM>, dim3((p.dk * p.dv + 1023) / 1024 + (MLSTM ? 1 : 0), p.H, p.segments), dim3(256), 0, stream, p);
     if (s != VK_OK) return s;
 #define GO(DK, DV)                                                                                                                       \
     return dtype == 0 ? cm_launch_out<MLSTM, DK, DV, float>(p, tokens, gate_off, norm_w, eps, out, stream)                               \
@@ -732,7 +722,7 @@ VK_API int vk_mlstm_chunked(const float* proj, int N, int H, int dk, int dv, con
     p.G = (double*)at; at += tok;
     p.F = (double*)at; at += tok;
     p.weight = (float*)at;
-    s = launch_dependent(mlstm_chunk_gates_kernel, dim3(H, segments), dim3(MG_THREADS), 0, stream, p, gate_bias, cap);
+    s = launch_plain(mlstm_chunk_gates_kernel, dim3(H, segments), dim3(MG_THREADS), 0, stream, p, gate_bias, cap);
     if (s != VK_OK) return s;
     return cm_launch<true>(p, tokens, gate_off, norm_w, eps, out, dtype, stream);
 }
@@ -752,7 +742,7 @@ VK_API int vk_gla_chunked(const float* proj, int N, int H, int dk, int dv, int a
     p.state_floats = (size_t)H * dk * dv;
     p.decay = (float*)((char*)scratch + cm_up((size_t)chunks * H * dk * dv * 4));
     p.logs = (float*)((char*)p.decay + cm_up((size_t)chunks * H * dk * 4));
-    s = launch_dependent(gla_chunk_decays_kernel, dim3(4 * chunks, (H * dk + GD_THREADS - 1) / GD_THREADS), dim3(GD_THREADS), smem, stream, p, a_off, rank, a2t, bias,
+    s = launch_plain(gla_chunk_decays_kernel, dim3(4 * chunks, (H * dk + GD_THREADS - 1) / GD_THREADS), dim3(GD_THREADS), smem, stream, p, a_off, rank, a2t, bias,
                          1.0f / tau);
     if (s != VK_OK) return s;
     return cm_launch<false>(p, tokens, gate_off, norm_w, eps, out, dtype, stream);
