@@ -66,6 +66,56 @@ __device__ __forceinline__ uint32_t at_pack(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
+// Two float32 values an instruction: the softmax warps are bound by what they issue (63 % of the issue slots at 32 heads and 2,048 tokens; measured there and at
+// 8,192 tokens with one value an instruction: 63 and 660 us).
+__device__ __forceinline__ uint64_t at_two(float a, float b) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ void at_split2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t at_fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+__device__ __forceinline__ uint64_t at_add2(uint64_t a, uint64_t b) {
+    uint64_t v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ float at_max3(float a, float b, float c) {
+    float v;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(a), "f"(b), "f"(c));
+    return v;
+}
+// The largest of N scores (N a multiple of 8).
+template <int N>
+__device__ __forceinline__ float at_largest(const uint32_t* s) {
+    float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int j = 0; j < N; j += 8)
+#pragma unroll
+        for (int u = 0; u < 4; u++) m[u] = at_max3(m[u], __uint_as_float(s[j + 2 * u]), __uint_as_float(s[j + 2 * u + 1]));
+    return fmaxf(at_max3(m[0], m[1], m[2]), m[3]);
+}
+// Eight scores -> probabilities 2^(s scale + shift) as high and low bfloat16 parts, and their sum in two halves.
+__device__ __forceinline__ void at_probabilities8(const uint32_t* s, uint64_t scale2, uint64_t shift2, uint32_t* hi, uint32_t* lo, uint64_t& sum2) {
+    const uint64_t minus = at_two(-1.0f, -1.0f);
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+        float x0, x1;
+        at_split2(at_fma2(at_two(__uint_as_float(s[j]), __uint_as_float(s[j + 1])), scale2, shift2), x0, x1);
+        const uint64_t p = at_two(at_ex2(x0), at_ex2(x1));
+        sum2 = at_add2(sum2, p);
+        float p0, p1, r0, r1;
+        at_split2(p, p0, p1);
+        const uint32_t h = at_pack(p0, p1);
+        at_split2(at_fma2(at_two(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus, p), r0, r1);
+        hi[j / 2] = h;
+        lo[j / 2] = at_pack(r0, r1);
+    }
+}
 
 // DBUF: two buffers of probabilities (132 KB of shared memory, one block a multiprocessor) instead of one (96 KB, two
 // blocks): the softmax warps then write a step's probabilities while the tensor core still reads the step's before.
@@ -260,9 +310,7 @@ __global__ void __launch_bounds__(AT_THREADS, DBUF ? 1 : 2) attention_prefill_tc
                         if (!(valid && kk <= my_pos && kk >= my_lo)) sr[j] = 0xff800000u;
                     }
                 }
-#pragma unroll
-                for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(sr[j]));
-                mx *= scale_log2;
+                mx = at_largest<32>(sr) * scale_log2;
             }
             xmax[((i & 1) * 2 + half) * AT_BM + r] = mx;
             asm volatile("bar.sync %0, 64;" ::"r"(bar_id) : "memory");
@@ -297,24 +345,19 @@ __global__ void __launch_bounds__(AT_THREADS, DBUF ? 1 : 2) attention_prefill_tc
                 if (!__all_sync(0xffffffffu, mbar_wait(&pv_done[pbuf(had)], ppar(had), wc.cycles))) { if (lane == 0) give_up(wc.error, &failed, 17); ok = false; }
             }
             if (ok) {
-                float sum = 0.0f;
+                const uint64_t scale2 = at_two(scale_log2, scale_log2), shift2 = at_two(-m_use, -m_use);
+                uint64_t sum2 = at_two(0.0f, 0.0f);
 #pragma unroll
                 for (int j8 = 0; j8 < 32; j8 += 8) {
                     uint32_t hi[4], lo[4];
-#pragma unroll
-                    for (int j = 0; j < 8; j += 2) {
-                        const float p0 = at_ex2(fmaf(__uint_as_float(sr[j8 + j]), scale_log2, -m_use));
-                        const float p1 = at_ex2(fmaf(__uint_as_float(sr[j8 + j + 1]), scale_log2, -m_use));
-                        sum += p0 + p1;
-                        const __nv_bfloat162 hv = __floats2bfloat162_rn(p0, p1);
-                        hi[j / 2] = *reinterpret_cast<const uint32_t*>(&hv);
-                        lo[j / 2] = at_pack(p0 - __bfloat162float(hv.x), p1 - __bfloat162float(hv.y));
-                    }
+                    at_probabilities8(sr + j8, scale2, shift2, hi, lo, sum2);
                     const int chunk = (half * 4 + (j8 >> 3)) ^ (r & 7);      // 128-byte swizzle: 16-byte piece index xor row mod 8
                     *reinterpret_cast<uint4*>(ph_row + pbuf(i) * P_BYTES + chunk * 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
                     *reinterpret_cast<uint4*>(pl_row + pbuf(i) * P_BYTES + chunk * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
                 }
-                l += sum;
+                float sum0, sum1;
+                at_split2(sum2, sum0, sum1);
+                l += sum0 + sum1;
                 // the values' rows beyond the last position (pages not loaded, slots not yet written): never counted,
                 // but 0 * garbage must not be NaN
                 if (kt0 + i == kt1 && (last_pos & (AT_BN - 1)) != AT_BN - 1 &&
@@ -651,15 +694,7 @@ __global__ void __launch_bounds__(AS_THREADS, 1) attention_prefill_streams_kerne
                         if (!(valid && kk <= my_pos && kk >= my_lo)) sr[j] = 0xff800000u;
                     }
                 }
-                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                for (int j = 0; j < 64; j += 4) {
-                    mx4[0] = fmaxf(mx4[0], __uint_as_float(sr[j]));
-                    mx4[1] = fmaxf(mx4[1], __uint_as_float(sr[j + 1]));
-                    mx4[2] = fmaxf(mx4[2], __uint_as_float(sr[j + 2]));
-                    mx4[3] = fmaxf(mx4[3], __uint_as_float(sr[j + 3]));
-                }
-                mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
+                mx = at_largest<64>(sr) * scale_log2;
             }
             // the group's last step has read this buffer of probabilities and added into O: both may change now
             if (ok && steps > 0) {
@@ -688,24 +723,18 @@ __global__ void __launch_bounds__(AS_THREADS, 1) attention_prefill_streams_kerne
             }
             const float m_use = m == -INFINITY ? 0.0f : m;
             if (ok) {
-                float sum0 = 0.0f, sum1 = 0.0f;
+                const uint64_t scale2 = at_two(scale_log2, scale_log2), shift2 = at_two(-m_use, -m_use);
+                uint64_t sum2 = at_two(0.0f, 0.0f);
 #pragma unroll
                 for (int j8 = 0; j8 < 64; j8 += 8) {
                     uint32_t hi[4], lo[4];
-#pragma unroll
-                    for (int j = 0; j < 8; j += 2) {
-                        const float p0 = at_ex2(fmaf(__uint_as_float(sr[j8 + j]), scale_log2, -m_use));
-                        const float p1 = at_ex2(fmaf(__uint_as_float(sr[j8 + j + 1]), scale_log2, -m_use));
-                        sum0 += p0;
-                        sum1 += p1;
-                        const __nv_bfloat162 hv = __floats2bfloat162_rn(p0, p1);
-                        hi[j / 2] = *reinterpret_cast<const uint32_t*>(&hv);
-                        lo[j / 2] = at_pack(p0 - __bfloat162float(hv.x), p1 - __bfloat162float(hv.y));
-                    }
+                    at_probabilities8(sr + j8, scale2, shift2, hi, lo, sum2);
                     const int chunk = (j8 >> 3) ^ (r & 7);      // 128-byte swizzle: 16-byte piece index xor row mod 8
                     *reinterpret_cast<uint4*>(ph_row + chunk * 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
                     *reinterpret_cast<uint4*>(pl_row + chunk * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
                 }
+                float sum0, sum1;
+                at_split2(sum2, sum0, sum1);
                 l += sum0 + sum1;
                 // the values' rows beyond the last position: never counted, but 0 * garbage must not be NaN
                 if (kt0 + i == kt1 && (last_pos & (AT_BN - 1)) != AT_BN - 1 &&
