@@ -66,6 +66,15 @@ __device__ __forceinline__ uint32_t at_pack(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
+// A box of one page's rows: column x, row y of the page's keys (or values), page z.
+__device__ __forceinline__ void at_load_page(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+// The low word of a descriptor of an N-major operand whose columns lie in panels of 64: the panels' distance is its leading byte offset.
+__device__ __forceinline__ uint32_t umma_desc_lo_panels(uint32_t smem_addr, uint32_t panel_bytes) { return ((smem_addr & 0x3FFFF) >> 4) | ((panel_bytes >> 4) << 16); }
 // Two float32 values an instruction: the softmax warps are bound by what they issue (63 % of the issue slots at 32 heads and 2,048 tokens; measured there and at
 // 8,192 tokens with one value an instruction: 63 and 660 us).
 __device__ __forceinline__ uint64_t at_two(float a, float b) {
@@ -121,20 +130,28 @@ __device__ __forceinline__ void at_probabilities8(const uint32_t* s, uint64_t sc
 // blocks): the softmax warps then write a step's probabilities while the tensor core still reads the step's before.
 // Measured, that loses where two blocks can share a multiprocessor, and where they cannot the kernel with two streams
 // further down is faster still: only the form with one buffer is launched.
-template <int HD, bool DBUF>
+//
+// Keys of HD and values of VD values, 64 or 128 each: rows of 128 lie as two panels of 64 columns, a box each.  With either of them 128 the walks are not cut (a
+// 128 x 64 step is long enough that a short launch's blocks are busy), rows of out may lie apart, and a head may have a gate (see attention_rows.cu).
+__host__ __device__ constexpr uint32_t at_smem_bytes(int HD, int VD, int STAGES, bool DBUF) {
+    return AT_BM * HD * 2 + STAGES * AT_BN * (HD + VD) * 2 + (DBUF ? 4 : 2) * AT_BM * AT_BN * 2 + 1024 + 256;
+}
+
+template <int HD, int VD, int STAGES, bool DBUF>
 __global__ void __launch_bounds__(AT_THREADS, DBUF ? 1 : 2) attention_prefill_tcgen05_kernel(
-    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv, const int32_t* __restrict__ block_tables,
-    const int32_t* __restrict__ tiles, __nv_bfloat16* __restrict__ out, int nh, int nkv, int page_size, int max_blocks, float scale,
-    int window, const WaitCtl wc, const AtScratch sc) {
-    static_assert(HD == 64, "one 128-byte row per key");
-    constexpr int STAGES = AT_STAGES;
-    constexpr uint32_t Q_BYTES = AT_BM * HD * 2, KV_BYTES = AT_BN * HD * 2, P_BYTES = AT_BM * AT_BN * 2;
-    constexpr uint32_t K_OFF = Q_BYTES, V_OFF = K_OFF + STAGES * KV_BYTES, PH_OFF = V_OFF + STAGES * KV_BYTES, PL_OFF = PH_OFF + (DBUF ? 2 : 1) * P_BYTES,
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+    const int32_t* __restrict__ block_tables, const int32_t* __restrict__ tiles, __nv_bfloat16* __restrict__ out, int nh, int nkv, int page_size, int max_blocks,
+    float scale, int window, int out_ld, const float* __restrict__ gate, int gate_ld, const WaitCtl wc, const AtScratch sc) {
+    static_assert((HD == 64 || HD == 128) && (VD == 64 || VD == 128), "panels of 128-byte rows");
+    constexpr int KP = HD / 64, VP = VD / 64;        // panels of a row
+    constexpr bool PARTS = HD == 64 && VD == 64;     // walks may be cut
+    constexpr uint32_t Q_BYTES = AT_BM * HD * 2, Q_PANEL = AT_BM * 128, KV_PANEL = AT_BN * 128, K_BYTES = KP * KV_PANEL, V_BYTES = VP * KV_PANEL, P_BYTES = AT_BM * AT_BN * 2;
+    constexpr uint32_t K_OFF = Q_BYTES, V_OFF = K_OFF + STAGES * K_BYTES, PH_OFF = V_OFF + STAGES * V_BYTES, PL_OFF = PH_OFF + (DBUF ? 2 : 1) * P_BYTES,
                        BAR_OFF = PL_OFF + (DBUF ? 2 : 1) * P_BYTES;
     // the probabilities of step i lie in buffer pbuf(i); its completions on p_full and pv_done have parity ppar(i)
     auto pbuf = [](int i) -> int { return DBUF ? (i & 1) : 0; };
     auto ppar = [](int i) -> uint32_t { return DBUF ? ((i >> 1) & 1) : (i & 1); };
-    constexpr uint32_t TMEM_COLS = 256;              // S in columns 0..63 and 64..127 (two buffers), O in 128..191
+    constexpr uint32_t TMEM_COLS = 256;              // S in columns 0..63 and 64..127 (two buffers), O in 128..191 or 255
     constexpr float RAISE = 8.0f;                    // the reference maximum follows when the step's exceeds it by 2^8
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -193,7 +210,7 @@ __global__ void __launch_bounds__(AT_THREADS, DBUF ? 1 : 2) attention_prefill_tc
         // ---- producer ------------------------------------------------------------------------------------
         if (lane == 0) {
             mbar_expect_tx(q_full, Q_BYTES);
-            tma_load_2d(smem, &map_q, h * HD, tok0, q_full);      // rows beyond the batch read as zero
+            for (int p = 0; p < KP; p++) tma_load_2d(smem + p * Q_PANEL, &map_q, h * HD + 64 * p, tok0, q_full);      // rows beyond the batch read as zero
         }
         const int32_t* bt = block_tables + (size_t)seg * max_blocks;
         const int box_rows = page_size < AT_BN ? page_size : AT_BN, boxes = AT_BN / box_rows;
@@ -219,7 +236,7 @@ __global__ void __launch_bounds__(AT_THREADS, DBUF ? 1 : 2) attention_prefill_tc
             int nb = (last_pos - key0) / box_rows + 1;
             nb = nb < boxes ? nb : boxes;
             const int off = (key0 + lane * box_rows) % page_size;
-            const uint32_t dst = s * KV_BYTES + lane * box_rows * (HD * 2);
+            const uint32_t dst = lane * box_rows * 128;
             if (i >= STAGES) {
                 const bool ok = mbar_wait(&k_empty[s], ((i / STAGES) - 1) & 1, wc.cycles);
                 if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) give_up(wc.error, &failed, 11); break; }
@@ -227,31 +244,34 @@ __global__ void __launch_bounds__(AT_THREADS, DBUF ? 1 : 2) attention_prefill_tc
             if (i != wc.skip_stage) {          // (a step named by wc.skip_stage gets no keys: a test of the give-up path)
                 if (lane == 0) mbar_expect_tx(&k_full[s], (uint32_t)nb * box_rows * HD * 2);
                 __syncwarp();
-                if (lane < nb) tma_load_2d(smem + K_OFF + dst, &map_kv, 0, (page * 2 * nkv + kvh) * page_size + off, &k_full[s]);
+                if (lane < nb)
+                    for (int p = 0; p < KP; p++) at_load_page(smem + K_OFF + s * K_BYTES + p * KV_PANEL + dst, &map_k, 64 * p, kvh * page_size + off, page, &k_full[s]);
             }
             if (i >= STAGES) {
                 const bool ok = mbar_wait(&v_empty[s], ((i / STAGES) - 1) & 1, wc.cycles);
                 if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) give_up(wc.error, &failed, 19); break; }
             }
-            if (lane == 0) mbar_expect_tx(&v_full[s], (uint32_t)nb * box_rows * HD * 2);
+            if (lane == 0) mbar_expect_tx(&v_full[s], (uint32_t)nb * box_rows * VD * 2);
             __syncwarp();
-            if (lane < nb) tma_load_2d(smem + V_OFF + dst, &map_kv, 0, ((page * 2 + 1) * nkv + kvh) * page_size + off, &v_full[s]);
+            if (lane < nb)
+                for (int p = 0; p < VP; p++) at_load_page(smem + V_OFF + s * V_BYTES + p * KV_PANEL + dst, &map_v, 64 * p, kvh * page_size + off, page, &v_full[s]);
         }
     } else if (warp == 9) {
         // ---- tensor core ---------------------------------------------------------------------------------
         if (lane == 0) {
             const uint32_t idesc_qk = umma_idesc_bf16(AT_BM, AT_BN);
-            const uint32_t idesc_pv = umma_idesc_bf16(AT_BM, HD) | (1u << 16);        // B (the values) is N-major
+            const uint32_t idesc_pv = umma_idesc_bf16(AT_BM, VD) | (1u << 16);        // B (the values) is N-major
             // the low words of the operands' descriptors (see umma_bf16_lo): stepped by bytes / 16
-            const uint32_t q_lo = umma_desc_lo(smem_u32(smem)), k_lo0 = umma_desc_lo(smem_u32(smem + K_OFF)), v_lo0 = umma_desc_lo(smem_u32(smem + V_OFF));
+            const uint32_t q_lo = umma_desc_lo(smem_u32(smem)), k_lo0 = umma_desc_lo(smem_u32(smem + K_OFF)), v_lo0 = umma_desc_lo_panels(smem_u32(smem + V_OFF), KV_PANEL);
             const uint32_t ph_lo0 = umma_desc_lo(smem_u32(smem + PH_OFF)), pl_lo0 = umma_desc_lo(smem_u32(smem + PL_OFF));
             auto scores = [&](int i) -> bool {        // S[i & 1] = Q K_i^T
                 const int s = i % STAGES;
                 if (!mbar_wait(&k_full[s], (i / STAGES) & 1, wc.cycles)) { give_up(wc.error, &failed, 13); return false; }
                 tc_fence_after();
-                const uint32_t k_lo = k_lo0 + s * (KV_BYTES >> 4), s_addr = tmem_s + (i & 1) * AT_BN;
+                const uint32_t k_lo = k_lo0 + s * (K_BYTES >> 4), s_addr = tmem_s + (i & 1) * AT_BN;
 #pragma unroll
-                for (int k = 0; k < HD / 16; k++) umma_bf16_lo(s_addr, q_lo + 2 * k, k_lo + 2 * k, idesc_qk, k != 0);
+                for (int k = 0; k < HD / 16; k++)
+                    umma_bf16_lo(s_addr, q_lo + (k / 4) * (Q_PANEL >> 4) + 2 * (k % 4), k_lo + (k / 4) * (KV_PANEL >> 4) + 2 * (k % 4), idesc_qk, k != 0);
                 umma_commit(&s_full[i & 1]);
                 umma_commit(&k_empty[s]);               // the keys' stage is free once these instructions have read it
                 return true;
@@ -266,7 +286,7 @@ __global__ void __launch_bounds__(AT_THREADS, DBUF ? 1 : 2) attention_prefill_tc
                 if (!mbar_wait(&p_full[pbuf(i)], ppar(i), wc.cycles)) { give_up(wc.error, &failed, 14); break; }
                 const uint32_t pb = (uint32_t)pbuf(i) * (P_BYTES >> 4);
                 tc_fence_after();
-                const uint32_t v_lo = v_lo0 + (i % STAGES) * (KV_BYTES >> 4), ph_lo = ph_lo0 + pb, pl_lo = pl_lo0 + pb;
+                const uint32_t v_lo = v_lo0 + (i % STAGES) * (V_BYTES >> 4), ph_lo = ph_lo0 + pb, pl_lo = pl_lo0 + pb;
                 // 16 keys an instruction: two groups of eight 128-byte rows of the values
 #pragma unroll
                 for (int k = 0; k < AT_BN / 16; k++) umma_bf16_lo(tmem_o, ph_lo + 2 * k, v_lo + k * (2048 >> 4), idesc_pv, (i | k) != 0);
@@ -325,12 +345,15 @@ __global__ void __launch_bounds__(AT_THREADS, DBUF ? 1 : 2) attention_prefill_tc
                     if (ok) {
                         tc_fence_after();
                         const float alpha = raise ? at_ex2(m - mx) : 1.0f;
-                        uint32_t orr[32];
-                        tmem_ld32(tmem_o + lane_off + half * 32, orr);
-                        tmem_loaded(orr);
 #pragma unroll
-                        for (int j = 0; j < 32; j++) orr[j] = __float_as_uint(__uint_as_float(orr[j]) * alpha);
-                        tmem_st32(tmem_o + lane_off + half * 32, orr);
+                        for (int c = 0; c < VD / 2; c += 32) {
+                            uint32_t orr[32];
+                            tmem_ld32(tmem_o + lane_off + half * (VD / 2) + c, orr);
+                            tmem_loaded(orr);
+#pragma unroll
+                            for (int j = 0; j < 32; j++) orr[j] = __float_as_uint(__uint_as_float(orr[j]) * alpha);
+                            tmem_st32(tmem_o + lane_off + half * (VD / 2) + c, orr);
+                        }
                         tmem_wait_st();
                         l *= alpha;
                         if (raise) m = mx;
@@ -363,9 +386,10 @@ __global__ void __launch_bounds__(AT_THREADS, DBUF ? 1 : 2) attention_prefill_tc
                 if (kt0 + i == kt1 && (last_pos & (AT_BN - 1)) != AT_BN - 1 &&
                     __all_sync(0xffffffffu, mbar_wait(&v_full[i % STAGES], (i / STAGES) & 1, wc.cycles))) {      // the values have landed
                     const int z0 = (last_pos & (AT_BN - 1)) + 1;
-                    uint8_t* vs = smem + V_OFF + (i % STAGES) * KV_BYTES;
+                    uint8_t* vs = smem + V_OFF + (i % STAGES) * V_BYTES;
                     for (int idx = half * AT_BM + r; idx < (AT_BN - z0) * 8; idx += 2 * AT_BM)
-                        *reinterpret_cast<uint4*>(vs + (z0 + idx / 8) * 128 + (idx & 7) * 16) = make_uint4(0, 0, 0, 0);
+                        for (int p = 0; p < VP; p++)
+                            *reinterpret_cast<uint4*>(vs + p * KV_PANEL + (z0 + idx / 8) * 128 + (idx & 7) * 16) = make_uint4(0, 0, 0, 0);
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // P (and the zeros) are for the tensor core
                 tc_fence_before();
@@ -380,24 +404,35 @@ __global__ void __launch_bounds__(AT_THREADS, DBUF ? 1 : 2) attention_prefill_tc
         uint32_t orr[32];
         if (ok) {
             tc_fence_after();
-            tmem_ld32(tmem_o + lane_off + half * 32, orr);
+            tmem_ld32(tmem_o + lane_off + half * (VD / 2), orr);
             tmem_loaded(orr);
         }
-        if (n_parts == 1) {
-            if (ok && valid) {
-                const float inv = 1.0f / l;
-                __nv_bfloat16* dst = out + ((size_t)(tok0 + r) * nh + h) * HD + half * 32;
+        if (!PARTS || n_parts == 1) {
+            if (ok) {                               // (the whole warp: a load from tensor memory is the warp's)
+                float inv = valid ? 1.0f / l : 0.0f;
+                if (!PARTS && gate && valid) inv = gated(inv, gate, gate_ld, tok0 + r, h);
+                __nv_bfloat16* dst = out + (size_t)(tok0 + r) * out_ld + (size_t)h * VD + half * (VD / 2);
 #pragma unroll
-                for (int d = 0; d < 32; d += 8) {
-                    uint4 v;
-                    v.x = at_pack(__uint_as_float(orr[d]) * inv, __uint_as_float(orr[d + 1]) * inv);
-                    v.y = at_pack(__uint_as_float(orr[d + 2]) * inv, __uint_as_float(orr[d + 3]) * inv);
-                    v.z = at_pack(__uint_as_float(orr[d + 4]) * inv, __uint_as_float(orr[d + 5]) * inv);
-                    v.w = at_pack(__uint_as_float(orr[d + 6]) * inv, __uint_as_float(orr[d + 7]) * inv);
-                    *reinterpret_cast<uint4*>(dst + d) = v;
+                for (int c = 0; c < VD / 2; c += 32) {
+                    if (c) {
+                        __syncwarp();
+                        tmem_ld32(tmem_o + lane_off + half * (VD / 2) + c, orr);
+                        tmem_loaded(orr);
+                    }
+                    if (valid) {
+#pragma unroll
+                        for (int d = 0; d < 32; d += 8) {
+                            uint4 v;
+                            v.x = at_pack(__uint_as_float(orr[d]) * inv, __uint_as_float(orr[d + 1]) * inv);
+                            v.y = at_pack(__uint_as_float(orr[d + 2]) * inv, __uint_as_float(orr[d + 3]) * inv);
+                            v.z = at_pack(__uint_as_float(orr[d + 4]) * inv, __uint_as_float(orr[d + 5]) * inv);
+                            v.w = at_pack(__uint_as_float(orr[d + 6]) * inv, __uint_as_float(orr[d + 7]) * inv);
+                            *reinterpret_cast<uint4*>(dst + c + d) = v;
+                        }
+                    }
                 }
             }
-        } else {
+        } else if constexpr (PARTS) {
             // this part's unnormalised output, reference maximum and sum; a row without a counted key in this part
             // (its keys all lie in earlier parts) leaves maximum -inf and nothing else
             const size_t slot = ((size_t)tile * nh + h) * sc.parts + part;
@@ -893,6 +928,32 @@ static bool at_make_map(CUtensorMap* map, const void* base, long long rows, int 
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The rows of `dim` values (keys or values) of every page: [pages][rows of a page][dim], pages page_elems elements apart, read in boxes of box_rows x 64 columns.
+static bool at_make_page_map(CUtensorMap* map, const void* base, int dim, int page_rows, long long pages, long long page_elems, int box_rows) {
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) return false;
+    cuuint64_t dims[3] = {(cuuint64_t)dim, (cuuint64_t)page_rows, (cuuint64_t)pages};
+    cuuint64_t strides[2] = {(cuuint64_t)dim * 2, (cuuint64_t)page_elems * 2};
+    cuuint32_t box[3] = {64u, (cuuint32_t)box_rows, 1u};
+    cuuint32_t elem[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int HD, int VD, int STAGES, bool DBUF>
+static int launch_at(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const int32_t* block_tables, const int32_t* tiles, void* out, int nh, int nkv,
+                     int page_size, int max_blocks, float scale, int window, int out_ld, const float* gate, int gate_ld, int* error, const AtScratch& sc,
+                     cudaStream_t stream) {
+    auto kern = attention_prefill_tcgen05_kernel<HD, VD, STAGES, DBUF>;
+    constexpr uint32_t smem = at_smem_bytes(HD, VD, STAGES, DBUF);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    // (an ordinary launch: started under programmatic dependent launch, with the kernel after it fetching its weights
+    // meanwhile, a 2,048-token prompt at the 135M sizes took 2.90 instead of 2.72 ms)
+    return launch_plain(kern, dim3(sc.n_tiles * sc.parts * nh), dim3(AT_THREADS), smem, stream, mq, mk, mv, block_tables, tiles, (__nv_bfloat16*)out, nh, nkv, page_size,
+                        max_blocks, scale, window, out_ld, gate, gate_ld, wait_ctl(error, WAIT_FAMILY_ATTENTION_PREFILL), sc);
+}
+
 }  // namespace vk
 
 using namespace vk;
@@ -975,13 +1036,42 @@ VK_API int vk_attention_prefill_tcgen05(const void* q, const void* cache, const 
         return launch_plain(kern2, dim3((unsigned)blocks), dim3(AS_THREADS), smem2, stream, mq, mkv, block_tables, tiles, (__nv_bfloat16*)out,
                             nh, nkv, page_size, max_blocks, scale, window, wait_ctl(error, WAIT_FAMILY_ATTENTION_PREFILL), sc);
     }
-    const bool dbuf = false;                                // (two buffers of probabilities: measured no better than the other kernel)
-    const size_t smem = (size_t)AT_BM * 64 * 2 + 2 * AT_STAGES * AT_BN * 64 * 2 + (dbuf ? 4 : 2) * AT_BM * AT_BN * 2 + 1024 + 256;
-    auto kern = attention_prefill_tcgen05_kernel<64, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    // (an ordinary launch: started under programmatic dependent launch, with the kernel after it fetching its weights
-    // meanwhile, a 2,048-token prompt at the 135M sizes took 2.90 instead of 2.72 ms)
-    return launch_plain(kern, dim3(n_tiles * sc.parts * nh), dim3(AT_THREADS), smem, stream, mq, mkv, block_tables, tiles, (__nv_bfloat16*)out, nh,
-                        nkv, page_size, max_blocks, scale, window, wait_ctl(error, WAIT_FAMILY_ATTENTION_PREFILL), sc);
+    CUtensorMap mk, mv;
+    const int box_rows = page_size < AT_BN ? page_size : AT_BN;
+    const long long page_elems = 2ll * nkv * page_size * hd;
+    if (!at_make_page_map(&mk, cache, hd, nkv * page_size, pages, page_elems, box_rows) ||
+        !at_make_page_map(&mv, (const __nv_bfloat16*)cache + (size_t)nkv * page_size * hd, hd, nkv * page_size, pages, page_elems, box_rows))
+        return VK_BAD_SHAPE;
+    return launch_at<64, 64, AT_STAGES, false>(mq, mk, mv, block_tables, tiles, out, nh, nkv, page_size, max_blocks, scale, window, nh * hd, nullptr, 0, error, sc, stream);
+}
+
+// The same for keys of hd and values of vd values, one of them 128 and the other 64 or 128 (a page holds its keys [nkv][page_size][hd], then its values
+// [nkv][page_size][vd]); rows of out are out_ld elements apart; gate float32 [n_tokens][gate_ld] or null: head h of token t times sigmoid(gate[t][h]).  Walks are not
+// cut and there is no scratch.  Blocks: 152 to 192 KB of shared memory and two buffers of probabilities (one a multiprocessor), but 96 KB, two a multiprocessor, for
+// 64 x 128 with two stages.
+VK_API int vk_attention_prefill_tcgen05_dims(const void* q, const void* cache, const int32_t* block_tables, const int32_t* tiles, void* out, int n_tokens, int n_tiles,
+                                             int pages, int nh, int nkv, int hd, int vd, int page_size, int max_blocks, float scale, int window, int out_ld,
+                                             const float* gate, int gate_ld, int* error, cudaStream_t stream) {
+    if (n_tiles <= 0) return VK_OK;
+    if (nh <= 0 || nkv <= 0 || nh % nkv != 0 || page_size <= 0 || max_blocks <= 0 || window < 0 || n_tokens <= 0 || pages <= 0 || !error) return VK_BAD_SHAPE;
+    if (page_size % 8 != 0 || (AT_BN % page_size != 0 && page_size % AT_BN != 0) || out_ld < nh * vd || out_ld % 8 != 0) return VK_BAD_SHAPE;
+    if (nh > 65535 || (long long)n_tiles * nh > 0x7fffffffll || (long long)nkv * page_size >= (1ll << 31)) return VK_TOO_LARGE;
+    if (((uintptr_t)q % 16) || ((uintptr_t)cache % 16) || ((uintptr_t)out % 16)) return VK_BAD_ALIGNMENT;
+    CUtensorMap mq, mk, mv;
+    const int box_rows = page_size < AT_BN ? page_size : AT_BN;
+    const long long page_elems = (long long)nkv * page_size * (hd + vd);
+    if (!at_make_map(&mq, q, n_tokens, nh * hd, (long long)nh * hd, AT_BM) || !at_make_page_map(&mk, cache, hd, nkv * page_size, pages, page_elems, box_rows) ||
+        !at_make_page_map(&mv, (const __nv_bfloat16*)cache + (size_t)nkv * page_size * hd, vd, nkv * page_size, pages, page_elems, box_rows))
+        return VK_BAD_SHAPE;
+    AtScratch sc = {};
+    sc.parts = 1;
+    sc.part_steps = 1 << 24;
+    sc.n_tiles = n_tiles;
+#define GO(HD, VD, STAGES, DBUF) \
+    return launch_at<HD, VD, STAGES, DBUF>(mq, mk, mv, block_tables, tiles, out, nh, nkv, page_size, max_blocks, scale, window, out_ld, gate, gate_ld, error, sc, stream)
+    if (hd == 128 && vd == 128) GO(128, 128, 3, true);
+    if (hd == 64 && vd == 128) GO(64, 128, 2, false);
+    if (hd == 128 && vd == 64) GO(128, 64, 3, true);
+#undef GO
+    return VK_BAD_SHAPE;
 }

@@ -1010,6 +1010,32 @@ def attention_prefill_biased(q: torch.Tensor, cache_layer: torch.Tensor, block_t
     return out
 
 
+def attention_prefill_tcgen05_dims_takes(q: torch.Tensor, cache_layer: torch.Tensor, out: torch.Tensor, hd: int, vd: int, page_size: int) -> bool:
+    """Whether the tcgen05 prompt-attention kernel takes keys of hd and values of vd values: bfloat16, one of them 128 and the other 64 or 128, pages
+    of 8, 16, 32 or a multiple of 64 slots, rows of q dense, everything on 16 bytes."""
+    return (q.dtype == torch.bfloat16 and (hd, vd) in ((128, 128), (64, 128), (128, 64)) and page_size % 8 == 0 and (64 % page_size == 0 or page_size % 64 == 0)
+            and q.dim() == 2 and q.stride(1) == 1 and q.stride(0) == q.shape[1] and q.data_ptr() % 16 == 0 and cache_layer.data_ptr() % 16 == 0
+            and cache_layer.is_contiguous() and out.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0)
+
+
+def attention_prefill_tcgen05_dims(q: torch.Tensor, cache_layer: torch.Tensor, block_tables: torch.Tensor, tiles: torch.Tensor, out: torch.Tensor, nh: int, nkv: int,
+                                   hd: int, vd: int, page_size: int, scale: float, window: int = 0, gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Causal attention of prompt portions on the tcgen05 tensor cores for keys of hd and values of vd values, one of them 128 and the other 64 or 128.
+    tiles int32 [n, 4]: first token, rows (1..128), position of the first token, segment.  gate: as in attention_rows_biased."""
+    _req(q, "q", torch.bfloat16, 2); _req(cache_layer, "cache_layer", torch.bfloat16)
+    _req(block_tables, "block_tables", torch.int32, 2); _req(tiles, "tiles", torch.int32, 2)
+    out_ld = _out_rows(out, torch.bfloat16, q.shape[0], nh * vd, "attention_prefill_tcgen05_dims")
+    gate_ld = _gate_rows(gate, q.shape[0], nh, "attention_prefill_tcgen05_dims")
+    if q.shape[1] != nh * hd or _page_size_of(cache_layer, nkv, hd, vd) != page_size or tiles.shape[1] != 4:
+        raise KernelError("attention_prefill_tcgen05_dims: shapes do not fit the head counts")
+    if not attention_prefill_tcgen05_dims_takes(q, cache_layer, out, hd, vd, page_size):
+        raise KernelError("attention_prefill_tcgen05_dims: bfloat16, keys and values of 64 and 128 values (not both 64) and pages of 8, 16, 32 or a multiple of 64 slots only")
+    _check(lib().vk_attention_prefill_tcgen05_dims(_p(q), _p(cache_layer), _p(block_tables), _p(tiles), _p(out), q.shape[0], tiles.shape[0], cache_layer.shape[0],
+                                                   nh, nkv, hd, vd, page_size, block_tables.shape[1], ctypes.c_float(scale), window, out_ld, _p(gate), gate_ld,
+                                                   _p(error_word()), _stream()), "attention_prefill_tcgen05_dims")
+    return out
+
+
 def attention_biased(q: torch.Tensor, pages: torch.Tensor, meta, ctx, out: torch.Tensor, nh: int, nkv: int, hd: int, vd: int,
                      page_size: int, scale: float, window: int = 0, dist_bias: Optional[torch.Tensor] = None,
                      v_in_key: bool = False, v_share: int = 1, gate: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -1033,7 +1059,10 @@ def attention_biased(q: torch.Tensor, pages: torch.Tensor, meta, ctx, out: torch
         scratch = ws.flat(f"att.decb/{nh}/{nkv}/{hd}/{vd}/{layout}", nbytes, torch.uint8, zero=True)
         attention_decode_biased(q, pages, meta.block_tables, ctx.token_seg, ctx.positions, out, scratch, cap, nh, nkv, hd, vd, page_size,
                                 scale, layout, min(layout, max(1, ctx.max_context)), window, dist_bias, ctx.dec_tokens, v_in_key, v_share, gate)
-    if pre_ok:
+    if (pre_ok and dist_bias is None and not v_in_key and v_share == 1 and getattr(ctx, "pre_tiles_big", None) is not None
+            and attention_prefill_tcgen05_dims_takes(q, pages, out, hd, vd, page_size)):
+        attention_prefill_tcgen05_dims(q, pages, meta.block_tables, ctx.pre_tiles_big, out, nh, nkv, hd, vd, page_size, scale, window, gate)
+    elif pre_ok:
         attention_prefill_biased(q, pages, meta.block_tables, ctx.pre_tiles, out, nh, nkv, hd, vd, page_size, scale, window, dist_bias, v_in_key, v_share,
                                  gate)
     if not pre_ok and attention_rows_tile_takes(q, pages, hd, vd, ctx):
