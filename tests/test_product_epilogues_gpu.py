@@ -1,4 +1,5 @@
-"""The tcgen05 products' float32 epilogues where rows do not start on 16 bytes, tiles end inside a warp's 32 x 32 and a block has several tiles."""
+"""The tcgen05 products' epilogues where rows do not start on 16 bytes, tiles end inside a warp's 32 x 32 and a block has several tiles, and the products of row
+groups where row tiles without a group lie between the others."""
 import pytest
 import torch
 
@@ -25,4 +26,38 @@ def test_float32_results_and_sums(shape):
     bound = K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)
     assert bool(((out.double() - want).abs() <= bound).all())
     assert bool(((acc.double() - want - base.double()).abs() <= bound + 2.0 ** -23 * (base.double().abs() + want.abs())).all())
+    assert bool((room[M * N:] == 5.0).all())
+
+
+# wide tiles (1,024 columns and more) and narrow ones; columns that end inside a tile, on a piece of eight and off it; bfloat16 (plain and relu squared) and float32
+@pytest.mark.parametrize("mode,act", [(0, 0), (0, 4), (1, 0)])
+@pytest.mark.parametrize("N,K,tiles", [(1024, 72, 19), (1064, 520, 16), (1027, 136, 40), (2304, 1056, 37), (1096, 72, 2), (520, 264, 9)])
+def test_row_groups(N, K, tiles, mode, act):
+    from vitna_anchor_b200 import ops
+    E, M = 5, tiles * 128
+    g = torch.Generator(device="cuda").manual_seed(N * K + tiles)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(E, N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    group = torch.randint(-1, E, (tiles,), generator=g, device="cuda", dtype=torch.int32)
+    group[tiles // 2] = -1
+    group[0] = 3
+    group[-max(1, tiles // 8):] = -1
+    dtype = torch.float32 if mode else torch.bfloat16
+    room = torch.full((M * N + 1024,), 5.0, device="cuda", dtype=dtype)
+    ops._check(ops.lib().vk_linear_tcgen05_grouped(x.data_ptr(), w.data_ptr(), room.data_ptr(), M, N, K, K, E, group.data_ptr(), mode, 0, act,
+                                                   ops._p(ops.error_word()), ops._stream()), "linear_tcgen05_grouped")
+    ops.check_device_errors()
+    out = room[:M * N].view(tiles, 128, N)
+    for i, e in enumerate(group.tolist()):
+        if e < 0:
+            assert bool((out[i] == 5.0).all())                       # rows without a group are left alone
+            continue
+        a, b = x[i * 128:(i + 1) * 128].double(), w[e].double()
+        want, off = a @ b.T, K * 2.0 ** -23 * (a.abs() @ b.abs().T)       # (as above)
+        if act:
+            off = 2 * want.abs() * off + off * off + 2.0 ** -23 * want * want
+            want = want.clamp(min=0.0) ** 2
+        if mode == 0:
+            off = off + 2.0 ** -8 * (want.abs() + off)                 # rounded to bfloat16
+        assert bool(((out[i].double() - want).abs() <= off).all())
     assert bool((room[M * N:] == 5.0).all())

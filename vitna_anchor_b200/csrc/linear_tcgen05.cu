@@ -54,6 +54,7 @@ struct TcExtra {
     // blocks leave at once).  The table is the output of a kernel before this one.  Null: one weight matrix for all rows.
     const int32_t* tile_group;
     int group_rows;
+    int band;                    // the wide kernel: row tiles of a band (see there)
     const __nv_bfloat16* tok_table;      // TC_TOKEN: [tok_vocab][tok_ld]
     const int32_t* tok_ids;
     int tok_ld, tok_off, tok_vocab;
@@ -83,6 +84,66 @@ __device__ __forceinline__ void store_rows_f32(float* box, const uint32_t* r, fl
         }
     }
     __syncwarp();
+}
+
+// The same for 32 columns that leave as bfloat16, packed in pairs: `dst` is where this lane's row's 64 bytes go (null: nowhere), `cols` how many of the
+// columns there are (a multiple of eight).  Through 2 KB of shared memory of the warp's own, so that an instruction writes eight rows' 64 bytes and not
+// 16 bytes of 32 rows, which are half a sector each (a routed
+// prompt's first product, 8,192 rows x 3,072 of 2,048 with the wide kernel: 119 -> 97 us; gate and up of an 8,192-token prompt: 360 -> 351 us).
+__device__ __forceinline__ void store_rows_bf16(uint8_t* box, const uint32_t* p, __nv_bfloat16* dst, int cols, int lane) {
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        *reinterpret_cast<uint4*>(box + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = make_uint4(p[4 * j], p[4 * j + 1], p[4 * j + 2], p[4 * j + 3]);
+    __syncwarp();
+    const int piece = lane & 3;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int row = 8 * i + (lane >> 2);
+        const uint4 v = *reinterpret_cast<const uint4*>(box + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4));
+        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst), row));
+        if (o && 8 * piece < cols) *reinterpret_cast<uint4*>(o + 8 * piece) = v;
+    }
+    __syncwarp();
+}
+// An activation on a row's 32 sums.  The kind is looked at once and not for every value: with every kind's code in every one of the 32 steps, and the steps
+// in every group of columns, a tile's last pass ran through hundreds of kilobytes of instructions.
+__device__ __forceinline__ void activate_row(int kind, uint32_t* r) {
+    if (kind == 4) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(activate_dense(4, __uint_as_float(r[j])));
+    } else if (kind == 3) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(activate_dense(3, __uint_as_float(r[j])));
+    } else if (kind == 2) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(activate_dense(2, __uint_as_float(r[j])));
+    } else if (kind == 1) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(activate_dense(1, __uint_as_float(r[j])));
+    }
+}
+// Gate and up of 32 columns, both rounded to bfloat16 first: f(gate) * up, packed in pairs; f = silu (act 0) or activate_rt's number act.
+__device__ __forceinline__ void gate_row(int act, const uint32_t* gr, const uint32_t* ur, uint32_t* packed) {
+    auto go = [&](auto f) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+            float v[2];
+#pragma unroll
+            for (int e = 0; e < 2; e++)
+                v[e] = f(__bfloat162float(__float2bfloat16_rn(__uint_as_float(gr[j + e]))), __bfloat162float(__float2bfloat16_rn(__uint_as_float(ur[j + e]))));
+            __nv_bfloat162 p = __floats2bfloat162_rn(v[0], v[1]);
+            packed[j / 2] = *reinterpret_cast<uint32_t*>(&p);
+        }
+    };
+    if (act == 0) go([](float g, float up) { return tc_silu_mul(g, up); });
+    else go([act](float g, float up) { return activate_rt(act, g) * up; });
+}
+__device__ __forceinline__ void pack_rows_bf16(const uint32_t* r, uint32_t* p) {
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+        p[j] = *reinterpret_cast<uint32_t*>(&v);
+    }
 }
 
 template <int BN, int EPI>
@@ -221,30 +282,11 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tcgen05_kernel(const __grid
                 tmem_ld32(lane_base + c, gr);
                 tmem_ld32(lane_base + BN / 2 + c, ur);
                 const int col = n0 + c;
-                if (row < M && col < ex.inter) {
-                    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out) + (size_t)row * ex.inter + col;
-                    uint32_t packed[16];
-#pragma unroll
-                    for (int j = 0; j < 32; j += 2) {
-                        float a[2];
-#pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            const float gte = __bfloat162float(__float2bfloat16_rn(__uint_as_float(gr[j + e])));
-                            const float up = __bfloat162float(__float2bfloat16_rn(__uint_as_float(ur[j + e])));
-                            a[e] = ex.act ? activate_rt(ex.act, gte) * up : tc_silu_mul(gte, up);
-                        }
-                        __nv_bfloat162 v = __floats2bfloat162_rn(a[0], a[1]);
-                        packed[j / 2] = *reinterpret_cast<uint32_t*>(&v);
-                    }
-                    if (col + 32 <= ex.inter && (ex.inter % 8 == 0)) {
-#pragma unroll
-                        for (int j = 0; j < 4; j++)
-                            *reinterpret_cast<uint4*>(o + 8 * j) = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
-                    } else {
-                        for (int j = 0; j < 32 && col + j < ex.inter; j++)
-                            o[j] = __ushort_as_bfloat16((unsigned short)((packed[j / 2] >> ((j & 1) * 16)) & 0xffffu));
-                    }
-                }
+                uint32_t packed[16];
+                gate_row(ex.act, gr, ur, packed);
+                // (inter is a multiple of eight; the stages are free: every product has read them)
+                store_rows_bf16(smem + quarter * 2048, packed, row < M ? reinterpret_cast<__nv_bfloat16*>(out) + (size_t)row * ex.inter + col : nullptr,
+                                ex.inter - col, lane);
             }
         } else if (EPI == TC_ROPE) {
             tc_fence_after();
@@ -269,34 +311,29 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tcgen05_kernel(const __grid
                 __syncwarp();
                 tmem_ld32(lane_base + c, ar);
                 tmem_ld32(lane_base + HALF + c, br);
-                if (dst) {
-                    uint32_t pa[16], pb[16];
+                uint32_t pa[16], pb[16];
 #pragma unroll
-                    for (int j = 0; j < 32; j += 2) {
-                        float ra[2], rb[2];
+                for (int j = 0; j < 32; j += 2) {
+                    float ra[2], rb[2];
 #pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            const float a = __bfloat162float(__float2bfloat16_rn(__uint_as_float(ar[j + e])));
-                            const float b = __bfloat162float(__float2bfloat16_rn(__uint_as_float(br[j + e])));
-                            if (is_q || is_k) {
-                                const int ti = c + j + e;                  // index into this row of the tables
-                                const float4 c4 = rc[ti / 4], s4 = rs[ti / 4];
-                                const float cs = (ti & 3) == 0 ? c4.x : (ti & 3) == 1 ? c4.y : (ti & 3) == 2 ? c4.z : c4.w;
-                                const float sn = (ti & 3) == 0 ? s4.x : (ti & 3) == 1 ? s4.y : (ti & 3) == 2 ? s4.z : s4.w;
-                                ra[e] = a * cs - b * sn;
-                                rb[e] = b * cs + a * sn;
-                            } else { ra[e] = a; rb[e] = b; }
-                        }
-                        __nv_bfloat162 va = __floats2bfloat162_rn(ra[0], ra[1]), vb = __floats2bfloat162_rn(rb[0], rb[1]);
-                        pa[j / 2] = *reinterpret_cast<uint32_t*>(&va);
-                        pb[j / 2] = *reinterpret_cast<uint32_t*>(&vb);
+                    for (int e = 0; e < 2; e++) {
+                        const float a = __bfloat162float(__float2bfloat16_rn(__uint_as_float(ar[j + e])));
+                        const float b = __bfloat162float(__float2bfloat16_rn(__uint_as_float(br[j + e])));
+                        if (is_q || is_k) {
+                            const int ti = c + j + e;                  // index into this row of the tables
+                            const float4 c4 = rc[ti / 4], s4 = rs[ti / 4];
+                            const float cs = (ti & 3) == 0 ? c4.x : (ti & 3) == 1 ? c4.y : (ti & 3) == 2 ? c4.z : c4.w;
+                            const float sn = (ti & 3) == 0 ? s4.x : (ti & 3) == 1 ? s4.y : (ti & 3) == 2 ? s4.z : s4.w;
+                            ra[e] = a * cs - b * sn;
+                            rb[e] = b * cs + a * sn;
+                        } else { ra[e] = a; rb[e] = b; }
                     }
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        *reinterpret_cast<uint4*>(dst + c + 8 * j) = make_uint4(pa[4 * j], pa[4 * j + 1], pa[4 * j + 2], pa[4 * j + 3]);
-                        *reinterpret_cast<uint4*>(dst + HALF + c + 8 * j) = make_uint4(pb[4 * j], pb[4 * j + 1], pb[4 * j + 2], pb[4 * j + 3]);
-                    }
+                    __nv_bfloat162 va = __floats2bfloat162_rn(ra[0], ra[1]), vb = __floats2bfloat162_rn(rb[0], rb[1]);
+                    pa[j / 2] = *reinterpret_cast<uint32_t*>(&va);
+                    pb[j / 2] = *reinterpret_cast<uint32_t*>(&vb);
                 }
+                store_rows_bf16(smem + quarter * 2048, pa, dst ? dst + c : nullptr, 32, lane);       // (the stages are free: every product has read them)
+                store_rows_bf16(smem + quarter * 2048, pb, dst ? dst + HALF + c : nullptr, 32, lane);
             }
         } else if (EPI == TC_ACC && ex.tma_out) {
             // The residual sum by TMA: the tile goes into shared memory (the stages are free: every product has read them)
@@ -330,14 +367,19 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tcgen05_kernel(const __grid
             }
         } else {
             tc_fence_after();
-#pragma unroll
+#pragma unroll (EPI == TC_ACC ? BN / 32 : 1)
             for (int c = 0; c < BN; c += 32) {
                 uint32_t r[32];
                 __syncwarp();
                 tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + c, r);
                 const int col = n0 + c;
                 const bool whole = col + 32 <= N;
-                if (EPI == TC_F32) {               // (the stages are free: every product has read them)
+                if (EPI == TC_SAME) activate_row(ex.act, r);
+                if (EPI == TC_SAME && N % 8 == 0) {
+                    uint32_t packed[16];
+                    pack_rows_bf16(r, packed);
+                    store_rows_bf16(smem + quarter * 2048, packed, row < M ? reinterpret_cast<__nv_bfloat16*>(out) + (size_t)row * N + col : nullptr, N - col, lane);
+                } else if (EPI == TC_F32) {               // (the stages are free: every product has read them)
                     store_rows_f32(reinterpret_cast<float*>(smem + quarter * 4096), r, reinterpret_cast<float*>(out), m0 + quarter * 32, col, M, N, lane);
                 } else if (row >= M || col >= N) {
                     // nothing of this thread's to store
@@ -367,25 +409,9 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tcgen05_kernel(const __grid
                     }
                 } else if (EPI == TC_SAME) {
                     __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out) + (size_t)row * N + col;
-                    if (ex.act) {
 #pragma unroll
-                        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(activate_dense(ex.act, __uint_as_float(r[j])));
-                    }
-                    if (whole && (N % 8 == 0)) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 8) {
-                            uint4 v;
-                            __nv_bfloat162 p0 = __floats2bfloat162_rn(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
-                            __nv_bfloat162 p1 = __floats2bfloat162_rn(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-                            __nv_bfloat162 p2 = __floats2bfloat162_rn(__uint_as_float(r[j + 4]), __uint_as_float(r[j + 5]));
-                            __nv_bfloat162 p3 = __floats2bfloat162_rn(__uint_as_float(r[j + 6]), __uint_as_float(r[j + 7]));
-                            v.x = *reinterpret_cast<uint32_t*>(&p0); v.y = *reinterpret_cast<uint32_t*>(&p1);
-                            v.z = *reinterpret_cast<uint32_t*>(&p2); v.w = *reinterpret_cast<uint32_t*>(&p3);
-                            *reinterpret_cast<uint4*>(o + j) = v;
-                        }
-                    } else {
-                        for (int j = 0; j < 32 && col + j < N; j++) o[j] = __float2bfloat16_rn(__uint_as_float(r[j]));
-                    }
+                    for (int j = 0; j < 32; j++)
+                        if (col + j < N) o[j] = __float2bfloat16_rn(__uint_as_float(r[j]));
                 } else {
                     float* o = reinterpret_cast<float*>(out) + (size_t)row * N + col;
                     if (whole && (N % 4 == 0)) {
@@ -407,7 +433,9 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tcgen05_kernel(const __grid
                             *reinterpret_cast<float4*>(o + 4 * j) = v;
                         }
                     } else {
-                        for (int j = 0; j < 32 && col + j < N; j++) {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) {
+                            if (col + j >= N) continue;
                             if (EPI == TC_ACC) o[j] += __uint_as_float(r[j]);
                             else o[j] = __uint_as_float(r[j]);
                         }
@@ -434,9 +462,12 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tcgen05_kernel(const __grid
 // SwiGLU: a tile is 128 gate rows and the 128 up rows of the same columns.  BNW, the tile's width in weight rows, is a
 // parameter of the kernel: 256, or 192 (96 gate and 96 up rows) where the launcher finds that a block's last round of
 // the wider tile would be mostly empty.
+// The tiles are walked in bands of row tiles (`band`), so that the tiles being worked on at one time need few different bytes of both matrices.  Down all rows
+// where x stays in the second-level cache; in bands of 24 row tiles where it does not (8,192 x 8,192 of x: 151 -> 142 us for this product and the output
+// projection, each); in bands of eight for row groups, whose neighbours in x share a weight matrix (8,192 rows, 16 groups, 2,048 x 3,072: 109 -> 96 us).
 constexpr int TW_BN = 256, TW_STAGES = 4, TW_THREADS = 320;      // warps 0 and 1 feed and issue; eight warps drain the accumulators
 
-__host__ __device__ constexpr uint32_t wide_boxes(int epi) { return epi == TC_ACC || epi == TC_F32 ? 8 * 4096 : 0; }
+__host__ __device__ constexpr uint32_t wide_boxes(int epi) { return epi == TC_ACC || epi == TC_F32 ? 8 * 4096 : 8 * 2048; }
 
 template <int EPI, int HD = 0, int BNW = TW_BN>
 __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x,
@@ -447,23 +478,23 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
     constexpr uint32_t TM_COLS = 2 * BNW <= 256 ? 256 : 512;      // the two accumulators; tensor memory comes in powers of two
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* boxes = smem + TW_STAGES * STAGE_BYTES;             // 4 KB an epilogue warp, where the epilogue goes through shared memory
+    uint8_t* boxes = smem + TW_STAGES * STAGE_BYTES;             // 4 KB (bfloat16 results: 2 KB) an epilogue warp
     uint64_t* full = reinterpret_cast<uint64_t*>(boxes + wide_boxes(EPI));
     uint64_t* empty = full + TW_STAGES;
     uint64_t* acc_full = empty + TW_STAGES;       // [2]
     uint64_t* acc_empty = acc_full + 2;           // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-    __shared__ int failed;
+    __shared__ int failed, used;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int num_kb = (K + TC_BK - 1) / TC_BK;
     const int tile_cols = EPI == TC_SWIGLU ? BNW / 2 : BNW;                // output columns of a tile
     const int out_cols = EPI == TC_SWIGLU ? ex.inter : N;
-    const int tiles_m = (M + TC_BM - 1) / TC_BM, tiles_n = (out_cols + tile_cols - 1) / tile_cols;
-    const int num_tiles = tiles_m * tiles_n;      // tile t: rows (t % tiles_m) * 128, columns (t / tiles_m) * tile_cols
+    const int tiles_n = (out_cols + tile_cols - 1) / tile_cols;
+    int tiles_m = (M + TC_BM - 1) / TC_BM;
 
     if (threadIdx.x == 0) {
-        failed = 0;
+        failed = used = 0;
         for (int s = 0; s < TW_STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -477,13 +508,29 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if (ex.tile_group) {                          // the row tiles end behind the last one that has a group
+        int last = 0;
+        for (int i = threadIdx.x; i < tiles_m; i += TW_THREADS)
+            if (ex.tile_group[i] >= 0) last = i + 1;
+        if (last) atomicMax(&used, last);
+        __syncthreads();
+        tiles_m = used;
+    }
+    const int num_tiles = tiles_m * tiles_n;      // tile t: rows tile_row(t) * 128, columns tile_col(t) * tile_cols
+    // Tile t in bands of `band` row tiles: down a band's rows, then along its columns, then the next band.
+    const int band = min(ex.band, tiles_m), per_band = band * tiles_n;
+    auto tile_row = [&](int t) { const int b0 = t / per_band * band, h = min(band, tiles_m - b0); return b0 + (t - t / per_band * per_band) % h; };
+    auto tile_col = [&](int t) { const int b0 = t / per_band * band, h = min(band, tiles_m - b0); return (t - t / per_band * per_band) / h; };
+    auto group_of = [&](int t) { return ex.tile_group ? ex.tile_group[tile_row(t)] : 0; };       // (negative: no tile)
 
     if (warp == 0) {
         if (lane == 0) {
             int kc = 0;                            // stages filled so far, over all of this block's tiles
             bool ok = true;
             for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-                const int m0 = (t % tiles_m) * TC_BM, n0 = (t / tiles_m) * tile_cols;
+                const int m0 = tile_row(t) * TC_BM, g = group_of(t);
+                if (g < 0) continue;
+                const int n0 = g * ex.group_rows + tile_col(t) * tile_cols;
                 for (int kb = 0; kb < num_kb; kb++, kc++) {
                     const int s = kc % TW_STAGES;
                     if (kc >= TW_STAGES && !mbar_wait(&empty[s], ((kc / TW_STAGES) - 1) & 1, wc.cycles)) { give_up(wc.error, &failed, 31); ok = false; break; }
@@ -506,6 +553,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
             int kc = 0, j = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, j++) {
+                if (group_of(t) < 0) { j--; continue; }
                 const int b = j & 1;
                 if (j >= 2 && !mbar_wait(&acc_empty[b], ((j >> 1) - 1) & 1, wc.cycles)) { give_up(wc.error, &failed, 32); break; }
                 tc_fence_after();
@@ -529,8 +577,9 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
         int j = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, j++) {
+            if (group_of(t) < 0) { j--; continue; }
             const int b = j & 1;
-            const int row = (t % tiles_m) * TC_BM + quarter * 32 + lane, n0 = (t / tiles_m) * tile_cols;
+            const int row = tile_row(t) * TC_BM + quarter * 32 + lane, n0 = tile_col(t) * tile_cols;
             if (ok && !__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (j >> 1) & 1, wc.cycles))) { if (lane == 0) give_up(wc.error, &failed, 34); ok = false; }
             // A residual sum goes out by TMA reductions from shared memory (see the narrow kernel), a box of 32 rows x 32 columns a warp: from the warp's
             // own box, or, for the block's last tile, whose epilogue hides behind no further tile, from the stages, which are free by now.
@@ -538,7 +587,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                 tc_fence_after();
                 const uint32_t acc = lane_base + b * BNW;
                 const bool last = t + (int)gridDim.x >= num_tiles;
-                const int row0 = (t % tiles_m) * TC_BM + quarter * 32;
+                const int row0 = tile_row(t) * TC_BM + quarter * 32;
 #pragma unroll 1
                 for (int c = half * (BNW / 2); c < (half + 1) * (BNW / 2); c += 32) {
                     uint32_t r[32];
@@ -566,10 +615,10 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                 tc_fence_after();
                 const uint32_t acc = lane_base + b * BNW;
                 if (EPI == TC_SWIGLU) {
-#pragma unroll 1
                     // the tile's gate columns in chunks of 32: the first of a lane quarter's two warps takes the first half of
                     // them (rounded up), the second the rest
                     constexpr int CHUNKS = BNW / 2 / 32, SPLIT = (CHUNKS + 1) / 2;
+#pragma unroll 1
                     for (int c = (half == 0 ? 0 : SPLIT) * 32; c < (half == 0 ? SPLIT : CHUNKS) * 32; c += 32) {
                         uint32_t gr[32], ur[32];
                         tmem_ld32_nowait(acc + c, gr);
@@ -578,30 +627,10 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                         tmem_loaded(gr);
                         tmem_loaded(ur);
                         const int col = n0 + c;
-                        if (row < M && col < ex.inter) {
-                            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out) + (size_t)row * ex.inter + col;
-                            uint32_t packed[16];
-#pragma unroll
-                            for (int q = 0; q < 32; q += 2) {
-                                float v[2];
-#pragma unroll
-                                for (int e = 0; e < 2; e++) {
-                                    const float gte = __bfloat162float(__float2bfloat16_rn(__uint_as_float(gr[q + e])));
-                                    const float up = __bfloat162float(__float2bfloat16_rn(__uint_as_float(ur[q + e])));
-                                    v[e] = ex.act ? activate_rt(ex.act, gte) * up : tc_silu_mul(gte, up);
-                                }
-                                __nv_bfloat162 pk = __floats2bfloat162_rn(v[0], v[1]);
-                                packed[q / 2] = *reinterpret_cast<uint32_t*>(&pk);
-                            }
-                            if (col + 32 <= ex.inter && (ex.inter % 8 == 0)) {
-#pragma unroll
-                                for (int q = 0; q < 4; q++)
-                                    *reinterpret_cast<uint4*>(o + 8 * q) = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-                            } else {
-                                for (int q = 0; q < 32 && col + q < ex.inter; q++)
-                                    o[q] = __ushort_as_bfloat16((unsigned short)((packed[q / 2] >> ((q & 1) * 16)) & 0xffffu));
-                            }
-                        }
+                        uint32_t packed[16];
+                        gate_row(ex.act, gr, ur, packed);
+                        store_rows_bf16(boxes + (warp - 2) * 2048, packed, row < M ? reinterpret_cast<__nv_bfloat16*>(out) + (size_t)row * ex.inter + col : nullptr,
+                                        ex.inter - col, lane);
                     }
                 } else if (EPI == TC_ROPE) {
                     // the tile is 256 / HD heads: q heads, then k heads, then v heads (see the narrow kernel)
@@ -630,7 +659,6 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                             tmem_wait_ld();
                             tmem_loaded(ar);
                             tmem_loaded(br);
-                            if (!dst) continue;
                             const float4* cp = reinterpret_cast<const float4*>(ex.cos_t + (size_t)p0 * HALF + c);
                             const float4* sp = reinterpret_cast<const float4*>(ex.sin_t + (size_t)p0 * HALF + c);
                             uint32_t pa[16], pb[16];
@@ -652,11 +680,27 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                                 pa[q / 2] = *reinterpret_cast<uint32_t*>(&va0); pa[q / 2 + 1] = *reinterpret_cast<uint32_t*>(&va1);
                                 pb[q / 2] = *reinterpret_cast<uint32_t*>(&vb0); pb[q / 2 + 1] = *reinterpret_cast<uint32_t*>(&vb1);
                             }
+                            store_rows_bf16(boxes + (warp - 2) * 2048, pa, dst ? dst + c : nullptr, 32, lane);
+                            store_rows_bf16(boxes + (warp - 2) * 2048, pb, dst ? dst + HALF + c : nullptr, 32, lane);
+                        }
+                    }
+                } else if (EPI == TC_SAME) {
+#pragma unroll 1
+                    for (int c = half * (BNW / 2); c < (half + 1) * (BNW / 2); c += 32) {
+                        uint32_t r[32];
+                        tmem_ld32(acc + c, r);
+                        tmem_loaded(r);
+                        const int col = n0 + c;
+                        __nv_bfloat16* o = row < M ? reinterpret_cast<__nv_bfloat16*>(out) + (size_t)row * N + col : nullptr;
+                        activate_row(ex.act, r);
+                        if (N % 8 == 0) {
+                            uint32_t packed[16];
+                            pack_rows_bf16(r, packed);
+                            store_rows_bf16(boxes + (warp - 2) * 2048, packed, o, N - col, lane);
+                        } else if (o) {
 #pragma unroll
-                            for (int q = 0; q < 4; q++) {
-                                *reinterpret_cast<uint4*>(dst + c + 8 * q) = make_uint4(pa[4 * q], pa[4 * q + 1], pa[4 * q + 2], pa[4 * q + 3]);
-                                *reinterpret_cast<uint4*>(dst + HALF + c + 8 * q) = make_uint4(pb[4 * q], pb[4 * q + 1], pb[4 * q + 2], pb[4 * q + 3]);
-                            }
+                            for (int q = 0; q < 32; q++)
+                                if (col + q < N) o[q] = __float2bfloat16_rn(__uint_as_float(r[q]));
                         }
                     }
                 } else {
@@ -669,52 +713,31 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                         if (EPI == TC_F32) {
                             if (col < N)
                                 store_rows_f32(reinterpret_cast<float*>(boxes + (warp - 2) * 4096), r, reinterpret_cast<float*>(out),
-                                               (t % tiles_m) * TC_BM + quarter * 32, col, M, N, lane);
+                                               tile_row(t) * TC_BM + quarter * 32, col, M, N, lane);
                             continue;
                         }
                         if (row >= M || col >= N) continue;
                         const bool whole = col + 32 <= N;
-                        if (EPI == TC_SAME) {
-                            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out) + (size_t)row * N + col;
-                            if (ex.act) {
+                        float* o = reinterpret_cast<float*>(out) + (size_t)row * N + col;
+                        if (whole && (N % 4 == 0)) {
+                            float4 prev[8];
+                            if (EPI == TC_ACC) {           // all eight reads are issued before any is used
 #pragma unroll
-                                for (int q = 0; q < 32; q++) r[q] = __float_as_uint(activate_dense(ex.act, __uint_as_float(r[q])));
+                                for (int q = 0; q < 8; q++) prev[q] = *reinterpret_cast<const float4*>(o + 4 * q);
                             }
-                            if (whole && (N % 8 == 0)) {
 #pragma unroll
-                                for (int q = 0; q < 32; q += 8) {
-                                    uint4 v;
-                                    __nv_bfloat162 p0 = __floats2bfloat162_rn(__uint_as_float(r[q]), __uint_as_float(r[q + 1]));
-                                    __nv_bfloat162 p1 = __floats2bfloat162_rn(__uint_as_float(r[q + 2]), __uint_as_float(r[q + 3]));
-                                    __nv_bfloat162 p2 = __floats2bfloat162_rn(__uint_as_float(r[q + 4]), __uint_as_float(r[q + 5]));
-                                    __nv_bfloat162 p3 = __floats2bfloat162_rn(__uint_as_float(r[q + 6]), __uint_as_float(r[q + 7]));
-                                    v.x = *reinterpret_cast<uint32_t*>(&p0); v.y = *reinterpret_cast<uint32_t*>(&p1);
-                                    v.z = *reinterpret_cast<uint32_t*>(&p2); v.w = *reinterpret_cast<uint32_t*>(&p3);
-                                    *reinterpret_cast<uint4*>(o + q) = v;
-                                }
-                            } else {
-                                for (int q = 0; q < 32 && col + q < N; q++) o[q] = __float2bfloat16_rn(__uint_as_float(r[q]));
+                            for (int q = 0; q < 8; q++) {
+                                float4 v = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]),
+                                                       __uint_as_float(r[4 * q + 3]));
+                                if (EPI == TC_ACC) { v.x += prev[q].x; v.y += prev[q].y; v.z += prev[q].z; v.w += prev[q].w; }
+                                *reinterpret_cast<float4*>(o + 4 * q) = v;
                             }
                         } else {
-                            float* o = reinterpret_cast<float*>(out) + (size_t)row * N + col;
-                            if (whole && (N % 4 == 0)) {
-                                float4 prev[8];
-                                if (EPI == TC_ACC) {           // all eight reads are issued before any is used
 #pragma unroll
-                                    for (int q = 0; q < 8; q++) prev[q] = *reinterpret_cast<const float4*>(o + 4 * q);
-                                }
-#pragma unroll
-                                for (int q = 0; q < 8; q++) {
-                                    float4 v = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]),
-                                                           __uint_as_float(r[4 * q + 3]));
-                                    if (EPI == TC_ACC) { v.x += prev[q].x; v.y += prev[q].y; v.z += prev[q].z; v.w += prev[q].w; }
-                                    *reinterpret_cast<float4*>(o + 4 * q) = v;
-                                }
-                            } else {
-                                for (int q = 0; q < 32 && col + q < N; q++) {
-                                    if (EPI == TC_ACC) o[q] += __uint_as_float(r[q]);
-                                    else o[q] = __uint_as_float(r[q]);
-                                }
+                            for (int q = 0; q < 32; q++) {
+                                if (col + q >= N) continue;
+                                if (EPI == TC_ACC) o[q] += __uint_as_float(r[q]);
+                                else o[q] = __uint_as_float(r[q]);
                             }
                         }
                     }
@@ -813,6 +836,7 @@ static int launch_wide(const CUtensorMap& mx, const CUtensorMap& mw, void* out, 
     CUtensorMap mo = mx;                               // (a valid map for the epilogues that do not use it)
     exx.tma_out = 0;
     if (EPI == TC_ACC && N % 4 == 0 && ((uintptr_t)out % 16 == 0) && make_out_map(&mo, out, M, N, 32)) exx.tma_out = 1;
+    exx.band = exx.tile_group ? 8 : (size_t)M * K * 2 > ((size_t)64 << 20) ? 24 : 1 << 20;
     auto kern = linear_tcgen05_wide_kernel<EPI, HD, BNW>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
@@ -961,6 +985,13 @@ VK_API int vk_linear_tcgen05_grouped(const void* x, const void* w, void* out, in
         return launch_tc<128, TC_SWIGLU>(mx, mw, out, M, 2 * N, K, error, stream, ex);
     }
     ex.group_rows = N;
+    // Tiles of 128 x 256 one after another where they are enough to fill the machine about half: 16 experts of which four, whole calls, cold: at width 2,048
+    // 341 -> 258 us (2,048 tokens) and 137 -> 125 (64), at 1,024 130 -> 104 (2,048) and 58 -> 57 (64 tokens: 18 row tiles at most, 4 and 5 across).
+    if (N >= 1024 && (long long)((M + TC_BM - 1) / TC_BM) * ((N + TW_BN - 1) / TW_BN) >= 64) {
+        if (!make_map(&mx, x, M, K, ldx, TC_BM) || !make_map(&mw, w, groups * N, K, K, TW_BN)) return VK_BAD_SHAPE;
+        if (mode == 0) return launch_wide<TC_SAME>(mx, mw, out, M, N, K, error, stream, ex);
+        return launch_wide<TC_F32>(mx, mw, out, M, N, K, error, stream, ex);
+    }
     const int bn = N >= 1024 ? 128 : 64;           // the weights differ from tile to tile: wider tiles pay sooner than with one matrix
     if (!make_map(&mx, x, M, K, ldx, TC_BM) || !make_map(&mw, w, groups * N, K, K, bn)) return VK_BAD_SHAPE;
     if (bn == 128) {
