@@ -44,7 +44,7 @@ def test_row_groups(N, K, tiles, mode, act):
     group[-max(1, tiles // 8):] = -1
     dtype = torch.float32 if mode else torch.bfloat16
     room = torch.full((M * N + 1024,), 5.0, device="cuda", dtype=dtype)
-    ops._check(ops.lib().vk_linear_tcgen05_grouped(x.data_ptr(), w.data_ptr(), room.data_ptr(), M, N, K, K, E, group.data_ptr(), mode, 0, act,
+    ops._check(ops.lib().vk_linear_tcgen05_grouped(ops._p(x), ops._p(w), ops._p(room), M, N, K, K, E, ops._p(group), mode, 0, act,
                                                    ops._p(ops.error_word()), ops._stream()), "linear_tcgen05_grouped")
     ops.check_device_errors()
     out = room[:M * N].view(tiles, 128, N)
