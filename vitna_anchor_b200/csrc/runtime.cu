@@ -67,7 +67,7 @@ VK_API int vk_set_wait_limit_ms(double ms) {
 }
 
 // For tests: the next launch of a kernel family (1 the tcgen05 product, 2 its wide variant, 3 the tcgen05 prompt
-// attention) leaves stage `stage` of every block unarmed and unfilled, so that the waits on it run out, the kernel
+// attention, 4 the persistent decode attention, 5 the delta rule's scan over chunks) leaves stage `stage` of every block unarmed and unfilled, so that the waits on it run out, the kernel
 // sets the error word and returns by itself.  No address is out of range and nothing traps.
 VK_API void vk_test_skip_stage(int family, int stage) {
     vk::g_skip_family = family;
