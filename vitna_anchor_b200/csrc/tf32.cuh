@@ -21,10 +21,16 @@ __device__ __forceinline__ float tf_exp2(float x) {
     return y;
 }
 // a float32 operand as two tf32 parts: its 11 leading bits rounded to the nearest, and the 11 leading bits (the tensor core does not read the others)
-// of what that leaves, rounded likewise
+// of what that leaves, rounded likewise.  cvt.rna and not a sum on the bits: a NaN stays one in the high part, whatever its bits (0x7fffffff, which the
+// arithmetic instructions make, carries over into the sign when something is added to it).
 struct Tf { uint32_t hi, lo; };
+__device__ __forceinline__ uint32_t tf_round(float x) {
+    uint32_t y;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(y) : "f"(x));
+    return y;
+}
 __device__ __forceinline__ Tf tf_split(float x) {
-    const uint32_t hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+    const uint32_t hi = tf_round(x);
     return Tf{hi, __float_as_uint(x - __uint_as_float(hi)) + 0x1000u};
 }
 __device__ __forceinline__ void tf_mma(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
