@@ -313,7 +313,8 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
                 const int i = j + step;
                 float s = 0.0f;
 #pragma unroll
-                for (int u = 0; u < 16; u++) s = fmaf(sT[(16 * i + r) * DC_LDA + 16 * i + u], sT[(16 * j + u) * DC_LDA + 16 * i + c], s);
+                for (int u = 0; u < 16; u++)
+                    if (u <= r) s = fmaf(sT[(16 * i + r) * DC_LDA + 16 * i + u], sT[(16 * j + u) * DC_LDA + 16 * i + c], s);
                 sT[(16 * i + r) * DC_LDA + 16 * j + c] = -s;
             }
             __syncthreads();
@@ -350,6 +351,22 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
             for (int m = ks / 2; m < 4; m++) tf_mma(acc[m], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[0].lo, b[1].lo);
 #pragma unroll
             for (int m = ks / 2; m < 4; m++) tf_mma(acc[m], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[0].hi, b[1].hi);
+        }
+        // a sum that is not finite again, term by term: zeros above T's diagonal meet what stands in the tokens behind (0 times a NaN), and the parts' products make a
+        // NaN of an infinity
+        float all = 0.0f;
+#pragma unroll
+        for (int m = 0; m < 4; m++) all += (acc[m][0] + acc[m][1]) + (acc[m][2] + acc[m][3]);
+        if (!tf_finite(all)) {
+#pragma unroll
+            for (int m = 0; m < 4; m++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int r = 16 * m + g + 8 * (e >> 1);
+                    acc[m][e] = 0.0f;
+#pragma unroll 1
+                    for (int k = 0; k <= r; k++) acc[m][e] = fmaf(sT[r * DC_LDA + k], fac[k] * src[k * ld + 2 * t4 + (e & 1) - g], acc[m][e]);
+                }
         }
         float* dst = is_w ? W_g : U_g;
         const int width = is_w ? LDQ : dv, c = c0 + 2 * t4;
@@ -630,6 +647,24 @@ __global__ void __launch_bounds__(256) delta_chunk_out_kernel(const DcArgs p, bo
             const int k = ks * 8 + 2 * t4;
             step(sP + (16 * m + g) * DC_LDA + k, DC_LDA, [&](int i) { const float* ub = sU + k * LDU + cw + 8 * i + g; return make_float2(ub[0], ub[LDU]); });
         }
+    }
+    // an output that is not finite again, term by term, without the tokens behind it (see delta_chunk_prepare)
+    float all = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NT; i++) all += (acc[i][0] + acc[i][1]) + (acc[i][2] + acc[i][3]);
+    if (!tf_finite(all)) {
+        auto again = [&](int r, int c) {
+            float s = 0.0f;
+#pragma unroll 1
+            for (int d = 0; d < dk; d++) s = fmaf(sQ[r * LDQ + d], sS[c * LDQ + d], s);
+#pragma unroll 1
+            for (int k = 0; k <= r; k++) s = fmaf(sP[r * DC_LDA + k], sU[k * LDU + c], s);
+            return s;
+        };
+#pragma unroll
+        for (int i = 0; i < NT; i++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[i][e] = again(16 * m + g + 8 * (e >> 1), cw + 8 * i + 2 * t4 + (e & 1));
     }
     if (!norm_w) {
 #pragma unroll

@@ -253,6 +253,25 @@ __global__ void __launch_bounds__(128) cm_add_kernel(const CmArgs p, int col_til
         }
         tf_mma3(d_, a, b);
     }
+    // a sum that is not finite again, term by term: the parts' products make a NaN of an infinity
+    float all = 0.0f;
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int n = 0; n < 4; n++) all += (acc[m][n][0] + acc[m][n][1]) + (acc[m][n][2] + acc[m][n][3]);
+    if (!tf_finite(all)) {
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int n = 0; n < 4; n++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int d = wd + 16 * m + g + 8 * (e >> 1), v = wv + n * 8 + 2 * t4 + (e & 1);
+                    acc[m][n][e] = 0.0f;
+#pragma unroll 1
+                    for (int r = 0; r < rows; r++) acc[m][n][e] = fmaf(sk[r * CM_LD + d], (MLSTM ? wt[r] : 1.0f) * sv[r * CM_LD + v], acc[m][n][e]);
+                }
+    }
     float* out = p.before + at * dk * dv;
 #pragma unroll
     for (int m = 0; m < 2; m++)
@@ -362,6 +381,13 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, wm = warp & 1, wn = warp >> 1;
     const int h = blockIdx.y, H = p.H, dk = p.dk, dv = p.dv, rows = ch.rows;
     const size_t at = (size_t)blockIdx.x * H + h;
+    const float qscale = 1.0f / sqrtf((float)dk);
+    const int col0 = wn * (DVP / 4);
+    float o[2][NT][4];
+    // The second time (where an output came out as no finite number): the outputs term by term, so that a token's NaN or infinity stays out of the tokens before it
+    // (a weight of zero times a NaN is one) and an infinity is not made a NaN by its parts.
+#pragma unroll 1
+    for (bool careful = false;; careful = true) {
     for (int e = tid; e < CM_Q * (DKP / 4); e += 256) {
         const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
         const bool on = r < rows && d < dk;
@@ -521,19 +547,16 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
     }
     __syncthreads();                                    // nobody reads k any more
     issue(1);
-    const float qscale = 1.0f / sqrtf((float)dk);
     if (MLSTM && tid < CM_Q) {
         const float nq = fmaf(row_f[tid], squares[0][tid], (sums[0][tid] + sums[1][tid]) + (sums[2][tid] + sums[3][tid])) * qscale;
         row_n[tid] = 1.0f / (fmaxf(fabsf(nq), row_n[tid]) + 1e-6f);
     }
-    float o[2][NT][4];
 #pragma unroll
     for (int m = 0; m < 2; m++)
 #pragma unroll
         for (int n = 0; n < NT; n++)
 #pragma unroll
             for (int e = 0; e < 4; e++) o[m][n][e] = 0.0f;
-    const int col0 = wn * (DVP / 4);
 #pragma unroll 1
     for (int s = 0; s < KS + 2; s++) {
         tf_wait<1>();
@@ -561,6 +584,23 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
         if (s < KS || 32 * (s - KS) <= 32 * wm + 31) {  // (rows 0..31 do not see tokens 32..63)
             const int lda = s < KS ? LDQ : LDP;
             const float* pa = sq + (32 * wm + g) * lda + (s < KS ? 32 * s : 32 * (s - KS));
+            if (careful) {
+#pragma unroll 1
+                for (int i = 0; i < 32; i++)
+#pragma unroll
+                    for (int m = 0; m < 2; m++)
+#pragma unroll
+                        for (int u = 0; u < 2; u++) {
+                            if (s >= KS && 32 * (s - KS) + i > 32 * wm + 16 * m + g + 8 * u) continue;
+                            float x = pa[(16 * m + 8 * u) * lda + i];
+                            if (!MLSTM && s < KS)
+                                for (int z = 0; z < 2 * wm + m; z++) x *= vec[z * DKP + 32 * s + i];
+#pragma unroll
+                            for (int n = 0; n < NT; n++)
+#pragma unroll
+                                for (int e = 0; e < 2; e++) o[m][n][2 * u + e] = fmaf(x, sb[i * LDB + n * 8 + 2 * t4 - g + e], o[m][n][2 * u + e]);
+                        }
+            } else
 #pragma unroll
             for (int ks = 0; ks < 4; ks++) {
                 Tf a[2][4];
@@ -594,6 +634,7 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
         issue(s + 2);
     }
     // the heads' norm and gate
+    bool odd = false;
 #pragma unroll
     for (int m = 0; m < 2; m++)
 #pragma unroll
@@ -611,8 +652,10 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
             ss += __shfl_xor_sync(0xffffffffu, ss, 1);
             ss += __shfl_xor_sync(0xffffffffu, ss, 2);
             if (t4 == 0) squares[wn][r] = ss;
+            odd = odd || (r < rows && !tf_finite(ss));
         }
-    __syncthreads();
+    if (!__syncthreads_or(odd && !careful)) break;
+    }
 #pragma unroll
     for (int m = 0; m < 2; m++)
 #pragma unroll
