@@ -345,12 +345,20 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
                 const float2 x = *reinterpret_cast<const float2*>(sT + (16 * m + g) * DC_LDA + k), y = *reinterpret_cast<const float2*>(sT + (16 * m + g + 8) * DC_LDA + k);
                 a[m][0] = tf_split(x.x); a[m][1] = tf_split(y.x); a[m][2] = tf_split(x.y); a[m][3] = tf_split(y.y);
             }
+            float t[4][4];
 #pragma unroll
-            for (int m = ks / 2; m < 4; m++) tf_mma(acc[m], a[m][0].lo, a[m][1].lo, a[m][2].lo, a[m][3].lo, b[0].hi, b[1].hi);
+            for (int m = ks / 2; m < 4; m++) {
+                t[m][0] = t[m][1] = t[m][2] = t[m][3] = 0.0f;
+                tf_mma(t[m], a[m][0].lo, a[m][1].lo, a[m][2].lo, a[m][3].lo, b[0].hi, b[1].hi);
+            }
 #pragma unroll
-            for (int m = ks / 2; m < 4; m++) tf_mma(acc[m], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[0].lo, b[1].lo);
+            for (int m = ks / 2; m < 4; m++) tf_mma(t[m], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[0].lo, b[1].lo);
 #pragma unroll
-            for (int m = ks / 2; m < 4; m++) tf_mma(acc[m], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[0].hi, b[1].hi);
+            for (int m = ks / 2; m < 4; m++) tf_mma(t[m], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[0].hi, b[1].hi);
+#pragma unroll
+            for (int m = ks / 2; m < 4; m++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) acc[m][e] += t[m][e];
         }
         // a sum that is not finite again, term by term: zeros above T's diagonal meet what stands in the tokens behind (0 times a NaN), and the parts' products make a
         // NaN of an infinity
@@ -462,12 +470,13 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
             const int cc = e / (DKP / 4), dd = 4 * (e % (DKP / 4));
             if (c0 + cc < dv && dd < dk) *reinterpret_cast<float4*>(in + s_off + (size_t)(c0 + cc) * dk + dd) = *reinterpret_cast<const float4*>(sS + cc * LDS + dd);
         }
-        // (a product of one sum waits some 70 cycles for the one before it: the steps take turns on four sets of sums)
-        float x[4][3][4];
+        // (a product of one sum waits some 70 cycles for the one before it: every step has sums of its own for the large products, added up in float32 (tf32.cuh says why),
+        // and the small ones of all steps take turns on two sets each)
+        float x[2][2][4], ws[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-        for (int j = 0; j < 4; j++)
+        for (int j = 0; j < 2; j++)
 #pragma unroll
-            for (int i = 0; i < 3; i++)
+            for (int i = 0; i < 2; i++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) x[j][i][e] = 0.0f;
         const float* wa = sW + ur * LDQ + 2 * t4;
@@ -477,17 +486,15 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
             const float2 a0 = *reinterpret_cast<const float2*>(wa + ks * 8), a1 = *reinterpret_cast<const float2*>(wa + 8 * LDQ + ks * 8);
             const float2 b0 = *reinterpret_cast<const float2*>(sb + ks * 8);
             const Tf a[4] = {tf_split(a0.x), tf_split(a1.x), tf_split(a0.y), tf_split(a1.y)}, b[2] = {tf_split(b0.x), tf_split(b0.y)};
-            tf_mma(x[ks & 3][0], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
-            tf_mma(x[ks & 3][1], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
-            tf_mma(x[ks & 3][2], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
-        }
-        float ws[4];
+            float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            tf_mma(t, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
+            tf_mma(x[ks & 1][0], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
+            tf_mma(x[ks & 1][1], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            ws[e] = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 3; i++) ws[e] += (x[0][i][e] + x[1][i][e]) + (x[2][i][e] + x[3][i][e]);
+            for (int e = 0; e < 4; e++) ws[e] += t[e];
         }
+#pragma unroll
+        for (int e = 0; e < 4; e++) ws[e] += (x[0][0][e] + x[1][0][e]) + (x[0][1][e] + x[1][1][e]);
         const float2 u[2] = {make_float2(up[0].x - ws[0], up[0].y - ws[1]), make_float2(up[1].x - ws[2], up[1].y - ws[3])};
         sU[uc * LDU + ur] = u[0].x;
         sU[(uc + 1) * LDU + ur] = u[0].y;
@@ -500,16 +507,16 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
         const float da = dec[0], db = dec[1];
         fetch(c + 1);
         __syncthreads();                            // U is there, and nobody reads the old state any more
-        constexpr int SETS = 4 / NT;
-        float y[NT][SETS][3][4];
+        constexpr int SETS = 2 / NT;
+        float y[NT][SETS][2][4], z[NT][4];
 #pragma unroll
         for (int i = 0; i < NT; i++)
 #pragma unroll
-            for (int q = 0; q < SETS; q++)
+            for (int e = 0; e < 4; e++) {
+                z[i][e] = 0.0f;
 #pragma unroll
-                for (int j = 0; j < 3; j++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) y[i][q][j][e] = 0.0f;
+                for (int q = 0; q < SETS; q++) y[i][q][0][e] = y[i][q][1][e] = 0.0f;
+            }
 #pragma unroll
         for (int ks = 0; ks < DC_C / 8; ks++) {
             const float* ka = sK + (ks * 8 + t4) * LDQ + d;
@@ -518,21 +525,21 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
             for (int i = 0; i < NT; i++) {
                 const float* ub = sU + (8 * i + g) * LDU + ks * 8 + t4;
                 const Tf b[2] = {tf_split(ub[0]), tf_split(ub[4])};
-                float (*z)[4] = y[i][ks % SETS];
-                tf_mma(z[0], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
-                tf_mma(z[1], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
-                tf_mma(z[2], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
+                float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                tf_mma(t, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
+                tf_mma(y[i][ks % SETS][0], a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
+                tf_mma(y[i][ks % SETS][1], a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
+#pragma unroll
+                for (int e = 0; e < 4; e++) z[i][e] += t[e];
             }
         }
 #pragma unroll
         for (int i = 0; i < NT; i++)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                float add = 0.0f;
+                float add = z[i][e];
 #pragma unroll
-                for (int j = 0; j < 3; j++)
-#pragma unroll
-                    for (int q = 0; q < SETS; q++) add += y[i][q][j][e];
+                for (int q = 0; q < SETS; q++) add += y[i][q][0][e] + y[i][q][1][e];
                 s[i][e] = fmaf(e < 2 ? da : db, s[i][e], add);
                 sS[(8 * i + 2 * t4 + (e & 1)) * LDS + d + 8 * (e >> 1)] = s[i][e];
             }
