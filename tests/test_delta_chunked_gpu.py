@@ -98,3 +98,27 @@ def test_neighbouring_tokens_are_prepared_as_single_ones():
                 part = run(lo, hi, st, i32([0, hi - lo]), i32([0] * (hi - lo)), i32([s]))
                 assert torch.equal(part[:, :C + 2 * H], whole[lo:hi, :C + 2 * H]), (taps, s, lo)
             at += n
+
+
+@pytest.mark.parametrize("G,dk", [(191, 4), (12, 64), (193, 4)])         # 1,528, 1,536 and 1,544 values of q and k: 47.75, 48 and 48.25 KB for eight tokens
+def test_neighbouring_tokens_at_the_limit_of_shared_memory(G, dk):
+    """Around the largest key heads that eight tokens a block have room for: a long step gives the bits of short ones, whichever kernel prepares it."""
+    from vitna_anchor_b200 import ops
+    H, dv, taps, T = G, 4, 4, 1184
+    g = torch.Generator(device="cuda").manual_seed(G)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    C, N = 2 * G * dk + H * dv, 2 * G * dk + 2 * H * dv + 2 * H
+    proj, conv, a_log, bias = r(T, N), r(C, taps), r(H), r(H)
+    state = r(1, ops.delta_state_floats(G, H, dk, dv, taps))
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+
+    def run(lo, hi, st):
+        n = hi - lo
+        prep = torch.zeros(n, ops.delta_prep_width(G, H, dk, dv), device="cuda")
+        ops.delta_rule(proj[lo:hi].contiguous(), conv, a_log, bias, torch.ones(dv, device="cuda"), 1e-5, i32([0] * n), i32([0, n]), i32([0]), st, prep,
+                       torch.empty(n, H * dv, device="cuda"), torch.empty(n, H * dv, device="cuda"), G, H, dk, dv, taps)
+        return prep[:, :C + 2 * H]
+
+    whole, st = run(0, T, state.clone()), state.clone()
+    for lo in range(0, T, 100):
+        assert torch.equal(run(lo, min(T, lo + 100), st), whole[lo:lo + 100]), lo

@@ -538,9 +538,9 @@ VK_API int vk_delta_prepare(const float* proj, const float* conv_w, const float*
     if (tokens <= DR_DEPENDENT_TOKENS)
         return launch_dependent(delta_prepare_kernel, dim3(tokens), dim3(threads), smem, stream, proj, conv_w, a_log, dt_bias, token_seg, seg_starts,
                                 seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps);
-    // from 148 blocks on: below, a block a token has the shorter way
+    // from 148 blocks on: below, a block a token has the shorter way.  (What a launch may have without asking, 48 KB, counts the kernel's `place` and `olds` too.)
     const size_t smem8 = (size_t)DP_TOKENS * 2 * G * dk * sizeof(float);
-    if (taps <= DP_TAPS && tokens >= 148 * DP_TOKENS && smem8 <= 48 * 1024)
+    if (taps <= DP_TAPS && tokens >= 148 * DP_TOKENS && smem8 + DP_TOKENS * (sizeof(int) + sizeof(float*)) <= 48 * 1024)
         return launch_plain(delta_prepare_tokens_kernel, dim3((tokens + DP_TOKENS - 1) / DP_TOKENS), dim3(256), smem8, stream, proj, conv_w, a_log, dt_bias, token_seg,
                             seg_starts, seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps, tokens);
     return launch_plain(delta_prepare_kernel, dim3(tokens), dim3(256), smem, stream, proj, conv_w, a_log, dt_bias, token_seg, seg_starts,
