@@ -130,3 +130,33 @@ def test_gated_linear_attention_in_chunks(sizes, tau):
     assert float((state[1] - 7.0).abs().max()) == 0.0
     for slot in (0, 2, 3, 4, 5, 6, 7):
         _close(state[slot].cpu(), S[slot].reshape(-1), PART * S_size[slot].reshape(-1), ("S", slot))
+
+
+@pytest.mark.parametrize("rank", [764, 768, 1100])          # around the most whose 16 tokens the chunks' kernel stages (767; rows come in whole pieces of four), and far more
+def test_ranks_around_what_the_chunks_take(rank, monkeypatch):
+    """A prompt's step through the part: a rank that the chunks do not take runs token after token, with the same results."""
+    from vitna_anchor_b200 import ops
+    from vitna_anchor_b200.cache import CacheManager
+    from vitna_anchor_b200.engine.context import ContextBuilder
+    from vitna_anchor_b200.parts.base import Workspace
+    from vitna_anchor_b200.parts.gla import GatedLinearAttention
+    W, H, dk, dv, T = 64, 1, 16, 16, 600
+    assert ops.memory_chunked_takes(2 * H * dk + 2 * H * dv + rank, dk, dv, rank) == (rank <= 767)
+    g = torch.Generator(device="cuda").manual_seed(rank)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    part = GatedLinearAttention(W, H, dk, dv, 8.0, (r(2 * H * dk + 2 * H * dv + rank, W) * W ** -0.5).bfloat16(), r(H * dk, rank) * rank ** -0.5, r(H * dk), 1 + 0.1 * r(dv),
+                                (r(W, H * dv) * dv ** -0.5).bfloat16(), 1e-6)
+    x, got = r(T, W).bfloat16(), []
+    for chunked in (True, False):
+        if not chunked:
+            monkeypatch.setattr(ops, "memory_chunked_takes", lambda *a: False)
+        cache = CacheManager([part.cache_spec()], page_size=16, num_pages=T // 16 + 1, max_requests=1, dtype=torch.bfloat16, device="cuda")
+        builder = ContextBuilder(cache, torch.bfloat16, Workspace(torch.device("cuda"), T, 1, T), max_batch_tokens=T, max_segments=1, max_model_len=608, device="cuda")
+        cache.open(0)
+        cache.reserve_step([(0, T)])
+        ctx, _ = builder.build([(0, [0] * T, [])])
+        ctx.caches[0].state.zero_()
+        y = torch.zeros(T, W, device="cuda")
+        part.forward(x, ctx, ctx.caches[0], y)
+        got.append(y)
+    assert float((got[0] - got[1]).abs().max()) <= 2e-2 * float(got[1].abs().max())         # bfloat16 outputs of the head in front of the last product

@@ -686,8 +686,13 @@ using namespace vk;
 static int cm_chunks(int tokens, int segments) { return tokens / CM_Q + (segments < tokens ? segments : tokens); }
 static size_t cm_up(size_t b) { return (b + 255) / 256 * 256; }
 
-// Whether the chunked kernels take these sizes: heads of up to 128 x 256 values in whole 16-byte pieces of the product's rows (N floats).
-VK_API int vk_memory_chunked_takes(int N, int dk, int dv) { return N % 4 == 0 && dk > 0 && dk % 4 == 0 && dk <= 128 && dv > 0 && dv % 4 == 0 && dv <= 256; }
+static size_t gla_decays_smem(int rank) { return (size_t)CM_LOCAL * rank * sizeof(float); }
+
+// Whether the chunked kernels take these sizes: heads of up to 128 x 256 values in whole 16-byte pieces of the product's rows (N floats), and a decays' narrow half
+// (rank values; none: 0) of which gla_chunk_decays has 16 tokens in the 48 KB that a block may have without asking, its own four numbers among them.
+VK_API int vk_memory_chunked_takes(int N, int dk, int dv, int rank) {
+    return N % 4 == 0 && dk > 0 && dk % 4 == 0 && dk <= 128 && dv > 0 && dv % 4 == 0 && dv <= 256 && rank >= 0 && gla_decays_smem(rank) + 4 * sizeof(int) <= 48 * 1024;
+}
 
 VK_API size_t vk_mlstm_chunked_scratch_bytes(int tokens, int segments, int H, int dk, int dv) {
     const size_t chunks = cm_chunks(tokens, segments);
@@ -733,7 +738,7 @@ static int cm_launch(const CmArgs& p, int tokens, int gate_off, const float* nor
 }
 
 static int cm_check(const CmArgs& p, int gate_off, const float* norm_w, const void* out, const void* scratch) {
-    if (p.H <= 0 || gate_off < 0 || gate_off % 2 || gate_off + p.H * p.dv > p.N || !vk_memory_chunked_takes(p.N, p.dk, p.dv)) return VK_BAD_SHAPE;
+    if (p.H <= 0 || gate_off < 0 || gate_off % 2 || gate_off + p.H * p.dv > p.N || !vk_memory_chunked_takes(p.N, p.dk, p.dv, 0)) return VK_BAD_SHAPE;
     if (p.H > 65535 || p.segments > 65535) return VK_TOO_LARGE;
     if ((uintptr_t)p.proj % 16 || (uintptr_t)norm_w % 8 || (uintptr_t)out % 4 || (uintptr_t)scratch % 16) return VK_BAD_ALIGNMENT;
     return VK_OK;
@@ -777,8 +782,8 @@ VK_API int vk_gla_chunked(const float* proj, int N, int H, int dk, int dv, int a
     if (segments <= 0 || tokens <= 0) return VK_OK;
     CmArgs p = cm_args(proj, N, H, dk, dv, seg_starts, seg_slots, state, scratch, segments);
     if (rank <= 0 || a_off < 0 || a_off + rank > N || !(tau > 0.0f) || N < 2 * H * dk + H * dv) return VK_BAD_SHAPE;
-    const size_t smem = (size_t)CM_LOCAL * rank * sizeof(float);
-    if (smem > 48 * 1024) return VK_TOO_LARGE;
+    const size_t smem = gla_decays_smem(rank);
+    if (!vk_memory_chunked_takes(N, dk, dv, rank)) return VK_BAD_SHAPE;
     int s = cm_check(p, gate_off, norm_w, out, scratch);
     if (s != VK_OK) return s;
     const int chunks = cm_chunks(tokens, segments);

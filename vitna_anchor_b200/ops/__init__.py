@@ -1436,9 +1436,10 @@ def mlstm_max_dim() -> int:
     return int(lib().vk_mlstm_max_dim())
 
 
-def memory_chunked_takes(proj_width: int, dim: int, vdim: int) -> bool:
-    """Whether the matrix memories' chunked form takes heads of dim x vdim behind a product of that many columns."""
-    return bool(lib().vk_memory_chunked_takes(proj_width, dim, vdim))
+def memory_chunked_takes(proj_width: int, dim: int, vdim: int, rank: int = 0) -> bool:
+    """Whether the matrix memories' chunked form takes heads of dim x vdim behind a product of that many columns, with decays from a narrow half
+    of `rank` values (0: none)."""
+    return bool(lib().vk_memory_chunked_takes(proj_width, dim, vdim, rank))
 
 
 def mlstm_chunked_scratch_bytes(tokens: int, segments: int, H: int, dim: int, vdim: int) -> int:

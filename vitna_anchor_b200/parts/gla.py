@@ -60,7 +60,7 @@ class GatedLinearAttention(Mixer):
         T, ws, HV = ctx.num_tokens, ctx.workspace, self.H * self.vdim
         proj = ops.linear(xn, self.w_in, ws.rows("gla.proj", T, self.w_in.shape[0], torch.float32), ops.LINEAR_F32)
         scratch = None
-        if T > self.CHUNKED_FROM and ctx.dtype == torch.bfloat16 and not ctx.decode_only and ops.memory_chunked_takes(proj.shape[1], self.dim, self.vdim):
+        if T > self.CHUNKED_FROM and ctx.dtype == torch.bfloat16 and not ctx.decode_only and ops.memory_chunked_takes(proj.shape[1], self.dim, self.vdim, self.a2t.shape[0]):
             scratch = ws.flat(f"gla.chunks/{self.H}/{self.dim}/{self.vdim}",
                               ops.gla_chunked_scratch_bytes(ws.max_tokens, ws.max_segments, self.H, self.dim, self.vdim), torch.uint8)
         out = ops.gla(proj, self.a_off, self.a2t, self.a_bias, self.tau, self.norm_weight, self.eps, ctx, cache.state,
