@@ -160,3 +160,26 @@ def test_ranks_around_what_the_chunks_take(rank, monkeypatch):
         part.forward(x, ctx, ctx.caches[0], y)
         got.append(y)
     assert float((got[0] - got[1]).abs().max()) <= 2e-2 * float(got[1].abs().max())         # bfloat16 outputs of the head in front of the last product
+
+
+@pytest.mark.parametrize("kind", ["mlstm", "gla"])
+def test_a_norm_weight_that_begins_anywhere(kind):
+    """A weight at an address off 8 bytes gives the bits of the same weight on 16."""
+    from vitna_anchor_b200 import ops
+    H, dk, dv, T, rank = 2, 20, 36, 100, 4
+    g = torch.Generator(device="cuda").manual_seed(1)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    n_nw = H * dv if kind == "mlstm" else dv
+    proj, bias, a2t, longer = r(T, 2 * H * dk + 2 * H * dv + 4), r(2 * H if kind == "mlstm" else H * dk), r(rank, H * dk), r(n_nw + 1)
+    got = []
+    for nw in (longer[1:], longer[1:].clone()):
+        ctx, out = _ctx((T,), (0,))[1], torch.empty(T, H * dv, device="cuda")
+        if kind == "mlstm":
+            ops.mlstm(proj, bias, 15.0, nw, 1e-5, ctx, torch.zeros(1, ops.mlstm_state_floats(H, dk, dv), device="cuda"), torch.empty(T, H * (dv + 2), device="cuda"), out, H, dk,
+                      dv, chunk_scratch=torch.empty(ops.mlstm_chunked_scratch_bytes(T, 1, H, dk, dv), dtype=torch.uint8, device="cuda"))
+        else:
+            ops.gla(proj, proj.shape[1] - rank, a2t, bias, 8.0, nw, 1e-5, ctx, torch.zeros(1, H * dk * dv, device="cuda"), torch.empty(T, H * dk, device="cuda"),
+                    torch.empty(T, H * dv, device="cuda"), out, H, dk, dv, 2 * H * dk + H * dv,
+                    chunk_scratch=torch.empty(ops.gla_chunked_scratch_bytes(T, 1, H, dk, dv), dtype=torch.uint8, device="cuda"))
+        got.append(out)
+    assert longer[1:].data_ptr() % 8 == 4 and torch.equal(got[0], got[1])

@@ -670,8 +670,8 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
             for (int n = 0; n < NT; n++) {
                 const int c = col0 + n * 8 + 2 * t4;
                 if (c >= dv) continue;
-                const float2 gt = *reinterpret_cast<const float2*>(gate + c), wt = *reinterpret_cast<const float2*>(wrow + c);
-                const float a = (o[m][n][2 * u] * inv) * wt.x, b = (o[m][n][2 * u + 1] * inv) * wt.y;
+                const float2 gt = *reinterpret_cast<const float2*>(gate + c);
+                const float a = (o[m][n][2 * u] * inv) * wrow[c], b = (o[m][n][2 * u + 1] * inv) * wrow[c + 1];      // (a weight may begin anywhere)
                 const float ra = (MLSTM ? a : a * gt.x) / (1.0f + expf(-gt.x)), rb = (MLSTM ? b : b * gt.y) / (1.0f + expf(-gt.y));
                 if (sizeof(T) == 2) *reinterpret_cast<__nv_bfloat162*>(orow + c) = __floats2bfloat162_rn(ra, rb);
                 else { orow[c] = from_f32<T>(ra); orow[c + 1] = from_f32<T>(rb); }
@@ -737,10 +737,10 @@ static int cm_launch(const CmArgs& p, int tokens, int gate_off, const float* nor
 #undef GO
 }
 
-static int cm_check(const CmArgs& p, int gate_off, const float* norm_w, const void* out, const void* scratch) {
+static int cm_check(const CmArgs& p, int gate_off, const void* out, const void* scratch) {
     if (p.H <= 0 || gate_off < 0 || gate_off % 2 || gate_off + p.H * p.dv > p.N || !vk_memory_chunked_takes(p.N, p.dk, p.dv, 0)) return VK_BAD_SHAPE;
     if (p.H > 65535 || p.segments > 65535) return VK_TOO_LARGE;
-    if ((uintptr_t)p.proj % 16 || (uintptr_t)norm_w % 8 || (uintptr_t)out % 4 || (uintptr_t)scratch % 16) return VK_BAD_ALIGNMENT;
+    if ((uintptr_t)p.proj % 16 || (uintptr_t)out % 4 || (uintptr_t)scratch % 16) return VK_BAD_ALIGNMENT;
     return VK_OK;
 }
 
@@ -758,7 +758,7 @@ VK_API int vk_mlstm_chunked(const float* proj, int N, int H, int dk, int dv, con
     if (segments <= 0 || tokens <= 0) return VK_OK;
     CmArgs p = cm_args(proj, N, H, dk, dv, seg_starts, seg_slots, state, scratch, segments);
     if (!(cap > 0.0f) || N < 2 * H * dk + 2 * H * dv + 2 * H) return VK_BAD_SHAPE;
-    int s = cm_check(p, gate_off, norm_w, out, scratch);
+    int s = cm_check(p, gate_off, out, scratch);
     if (s != VK_OK) return s;
     const size_t chunks = cm_chunks(tokens, segments), tok = cm_up((size_t)tokens * H * 8);
     char* at = (char*)scratch + cm_up(chunks * H * dk * dv * 4);
@@ -784,7 +784,7 @@ VK_API int vk_gla_chunked(const float* proj, int N, int H, int dk, int dv, int a
     if (rank <= 0 || a_off < 0 || a_off + rank > N || !(tau > 0.0f) || N < 2 * H * dk + H * dv) return VK_BAD_SHAPE;
     const size_t smem = gla_decays_smem(rank);
     if (!vk_memory_chunked_takes(N, dk, dv, rank)) return VK_BAD_SHAPE;
-    int s = cm_check(p, gate_off, norm_w, out, scratch);
+    int s = cm_check(p, gate_off, out, scratch);
     if (s != VK_OK) return s;
     const int chunks = cm_chunks(tokens, segments);
     p.state_floats = (size_t)H * dk * dv;
