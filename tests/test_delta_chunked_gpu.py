@@ -122,3 +122,41 @@ def test_neighbouring_tokens_at_the_limit_of_shared_memory(G, dk):
     whole, st = run(0, T, state.clone()), state.clone()
     for lo in range(0, T, 100):
         assert torch.equal(run(lo, min(T, lo + 100), st), whole[lo:lo + 100]), lo
+
+
+@pytest.mark.parametrize("strong", [3.0, 200.0, 1e30, float("inf")])       # sums to -100, -6,400, and beyond what any sum holds
+@pytest.mark.parametrize("dk", [64, 128])
+def test_strong_decays_beside_weak_ones(dk, strong):
+    """Tokens that leave almost nothing of the state in front of tokens that leave almost all, inside one chunk, against the recurrence in 64 bits."""
+    from vitna_anchor_b200 import ops
+    G, H, dv, taps, T = 1, 2, 32, 1, 192
+    rng = np.random.default_rng(dk)
+    N = 2 * G * dk + 2 * H * dv + 2 * H
+    proj = rng.standard_normal((T, N)).astype(np.float32)
+    a = np.where((np.arange(T) // 8) % 4 < 2, strong, -2.25)[:, None] + 0.05 * rng.standard_normal((T, H))      # softplus(-2.25) is 0.1
+    proj[:, N - H:] = a
+    conv, nw = rng.standard_normal((2 * G * dk + H * dv, taps)).astype(np.float32), np.ones(dv, np.float32)
+    dev = lambda x: torch.from_numpy(x).cuda()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    state = torch.zeros(1, ops.delta_state_floats(G, H, dk, dv, taps), device="cuda")
+    out = torch.empty(T, H * dv, device="cuda")
+    ops.delta_rule(dev(proj), dev(conv), torch.zeros(H, device="cuda"), torch.zeros(H, device="cuda"), dev(nw), 1e-6, i32([0] * T), i32([0, T]), i32([0]), state,
+                   torch.empty(T, ops.delta_prep_width(G, H, dk, dv), device="cuda"), torch.empty(T, H * dv, device="cuda"), out, G, H, dk, dv, taps,
+                   chunk_scratch=torch.full((ops.delta_chunked_scratch_floats(T, 1, H, dk, dv),), float("nan"), device="cuda"))
+    p = proj.astype(np.float64)
+    z = p[:, :2 * G * dk + H * dv] * conv[:, 0]
+    act = z / (1 + np.exp(-z))
+    unit = lambda x: x / np.sqrt((x ** 2).sum(-1, keepdims=True) + 1e-6)
+    q, k, v = unit(act[:, :dk]) * dk ** -0.5, unit(act[:, dk:2 * dk]), act[:, 2 * dk:].reshape(T, H, dv)
+    gate, beta = p[:, 2 * dk + H * dv:2 * dk + 2 * H * dv].reshape(T, H, dv), 1 / (1 + np.exp(-p[:, N - 2 * H:N - H]))
+    g = np.exp(-np.logaddexp(0.0, p[:, N - H:]))
+    S, want = np.zeros((H, dk, dv)), np.zeros((T, H, dv))
+    for t in range(T):
+        S *= g[t][:, None, None]
+        S += k[t][None, :, None] * (beta[t][:, None] * (v[t] - np.einsum("hkv,k->hv", S, k[t])))[:, None, :]
+        want[t] = np.einsum("hkv,k->hv", S, q[t])
+    want = want / np.sqrt((want ** 2).mean(-1, keepdims=True) + 1e-6) * gate / (1 + np.exp(-gate))
+    # float32 sums of up to 64 tokens' contributions, as in test_chunks_against_tokens; a ratio of decays from float32 sums of -6,400 would be 5e-4 off
+    assert np.abs(out.double().cpu().numpy().reshape(T, H, dv) - want).max() <= 2e-5 * np.abs(want).max()
+    got = state[0, :H * dv * dk].double().cpu().numpy().reshape(H, dv, dk).transpose(0, 2, 1)
+    assert np.abs(got - S).max() <= 2e-5 * max(1.0, np.abs(S).max())

@@ -67,7 +67,8 @@ template <int DKP, bool CH>
 __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p) {
     constexpr int LDQ = DKP + 8;
     extern __shared__ __align__(16) float dp_smem[];
-    __shared__ float L[DC_C], beta[DC_C];
+    __shared__ double L[CH ? 1 : DC_C];             // (float64: what counts are differences of neighbours, and behind a strongly decaying token the sum is in the thousands)
+    __shared__ float beta[DC_C], factor[DC_C];
     __shared__ int find[4];
     const int LDV = dc_ldv(p.dv);
     float* sq = dp_smem;                            // [64][LDQ]
@@ -98,17 +99,19 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
     }
     tf_commit();
     if (tid < 32) {                                 // beta, and the sums of the decays' logarithms
-        float carry = 0.0f;
+        double carry = 0.0;
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int r = 32 * u + tid;
             const float* row = row0 + (size_t)(r < rows ? r : 0) * p.P + Cq;
             beta[r] = r < rows ? row[(CH ? p.H * dk : p.H) + h] : 0.0f;
             if (!CH) {
-                float s = r < rows ? row[h] : 0.0f;
+                // (a token that leaves less than e^-10000 leaves nothing either way, and one that leaves e^-inf must not make the sums infinite)
+                const float l = r < rows ? row[h] : 0.0f;
+                double s = l < -1e4f ? -1e4 : (double)l;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
-                    const float v = __shfl_up_sync(0xffffffffu, s, o);
+                    const double v = __shfl_up_sync(0xffffffffu, s, o);
                     if (tid >= o) s += v;
                 }
                 L[r] = carry + s;
@@ -240,7 +243,7 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
                 float a[2], w[2];
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
-                    const float ratio = i + e <= r ? (CH ? 1.0f : expf(L[r] - L[i + e])) : 0.0f;
+                    const float ratio = i + e <= r ? (CH ? 1.0f : expf((float)(L[r] - L[i + e]))) : 0.0f;
                     a[e] = i + e < r ? beta[r] * ratio * kk[m][n][2 * u + e] : 0.0f;
                     w[e] = i + e <= r ? ratio * qk[m][n][2 * u + e] : 0.0f;
                 }
@@ -266,7 +269,7 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
             }
             *reinterpret_cast<float4*>(sk + r * LDQ + d) = kw;
         } else {
-            const float fq = expf(L[r]), fk = expf(L[DC_C - 1] - L[r]);
+            const float fq = expf((float)L[r]), fk = expf((float)(L[DC_C - 1] - L[r]));
             kq = *reinterpret_cast<const float4*>(sq + r * LDQ + d);
             kb = *reinterpret_cast<const float4*>(sk + r * LDQ + d);
             kq.x *= fq; kq.y *= fq; kq.z *= fq; kq.w *= fq;
@@ -277,7 +280,7 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
     }
     if (CH) {
         for (int d = tid; d < dk; d += 256) E_g[d] = (vec[d] * vec[DKP + d]) * (vec[2 * DKP + d] * vec[3 * DKP + d]);
-    } else if (tid == 0) E_g[0] = expf(L[DC_C - 1]);
+    } else if (tid == 0) E_g[0] = expf((float)L[DC_C - 1]);
     __syncthreads();
 
     // T = (I + A)^-1.  The blocks on the diagonal, a column a thread ..
@@ -321,7 +324,7 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
         }
     }
     // W = T diag(beta e^L) K and U' = T diag(beta) V, eight columns a warp at a time
-    if (tid < DC_C) L[tid] = CH ? beta[tid] : beta[tid] * expf(L[tid]);         // (the factor of k's rows from here on)
+    if (tid < DC_C) factor[tid] = CH ? beta[tid] : beta[tid] * expf((float)L[tid]);      // of k's rows
     __syncthreads();
     constexpr int nw = DKP / 8;
     const int nv = (dv + 7) / 8;
@@ -329,7 +332,7 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
         const bool is_w = n < nw;
         const int c0 = (is_w ? n : n - nw) * 8, ld = is_w ? LDQ : LDV;
         const float* src = (is_w ? sk : sv) + c0 + g;
-        const float* fac = is_w ? L : beta;
+        const float* fac = is_w ? factor : beta;
         float acc[4][4];
 #pragma unroll
         for (int m = 0; m < 4; m++)
