@@ -183,3 +183,60 @@ def test_a_norm_weight_that_begins_anywhere(kind):
                     chunk_scratch=torch.empty(ops.gla_chunked_scratch_bytes(T, 1, H, dk, dv), dtype=torch.uint8, device="cuda"))
         got.append(out)
     assert longer[1:].data_ptr() % 8 == 4 and torch.equal(got[0], got[1])
+
+
+def _part_and_batch(kind, lens, max_tokens, max_requests):
+    from vitna_anchor_b200.cache import CacheManager
+    from vitna_anchor_b200.engine.context import ContextBuilder
+    from vitna_anchor_b200.parts.base import Workspace
+    from vitna_anchor_b200.parts.gla import GatedLinearAttention
+    from vitna_anchor_b200.parts.mlstm import MatrixLSTM
+    W, H, dk, dv, rank = 64, 2, 16, 32, 4
+    g = torch.Generator(device="cuda").manual_seed(len(lens))
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    m = lambda rows, cols: (r(rows, cols) * cols ** -0.5).bfloat16()
+    if kind == "mlstm":
+        part = MatrixLSTM(W, H, dk, dv, 15.0, m(2 * H * dk + 2 * H * dv + 2 * H, W), r(2 * H), 1 + 0.1 * r(H * dv), m(W, H * dv), 1e-6)
+    else:
+        part = GatedLinearAttention(W, H, dk, dv, 8.0, m(2 * H * dk + 2 * H * dv + rank, W), r(H * dk, rank) * 0.5, r(H * dk), 1 + 0.1 * r(dv), m(W, H * dv), 1e-6)
+    cache = CacheManager([part.cache_spec()], page_size=16, num_pages=64, max_requests=max_requests, dtype=torch.bfloat16, device="cuda")
+    builder = ContextBuilder(cache, torch.bfloat16, Workspace(torch.device("cuda"), max_tokens, max_requests, 4096), max_batch_tokens=max_tokens, max_segments=max_requests,
+                             max_model_len=4096, device="cuda")
+    for i in range(len(lens)):
+        cache.open(i)
+    cache.reserve_step([(i, n) for i, n in enumerate(lens)])
+    ctx, _ = builder.build([(i, [0] * n, []) for i, n in enumerate(lens)])
+    ctx.caches[0].state.copy_(0.1 * r(*ctx.caches[0].state.shape))
+    return part, ctx, r(sum(lens), W).bfloat16()
+
+
+@pytest.mark.parametrize("lens", [(600, 1, 1, 32, 33, 1), (1, 433, 2), (33, 32, 700), (1, 1, 40, 1), (500,), (1200, 900)])
+@pytest.mark.parametrize("few", [1, 100])
+@pytest.mark.parametrize("kind", ["mlstm", "gla"])
+def test_a_step_of_segments_of_every_length(kind, lens, few, monkeypatch):
+    """Long segments in chunks, with short ones token after token or among them: all have the results and states of the token-by-token kernels, and those that run token
+    after token their bits."""
+    from vitna_anchor_b200.parts.base import StepContext
+    got = []
+    for plain in (False, True):
+        if plain:
+            monkeypatch.setattr(StepContext, "chunk_plan", lambda *a: None)
+        part, ctx, x = _part_and_batch(kind, lens, sum(lens), len(lens))
+        part.chunk_rule = part.chunk_rule._replace(few=few)
+        assert plain or (ctx.chunk_plan(part.chunk_rule) is not None) == (max(lens) > 432)
+        y = torch.zeros(x.shape[0], 64, device="cuda")
+        part.forward(x, ctx, ctx.caches[0], y)
+        got.append((y, ctx.caches[0].state.clone(), ctx.host_seg_slots))
+    (y, st, slots), (want, want_st, _) = got
+    assert float((y - want).abs().max()) <= 2e-2 * float(want.abs().max())         # bfloat16 outputs of the heads in front of the last product
+    assert float((st - want_st).abs().max()) <= 2e-4 * float(want_st.abs().max())
+    for n, slot in zip(lens, slots):
+        if n <= 32 and few == 1:
+            assert torch.equal(st[slot], want_st[slot]), n
+
+
+def test_scratch_follows_the_segments_that_can_be_long():
+    """Steps of up to 2,048 tokens and 256 requests: of more than 32 tokens there are at most 62 segments, and only those have chunks."""
+    from vitna_anchor_b200 import ops
+    assert ops.mlstm_chunked_scratch_bytes(2048, 256, 8, 128, 256, 32) == ops.mlstm_chunked_scratch_bytes(2048, 62, 8, 128, 256)
+    assert 3 * ops.mlstm_chunked_scratch_bytes(2048, 256, 8, 128, 256, 32) < ops.mlstm_chunked_scratch_bytes(2048, 256, 8, 128, 256)

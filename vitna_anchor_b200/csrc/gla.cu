@@ -37,13 +37,20 @@ __device__ __forceinline__ void gla_cp16(float* dst, const float* src) {
 }
 
 // proj float32 [tokens][N] with the narrow half at columns a_off .. a_off + rank - 1; a2t float32 [rank][C]; bias float32 [C];
-// decay float32 [tokens][C], C = H dim.
+// decay float32 [tokens][C], C = H dim.  SOME: only for the tokens of segments of up to `upto` tokens.
+template <bool SOME>
 __global__ void __launch_bounds__(256) gla_prepare_kernel(const float* __restrict__ proj, int N, int a_off, int rank, const float* __restrict__ a2t,
-                                                          const float* __restrict__ bias, float inv_tau, int C, float* __restrict__ decay, int tokens) {
+                                                          const float* __restrict__ bias, float inv_tau, int C, float* __restrict__ decay, int tokens,
+                                                          const int32_t* __restrict__ token_seg, const int32_t* __restrict__ seg_starts, int upto) {
     extern __shared__ float gp_sh[];                    // [GLA_PREP_TOKENS][rank]
     dependency_wait();
     let_dependents_start();
     const int t0 = blockIdx.x * GLA_PREP_TOKENS, cnt = min(GLA_PREP_TOKENS, tokens - t0);
+    if (SOME) {                                         // nothing to do where all the tokens are of longer segments
+        bool any = false;
+        for (int t = t0; t < t0 + cnt; t++) any = any || seg_starts[token_seg[t] + 1] - seg_starts[token_seg[t]] <= upto;
+        if (!any) return;
+    }
     for (int i = threadIdx.x; i < cnt * rank; i += blockDim.x) gp_sh[i] = proj[(size_t)(t0 + i / rank) * N + a_off + i % rank];
     __syncthreads();
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
@@ -79,7 +86,7 @@ template <int DPT, int C, int RG>
 __global__ void __launch_bounds__(GLA_THREADS) gla_recurrence_kernel(const float* __restrict__ proj, int N, int H, int dim, int vdim,
                                                                      const float* __restrict__ decay, float qscale,
                                                                      const int32_t* __restrict__ seg_starts, const int32_t* __restrict__ seg_slots,
-                                                                     float* __restrict__ state, size_t state_floats, float* __restrict__ o, int vec) {
+                                                                     float* __restrict__ state, size_t state_floats, float* __restrict__ o, int vec, int upto) {
     constexpr int DP = RG * DPT;                                                // rows of the state as the registers hold them (dim rounded up)
     constexpr int CPW = 32 / RG, COLS = 4 * CPW;                                // columns of a warp and of a block
     constexpr int STAGE = gla_stage_floats(C, DPT, RG);
@@ -92,7 +99,7 @@ __global__ void __launch_bounds__(GLA_THREADS) gla_recurrence_kernel(const float
     const int cl = warp * CPW + lane % CPW;
     const int col0 = blockIdx.x * COLS, col = col0 + cl;
     const int first = seg_starts[seg], end = seg_starts[seg + 1], slot = seg_slots[seg];
-    if (first >= end) return;
+    if (first >= end || end - first > upto) return;
     float* st = slot >= 0 ? state + (size_t)slot * state_floats : nullptr;
     float* col_st = (!st || col >= vdim) ? nullptr : st + (size_t)h * dim * vdim + col;
     float S[DPT];
@@ -276,10 +283,12 @@ __global__ void __launch_bounds__(GLA_THREADS) gla_decode_kernel(const float* __
 
 template <typename T>
 __global__ void __launch_bounds__(256) gla_gate_kernel(const float* __restrict__ o, const float* __restrict__ proj, int N, int gate_off,
-                                                       const float* __restrict__ w, float eps, int H, int vdim, T* __restrict__ out) {
+                                                       const float* __restrict__ w, float eps, int H, int vdim, T* __restrict__ out,
+                                                       const int32_t* __restrict__ token_seg, const int32_t* __restrict__ seg_starts, int upto) {
     dependency_wait();
     let_dependents_start();
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    if (token_seg && seg_starts[token_seg[t] + 1] - seg_starts[token_seg[t]] > upto) return;
     for (int h = warp; h < H; h += nwarps) {
         const float* in = o + ((size_t)t * H + h) * vdim;
         float ss = 0.0f;
@@ -305,21 +314,22 @@ VK_API int vk_gla_max_dim() { return 256; }
 // the one-launch form for single tokens makes the same one, so that a token's sums meet in one order wherever it is worked out.
 static inline bool gla_sixteen_lanes(int H, int dim, int vdim) { return dim > 32 && (long long)((vdim + 7) / 8) * H <= 148; }
 
-// decay float32 [tokens][H dim] <- exp(log sigmoid(a2t^T proj[:, a_off : a_off + rank] + bias) / tau)
+// decay float32 [tokens][H dim] <- exp(log sigmoid(a2t^T proj[:, a_off : a_off + rank] + bias) / tau).  Here and below, segments of more than `upto` tokens are
+// left alone (vk_gla_chunked has them); vk_gla_prepare and vk_gla_gate then need token_seg and seg_starts, and null token_seg otherwise.
 VK_API int vk_gla_prepare(const float* proj, int N, int a_off, int rank, const float* a2t, const float* bias, float tau, int channels, float* decay,
-                          int tokens, cudaStream_t stream) {
+                          int tokens, const int32_t* token_seg, const int32_t* seg_starts, int upto, cudaStream_t stream) {
     if (tokens <= 0) return VK_OK;
     if (rank <= 0 || a_off < 0 || a_off + rank > N || channels <= 0 || !(tau > 0.0f)) return VK_BAD_SHAPE;
     const size_t smem = (size_t)GLA_PREP_TOKENS * rank * sizeof(float);
     if (smem > 48 * 1024) return VK_TOO_LARGE;
-    return launch_dependent(gla_prepare_kernel, dim3((tokens + GLA_PREP_TOKENS - 1) / GLA_PREP_TOKENS), dim3(256), smem, stream, proj, N, a_off, rank,
-                            a2t, bias, 1.0f / tau, channels, decay, tokens);
+    return launch_dependent(token_seg ? gla_prepare_kernel<true> : gla_prepare_kernel<false>, dim3((tokens + GLA_PREP_TOKENS - 1) / GLA_PREP_TOKENS), dim3(256), smem, stream, proj, N, a_off, rank,
+                            a2t, bias, 1.0f / tau, channels, decay, tokens, token_seg, seg_starts, upto);
 }
 
 // proj float32 [tokens][N] = q [H dim] | k [H dim] | v [H vdim] | ...;  decay float32 [tokens][H dim];  state float32 [slots][H dim vdim];
 // o float32 [tokens][H][vdim].  A block a (16 columns, head, segment): segments is the step's count, whatever their lengths.
 VK_API int vk_gla_recurrence(const float* proj, int N, int H, int dim, int vdim, const float* decay, const int32_t* seg_starts,
-                             const int32_t* seg_slots, float* state, float* o, int segments, cudaStream_t stream) {
+                             const int32_t* seg_slots, float* state, float* o, int segments, int upto, cudaStream_t stream) {
     if (segments <= 0) return VK_OK;
     if (H <= 0 || dim <= 0 || vdim <= 0 || N < 2 * H * dim + H * vdim) return VK_BAD_SHAPE;
     if (dim > 256 || H > 65535 || segments > 65535) return VK_TOO_LARGE;
@@ -335,7 +345,7 @@ VK_API int vk_gla_recurrence(const float* proj, int N, int H, int dim, int vdim,
         if (e != cudaSuccess) return (int)e;                                                                                                 \
         const int cols = 128 / RG;                                                                                                           \
         return launch_dependent(kern, dim3((vdim + cols - 1) / cols, H, segments), dim3(GLA_THREADS), smem, stream, proj, N, H, dim, vdim,   \
-                                decay, qscale, seg_starts, seg_slots, state, state_floats, o, vec);                                          \
+                                decay, qscale, seg_starts, seg_slots, state, state_floats, o, vec, upto);                                          \
     } while (0)
     if (dim <= 32) VK_GLA(4, 32, 8);
     if (gla_sixteen_lanes(H, dim, vdim)) {
@@ -376,11 +386,12 @@ VK_API int vk_gla_decode(const float* proj, int N, int H, int dim, int vdim, int
 
 // out [tokens][H vdim] in dtype = o / rms(o) per head * w [vdim] * silu(proj[:, gate_off + ...])
 VK_API int vk_gla_gate(const float* o, const float* proj, int N, int gate_off, const float* w, float eps, int H, int vdim, void* out, int tokens,
-                       int dtype, cudaStream_t stream) {
+                       const int32_t* token_seg, const int32_t* seg_starts, int upto, int dtype, cudaStream_t stream) {
     if (tokens <= 0) return VK_OK;
     if (H <= 0 || vdim <= 0 || gate_off < 0 || gate_off + H * vdim > N) return VK_BAD_SHAPE;
     if (dtype == 0)
-        return launch_dependent(gla_gate_kernel<float>, dim3(tokens), dim3(256), 0, stream, o, proj, N, gate_off, w, eps, H, vdim, (float*)out);
+        return launch_dependent(gla_gate_kernel<float>, dim3(tokens), dim3(256), 0, stream, o, proj, N, gate_off, w, eps, H, vdim, (float*)out, token_seg,
+                                seg_starts, upto);
     return launch_dependent(gla_gate_kernel<__nv_bfloat16>, dim3(tokens), dim3(256), 0, stream, o, proj, N, gate_off, w, eps, H, vdim,
-                            (__nv_bfloat16*)out);
+                            (__nv_bfloat16*)out, token_seg, seg_starts, upto);
 }

@@ -37,7 +37,7 @@ __device__ __forceinline__ float cm_log_sigmoid(float z) { return fminf(z, 0.0f)
 
 struct CmArgs {
     const float* proj;              // [tokens][N]: q | k | v | ..
-    int N, H, dk, dv, segments;
+    int N, H, dk, dv, segments, from;       // segments of up to `from` tokens are left alone
     const int32_t* seg_starts;
     const int32_t* seg_slots;
     float* state;                   // [slots][state_floats]
@@ -64,9 +64,9 @@ __global__ void __launch_bounds__(MG_THREADS) mlstm_chunk_gates_kernel(const CmA
     __shared__ int base_sh;
     const int h = blockIdx.x, seg = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = p.H;
     const int first = p.seg_starts[seg], end = p.seg_starts[seg + 1], slot = p.seg_slots[seg];
-    if (first >= end) return;
+    if (end - first <= p.from) return;
     if (warp == 0) {
-        const int b = first_chunk_of<CM_Q>(seg, p.seg_starts);
+        const int b = first_chunk_of<CM_Q>(seg, p.seg_starts, p.from);
         if (lane == 0) base_sh = b;
     }
     const int chunks = (end - first + CM_Q - 1) / CM_Q;
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(GD_THREADS) gla_chunk_decays_kernel(const CmAr
                                                                       const float* __restrict__ bias, float inv_tau) {
     extern __shared__ float gd_sh[];                    // [rank][16]
     __shared__ int find[4];
-    const Chunk ch = find_chunk<CM_Q>(blockIdx.x / 4, p.seg_starts, p.segments, find);
+    const Chunk ch = find_chunk<CM_Q>(blockIdx.x / 4, p.seg_starts, p.segments, find, p.from);
     const int r0 = (blockIdx.x & 3) * CM_LOCAL, cnt = ch.seg < 0 ? 0 : min(CM_LOCAL, ch.rows - r0);
     if (cnt <= 0) return;
     const int first = ch.first + r0, c = blockIdx.y * GD_THREADS + threadIdx.x, C = p.H * p.dk;
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(128) cm_add_kernel(const CmArgs p, int col_til
     float* sk = ca_smem;                            // [64][CM_LD] k
     float* sv = sk + CM_Q * CM_LD;                  // [64][CM_LD] v
     float* sl = sv + CM_Q * CM_LD;                  // [64][CM_LD] the decays' logarithms (gated linear attention)
-    const Chunk ch = find_chunk<CM_Q>(blockIdx.x, p.seg_starts, p.segments, find);
+    const Chunk ch = find_chunk<CM_Q>(blockIdx.x, p.seg_starts, p.segments, find, p.from);
     if (ch.seg < 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, wd = (warp & 1) * 32, wv = (warp >> 1) * 32;
     const int h = blockIdx.y, H = p.H, dk = p.dk, dv = p.dv, rows = ch.rows;
@@ -301,9 +301,9 @@ __global__ void __launch_bounds__(256) cm_scan_kernel(const CmArgs p) {
     __shared__ int base_sh;
     const int seg = blockIdx.z, h = blockIdx.y, H = p.H, dk = p.dk, dv = p.dv;
     const int first = p.seg_starts[seg], end = p.seg_starts[seg + 1], slot = p.seg_slots[seg];
-    if (first >= end) return;
+    if (end - first <= p.from) return;
     if (threadIdx.x < 32) {
-        const int b = first_chunk_of<CM_Q>(seg, p.seg_starts);
+        const int b = first_chunk_of<CM_Q>(seg, p.seg_starts, p.from);
         if (threadIdx.x == 0) base_sh = b;
     }
     __syncthreads();
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
     float* sq = co_smem;
     float* ring = co_smem + CM_Q * LDQ;
     float* sk = ring + L::SLOT;                         // k waits in the second slot
-    const Chunk ch = find_chunk<CM_Q>(blockIdx.x, p.seg_starts, p.segments, find);
+    const Chunk ch = find_chunk<CM_Q>(blockIdx.x, p.seg_starts, p.segments, find, p.from);
     if (ch.seg < 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, wm = warp & 1, wn = warp >> 1;
     const int h = blockIdx.y, H = p.H, dk = p.dk, dv = p.dv, rows = ch.rows;
@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
 
 using namespace vk;
 
-static int cm_chunks(int tokens, int segments) { return tokens / CM_Q + (segments < tokens ? segments : tokens); }
+static int cm_chunks(int tokens, int segments, int from) { return most_chunks(CM_Q, tokens, segments, from); }
 static size_t cm_up(size_t b) { return (b + 255) / 256 * 256; }
 
 static size_t gla_decays_smem(int rank) { return (size_t)CM_LOCAL * rank * sizeof(float); }
@@ -694,12 +694,13 @@ VK_API int vk_memory_chunked_takes(int N, int dk, int dv, int rank) {
     return N % 4 == 0 && dk > 0 && dk % 4 == 0 && dk <= 128 && dv > 0 && dv % 4 == 0 && dv <= 256 && rank >= 0 && gla_decays_smem(rank) + 4 * sizeof(int) <= 48 * 1024;
 }
 
-VK_API size_t vk_mlstm_chunked_scratch_bytes(int tokens, int segments, int H, int dk, int dv) {
-    const size_t chunks = cm_chunks(tokens, segments);
+// (from: as for the kernels; the larger it is, the fewer chunks a step of many segments can have, each with a head's whole state)
+VK_API size_t vk_mlstm_chunked_scratch_bytes(int tokens, int segments, int H, int dk, int dv, int from) {
+    const size_t chunks = cm_chunks(tokens, segments, from);
     return cm_up(chunks * H * dk * dv * 4) + cm_up(chunks * H * dk * 4) + 2 * cm_up(chunks * H * 8) + 4 * cm_up((size_t)tokens * H * 8);
 }
-VK_API size_t vk_gla_chunked_scratch_bytes(int tokens, int segments, int H, int dk, int dv) {
-    const size_t chunks = cm_chunks(tokens, segments);
+VK_API size_t vk_gla_chunked_scratch_bytes(int tokens, int segments, int H, int dk, int dv, int from) {
+    const size_t chunks = cm_chunks(tokens, segments, from);
     return cm_up(chunks * H * dk * dv * 4) + cm_up(chunks * H * dk * 4) + cm_up((size_t)tokens * H * dk * 4);
 }
 
@@ -709,7 +710,7 @@ static int cm_launch_out(const CmArgs& p, int tokens, int gate_off, const float*
     const int smem = CmOut<DK, DV>::FLOATS * (int)sizeof(float);
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
-    return launch_plain(kern, dim3(cm_chunks(tokens, p.segments), p.H), dim3(256), smem, stream, p, gate_off, norm_w, eps, (T*)out);
+    return launch_plain(kern, dim3(cm_chunks(tokens, p.segments, p.from), p.H), dim3(256), smem, stream, p, gate_off, norm_w, eps, (T*)out);
 }
 
 template <bool MLSTM>
@@ -719,7 +720,7 @@ static int cm_launch(const CmArgs& p, int tokens, int gate_off, const float* nor
     const cudaError_t e = cudaFuncSetAttribute(add, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     const int col_tiles = (p.dv + CM_T - 1) / CM_T, row_tiles = (p.dk + CM_T - 1) / CM_T;
-    int s = launch_plain(add, dim3(cm_chunks(tokens, p.segments), p.H, row_tiles * col_tiles), dim3(128), smem, stream, p, col_tiles);
+    int s = launch_plain(add, dim3(cm_chunks(tokens, p.segments, p.from), p.H, row_tiles * col_tiles), dim3(128), smem, stream, p, col_tiles);
     if (s != VK_OK) return s;
     s = launch_plain(cm_scan_kernel<MLSTM>, dim3((p.dk * p.dv + 1023) / 1024 + (MLSTM ? 1 : 0), p.H, p.segments), dim3(256), 0, stream, p);
     if (s != VK_OK) return s;
@@ -744,23 +745,24 @@ static int cm_check(const CmArgs& p, int gate_off, const void* out, const void* 
     return VK_OK;
 }
 
-static CmArgs cm_args(const float* proj, int N, int H, int dk, int dv, const int32_t* seg_starts, const int32_t* seg_slots, float* state, void* scratch, int segments) {
+static CmArgs cm_args(const float* proj, int N, int H, int dk, int dv, const int32_t* seg_starts, const int32_t* seg_slots, float* state, void* scratch, int segments, int from) {
     CmArgs p = {};
-    p.proj = proj; p.N = N; p.H = H; p.dk = dk; p.dv = dv; p.segments = segments;
+    p.proj = proj; p.N = N; p.H = H; p.dk = dk; p.dv = dv; p.segments = segments; p.from = from;
     p.seg_starts = seg_starts; p.seg_slots = seg_slots; p.state = state; p.before = (float*)scratch;
     return p;
 }
 
-// proj, state and norm as for vk_mlstm_recurrence and vk_mlstm_gate; out [tokens][H dv] in dtype; four kernels.
+// proj, state and norm as for vk_mlstm_recurrence and vk_mlstm_gate; out [tokens][H dv] in dtype; four kernels.  Segments of up to `from` tokens are left alone: their
+// states and their rows of out are for the token-by-token kernels.
 VK_API int vk_mlstm_chunked(const float* proj, int N, int H, int dk, int dv, const float* gate_bias, float cap, int gate_off, const float* norm_w, float eps,
-                            const int32_t* seg_starts, const int32_t* seg_slots, float* state, void* scratch, void* out, int tokens, int segments, int dtype,
-                            cudaStream_t stream) {
+                            const int32_t* seg_starts, const int32_t* seg_slots, float* state, void* scratch, void* out, int tokens, int segments, int from,
+                            int dtype, cudaStream_t stream) {
     if (segments <= 0 || tokens <= 0) return VK_OK;
-    CmArgs p = cm_args(proj, N, H, dk, dv, seg_starts, seg_slots, state, scratch, segments);
-    if (!(cap > 0.0f) || N < 2 * H * dk + 2 * H * dv + 2 * H) return VK_BAD_SHAPE;
+    CmArgs p = cm_args(proj, N, H, dk, dv, seg_starts, seg_slots, state, scratch, segments, from);
+    if (from < 0 || !(cap > 0.0f) || N < 2 * H * dk + 2 * H * dv + 2 * H) return VK_BAD_SHAPE;
     int s = cm_check(p, gate_off, out, scratch);
     if (s != VK_OK) return s;
-    const size_t chunks = cm_chunks(tokens, segments), tok = cm_up((size_t)tokens * H * 8);
+    const size_t chunks = cm_chunks(tokens, segments, from), tok = cm_up((size_t)tokens * H * 8);
     char* at = (char*)scratch + cm_up(chunks * H * dk * dv * 4);
     p.state_floats = (size_t)H * dk * dv + (size_t)H * dk + H;
     p.n_before = (float*)at; at += cm_up(chunks * H * dk * 4);
@@ -778,15 +780,15 @@ VK_API int vk_mlstm_chunked(const float* proj, int N, int H, int dk, int dv, con
 // proj, decays and state as for vk_gla_prepare and vk_gla_recurrence, norm and gate as for vk_gla_gate; four kernels.
 VK_API int vk_gla_chunked(const float* proj, int N, int H, int dk, int dv, int a_off, int rank, const float* a2t, const float* bias, float tau, int gate_off,
                           const float* norm_w, float eps, const int32_t* seg_starts, const int32_t* seg_slots, float* state, void* scratch, void* out,
-                          int tokens, int segments, int dtype, cudaStream_t stream) {
+                          int tokens, int segments, int from, int dtype, cudaStream_t stream) {
     if (segments <= 0 || tokens <= 0) return VK_OK;
-    CmArgs p = cm_args(proj, N, H, dk, dv, seg_starts, seg_slots, state, scratch, segments);
-    if (rank <= 0 || a_off < 0 || a_off + rank > N || !(tau > 0.0f) || N < 2 * H * dk + H * dv) return VK_BAD_SHAPE;
+    CmArgs p = cm_args(proj, N, H, dk, dv, seg_starts, seg_slots, state, scratch, segments, from);
+    if (from < 0 || rank <= 0 || a_off < 0 || a_off + rank > N || !(tau > 0.0f) || N < 2 * H * dk + H * dv) return VK_BAD_SHAPE;
     const size_t smem = gla_decays_smem(rank);
     if (!vk_memory_chunked_takes(N, dk, dv, rank)) return VK_BAD_SHAPE;
     int s = cm_check(p, gate_off, out, scratch);
     if (s != VK_OK) return s;
-    const int chunks = cm_chunks(tokens, segments);
+    const int chunks = cm_chunks(tokens, segments, from);
     p.state_floats = (size_t)H * dk * dv;
     p.decay = (float*)((char*)scratch + cm_up((size_t)chunks * H * dk * dv * 4));
     p.logs = (float*)((char*)p.decay + cm_up((size_t)chunks * H * dk * 4));

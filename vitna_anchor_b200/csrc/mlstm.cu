@@ -49,7 +49,7 @@ template <int DPT, int C>
 __global__ void __launch_bounds__(ML_THREADS) mlstm_recurrence_kernel(const float* __restrict__ proj, int N, int H, int dim, int vdim,
                                                                       const float* __restrict__ gate_bias, float cap, float qscale,
                                                                       const int32_t* __restrict__ seg_starts, const int32_t* __restrict__ seg_slots,
-                                                                      float* __restrict__ state, size_t state_floats, float* __restrict__ o, int vec) {
+                                                                      float* __restrict__ state, size_t state_floats, float* __restrict__ o, int vec, int upto) {
     constexpr int DP = ML_ROW_GROUPS * DPT;                                     // rows of the state as the registers hold them (dim rounded up)
     constexpr int STAGE = ml_stage_floats(C, DPT);
     extern __shared__ __align__(16) float ml_smem[];
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(ML_THREADS) mlstm_recurrence_kernel(const floa
     const int cl = warp * 4 + (lane & 3);
     const int col0 = blockIdx.x * ML_COLS, col = col0 + cl;
     const int first = seg_starts[seg], end = seg_starts[seg + 1], slot = seg_slots[seg];
-    if (first >= end) return;
+    if (first >= end || end - first > upto) return;
     float* st = slot >= 0 ? state + (size_t)slot * state_floats : nullptr;
     // column vdim is n: its rows lie one after another in the state
     float* col_st = !st || col > vdim ? nullptr
@@ -190,19 +190,20 @@ template <typename T>
 __global__ void __launch_bounds__(256) mlstm_gate_kernel(const float* __restrict__ o, const float* __restrict__ proj, int N, int gate_off,
                                                          const float* __restrict__ w, float eps, int H, int dim, int vdim, T* __restrict__ out,
                                                          int tokens, const int32_t* __restrict__ seg_starts, const int32_t* __restrict__ seg_slots,
-                                                         float* __restrict__ state, size_t state_floats) {
+                                                         float* __restrict__ state, size_t state_floats, const int32_t* __restrict__ token_seg, int upto) {
     dependency_wait();
     let_dependents_start();
     const int OW = vdim + 2;
     if ((int)blockIdx.x >= tokens) {                     // a segment's block: m after its last token goes into the state
         const int seg = blockIdx.x - tokens;
         const int first = seg_starts[seg], end = seg_starts[seg + 1], slot = seg_slots[seg];
-        if (first >= end || slot < 0) return;
+        if (first >= end || slot < 0 || end - first > upto) return;
         float* m_st = state + (size_t)slot * state_floats + (size_t)H * dim * vdim + (size_t)H * dim;
         for (int h = threadIdx.x; h < H; h += blockDim.x) m_st[h] = o[((size_t)(end - 1) * H + h) * OW + vdim + 1];
         return;
     }
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    if (token_seg && seg_starts[token_seg[t] + 1] - seg_starts[token_seg[t]] > upto) return;
     for (int h = warp; h < H; h += nwarps) {
         const float* in = o + ((size_t)t * H + h) * OW;
         const float inv_den = 1.0f / (fmaxf(fabsf(in[vdim]), expf(-in[vdim + 1])) + 1e-6f);
@@ -227,9 +228,10 @@ VK_API int vk_mlstm_max_dim() { return 256; }
 
 // proj float32 [tokens][N] = q [H dim] | k [H dim] | v [H vdim] | gate [H vdim] | a [H] | b [H];  gate_bias float32 [2H] (a's, then b's);
 // state float32 [slots][H dim vdim + H dim + H];  o float32 [tokens][H][vdim + 2] (numerators, n . q, m).  A block a (16 columns, head,
-// segment): segments is the step's count, whatever their lengths.  S and n of the state are written here, m by vk_mlstm_gate.
+// segment): segments is the step's count, whatever their lengths.  S and n of the state are written here, m by vk_mlstm_gate.  Segments of more than
+// `upto` tokens are left alone by both (vk_mlstm_chunked has them); vk_mlstm_gate then needs token_seg, and null otherwise.
 VK_API int vk_mlstm_recurrence(const float* proj, int N, int H, int dim, int vdim, const float* gate_bias, float cap, const int32_t* seg_starts,
-                               const int32_t* seg_slots, float* state, float* o, int segments, cudaStream_t stream) {
+                               const int32_t* seg_slots, float* state, float* o, int segments, int upto, cudaStream_t stream) {
     if (segments <= 0) return VK_OK;
     if (H <= 0 || dim <= 0 || vdim <= 0 || !(cap > 0.0f) || N < 2 * H * dim + 2 * H * vdim + 2 * H) return VK_BAD_SHAPE;
     if (dim > 256 || H > 65535 || segments > 65535) return VK_TOO_LARGE;
@@ -245,7 +247,7 @@ VK_API int vk_mlstm_recurrence(const float* proj, int N, int H, int dim, int vdi
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                                  \
         if (e != cudaSuccess) return (int)e;                                                                                                 \
         return launch_dependent(kern, grid, dim3(ML_THREADS), smem, stream, proj, N, H, dim, vdim, gate_bias, cap, qscale, seg_starts,       \
-                                seg_slots, state, state_floats, o, vec);                                                                     \
+                                seg_slots, state, state_floats, o, vec, upto);                                                                     \
     } while (0)
     if (dim <= 32) VK_MLSTM(4, 32);
     if (dim <= 64) VK_MLSTM(8, 32);
@@ -255,15 +257,15 @@ VK_API int vk_mlstm_recurrence(const float* proj, int N, int H, int dim, int vdi
 }
 
 VK_API int vk_mlstm_gate(const float* o, const float* proj, int N, int gate_off, const float* w, float eps, int H, int dim, int vdim, void* out,
-                         int tokens, const int32_t* seg_starts, const int32_t* seg_slots, float* state, int segments, int dtype,
-                         cudaStream_t stream) {
+                         int tokens, const int32_t* seg_starts, const int32_t* seg_slots, float* state, int segments, const int32_t* token_seg,
+                         int upto, int dtype, cudaStream_t stream) {
     if (tokens <= 0) return VK_OK;
     if (H <= 0 || dim <= 0 || vdim <= 0 || gate_off < 0 || gate_off + H * vdim > N || segments < 0) return VK_BAD_SHAPE;
     const size_t state_floats = (size_t)H * dim * vdim + (size_t)H * dim + H;
     const dim3 grid(tokens + segments);
     if (dtype == 0)
         return launch_dependent(mlstm_gate_kernel<float>, grid, dim3(256), 0, stream, o, proj, N, gate_off, w, eps, H, dim, vdim, (float*)out, tokens,
-                                seg_starts, seg_slots, state, state_floats);
+                                seg_starts, seg_slots, state, state_floats, token_seg, upto);
     return launch_dependent(mlstm_gate_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, o, proj, N, gate_off, w, eps, H, dim, vdim,
-                            (__nv_bfloat16*)out, tokens, seg_starts, seg_slots, state, state_floats);
+                            (__nv_bfloat16*)out, tokens, seg_starts, seg_slots, state, state_floats, token_seg, upto);
 }

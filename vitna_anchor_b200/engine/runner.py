@@ -102,6 +102,7 @@ class ModelRunner:
         self.steps_run = 0
         # A model is run from captured graphs only if every part of it says that a capture replays it faithfully.
         self.cuda_graphs = bool(cuda_graphs) and model.capture_safe
+        self._chunk_rules = list(getattr(model, "chunk_rules", ()))      # the parts' launches also depend on what these say of a step
         self._decode_graphs: "OrderedDict[tuple, tuple]" = OrderedDict()    # (batch bucket, context bucket) -> (graph, kernels)
         self._mixed_graphs: Dict[tuple, tuple] = {}                          # the counts of a mixed step -> (graph, logits, kernels)
         self._seen_shapes: Dict[tuple, int] = {}
@@ -362,6 +363,7 @@ class ModelRunner:
         key = ("mixed", T, len(entries), R, n_dec, n_tiles, n_big)
         ctx, rows = self.builder.build([(e.request_id, e.tokens, e.want) for e in entries], fixed_blocks=self.max_blocks,
                                        for_graph=True)
+        key += tuple(ctx.chunk_plan(r) for r in self._chunk_rules)
         out = self._logits_buffer()[:R] if R else None
         held = self._mixed_graphs.get(key)
         if held is not None:

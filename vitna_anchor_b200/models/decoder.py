@@ -24,7 +24,7 @@ from typing import List, Optional, Sequence
 import torch
 
 from ..cache.manager import CacheSpec
-from ..parts.base import Block, LogitsOutput, Norm, Part, PositionEncoding, StepContext, TokenInput
+from ..parts.base import Block, ChunkRule, LogitsOutput, Norm, Part, PositionEncoding, StepContext, TokenInput
 
 
 @dataclass(frozen=True)
@@ -99,6 +99,18 @@ class DecoderModel:
                 return False
             return all(safe(sub) for sub in vars(part).values() if isinstance(sub, Part))
         return all(safe(p) for p in self.parts() if p is not None) and (self.position is None or safe(self.position))
+
+    @property
+    def chunk_rules(self) -> List[ChunkRule]:
+        """The parts' rules for running segments in chunks, each once (Part.chunk_rule)."""
+        def of(part):
+            rule = getattr(part, "chunk_rule", None)
+            out = set() if rule is None else {rule}
+            for sub in vars(part).values():
+                if isinstance(sub, Part):
+                    out |= of(sub)
+            return out
+        return sorted(set().union(*(of(p) for p in self.parts() if p is not None)))
 
     def forward(self, ctx: StepContext, logit_rows: Optional[torch.Tensor], out: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
         """Run the batch; float32 logits [len(logit_rows), vocab] for the flat token indices in logit_rows

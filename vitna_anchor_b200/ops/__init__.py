@@ -1442,18 +1442,23 @@ def memory_chunked_takes(proj_width: int, dim: int, vdim: int, rank: int = 0) ->
     return bool(lib().vk_memory_chunked_takes(proj_width, dim, vdim, rank))
 
 
-def mlstm_chunked_scratch_bytes(tokens: int, segments: int, H: int, dim: int, vdim: int) -> int:
+ANY_LENGTH = 2 ** 31 - 1          # what the token-by-token kernels take for "segments of whatever length"
+
+
+def mlstm_chunked_scratch_bytes(tokens: int, segments: int, H: int, dim: int, vdim: int, chunked_from: int = 0) -> int:
     fn = lib().vk_mlstm_chunked_scratch_bytes
     fn.restype = ctypes.c_size_t
-    return int(fn(tokens, segments, H, dim, vdim))
+    return int(fn(tokens, segments, H, dim, vdim, chunked_from))
 
 
 def mlstm(proj: torch.Tensor, gate_bias: torch.Tensor, cap: float, norm_w: torch.Tensor, eps: float, ctx, state: torch.Tensor,
-          o: torch.Tensor, out: torch.Tensor, H: int, dim: int, vdim: int, chunk_scratch: Optional[torch.Tensor] = None) -> torch.Tensor:
+          o: torch.Tensor, out: torch.Tensor, H: int, dim: int, vdim: int, chunk_scratch: Optional[torch.Tensor] = None, chunked_from: int = 0,
+          others: bool = False) -> torch.Tensor:
     """proj float32 [T, N] = q | k | v | gate | a | b; the recurrence token after token per segment from and into `state`
     [slots, mlstm_state_floats]; o float32 [T, H * (vdim + 2)] receives each head's numerators, n . q and m;
     out [T, H * vdim] = o / rms(o) * norm_w * sigmoid(gate) in out's dtype.  With chunk_scratch (bytes, mlstm_chunked_scratch_bytes(T, segments, ...);
-    sizes that memory_chunked_takes) the recurrence runs in chunks of 64 tokens on the tensor cores, four launches, and o is not used."""
+    sizes that memory_chunked_takes) the segments of more than chunked_from tokens run in chunks of 64 tokens on the tensor cores, four launches; others:
+    there are shorter ones, which then run token after token (else o is not used)."""
     _req(proj, "proj", torch.float32, 2); _req(gate_bias, "gate_bias", torch.float32, 1); _req(norm_w, "norm_w", torch.float32, 1)
     _req(state, "state", torch.float32); _req(o, "o", torch.float32, 2); _req(out, "out", dims=2)
     T, N = proj.shape
@@ -1462,17 +1467,19 @@ def mlstm(proj: torch.Tensor, gate_bias: torch.Tensor, cap: float, norm_w: torch
         raise KernelError("mlstm: shapes do not fit the head counts")
     if chunk_scratch is not None:
         _req(chunk_scratch, "chunk_scratch", torch.uint8, 1)
-        if chunk_scratch.numel() < mlstm_chunked_scratch_bytes(T, ctx.num_segments, H, dim, vdim):
+        if chunk_scratch.numel() < mlstm_chunked_scratch_bytes(T, ctx.num_segments, H, dim, vdim, chunked_from):
             raise KernelError("mlstm: the scratch of the chunked form is too small")
         _check(lib().vk_mlstm_chunked(_p(proj), N, H, dim, vdim, _p(gate_bias), ctypes.c_float(cap), 2 * H * dim + H * vdim, _p(norm_w), ctypes.c_float(eps),
-                                      _p(ctx.seg_starts), _p(ctx.seg_slots), _p(state), _p(chunk_scratch), _p(out), T, ctx.num_segments, _dt(out), _stream()),
-               "mlstm_chunked")
+                                      _p(ctx.seg_starts), _p(ctx.seg_slots), _p(state), _p(chunk_scratch), _p(out), T, ctx.num_segments, chunked_from, _dt(out),
+                                      _stream()), "mlstm_chunked")
         add_launches(3)                                 # four kernels
-        return out
+        if not others:
+            return out
+    upto, token_seg = (ANY_LENGTH, None) if chunk_scratch is None else (chunked_from, ctx.token_seg)
     _check(lib().vk_mlstm_recurrence(_p(proj), N, H, dim, vdim, _p(gate_bias), ctypes.c_float(cap), _p(ctx.seg_starts), _p(ctx.seg_slots),
-                                     _p(state), _p(o), ctx.num_segments, _stream()), "mlstm_recurrence")
+                                     _p(state), _p(o), ctx.num_segments, upto, _stream()), "mlstm_recurrence")
     _check(lib().vk_mlstm_gate(_p(o), _p(proj), N, 2 * H * dim + H * vdim, _p(norm_w), ctypes.c_float(eps), H, dim, vdim, _p(out), T,
-                               _p(ctx.seg_starts), _p(ctx.seg_slots), _p(state), ctx.num_segments, _dt(out), _stream()), "mlstm_gate")
+                               _p(ctx.seg_starts), _p(ctx.seg_slots), _p(state), ctx.num_segments, _p(token_seg), upto, _dt(out), _stream()), "mlstm_gate")
     return out
 
 
@@ -1708,21 +1715,22 @@ def gla_max_dim() -> int:
     return int(lib().vk_gla_max_dim())
 
 
-def gla_chunked_scratch_bytes(tokens: int, segments: int, H: int, dim: int, vdim: int) -> int:
+def gla_chunked_scratch_bytes(tokens: int, segments: int, H: int, dim: int, vdim: int, chunked_from: int = 0) -> int:
     fn = lib().vk_gla_chunked_scratch_bytes
     fn.restype = ctypes.c_size_t
-    return int(fn(tokens, segments, H, dim, vdim))
+    return int(fn(tokens, segments, H, dim, vdim, chunked_from))
 
 
 def gla(proj: torch.Tensor, a_off: int, a2t: torch.Tensor, bias: torch.Tensor, tau: float, norm_w: torch.Tensor, eps: float, ctx,
         state: torch.Tensor, decay: torch.Tensor, o: torch.Tensor, out: torch.Tensor, H: int, dim: int, vdim: int, gate_off: int,
-        chunk_scratch: Optional[torch.Tensor] = None) -> torch.Tensor:
+        chunk_scratch: Optional[torch.Tensor] = None, chunked_from: int = 0, others: bool = False) -> torch.Tensor:
     """proj float32 [T, N] = q | k | v | ... with the gate's H vdim columns at gate_off and the decays' narrow half (rank = a2t.shape[0]
     columns) at a_off; a2t float32 [rank, H dim], bias [H dim]; the recurrence S <- diag(a) S + k v^T, o = S^T q dim^-1/2 token after token
     per segment from and into state [slots, H dim vdim]; decay float32 [T, H dim] and o float32 [T, H vdim] are scratch; out [T, H vdim] =
     o / rms(o) per head * norm_w [vdim] * silu(gate) in out's dtype.  A batch of single tokens takes one launch for decays and step.  With
-    chunk_scratch (bytes, gla_chunked_scratch_bytes(T, segments, ...); sizes that memory_chunked_takes) the recurrence runs in chunks of 64
-    tokens on the tensor cores, four launches, and decay and o are not used."""
+    chunk_scratch (bytes, gla_chunked_scratch_bytes(T, segments, ...); sizes that memory_chunked_takes) the segments of more than chunked_from tokens
+    run in chunks of 64 tokens on the tensor cores, four launches; others: there are shorter ones, which then run token after token (else decay
+    and o are not used)."""
     _req(proj, "proj", torch.float32, 2); _req(a2t, "a2t", torch.float32, 2); _req(bias, "bias", torch.float32, 1); _req(norm_w, "norm_w", torch.float32, 1)
     _req(state, "state", torch.float32); _req(decay, "decay", torch.float32, 2); _req(o, "o", torch.float32, 2); _req(out, "out", dims=2)
     T, N = proj.shape
@@ -1733,21 +1741,25 @@ def gla(proj: torch.Tensor, a_off: int, a2t: torch.Tensor, bias: torch.Tensor, t
     L = lib()
     if chunk_scratch is not None:
         _req(chunk_scratch, "chunk_scratch", torch.uint8, 1)
-        if chunk_scratch.numel() < gla_chunked_scratch_bytes(T, ctx.num_segments, H, dim, vdim):
+        if chunk_scratch.numel() < gla_chunked_scratch_bytes(T, ctx.num_segments, H, dim, vdim, chunked_from):
             raise KernelError("gla: the scratch of the chunked form is too small")
         _check(L.vk_gla_chunked(_p(proj), N, H, dim, vdim, a_off, rank, _p(a2t), _p(bias), ctypes.c_float(tau), gate_off, _p(norm_w), ctypes.c_float(eps),
-                                _p(ctx.seg_starts), _p(ctx.seg_slots), _p(state), _p(chunk_scratch), _p(out), T, ctx.num_segments, _dt(out), _stream()),
+                                _p(ctx.seg_starts), _p(ctx.seg_slots), _p(state), _p(chunk_scratch), _p(out), T, ctx.num_segments, chunked_from, _dt(out), _stream()),
                "gla_chunked")
         add_launches(3)                                 # four kernels
-        return out
+        if not others:
+            return out
+    upto, token_seg = (ANY_LENGTH, None) if chunk_scratch is None else (chunked_from, ctx.token_seg)
     if ctx.decode_only and not (proj.dtype == torch.float32 and out.dtype == torch.float32 and _float32_exact):
         _check(L.vk_gla_decode(_p(proj), N, H, dim, vdim, a_off, rank, _p(a2t), _p(bias), ctypes.c_float(tau), _p(ctx.seg_starts), _p(ctx.seg_slots),
                                _p(state), _p(o), ctx.num_segments, _stream()), "gla_decode")
     else:
-        _check(L.vk_gla_prepare(_p(proj), N, a_off, rank, _p(a2t), _p(bias), ctypes.c_float(tau), C, _p(decay), T, _stream()), "gla_prepare")
+        _check(L.vk_gla_prepare(_p(proj), N, a_off, rank, _p(a2t), _p(bias), ctypes.c_float(tau), C, _p(decay), T, _p(token_seg),
+                                _p(ctx.seg_starts), upto, _stream()), "gla_prepare")
         _check(L.vk_gla_recurrence(_p(proj), N, H, dim, vdim, _p(decay), _p(ctx.seg_starts), _p(ctx.seg_slots), _p(state), _p(o), ctx.num_segments,
-                                   _stream()), "gla_recurrence")
-    _check(L.vk_gla_gate(_p(o), _p(proj), N, gate_off, _p(norm_w), ctypes.c_float(eps), H, vdim, _p(out), T, _dt(out), _stream()), "gla_gate")
+                                   upto, _stream()), "gla_recurrence")
+    _check(L.vk_gla_gate(_p(o), _p(proj), N, gate_off, _p(norm_w), ctypes.c_float(eps), H, vdim, _p(out), T, _p(token_seg), _p(ctx.seg_starts), upto,
+                         _dt(out), _stream()), "gla_gate")
     return out
 
 

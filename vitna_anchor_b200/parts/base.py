@@ -9,7 +9,7 @@ do the sum in its epilogue (float32 either way).
 from __future__ import annotations
 
 from dataclasses import dataclass, field
-from typing import Callable, Dict, List, Optional, Sequence
+from typing import Callable, Dict, List, NamedTuple, Optional, Sequence, Tuple
 
 import torch
 
@@ -60,6 +60,22 @@ class GroupMeta:
     max_blocks: int
 
 
+class ChunkRule(NamedTuple):
+    """When a recurrence runs segments in chunks of 64 tokens side by side and not token after token; measured by the part that has it.
+
+    length: a step with a segment of more tokens than this does, and (total > 0) one whose segments of several tokens have `total` together and 48 each on
+    average.  a_single: a single decoded token beside them moves both lines up by so many tokens, since token after token its step hides behind the long
+    segment's chain.  few: fewer segments of up to SHORT_SEGMENT tokens than this go in chunks with the long ones (launches of their own would cost more), more
+    of them run token after token: a chunk costs a head's whole state four times through memory however few its tokens are."""
+    length: int
+    total: int = 0
+    a_single: int = 0
+    few: int = 1
+
+
+SHORT_SEGMENT = 32
+
+
 @dataclass
 class StepContext:
     """One batch: S segments (request, its next tokens), T tokens in all, flat and in segment order."""
@@ -96,17 +112,36 @@ class StepContext:
     extra: dict = field(default_factory=dict)
     after_run: Optional[Callable[[int], None]] = None    # called by the decoder after each run of its schedule (tests)
 
+    def chunk_plan(self, rule: ChunkRule) -> Optional[Tuple[int, bool]]:
+        """What of this step a recurrence with this rule runs in chunks: None (nothing), or the segments of more than the first number of tokens, and whether there are
+        others, which then run token after token.  One of the step's counts for a captured graph (Part.chunk_rule)."""
+        if rule not in self.extra:
+            self.extra[rule] = None
+            lens, more = self.host_seg_lens, rule.a_single * self.num_dec
+            portions = self.num_segments - self.num_dec
+            if not self.decode_only and (max(lens, default=0) > rule.length + more
+                                         or rule.total > 0 and self.num_pre >= max(rule.total + more, 48 * portions)):
+                short = sum(1 for n in lens if n <= SHORT_SEGMENT)
+                self.extra[rule] = (0, False) if short < rule.few else (SHORT_SEGMENT, True)
+        return self.extra[rule]
+
+
+def chunked_segments(ws: Workspace, rule: ChunkRule) -> int:
+    """The most segments that a step's chunks are of (scratch is laid out for them)."""
+    return min(ws.max_segments, ws.max_tokens // (SHORT_SEGMENT + 1) + rule.few)
+
 
 class Part:
     """Common base: a part may hold device tensors and says how many bytes of weights it reads per step.
 
     capture_safe: whether a CUDA graph captured from one batch replays this part faithfully for any other batch
-    with the same counts (tokens, segments, wanted rows, single-token segments, prompt tiles).  True means: the
-    part's launches and their arguments depend only on those counts, on its own constants and on the context's
+    with the same counts (tokens, segments, wanted rows, single-token segments, prompt tiles, and what
+    StepContext.chunk_plan says of its chunk_rule).  True means: the part's launches and their arguments depend only on those counts, on its own constants and on the context's
     device arrays (a padding segment of a decode batch has seg_slots -1 and slot mapping -1), and it neither
     synchronises nor allocates per batch.  A model with a part that says False is never captured."""
 
     capture_safe: bool = True
+    chunk_rule: Optional[ChunkRule] = None   # of a recurrence that runs long segments in chunks
 
     def weight_bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in self.tensors())
