@@ -160,3 +160,75 @@ def test_strong_decays_beside_weak_ones(dk, strong):
     assert np.abs(out.double().cpu().numpy().reshape(T, H, dv) - want).max() <= 2e-5 * np.abs(want).max()
     got = state[0, :H * dv * dk].double().cpu().numpy().reshape(H, dv, dk).transpose(0, 2, 1)
     assert np.abs(got - S).max() <= 2e-5 * max(1.0, np.abs(S).max())
+
+
+@pytest.mark.parametrize("lens", [(600, 1, 1, 32, 33, 1), (1, 161, 2), (33, 32, 700), (1, 1, 40, 1), (200,), (1200, 900)])
+@pytest.mark.parametrize("few", [1, 100])
+@pytest.mark.parametrize("channel,dk,dv", [(False, 16, 32), (False, 72, 132), (True, 16, 32), (True, 72, 36)])
+def test_a_step_of_segments_of_every_length(channel, dk, dv, lens, few, monkeypatch):
+    """Long segments in chunks, with short ones token after token or among them: all have the results and states of the token-by-token kernels, and those that run token
+    after token their bits."""
+    from vitna_anchor_b200.cache import CacheManager
+    from vitna_anchor_b200.engine.context import ContextBuilder
+    from vitna_anchor_b200.parts.base import StepContext, Workspace
+    from vitna_anchor_b200.parts.delta import ChannelDeltaRule, GatedDeltaRule
+    W, G, H, taps, rank, T = 64, 1, 2, 4, 4, sum(lens)
+    got = []
+    for plain in (False, True):
+        if plain:
+            monkeypatch.setattr(StepContext, "chunk_plan", lambda *a: None)
+        g = torch.Generator(device="cuda").manual_seed(dk)
+        r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+        m = lambda rows, cols: (r(rows, cols) * cols ** -0.5).bfloat16()
+        C = 2 * G * dk + H * dv
+        if channel:
+            part = ChannelDeltaRule(W, H, G, dk, dv, taps, m(C + H + 2 * rank, W), r(C, taps), 0.5 * r(H), r(H * dk) - 2, 0.5 * r(H * dk, rank), r(H * dv, rank), 1 + 0.1 * r(dv),
+                                    m(W, H * dv), 1e-6)
+        else:
+            part = GatedDeltaRule(W, H, G, dk, dv, taps, m(C + H * dv + 2 * H, W), r(C, taps), 0.5 * r(H), r(H) - 2, 1 + 0.1 * r(dv), m(W, H * dv), 1e-6)
+        cache = CacheManager([part.cache_spec()], page_size=16, num_pages=64, max_requests=len(lens), dtype=torch.bfloat16, device="cuda")
+        builder = ContextBuilder(cache, torch.bfloat16, Workspace(torch.device("cuda"), T, len(lens), 4096), max_batch_tokens=T, max_segments=len(lens), max_model_len=4096,
+                                 device="cuda")
+        for i in range(len(lens)):
+            cache.open(i)
+        cache.reserve_step([(i, n) for i, n in enumerate(lens)])
+        ctx, _ = builder.build([(i, [0] * n, []) for i, n in enumerate(lens)])
+        ctx.caches[0].state.copy_(0.1 * r(*ctx.caches[0].state.shape))
+        x, y = r(T, W).bfloat16(), torch.zeros(T, W, device="cuda")
+        part.chunk_rule = part.chunk_rule._replace(few=few)
+        assert plain or (ctx.chunk_plan(part.chunk_rule) is not None) == (max(lens) > 160)
+        part.forward(x, ctx, ctx.caches[0], y)
+        got.append((y, ctx.caches[0].state.clone(), ctx.host_seg_slots))
+    (y, st, slots), (want, want_st, _) = got
+    assert float((y - want).abs().max()) <= 2e-2 * float(want.abs().max())         # bfloat16 outputs of the heads in front of the last product
+    assert float((st - want_st).abs().max()) <= 2e-5 * max(1.0, float(want_st.abs().max()))
+    for n, slot in zip(lens, slots):
+        if n <= 32 and few == 1:
+            assert torch.equal(st[slot], want_st[slot]), n
+
+
+
+def test_a_captured_step_is_not_played_for_one_with_longer_segments(tmp_path):
+    """Two steps whose counts of tokens, requests and tiles are the same (70 + 60 and 100 + 30 tokens) take different launches, because only the second has a segment
+    long enough for chunks: the graph captured for the one must not be played for the other."""
+    import lupanex_models as LM
+    from vitna_anchor_b200.engine.loading import load_model
+    from vitna_anchor_b200.engine.runner import ModelRunner, StepEntry
+    model_dir = LM.make_model(str(tmp_path / "m"), "streams", 5)
+    rows = {}
+    for graphs in (True, False):
+        model = load_model(model_dir, "bfloat16", "cuda")
+        assert model.chunk_rules
+        runner = ModelRunner(model, page_size=16, num_pages=64, max_requests=2, max_batch_tokens=256, max_model_len=model.max_positions, device="cuda", cuda_graphs=graphs)
+        rng, got = np.random.default_rng(3), []
+        for lens in ((70, 60), (70, 60), (70, 60), (100, 30), (30, 100), (100, 30), (70, 60)):
+            for i, n in enumerate(lens):
+                runner.open(i)
+            ids = [rng.integers(0, model.vocab_size, n).tolist() for n in lens]
+            got.append(runner.step([StepEntry(i, t, [len(t) - 1]) for i, t in enumerate(ids)]).clone())
+            for i in range(2):
+                runner.close(i)
+        runner.check(sync=True)
+        rows[graphs] = torch.stack(got)
+        assert not graphs or runner.graph_replays > 0
+    assert float((rows[True] - rows[False]).abs().max()) <= 1e-5 * max(1.0, float(rows[False].abs().max()))        # the same launches either way

@@ -85,3 +85,29 @@ def test_the_plain_pieces():
     assert np.allclose(y[:, 0], [1, 12, 123, 234, 345])          # the last tap is the current token's, zeros before the start
     v = np.array([[3.0, 4.0]])
     assert np.allclose(PL.rms(v, 0.0), v / math.sqrt(12.5))
+
+
+def test_when_segments_run_in_chunks():
+    """What a step's launches hang on besides its counts of tokens and requests: what each rule says of it."""
+    import torch
+    from vitna_anchor_b200.parts.base import ChunkRule, StepContext
+    cfg = LM.CONFIGS["streams"]
+    arch = resolve(cfg)
+    made = {k: torch.from_numpy(v) for k, v in LM.make_tensors(cfg, 1, LM.REL_ROWS["streams"]).items()}
+    model = arch.build(arch.parse_config(cfg), made, torch.float32, "cpu")
+    rules = model.chunk_rules
+    assert rules == sorted({b.mixer.chunk_rule for b in model.blocks if getattr(b.mixer, "chunk_rule", None)}) and all(r.length == 80 for r in rules)
+
+    def plan(lens, **rule):
+        ctx = StepContext.__new__(StepContext)
+        ctx.host_seg_lens, ctx.num_segments, ctx.num_dec, ctx.extra = lens, len(lens), lens.count(1), {}
+        ctx.num_pre, ctx.decode_only = sum(lens) - ctx.num_dec, set(lens) == {1}
+        return ctx.chunk_plan(ChunkRule(**rule))
+
+    assert plan([60, 60], length=60) is None and plan([60, 60], length=59) == (0, False)
+    assert plan([60, 60], length=60, total=120) == (0, False) and plan([60, 60], length=60, total=121) is None
+    assert plan([40, 40, 40], length=60, total=100) is None                                       # under 48 each
+    # single tokens move both lines, and short segments that are not few go token after token
+    assert plan([1, 1, 60, 60], length=39, a_single=10) == (32, True) and plan([1, 1, 60, 60], length=40, a_single=10) is None
+    assert plan([1, 1, 60, 60], length=60, total=100, a_single=10, few=3) == (0, False) and plan([1, 1, 60, 60], length=60, total=101, a_single=10) is None
+    assert plan([32, 33, 90], length=80) == (32, True) and plan([33, 33, 90], length=80) == (0, False) and plan([1] * 100, length=0) is None

@@ -161,7 +161,7 @@ template <int KPT, int M>
 __global__ void __launch_bounds__(256) delta_recurrence_kernel(
     const float* __restrict__ prep, int P, const float* __restrict__ proj, const int32_t* __restrict__ seg_starts,
     const int32_t* __restrict__ seg_slots, float* __restrict__ state, size_t state_stride, size_t conv_off, float* __restrict__ o, int G, int H,
-    int dk, int dv, int taps, int R, int cols, int chunk, int vec) {
+    int dk, int dv, int taps, int R, int cols, int chunk, int vec, int upto) {
     extern __shared__ __align__(16) float sm[];
     const int seg = blockIdx.x, h = blockIdx.y, part = blockIdx.z, tid = threadIdx.x;
     dependency_wait();
@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(256) delta_recurrence_kernel(
     const int slot = seg_slots[seg];
     if (slot < 0) return;                                    // a padding segment of a captured batch
     const int start = seg_starts[seg], n = seg_starts[seg + 1] - start;
+    if (n > upto) return;
     const int C = 2 * G * dk + H * dv, N = C + H * dv + 2 * H;
     const int g = h / (H / G);
     const int dkp = R * KPT;                                 // dk rounded up to what the lanes hold (a power of two)
@@ -372,12 +373,14 @@ __global__ void __launch_bounds__(256) delta_recurrence_kernel(
 // A warp per (token, head): out = o / rms(o) * w * silu(gate).
 template <typename T>
 __global__ void __launch_bounds__(256) delta_gate_kernel(const float* __restrict__ o, const float* __restrict__ proj, const float* __restrict__ norm_w,
-                                                         float eps, T* __restrict__ out, int tokens, int G, int H, int dk, int dv) {
+                                                         float eps, T* __restrict__ out, int tokens, int G, int H, int dk, int dv,
+                                                         const int32_t* __restrict__ token_seg, const int32_t* __restrict__ seg_starts, int upto) {
     const int unit = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     dependency_wait();
     let_dependents_start();
     if (unit >= tokens * H) return;
     const int t = unit / H, h = unit % H;
+    if (token_seg && seg_starts[token_seg[t] + 1] - seg_starts[token_seg[t]] > upto) return;
     const int C = 2 * G * dk + H * dv, N = C + H * dv + 2 * H;
     const float* in = o + (size_t)unit * dv;
     const float* gate = proj + (size_t)t * N + C + (size_t)h * dv;
@@ -547,8 +550,10 @@ VK_API int vk_delta_prepare(const float* proj, const float* conv_w, const float*
                         seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps);
 }
 
+// Segments of more than `upto` tokens are left alone by this and by vk_delta_gate (vk_delta_chunked has them); vk_delta_gate then needs token_seg and
+// seg_starts, and null token_seg otherwise.
 VK_API int vk_delta_recurrence(const float* prep, const float* proj, const int32_t* seg_starts, const int32_t* seg_slots, float* state,
-                               size_t state_stride, float* o, int segments, int tokens, int G, int H, int dk, int dv, int taps,
+                               size_t state_stride, float* o, int segments, int upto, int tokens, int G, int H, int dk, int dv, int taps,
                                cudaStream_t stream) {
     if (segments <= 0) return VK_OK;
     if (G <= 0 || H <= 0 || H % G || dk <= 0 || dv <= 0 || taps < 1) return VK_BAD_SHAPE;
@@ -570,7 +575,7 @@ VK_API int vk_delta_recurrence(const float* prep, const float* proj, const int32
     while ((long long)segments * H * ((dv + cols - 1) / cols) < 148 && cols * R > 64 && cols % 2 == 0) cols /= 2;
     const int parts = (dv + cols - 1) / cols;
     const int threads = ((cols * R + 31) / 32) * 32;
-    const int longest = tokens > 0 ? tokens : 1;             // no segment is longer than the step
+    const int longest = upto < tokens ? (upto > 0 ? upto : 1) : (tokens > 0 ? tokens : 1);      // no segment is longer than the step
     const int M = longest > 1 ? 4 : 1;                       // tokens taken together (see the kernel)
     int chunk = 64;
     while (chunk > 8 && (chunk / 2 >= longest || (size_t)2 * chunk * (2 * R * kpt + cols + 2 + 2 * M) * sizeof(float) > 64 * 1024)) chunk /= 2;
@@ -582,9 +587,9 @@ VK_API int vk_delta_recurrence(const float* prep, const float* proj, const int32
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                     \
         if (tokens <= DR_DEPENDENT_TOKENS)                                                                                             \
             return launch_dependent(kern, dim3(segments, H, parts), dim3(threads), smem, stream, prep, P, proj, seg_starts, seg_slots, \
-                                    state, state_stride, (size_t)H * dv * dk, o, G, H, dk, dv, taps, R, cols, chunk, vec);            \
+                                    state, state_stride, (size_t)H * dv * dk, o, G, H, dk, dv, taps, R, cols, chunk, vec, upto);            \
         return launch_plain(kern, dim3(segments, H, parts), dim3(threads), smem, stream, prep, P, proj, seg_starts, seg_slots, state,  \
-                            state_stride, (size_t)H * dv * dk, o, G, H, dk, dv, taps, R, cols, chunk, vec);                           \
+                            state_stride, (size_t)H * dv * dk, o, G, H, dk, dv, taps, R, cols, chunk, vec, upto);                           \
     }
     if (M == 1) {
         if (kpt == 4) GO(4, 1) else if (kpt == 8) GO(8, 1) else if (kpt == 16) GO(16, 1) else GO(32, 1)
@@ -596,16 +601,16 @@ VK_API int vk_delta_recurrence(const float* prep, const float* proj, const int32
 }
 
 VK_API int vk_delta_gate(const float* o, const float* proj, const float* norm_w, float eps, void* out, int tokens, int G, int H, int dk, int dv,
-                         int dtype, cudaStream_t stream) {
+                         const int32_t* token_seg, const int32_t* seg_starts, int upto, int dtype, cudaStream_t stream) {
     if (tokens <= 0) return VK_OK;
     if (G <= 0 || H <= 0 || dk <= 0 || dv <= 0) return VK_BAD_SHAPE;
     const int grid = (tokens * H + 7) / 8;
     if (tokens <= DR_DEPENDENT_TOKENS) {
-        if (dtype == 0) return launch_dependent(delta_gate_kernel<float>, dim3(grid), dim3(256), 0, stream, o, proj, norm_w, eps, (float*)out, tokens, G, H, dk, dv);
-        return launch_dependent(delta_gate_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, stream, o, proj, norm_w, eps, (__nv_bfloat16*)out, tokens, G, H, dk, dv);
+        if (dtype == 0) return launch_dependent(delta_gate_kernel<float>, dim3(grid), dim3(256), 0, stream, o, proj, norm_w, eps, (float*)out, tokens, G, H, dk, dv, token_seg, seg_starts, upto);
+        return launch_dependent(delta_gate_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, stream, o, proj, norm_w, eps, (__nv_bfloat16*)out, tokens, G, H, dk, dv, token_seg, seg_starts, upto);
     }
-    if (dtype == 0) return launch_plain(delta_gate_kernel<float>, dim3(grid), dim3(256), 0, stream, o, proj, norm_w, eps, (float*)out, tokens, G, H, dk, dv);
-    return launch_plain(delta_gate_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, stream, o, proj, norm_w, eps, (__nv_bfloat16*)out, tokens, G, H, dk, dv);
+    if (dtype == 0) return launch_plain(delta_gate_kernel<float>, dim3(grid), dim3(256), 0, stream, o, proj, norm_w, eps, (float*)out, tokens, G, H, dk, dv, token_seg, seg_starts, upto);
+    return launch_plain(delta_gate_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, stream, o, proj, norm_w, eps, (__nv_bfloat16*)out, tokens, G, H, dk, dv, token_seg, seg_starts, upto);
 }
 
 // Whether the one-kernel form for single decoded tokens takes these sizes.

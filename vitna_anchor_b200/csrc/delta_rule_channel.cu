@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(1024) cdelta_prepare_kernel(
 template <int M>
 __global__ void __launch_bounds__(256) cdelta_groups_kernel(const float* __restrict__ prep, int P, const int32_t* __restrict__ token_seg,
                                                             const int32_t* __restrict__ seg_starts, float* __restrict__ grp, int tokens, int G,
-                                                            int H, int dk, int dv) {
+                                                            int H, int dk, int dv, int upto) {
     dependency_wait();
     let_dependents_start();
     const int unit = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(256) cdelta_groups_kernel(const float* __restr
     const int g = h / (H / G);
     const int seg = token_seg[t];
     const int first = seg_starts[seg], i = t - first, n = seg_starts[seg + 1] - first;
+    if (n > upto) return;
     const int p = i % M, t0 = t - p;
     const int gl = n - (i - p) < M ? n - (i - p) : M;           // tokens of this group
     const int C = 2 * G * dk + H * dv, dkr = (dk + 3) / 4 * 4, GW = 4 * dkr + 8;      // eight floats for the products whatever M is: rows stay 16-byte aligned
@@ -186,7 +187,7 @@ template <int KPT, int M>
 __global__ void __launch_bounds__(256) cdelta_recurrence_kernel(
     const float* __restrict__ prep, int P, const float* __restrict__ grp, const float* __restrict__ proj, int N,
     const int32_t* __restrict__ seg_starts, const int32_t* __restrict__ seg_slots, float* __restrict__ state, size_t state_stride,
-    size_t conv_off, float* __restrict__ o, int G, int H, int dk, int dv, int taps, int R, int cols, int chunk, int vec) {
+    size_t conv_off, float* __restrict__ o, int G, int H, int dk, int dv, int taps, int R, int cols, int chunk, int vec, int upto) {
     extern __shared__ __align__(16) float sm[];
     const int seg = blockIdx.x, h = blockIdx.y, part = blockIdx.z, tid = threadIdx.x;
     dependency_wait();
@@ -194,6 +195,7 @@ __global__ void __launch_bounds__(256) cdelta_recurrence_kernel(
     const int slot = seg_slots[seg];
     if (slot < 0) return;                                    // a padding segment of a captured batch
     const int start = seg_starts[seg], n = seg_starts[seg + 1] - start;
+    if (n > upto) return;
     const int C = 2 * G * dk + H * dv;
     const int dkp = R * KPT;                                 // dk rounded up to what the lanes hold (a power of two)
     const int dkr = (dk + 3) / 4 * 4, dkr4 = dkr / 4, dkp4 = dkp / 4, GW = 4 * dkr + 8;      // eight floats for the products whatever M is: rows stay 16-byte aligned
@@ -552,9 +554,9 @@ VK_API int vk_cdelta_prepare(const float* proj, const float* conv_w, const float
 VK_API size_t vk_cdelta_group_floats(int tokens, int H, int dk) { return (size_t)tokens * H * (4 * ((dk + 3) / 4 * 4) + 8); }
 
 // Two launches: the groups' vectors and products for all tokens side by side (into grp, vk_cdelta_group_floats), then the
-// recurrence, which also writes the state and the convolution's memory.
+// recurrence, which also writes the state and the convolution's memory.  Segments of more than `upto` tokens are left alone (vk_cdelta_chunked has them).
 VK_API int vk_cdelta_recurrence(const float* prep, const float* proj, int proj_width, const int32_t* token_seg, const int32_t* seg_starts,
-                                const int32_t* seg_slots, float* state, size_t state_stride, float* grp, float* o, int segments, int tokens,
+                                const int32_t* seg_slots, float* state, size_t state_stride, float* grp, float* o, int segments, int upto, int tokens,
                                 int G, int H, int dk, int dv, int taps, cudaStream_t stream) {
     if (segments <= 0 || tokens <= 0) return VK_OK;
     if (G <= 0 || H <= 0 || H % G || dk <= 0 || dv <= 0 || taps < 1) return VK_BAD_SHAPE;
@@ -567,10 +569,10 @@ VK_API int vk_cdelta_recurrence(const float* prep, const float* proj, int proj_w
     {
         const int grid = (tokens * H + 7) / 8;
         int rc;
-        if (M == 1) rc = dependent ? launch_dependent(cdelta_groups_kernel<1>, dim3(grid), dim3(256), 0, stream, prep, P, token_seg, seg_starts, grp, tokens, G, H, dk, dv)
-                                   : launch_plain(cdelta_groups_kernel<1>, dim3(grid), dim3(256), 0, stream, prep, P, token_seg, seg_starts, grp, tokens, G, H, dk, dv);
-        else rc = dependent ? launch_dependent(cdelta_groups_kernel<4>, dim3(grid), dim3(256), 0, stream, prep, P, token_seg, seg_starts, grp, tokens, G, H, dk, dv)
-                            : launch_plain(cdelta_groups_kernel<4>, dim3(grid), dim3(256), 0, stream, prep, P, token_seg, seg_starts, grp, tokens, G, H, dk, dv);
+        if (M == 1) rc = dependent ? launch_dependent(cdelta_groups_kernel<1>, dim3(grid), dim3(256), 0, stream, prep, P, token_seg, seg_starts, grp, tokens, G, H, dk, dv, upto)
+                                   : launch_plain(cdelta_groups_kernel<1>, dim3(grid), dim3(256), 0, stream, prep, P, token_seg, seg_starts, grp, tokens, G, H, dk, dv, upto);
+        else rc = dependent ? launch_dependent(cdelta_groups_kernel<4>, dim3(grid), dim3(256), 0, stream, prep, P, token_seg, seg_starts, grp, tokens, G, H, dk, dv, upto)
+                            : launch_plain(cdelta_groups_kernel<4>, dim3(grid), dim3(256), 0, stream, prep, P, token_seg, seg_starts, grp, tokens, G, H, dk, dv, upto);
         if (rc != 0) return rc;
     }
     int R = 1;
@@ -595,9 +597,9 @@ VK_API int vk_cdelta_recurrence(const float* prep, const float* proj, int proj_w
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                       \
         if (dependent)                                                                                                                   \
             return launch_dependent(kern, dim3(segments, H, parts), dim3(threads), smem, stream, prep, P, grp, proj, proj_width, seg_starts, \
-                                    seg_slots, state, state_stride, (size_t)H * dv * dk, o, G, H, dk, dv, taps, R, cols, chunk, vec);    \
+                                    seg_slots, state, state_stride, (size_t)H * dv * dk, o, G, H, dk, dv, taps, R, cols, chunk, vec, upto);    \
         return launch_plain(kern, dim3(segments, H, parts), dim3(threads), smem, stream, prep, P, grp, proj, proj_width, seg_starts,     \
-                            seg_slots, state, state_stride, (size_t)H * dv * dk, o, G, H, dk, dv, taps, R, cols, chunk, vec);            \
+                            seg_slots, state, state_stride, (size_t)H * dv * dk, o, G, H, dk, dv, taps, R, cols, chunk, vec, upto);            \
     }
     if (M == 1) {
         if (kpt == 4) GO(4, 1) else if (kpt == 8) GO(8, 1) else if (kpt == 16) GO(16, 1) else GO(32, 1)

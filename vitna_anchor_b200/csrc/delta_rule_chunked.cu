@@ -52,7 +52,7 @@ struct DcArgs {
     int P;                                  // floats of a row of prep
     const int32_t* seg_starts;
     const int32_t* seg_slots;
-    int segments;
+    int segments, from;                     // segments of up to `from` tokens are left alone
     float* scratch;
     int G, H, dk, dv;
 };
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
     float* sl = sT + DC_C * DC_LDA;                 // CH: [64][LDQ] the decays' logarithms, then k times what its sixteen leaves behind it
     float* vec = sl + (CH ? DC_C * LDQ : 0);        // CH: [4][DKP] what whole sixteens leave
     float* sv = vec + (CH ? 4 * DKP : 0);           // [64][LDV]
-    const Chunk ch = find_chunk<DC_C>(blockIdx.x, p.seg_starts, p.segments, find);
+    const Chunk ch = find_chunk<DC_C>(blockIdx.x, p.seg_starts, p.segments, find, p.from);
     if (ch.seg < 0 || p.seg_slots[ch.seg] < 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, wm = warp & 1, wn = warp >> 1;
     const int h = blockIdx.y, dk = p.dk, dv = p.dv, rows = ch.rows, kh = h / (p.H / p.G), Cq = 2 * p.G * dk + p.H * dv;
@@ -408,9 +408,9 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
     float* sU = sS + COLS * LDS;                    // [COLS][LDU]
     const int seg = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int slot = p.seg_slots[seg], start = p.seg_starts[seg], n = p.seg_starts[seg + 1] - start;
-    if (slot < 0 || n <= 0) return;
+    if (slot < 0 || n <= p.from) return;
     if (warp == 0) {
-        const int b = first_chunk_of<DC_C>(seg, p.seg_starts);
+        const int b = first_chunk_of<DC_C>(seg, p.seg_starts, p.from);
         if (lane == 0) {
             base_sh = b;
             failed = 0;
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(256) delta_chunk_out_kernel(const DcArgs p, bo
     float* sS = sQ + DC_C * LDQ;                    // [COLS columns][LDQ]
     float* sP = sS + COLS * LDQ;                    // [64][DC_LDA]
     float* sU = sP + DC_C * DC_LDA;                 // [64][LDU]
-    const Chunk ch = find_chunk<DC_C>(blockIdx.x, p.seg_starts, p.segments, find);
+    const Chunk ch = find_chunk<DC_C>(blockIdx.x, p.seg_starts, p.segments, find, p.from);
     if (ch.seg < 0 || p.seg_slots[ch.seg] < 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, m = warp & 3, half = warp >> 2, cw = (COLS / 2) * half;
     const int h = blockIdx.y, c0 = blockIdx.z * COLS, dk = p.dk, dv = p.dv;
@@ -725,16 +725,17 @@ __global__ void __launch_bounds__(256) delta_chunk_out_kernel(const DcArgs p, bo
 
 using namespace vk;
 
-static int dc_chunks(int tokens, int segments) { return tokens / DC_C + (segments < tokens ? segments : tokens); }
+static int dc_chunks(int tokens, int segments, int from) { return most_chunks(DC_C, tokens, segments, from); }
 
 // Whether the chunked kernels take these sizes (else the token-by-token kernel does the work).
 VK_API int vk_delta_chunked_takes(int G, int H, int dk, int dv, int taps) {
     return G > 0 && H > 0 && H % G == 0 && dk % 4 == 0 && dk >= 8 && dk <= 128 && dv > 0 && dv % 4 == 0 && dv <= 256 && taps >= 1 && taps <= DC_MAX_TAPS;
 }
 
-// Bytes of scratch for a step of `tokens` tokens in `segments` segments.
-VK_API size_t vk_delta_chunked_scratch_bytes(int tokens, int segments, int H, int dk, int dv) {
-    return (size_t)dc_chunks(tokens, segments) * H * dc_stride(dk, dv, false) * sizeof(float);
+// Bytes of scratch for a step of `tokens` tokens in `segments` segments (from: as for the kernels; the larger it is, the fewer chunks a step of many segments can
+// have, each with its operands and a head's whole state: 0.22 MB a head of 128 x 128).
+VK_API size_t vk_delta_chunked_scratch_bytes(int tokens, int segments, int H, int dk, int dv, int from) {
+    return (size_t)dc_chunks(tokens, segments, from) * H * dc_stride(dk, dv, false) * sizeof(float);
 }
 
 // Whether delta_chunk_out norms and gates the outputs itself (else the gate kernel follows): a head's values lie in one of its blocks.
@@ -763,7 +764,7 @@ template <int DKP, bool CH>
 static int delta_chunked_launch(const DcArgs& p, const float* proj, int proj_width, float* state, size_t state_stride, const DcOut& f, int tokens, int taps,
                                 int* error, cudaStream_t stream) {
     constexpr int COLS = DKP / 8;
-    const int chunks = dc_chunks(tokens, p.segments);
+    const int chunks = dc_chunks(tokens, p.segments, p.from);
     const int smem1 = (dc_prepare_floats_fixed<DKP, CH>() + DC_C * dc_ldv(p.dv)) * (int)sizeof(float);
     const int smem2 = (DC_STAGES * 2 * DC_C * (DKP + 8) + COLS * (DKP + 4) + COLS * (DC_C + 4)) * (int)sizeof(float);
     auto k1 = delta_chunk_prepare_kernel<DKP, CH>;
@@ -784,37 +785,37 @@ static int delta_chunked_launch(const DcArgs& p, const float* proj, int proj_wid
 
 template <bool CH>
 static int delta_chunked(const float* prep, int prep_width, const float* proj, int proj_width, const int32_t* seg_starts, const int32_t* seg_slots, float* state,
-                         size_t state_stride, const DcOut& f, float* scratch, int segments, int tokens, int G, int H, int dk, int dv, int taps, int* error,
-                         cudaStream_t stream) {
+                         size_t state_stride, const DcOut& f, float* scratch, int segments, int from, int tokens, int G, int H, int dk, int dv, int taps,
+                         int* error, cudaStream_t stream) {
     if (segments <= 0 || tokens <= 0) return VK_OK;
-    if (!vk_delta_chunked_takes(G, H, dk, dv, taps) || prep_width % 4 || !error || (f.norm_w && !vk_delta_chunked_gates(dv))) return VK_BAD_SHAPE;
+    if (!vk_delta_chunked_takes(G, H, dk, dv, taps) || prep_width % 4 || from < 0 || !error || (f.norm_w && !vk_delta_chunked_gates(dv))) return VK_BAD_SHAPE;
     if ((uintptr_t)scratch % 16 || (uintptr_t)prep % 16 || (uintptr_t)f.o % 8 || (f.norm_w && (uintptr_t)f.out % 4)) return VK_BAD_ALIGNMENT;
     if (H > 65535) return VK_TOO_LARGE;
-    const DcArgs p = {prep, prep_width, seg_starts, seg_slots, segments, scratch, G, H, dk, dv};
+    const DcArgs p = {prep, prep_width, seg_starts, seg_slots, segments, from, scratch, G, H, dk, dv};
     return dk <= 64 ? delta_chunked_launch<64, CH>(p, proj, proj_width, state, state_stride, f, tokens, taps, error, stream)
                     : delta_chunked_launch<128, CH>(p, proj, proj_width, state, state_stride, f, tokens, taps, error, stream);
 }
 
 // prep [tokens][prep width] as delta_prepare leaves it; proj as for the token-by-token kernel; three kernels.  norm_w null: o [tokens][H*dv] float32 gets the outputs.
-// Else (sizes that vk_delta_chunked_gates) out [tokens][H*dv] in dtype gets them as vk_delta_gate makes them.  error: as for vk_linear_tcgen05.
+// Segments of up to `from` tokens are left alone: their states and rows are for the token-by-token kernels.  norm_w given (sizes that vk_delta_chunked_gates): out [tokens][H*dv] in dtype gets them as vk_delta_gate makes them.  error: as for vk_linear_tcgen05.
 VK_API int vk_delta_chunked(const float* prep, int prep_width, const float* proj, const int32_t* seg_starts, const int32_t* seg_slots, float* state,
-                            size_t state_stride, float* o, float* scratch, const float* norm_w, float eps, void* out, int dtype, int segments, int tokens, int G,
-                            int H, int dk, int dv, int taps, int* error, cudaStream_t stream) {
+                            size_t state_stride, float* o, float* scratch, const float* norm_w, float eps, void* out, int dtype, int segments, int from,
+                            int tokens, int G, int H, int dk, int dv, int taps, int* error, cudaStream_t stream) {
     const int N = 2 * G * dk + 2 * H * dv + 2 * H;
     const DcOut f = {o, proj, N, 2 * G * dk + H * dv, norm_w, eps, out, dtype};
-    return delta_chunked<false>(prep, prep_width, proj, N, seg_starts, seg_slots, state, state_stride, f, scratch, segments, tokens, G, H, dk, dv, taps, error, stream);
+    return delta_chunked<false>(prep, prep_width, proj, N, seg_starts, seg_slots, state, state_stride, f, scratch, segments, from, tokens, G, H, dk, dv, taps, error, stream);
 }
 
 // The form with a decay per head and key channel: prep as cdelta_prepare leaves it, proj rows of proj_width floats (the
 // convolution's inputs first).  The sizes are those vk_delta_chunked_takes.
-VK_API size_t vk_cdelta_chunked_scratch_bytes(int tokens, int segments, int H, int dk, int dv) {
-    return (size_t)dc_chunks(tokens, segments) * H * dc_stride(dk, dv, true) * sizeof(float);
+VK_API size_t vk_cdelta_chunked_scratch_bytes(int tokens, int segments, int H, int dk, int dv, int from) {
+    return (size_t)dc_chunks(tokens, segments, from) * H * dc_stride(dk, dv, true) * sizeof(float);
 }
 
 VK_API int vk_cdelta_chunked(const float* prep, int prep_width, const float* proj, int proj_width, const int32_t* seg_starts,
-                             const int32_t* seg_slots, float* state, size_t state_stride, float* o, float* scratch, int segments, int tokens,
+                             const int32_t* seg_slots, float* state, size_t state_stride, float* o, float* scratch, int segments, int from, int tokens,
                              int G, int H, int dk, int dv, int taps, int* error, cudaStream_t stream) {
     const DcOut f = {o, nullptr, 0, 0, nullptr, 0.0f, nullptr, 0};
-    return delta_chunked<true>(prep, prep_width, proj, proj_width, seg_starts, seg_slots, state, state_stride, f, scratch, segments, tokens, G, H, dk, dv, taps,
+    return delta_chunked<true>(prep, prep_width, proj, proj_width, seg_starts, seg_slots, state, state_stride, f, scratch, segments, from, tokens, G, H, dk, dv, taps,
                                error, stream);
 }

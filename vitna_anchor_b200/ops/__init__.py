@@ -894,23 +894,24 @@ def delta_chunked_takes(G: int, H: int, dk: int, dv: int, taps: int) -> bool:
     return bool(lib().vk_delta_chunked_takes(G, H, dk, dv, taps))
 
 
-def delta_chunked_scratch_floats(tokens: int, segments: int, H: int, dk: int, dv: int) -> int:
+def delta_chunked_scratch_floats(tokens: int, segments: int, H: int, dk: int, dv: int, chunked_from: int = 0) -> int:
     fn = lib().vk_delta_chunked_scratch_bytes
     fn.restype = ctypes.c_size_t
-    return int(fn(tokens, segments, H, dk, dv)) // 4
+    return int(fn(tokens, segments, H, dk, dv, chunked_from)) // 4
 
 
 def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor, norm_w: torch.Tensor, eps: float,
                token_seg: torch.Tensor, seg_starts: torch.Tensor, seg_slots: torch.Tensor, state: torch.Tensor, prep: torch.Tensor,
                o: torch.Tensor, out: torch.Tensor, G: int, H: int, dk: int, dv: int, taps: int,
-               chunk_scratch: Optional[torch.Tensor] = None, single_tokens: bool = False) -> torch.Tensor:
+               chunk_scratch: Optional[torch.Tensor] = None, single_tokens: bool = False, chunked_from: int = 0, others: bool = False) -> torch.Tensor:
     """The gated delta rule on a batch of segments, from the projections to the input of the output projection.
     proj float32 [T, 2 G dk + 2 H dv + 2 H] = q | k | v | gate | b | a;  conv_w float32 [2 G dk + H dv, taps];  a_log, dt_bias [H];
     norm_w [dv];  state float32 [slots, delta_state_floats];  prep [T, delta_prep_width] and o [T, H dv] float32 scratch;
     out [T, H dv] in the compute dtype.  Three launches: prepare, recurrence (which also writes the state), gate.  With
-    chunk_scratch (float32, delta_chunked_scratch_floats(T, segments, ...)) the recurrence runs in its chunked form, three launches:
+    chunk_scratch (float32, delta_chunked_scratch_floats(T, segments, ...)) the segments of more than chunked_from tokens run in chunks, three launches:
     what does not need the state for all chunks side by side, then the chunks of every request in order, then the outputs side by side
-    (normed and gated there where vk_delta_chunked_gates(dv); o is then not used).  With single_tokens
+    (normed and gated there where vk_delta_chunked_gates(dv); o is then not used for them); others: there are shorter ones, which then run token
+    after token.  With single_tokens
     (every segment is one token; sizes that delta_decode_takes) everything is ONE launch."""
     C = 2 * G * dk + H * dv
     _req(proj, "proj", torch.float32, 2); _req(conv_w, "conv_w", torch.float32, 2); _req(a_log, "a_log", torch.float32, 1)
@@ -931,19 +932,21 @@ def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt
                                   _p(prep), T, G, H, dk, dv, taps, _stream()), "delta_prepare")
     if chunk_scratch is not None:
         _req(chunk_scratch, "chunk_scratch", torch.float32, 1)
-        if chunk_scratch.numel() < delta_chunked_scratch_floats(T, S, H, dk, dv):
+        if chunk_scratch.numel() < delta_chunked_scratch_floats(T, S, H, dk, dv, chunked_from):
             raise KernelError("delta_rule: the scratch of the chunked form is too small")
         gated_here = bool(lib().vk_delta_chunked_gates(dv))
         _check(lib().vk_delta_chunked(_p(prep), prep.shape[1], _p(proj), _p(seg_starts), _p(seg_slots), _p(state), stride, _p(o), _p(chunk_scratch),
-                                      _p(norm_w if gated_here else None), ctypes.c_float(eps), _p(out), _dt(out), S, T, G, H, dk, dv, taps, _p(error_word()),
-                                      _stream()), "delta_chunked")
+                                      _p(norm_w if gated_here else None), ctypes.c_float(eps), _p(out), _dt(out), S, chunked_from, T, G, H, dk, dv, taps,
+                                      _p(error_word()), _stream()), "delta_chunked")
         add_launches(2)                             # three kernels
-        if gated_here:
+        if gated_here and not others:
             return out
-    else:
-        _check(lib().vk_delta_recurrence(_p(prep), _p(proj), _p(seg_starts), _p(seg_slots), _p(state), stride, _p(o), S, T, G, H, dk, dv, taps,
-                                         _stream()), "delta_recurrence")
-    _check(lib().vk_delta_gate(_p(o), _p(proj), _p(norm_w), ctypes.c_float(eps), _p(out), T, G, H, dk, dv, _dt(out), _stream()), "delta_gate")
+    if chunk_scratch is None or others:
+        _check(lib().vk_delta_recurrence(_p(prep), _p(proj), _p(seg_starts), _p(seg_slots), _p(state), stride, _p(o), S,
+                                         ANY_LENGTH if chunk_scratch is None else chunked_from, T, G, H, dk, dv, taps, _stream()), "delta_recurrence")
+    short_alone = chunk_scratch is not None and gated_here
+    _check(lib().vk_delta_gate(_p(o), _p(proj), _p(norm_w), ctypes.c_float(eps), _p(out), T, G, H, dk, dv, _p(token_seg if short_alone else None), _p(seg_starts),
+                               chunked_from, _dt(out), _stream()), "delta_gate")
     return out
 
 
@@ -1205,10 +1208,10 @@ def channel_delta_group_floats(tokens: int, H: int, dk: int) -> int:
     return tokens * H * (4 * ((dk + 3) // 4 * 4) + 8)
 
 
-def channel_delta_chunked_scratch_floats(tokens: int, segments: int, H: int, dk: int, dv: int) -> int:
+def channel_delta_chunked_scratch_floats(tokens: int, segments: int, H: int, dk: int, dv: int, chunked_from: int = 0) -> int:
     fn = lib().vk_cdelta_chunked_scratch_bytes
     fn.restype = ctypes.c_size_t
-    return int(fn(tokens, segments, H, dk, dv)) // 4
+    return int(fn(tokens, segments, H, dk, dv, chunked_from)) // 4
 
 
 def channel_delta_decode_takes(G: int, H: int, dk: int, dv: int, taps: int, ra: int, rg: int) -> bool:
@@ -1220,16 +1223,16 @@ def channel_delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Te
                        g2t: torch.Tensor, norm_w: torch.Tensor, eps: float, token_seg: torch.Tensor, seg_starts: torch.Tensor,
                        seg_slots: torch.Tensor, state: torch.Tensor, prep: torch.Tensor, groups: torch.Tensor, o: torch.Tensor, out: torch.Tensor,
                        G: int, H: int, dk: int, dv: int, taps: int, single_tokens: bool = False,
-                       chunk_scratch: Optional[torch.Tensor] = None) -> torch.Tensor:
+                       chunk_scratch: Optional[torch.Tensor] = None, chunked_from: int = 0, others: bool = False) -> torch.Tensor:
     """The delta rule whose decay differs by head and key channel, from the projections to the input of the output projection.
     proj float32 [T, 2 G dk + H dv + H + ra + rg] = q | k | v | b | a1 | g1;  a2t float32 [ra, H dk] and g2t [rg, H dv], the wide
     halves of the two low-rank projections, transposed;  dt_bias [H dk];  a_log [H];  norm_w [dv];  state float32
     [slots, delta_state_floats];  prep [T, channel_delta_prep_width], groups (flat, channel_delta_group_floats(T, H, dk)) and o [T, H dv]
     float32 scratch;  out [T, H dv] in the compute dtype.  Four launches: prepare, what the groups of tokens need besides the state
     (all groups side by side), the recurrence (which also writes the state), gate.  With chunk_scratch (float32,
-    channel_delta_chunked_scratch_floats(T, segments, ...); sizes that delta_chunked_takes) the recurrence runs in its chunked form
-    instead: what does not need the state for all chunks side by side, then the chunks of every request in order.  With
-    single_tokens (every segment is one token; sizes that channel_delta_decode_takes) everything is ONE launch."""
+    channel_delta_chunked_scratch_floats(T, segments, ...); sizes that delta_chunked_takes) the segments of more than chunked_from tokens run in
+    chunks instead: what does not need the state for all chunks side by side, then the chunks of every request in order, then the
+    outputs; others: there are shorter ones, which then run in groups as ever.  With single_tokens (every segment is one token; sizes that channel_delta_decode_takes) everything is ONE launch."""
     C = 2 * G * dk + H * dv
     for name, t, d in (("proj", proj, 2), ("conv_w", conv_w, 2), ("a_log", a_log, 1), ("dt_bias", dt_bias, 1), ("a2t", a2t, 2), ("g2t", g2t, 2),
                        ("norm_w", norm_w, 1), ("state", state, 2), ("prep", prep, 2), ("o", o, 2), ("groups", groups, 1)):
@@ -1254,14 +1257,15 @@ def channel_delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Te
                                    _p(state), stride, _p(prep), T, G, H, dk, dv, taps, ra, rg, _stream()), "cdelta_prepare")
     if chunk_scratch is not None:
         _req(chunk_scratch, "chunk_scratch", torch.float32, 1)
-        if chunk_scratch.numel() < channel_delta_chunked_scratch_floats(T, S, H, dk, dv):
+        if chunk_scratch.numel() < channel_delta_chunked_scratch_floats(T, S, H, dk, dv, chunked_from):
             raise KernelError("channel_delta_rule: the scratch of the chunked form is too small")
         _check(lib().vk_cdelta_chunked(_p(prep), prep.shape[1], _p(proj), proj.shape[1], _p(seg_starts), _p(seg_slots), _p(state), stride, _p(o),
-                                       _p(chunk_scratch), S, T, G, H, dk, dv, taps, _p(error_word()), _stream()), "cdelta_chunked")
+                                       _p(chunk_scratch), S, chunked_from, T, G, H, dk, dv, taps, _p(error_word()), _stream()), "cdelta_chunked")
         add_launches(2)                             # three kernels
-    else:
+    if chunk_scratch is None or others:
         _check(lib().vk_cdelta_recurrence(_p(prep), _p(proj), proj.shape[1], _p(token_seg), _p(seg_starts), _p(seg_slots), _p(state), stride,
-                                          _p(groups), _p(o), S, T, G, H, dk, dv, taps, _stream()), "cdelta_recurrence")
+                                          _p(groups), _p(o), S, ANY_LENGTH if chunk_scratch is None else chunked_from, T, G, H, dk, dv, taps, _stream()),
+               "cdelta_recurrence")
         add_launches(1)                             # two kernels
     _check(lib().vk_cdelta_gate(_p(o), _p(prep), _p(norm_w), ctypes.c_float(eps), _p(out), T, G, H, dk, dv, _dt(out), _stream()), "cdelta_gate")
     return out

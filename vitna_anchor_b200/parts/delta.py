@@ -21,12 +21,10 @@ import torch
 
 from .. import ops
 from ..cache.manager import LayerCacheView, StateSpec
-from .base import Mixer, StepContext
+from .base import ChunkRule, Mixer, StepContext, chunked_segments
 
 
 class GatedDeltaRule(Mixer):
-    CHUNKED_FROM = 64       # steps of more tokens than this run the recurrence in chunks
-
     def __init__(self, hidden: int, num_heads: int, num_key_heads: int, key_dim: int, value_dim: int, taps: int, w_in: torch.Tensor,
                  conv: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor, norm_weight: torch.Tensor, wo: torch.Tensor, eps: float):
         """w_in: the projections stacked by rows, q | k | v | g | b | a ([2 G dk + 2 H dv + 2 H, hidden], compute dtype);
@@ -44,6 +42,10 @@ class GatedDeltaRule(Mixer):
         f32 = lambda t: t.to(torch.float32).contiguous()
         self.conv, self.a_log, self.dt_bias, self.norm_weight = f32(conv), f32(a_log), f32(dt_bias), f32(norm_weight)
         self.channels = C
+        # Measured, us a mixer, token after token / in chunks, 9 heads of 64 x 64 and 16 of 128 x 128:  one segment of 72: 50 / 52, 79 / 90; of 88: 55 / 52, 84 / 90; of 104:
+        # 61 / 52, 92 / 90;  four of 64: 49 / 53, 121 / 116;  sixteen of 64: 68 / 81, 345 / 286; of 32: 45 / 73, 193 / 254;  one of 512 beside 32 single tokens: all in chunks
+        # 113, 500, the single ones token after token 85, 210.
+        self.chunk_rule = ChunkRule(80 if dk <= 64 else 100, total=(1 << 19) // (H * dv), few=max(1, 294912 // (H * dk * dv)))
 
     def tensors(self):
         return [self.w_in, self.conv, self.a_log, self.dt_bias, self.norm_weight, self.wo]
@@ -57,17 +59,15 @@ class GatedDeltaRule(Mixer):
             raise ValueError("a recurrent mixer has no cache that another run could read")
         T, ws = ctx.num_tokens, ctx.workspace
         proj = ops.linear(xn, self.w_in, ws.rows("delta.proj", T, self.w_in.shape[0], torch.float32), ops.LINEAR_F32)
-        # a prompt's step takes the chunked form (the exact 32-bit routing keeps one kernel for every step)
-        scratch = None
-        if (T > self.CHUNKED_FROM and not (ctx.dtype == torch.float32 and ops.float32_exact())
-                and ops.delta_chunked_takes(self.G, self.H, self.dk, self.dv, self.taps)):
-            scratch = ws.flat(f"delta.chunks/{self.H}/{self.dk}/{self.dv}",
-                              ops.delta_chunked_scratch_floats(ws.max_tokens, ws.max_segments, self.H, self.dk, self.dv), torch.float32)
+        # long segments take the chunked form (the exact 32-bit routing keeps one kernel for every step)
+        serving = not (ctx.dtype == torch.float32 and ops.float32_exact())
+        plan = ctx.chunk_plan(self.chunk_rule) if serving and ops.delta_chunked_takes(self.G, self.H, self.dk, self.dv, self.taps) else None
+        scratch = None if plan is None else ws.flat(f"delta.chunks/{self.H}/{self.dk}/{self.dv}",
+                                                    ops.delta_chunked_scratch_floats(ws.max_tokens, chunked_segments(ws, self.chunk_rule), self.H, self.dk, self.dv), torch.float32)
         out = ops.delta_rule(proj, self.conv, self.a_log, self.dt_bias, self.norm_weight, self.eps, ctx.token_seg, ctx.seg_starts,
                              ctx.seg_slots, cache.state, ws.rows("delta.prep", T, ops.delta_prep_width(self.G, self.H, self.dk, self.dv), torch.float32),
                              ws.rows("delta.o", T, self.H * self.dv, torch.float32), ws.rows("delta.out", T, self.H * self.dv, ctx.dtype),
-                             self.G, self.H, self.dk, self.dv, self.taps, chunk_scratch=scratch,
-                             single_tokens=ctx.decode_only and not (ctx.dtype == torch.float32 and ops.float32_exact()))
+                             self.G, self.H, self.dk, self.dv, self.taps, scratch, ctx.decode_only and serving, *(plan or ()))
         ops.linear(out, self.wo, residual, ops.LINEAR_ACC_F32)
 
 
@@ -103,6 +103,9 @@ class ChannelDeltaRule(Mixer):
         self.w_in, self.wo = w_in.contiguous(), wo.contiguous()
         f32 = lambda t: t.to(torch.float32).contiguous()
         self.conv, self.a_log, self.dt_bias, self.norm_weight = f32(conv), f32(a_log), f32(dt_bias), f32(norm_weight)
+        # Measured, us a mixer, in groups of four tokens / in chunks, 9 heads of 64 x 64 and 16 of 128 x 128:  one segment of 112: 82 / 85, 146 / 161; of 136: 90 / 87,
+        # 157 / 165; of 176: 100 / 87, 172 / 165;  eight of 100: 94 / 106, 306 / 330;  one of 512 beside 32 single tokens: all in chunks 158, 693, the single ones apart 118, 280.
+        self.chunk_rule = ChunkRule(124 if dk <= 64 else 160, few=max(1, 294912 // (H * dk * dv)))
         self.a2t, self.g2t = f32(w_a2.to(torch.float32).t()), f32(w_g2.to(torch.float32).t())
 
     def tensors(self):
@@ -118,16 +121,16 @@ class ChannelDeltaRule(Mixer):
         T, ws = ctx.num_tokens, ctx.workspace
         proj = ops.linear(xn, self.w_in, ws.rows("cdelta.proj", T, self.w_in.shape[0], torch.float32), ops.LINEAR_F32)
         serving = not (ctx.dtype == torch.float32 and ops.float32_exact())
-        # a prompt's step takes the chunked form (the exact 32-bit routing keeps one set of kernels for every step)
-        scratch = None
-        if T > GatedDeltaRule.CHUNKED_FROM and serving and ops.delta_chunked_takes(self.G, self.H, self.dk, self.dv, self.taps):
-            scratch = ws.flat(f"cdelta.chunks/{self.H}/{self.dk}/{self.dv}",
-                              ops.channel_delta_chunked_scratch_floats(ws.max_tokens, ws.max_segments, self.H, self.dk, self.dv), torch.float32)
+        # long segments take the chunked form (the exact 32-bit routing keeps one set of kernels for every step)
+        plan = ctx.chunk_plan(self.chunk_rule) if serving and ops.delta_chunked_takes(self.G, self.H, self.dk, self.dv, self.taps) else None
+        scratch = None if plan is None else ws.flat(f"cdelta.chunks/{self.H}/{self.dk}/{self.dv}",
+                                                    ops.channel_delta_chunked_scratch_floats(ws.max_tokens, chunked_segments(ws, self.chunk_rule), self.H, self.dk, self.dv),
+                                                    torch.float32)
         out = ops.channel_delta_rule(proj, self.conv, self.a_log, self.dt_bias, self.a2t, self.g2t, self.norm_weight, self.eps, ctx.token_seg,
                                      ctx.seg_starts, ctx.seg_slots, cache.state,
                                      ws.rows("cdelta.prep", T, ops.channel_delta_prep_width(self.G, self.H, self.dk, self.dv), torch.float32),
                                      ws.flat(f"cdelta.groups/{self.H}/{self.dk}", ops.channel_delta_group_floats(ws.max_tokens, self.H, self.dk),
                                              torch.float32),
                                      ws.rows("delta.o", T, self.H * self.dv, torch.float32), ws.rows("delta.out", T, self.H * self.dv, ctx.dtype),
-                                     self.G, self.H, self.dk, self.dv, self.taps, single_tokens=ctx.decode_only and serving, chunk_scratch=scratch)
+                                     self.G, self.H, self.dk, self.dv, self.taps, ctx.decode_only and serving, scratch, *(plan or ()))
         ops.linear(out, self.wo, residual, ops.LINEAR_ACC_F32)
