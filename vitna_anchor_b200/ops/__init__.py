@@ -1033,10 +1033,23 @@ def attention_prefill_tcgen05_dims(q: torch.Tensor, cache_layer: torch.Tensor, b
         raise KernelError("attention_prefill_tcgen05_dims: shapes do not fit the head counts")
     if not attention_prefill_tcgen05_dims_takes(q, cache_layer, out, hd, vd, page_size):
         raise KernelError("attention_prefill_tcgen05_dims: bfloat16, keys and values of 64 and 128 values (not both 64) and pages of 8, 16, 32 or a multiple of 64 slots only")
+    return _prefill_tcgen05_dims(q, cache_layer, block_tables, tiles, out, out_ld, nh, nkv, hd, vd, page_size, scale, window, gate, gate_ld)
+
+
+def _prefill_tcgen05_dims(q, cache_layer, block_tables, tiles, out, out_ld, nh, nkv, hd, vd, page_size, scale, window, gate, gate_ld):
+    """The launch alone, for operands that have been looked at."""
     _check(lib().vk_attention_prefill_tcgen05_dims(_p(q), _p(cache_layer), _p(block_tables), _p(tiles), _p(out), q.shape[0], tiles.shape[0], cache_layer.shape[0],
                                                    nh, nkv, hd, vd, page_size, block_tables.shape[1], ctypes.c_float(scale), window, out_ld, _p(gate), gate_ld,
                                                    _p(error_word()), _stream()), "attention_prefill_tcgen05_dims")
     return out
+
+
+def prefill_tcgen05_dims_pays(ctx, hd: int) -> bool:
+    """Whether a step's prompt portions are long enough for attention_prefill_tcgen05_dims: its tiles are 128 rows (half as many blocks as attention_prefill_biased
+    makes) and a block of its is longer to set up.  By the step's counts alone, so the portions' average length.  Measured, us a mixer, that kernel / this one, nothing
+    cached before:  8 heads of 64 x 128:  one portion of 32 tokens 16.1 / 16.9, of 128 27.2 / 27.5, of 200 31.2 / 29.7; four of 100 27.9 / 28.4, of 200 35.3 / 32.8;
+    16 heads of 128 x 128:  one of 16 25.1 / 26.7, of 40 27.6 / 27.9, of 65 37.4 / 37.1; four of 100 45.9 / 40.2."""
+    return ctx.num_pre > (128 if hd == 64 else 48) * max(1, ctx.num_segments - ctx.num_dec)
 
 
 def attention_biased(q: torch.Tensor, pages: torch.Tensor, meta, ctx, out: torch.Tensor, nh: int, nkv: int, hd: int, vd: int,
@@ -1063,8 +1076,12 @@ def attention_biased(q: torch.Tensor, pages: torch.Tensor, meta, ctx, out: torch
         attention_decode_biased(q, pages, meta.block_tables, ctx.token_seg, ctx.positions, out, scratch, cap, nh, nkv, hd, vd, page_size,
                                 scale, layout, min(layout, max(1, ctx.max_context)), window, dist_bias, ctx.dec_tokens, v_in_key, v_share, gate)
     if (pre_ok and dist_bias is None and not v_in_key and v_share == 1 and getattr(ctx, "pre_tiles_big", None) is not None
-            and attention_prefill_tcgen05_dims_takes(q, pages, out, hd, vd, page_size)):
-        attention_prefill_tcgen05_dims(q, pages, meta.block_tables, ctx.pre_tiles_big, out, nh, nkv, hd, vd, page_size, scale, window, gate)
+            and prefill_tcgen05_dims_pays(ctx, hd) and attention_prefill_tcgen05_dims_takes(q, pages, out, hd, vd, page_size)):
+        T = q.shape[0]
+        out_ld, gate_ld = _out_rows(out, torch.bfloat16, T, nh * vd, "attention_biased"), _gate_rows(gate, T, nh, "attention_biased")
+        if not (q.is_cuda and pages.is_cuda) or q.shape[1] != nh * hd or _page_size_of(pages, nkv, hd, vd) != page_size:
+            raise KernelError("attention_biased: shapes do not fit the head counts")
+        _prefill_tcgen05_dims(q, pages, meta.block_tables, ctx.pre_tiles_big, out, out_ld, nh, nkv, hd, vd, page_size, scale, window, gate, gate_ld)
     elif pre_ok:
         attention_prefill_biased(q, pages, meta.block_tables, ctx.pre_tiles, out, nh, nkv, hd, vd, page_size, scale, window, dist_bias, v_in_key, v_share,
                                  gate)
