@@ -1004,9 +1004,9 @@ VK_API int vk_attention_prefill_tcgen05(const void* q, const void* cache, const 
     const long long cache_rows = (long long)pages * 2 * nkv * page_size;
     if (cache_rows >= (1ll << 31)) return VK_TOO_LARGE;
     if (((uintptr_t)q % 16) || ((uintptr_t)cache % 16) || ((uintptr_t)out % 16) || ((uintptr_t)scratch % 16)) return VK_BAD_ALIGNMENT;
-    CUtensorMap mq, mkv;
+    const int box_rows = page_size < AT_BN ? page_size : AT_BN;
+    CUtensorMap mq;
     if (!at_make_map(&mq, q, n_tokens, nh * hd, (long long)nh * hd, AT_BM)) return VK_BAD_SHAPE;
-    if (!at_make_map(&mkv, cache, cache_rows, hd, hd, page_size < AT_BN ? page_size : AT_BN)) return VK_BAD_SHAPE;
     const size_t max_parts = (size_t)((max_context - 1) / AT_BN) / AT_PART + 1;
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     AtScratch sc;
@@ -1031,6 +1031,8 @@ VK_API int vk_attention_prefill_tcgen05(const void* q, const void* cache, const 
     const int forced_kernel = prefill_streams_mode();
     const long long blocks = (long long)n_tiles * sc.parts * nh;
     if (forced_kernel == 1 || (forced_kernel == 2 && blocks < 370)) {
+        CUtensorMap mkv;
+        if (!at_make_map(&mkv, cache, cache_rows, hd, hd, box_rows)) return VK_BAD_SHAPE;
         const size_t smem2 = (size_t)AT_BM * 64 * 2 + 2 * AS_STAGES * AT_BN * 64 * 2 + 4 * AT_BM * AT_BN * 2 + 1024 + 256;
         auto kern2 = attention_prefill_streams_kernel<64>;
         cudaError_t e2 = cudaFuncSetAttribute(kern2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
@@ -1039,7 +1041,6 @@ VK_API int vk_attention_prefill_tcgen05(const void* q, const void* cache, const 
                             nh, nkv, page_size, max_blocks, scale, window, wait_ctl(error, WAIT_FAMILY_ATTENTION_PREFILL), sc);
     }
     CUtensorMap mk, mv;
-    const int box_rows = page_size < AT_BN ? page_size : AT_BN;
     const long long page_elems = 2ll * nkv * page_size * hd;
     if (!at_make_page_map(&mk, cache, hd, nkv * page_size, pages, page_elems, box_rows) ||
         !at_make_page_map(&mv, (const __nv_bfloat16*)cache + (size_t)nkv * page_size * hd, hd, nkv * page_size, pages, page_elems, box_rows))
