@@ -462,7 +462,9 @@ __global__ void __launch_bounds__(DKP * 2) delta_chunk_scan_kernel(const DcArgs 
         if (!mbar_wait(&full[c % DC_STAGES], (c / DC_STAGES) & 1, wc.cycles)) give_up(wc.error, &failed, 61);
         __syncthreads();                            // the chunk's operands are there, the state's slice is written, and everybody has left the chunk before
         if (*reinterpret_cast<volatile int*>(&failed)) {        // the same for every thread: all have written it before the barrier or nobody has
-            __nanosleep(200000);                    // let copies in flight land
+            // this chunk's copy and the next one's may be in flight: they land before the block's memory goes, or the limit runs out again
+            for (int d = c; d < chunks && d < c + 2; d++)
+                if (d != wc.skip_stage) mbar_wait(&full[d % DC_STAGES], (d / DC_STAGES) & 1, wc.cycles);
             return;
         }
         if (tid == 0) issue(c + 2);
