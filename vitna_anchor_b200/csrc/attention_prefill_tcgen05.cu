@@ -128,8 +128,8 @@ __device__ __forceinline__ void at_probabilities8(const uint32_t* s, uint64_t sc
 
 // DBUF: two buffers of probabilities (132 KB of shared memory, one block a multiprocessor) instead of one (96 KB, two
 // blocks): the softmax warps then write a step's probabilities while the tensor core still reads the step's before.
-// Measured, that loses where two blocks can share a multiprocessor, and where they cannot the kernel with two streams
-// further down is faster still: only the form with one buffer is launched.
+// Measured, that loses where two blocks can share a multiprocessor, so keys and values of 64 values each, and 64 x 128, have one buffer (where few blocks of 64 x 64 make
+// it pay, the kernel with two streams further down is faster still); 128 x 128 and 128 x 64 leave room for one block, which takes two.
 //
 // Keys of HD and values of VD values, 64 or 128 each: rows of 128 lie as two panels of 64 columns, a box each.  With either of them 128 the walks are not cut (a
 // 128 x 64 step is long enough that a short launch's blocks are busy), rows of out may lie apart, and a head may have a gate (see attention_rows.cu).  Measured, 2,048

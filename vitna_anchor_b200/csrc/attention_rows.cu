@@ -2,8 +2,9 @@
 //
 // This is the engine's attention for every size and both storage types: any
 // head size, any number of heads and groups, any page size, an optional
-// window.  The 32-bit path always runs it; the bfloat16 path runs it where
-// the specialised kernels do not take the sizes.  A token of a prompt portion
+// window.  The 32-bit path runs it for single tokens, and for prompt portions
+// whose sizes attention_rows_tile.cu (the same sums in the same order) does not
+// take; the bfloat16 path where the specialised kernels do not take the sizes.  A token of a prompt portion
 // and a single decoded token take the same code: a query at position p of a
 // request reads keys lo..p of that request through its block table
 // (lo = 0, or p - window + 1 with a window).

@@ -19,9 +19,9 @@
 //
 // Products take float32 operands as two tf32 parts (tf32.cuh).
 //
-// Measured, a whole mixer with its two products: mLSTM, one request of 2,048 tokens, 8 heads of 128 x 256: 599 us token after token, 196 us here (gates 14,
-// cm_add 26, cm_scan 10, cm_out 64: the tensor cores' rate for three tf32 products is 23 us of it on the multiprocessors that have two of its blocks);
-// gated linear attention, 1,204 + 807 tokens, 4 heads of 64 x 256: 279 and 109 us (decays 7, cm_add 9, cm_scan 8, cm_out 39: 128 blocks of one wave).  A first form
+// Measured, a whole mixer with its two products: mLSTM, one request of 2,048 tokens, 8 heads of 128 x 256: 599 us token after token, 200 us here (gates 14,
+// cm_add 26, cm_scan 10, cm_out 64 to 70: the tensor cores' rate for three tf32 products is 23 us of it on the multiprocessors that have two of its blocks);
+// gated linear attention, 1,204 + 807 tokens, 4 heads of 64 x 256: 279 and 110 us (decays 7, cm_add 9, cm_scan 8, cm_out 39: 128 blocks of one wave).  A first form
 // whose blocks walked the chunks in order with their tile of the state in the accumulators took 2.9 us a chunk, 90 us for cm_add's and cm_scan's work.
 #include "chunks.cuh"
 #include "common.cuh"
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(128) cm_add_kernel(const CmArgs p, int col_til
     }
 }
 
-// grid (blocks of 1,024 elements of S, and with MLSTM one more for n; H; segments).  What a chunk adds is read four chunks ahead.
+// grid (blocks of 1,024 elements of S, and with MLSTM one more for n; H; segments).  What the chunks add is read eight at a time.
 template <bool MLSTM>
 __global__ void __launch_bounds__(256) cm_scan_kernel(const CmArgs p) {
     __shared__ int base_sh;
