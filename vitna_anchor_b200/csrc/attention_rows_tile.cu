@@ -16,10 +16,6 @@ namespace vk {
 
 constexpr int RT_THREADS = 256, RT_Q = 32, RT_KEYS = 128;
 
-__device__ __forceinline__ void rt_cp16(float* dst, const float* src, bool there) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
-}
-
 // HD: the head size rounded up to 64 or 128 (sizes that are multiples of 4); warp w has queries 4 w .. 4 w + 3, lane l keys l, l + 32, l + 64, l + 96
 // of a run and, for the outputs, values (HD / 32) l ..
 template <int HD>
@@ -46,7 +42,7 @@ __global__ void __launch_bounds__(RT_THREADS) attention_rows_tile_kernel(
     const int v_stride = v_in_key ? hd : vd;
     for (int e = tid; e < RT_Q * (HD / 4); e += RT_THREADS) {
         const int r = e / (HD / 4), d = 4 * (e % (HD / 4));
-        rt_cp16(qs + r * LDK + d, q + ((size_t)(first + (r < rows ? r : 0)) * nh + h) * hd + (d < hd ? d : 0), r < rows && d < hd);
+        copy16_or_zero(qs + r * LDK + d, q + ((size_t)(first + (r < rows ? r : 0)) * nh + h) * hd + (d < hd ? d : 0), r < rows && d < hd);
     }
     float m[4], l[4], acc[4][DV];
 #pragma unroll
@@ -64,8 +60,8 @@ __global__ void __launch_bounds__(RT_THREADS) attention_rows_tile_kernel(
             const bool there = key >= lo_first && key <= last;
             const int page = there ? bt[key / page_size] : 0, at = there ? key % page_size : 0;
             const float* base = cache + (size_t)page * page_stride;
-            rt_cp16(ks + j * LDK + d, base + ((size_t)kvh * page_size + at) * hd + (d < hd ? d : 0), there && d < hd);
-            rt_cp16(vs + j * HD + d, base + v_base + ((size_t)(kvh / v_share) * page_size + at) * v_stride + (d < vd ? d : 0), there && d < vd);
+            copy16_or_zero(ks + j * LDK + d, base + ((size_t)kvh * page_size + at) * hd + (d < hd ? d : 0), there && d < hd);
+            copy16_or_zero(vs + j * HD + d, base + v_base + ((size_t)(kvh / v_share) * page_size + at) * v_stride + (d < vd ? d : 0), there && d < vd);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 0;" ::: "memory");

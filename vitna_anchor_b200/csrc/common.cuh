@@ -86,6 +86,13 @@ template <> __device__ __forceinline__ void load16<__nv_bfloat16>(const __nv_bfl
     }
 }
 
+// Sixteen bytes from memory into shared memory by cp.async, or zeros (src must be readable either way).
+__device__ __forceinline__ void copy16_or_zero(float* dst, const float* src, bool there) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+
+__device__ __forceinline__ float log_sigmoid(float z) { return fminf(z, 0.0f) - log1pf(expf(-fabsf(z))); }
+
 // An activation chosen at run time, for epilogues: 0 none, 1 gelu in its erf form 0.5 z (1 + erf(z / sqrt 2)), 2 gelu in
 // its tanh form, 3 silu.  (The element-wise kernel numbers them from 0 without "none".)
 __device__ __forceinline__ float activate_rt(int kind, float z) {

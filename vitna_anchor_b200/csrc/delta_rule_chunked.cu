@@ -87,15 +87,15 @@ __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(const DcArgs p
         const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
         const bool on = r < rows && d < dk;
         const float* row = row0 + (size_t)(on ? r : 0) * p.P + (on ? d : 0);
-        tf_cp16(sq + r * LDQ + d, row + kh * dk, on);
-        tf_cp16(sk + r * LDQ + d, row + (p.G + kh) * dk, on);
-        if (CH) tf_cp16(sl + r * LDQ + d, row + Cq + h * dk, on);
+        copy16_or_zero(sq + r * LDQ + d, row + kh * dk, on);
+        copy16_or_zero(sk + r * LDQ + d, row + (p.G + kh) * dk, on);
+        if (CH) copy16_or_zero(sl + r * LDQ + d, row + Cq + h * dk, on);
     }
     const int vp = (LDV - 4) / 4;
     for (int e = tid; e < DC_C * vp; e += 256) {
         const int r = e / vp, c = 4 * (e - r * vp);
         const bool on = r < rows && c < dv;
-        tf_cp16(sv + r * LDV + c, row0 + (size_t)(on ? r : 0) * p.P + 2 * p.G * dk + h * dv + (on ? c : 0), on);
+        copy16_or_zero(sv + r * LDV + c, row0 + (size_t)(on ? r : 0) * p.P + 2 * p.G * dk + h * dv + (on ? c : 0), on);
     }
     tf_commit();
     if (tid < 32) {                                 // beta, and the sums of the decays' logarithms
@@ -594,21 +594,21 @@ __global__ void __launch_bounds__(256) delta_chunk_out_kernel(const DcArgs p, bo
     const float* in = p.scratch + ((size_t)blockIdx.x * p.H + h) * dc_stride(dk, dv, ch_decay);
     for (int e = tid; e < DC_C * (DKP / 4); e += 256) {
         const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
-        tf_cp16(sQ + r * LDQ + d, in + dc_q_off(dk) + (d < dk ? (size_t)r * dk + d : 0), d < dk);
+        copy16_or_zero(sQ + r * LDQ + d, in + dc_q_off(dk) + (d < dk ? (size_t)r * dk + d : 0), d < dk);
     }
     for (int e = tid; e < COLS * (DKP / 4); e += 256) {
         const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
         const bool on = d < dk && c0 + r < dv;
-        tf_cp16(sS + r * LDQ + d, in + dc_s_off(dk, dv) + (on ? (size_t)(c0 + r) * dk + d : 0), on);
+        copy16_or_zero(sS + r * LDQ + d, in + dc_s_off(dk, dv) + (on ? (size_t)(c0 + r) * dk + d : 0), on);
     }
     for (int e = tid; e < DC_C * 16; e += 256) {
         const int r = e / 16, c = 4 * (e % 16);
-        tf_cp16(sP + r * DC_LDA + c, in + dc_p_off(dk) + r * DC_C + c, true);
+        copy16_or_zero(sP + r * DC_LDA + c, in + dc_p_off(dk) + r * DC_C + c, true);
     }
     for (int e = tid; e < DC_C * (COLS / 4); e += 256) {
         const int r = e / (COLS / 4), c = 4 * (e % (COLS / 4));
         const bool on = c0 + c < dv;
-        tf_cp16(sU + r * LDU + c, in + dc_u_off(dk) + (on ? (size_t)r * dv + c0 + c : 0), on);
+        copy16_or_zero(sU + r * LDU + c, in + dc_u_off(dk) + (on ? (size_t)r * dv + c0 + c : 0), on);
     }
     tf_commit();
     // the gate's values are asked for with the operands

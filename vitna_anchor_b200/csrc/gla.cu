@@ -24,8 +24,6 @@
 
 namespace vk {
 
-__device__ __forceinline__ float gla_log_sigmoid(float z) { return fminf(z, 0.0f) - log1pf(expf(-fabsf(z))); }
-
 constexpr int GLA_THREADS = 128;
 constexpr int GLA_PREP_TOKENS = 4;
 
@@ -65,7 +63,7 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(const float* __restric
         const float b = bias[c];
 #pragma unroll
         for (int t = 0; t < GLA_PREP_TOKENS; t++)
-            if (t < cnt) decay[(size_t)(t0 + t) * C + c] = expf(gla_log_sigmoid(z[t] + b) * inv_tau);
+            if (t < cnt) decay[(size_t)(t0 + t) * C + c] = expf(log_sigmoid(z[t] + b) * inv_tau);
     }
 }
 
@@ -248,7 +246,7 @@ __global__ void __launch_bounds__(GLA_THREADS) gla_decode_kernel(const float* __
         if (d < dim) {
             float z = 0.0f;
             for (int j = 0; j < rank; j++) z = fmaf(gd_a1[j], a2t[(size_t)j * C + h * dim + d], z);
-            a = expf(gla_log_sigmoid(z + bias[h * dim + d]) * inv_tau);
+            a = expf(log_sigmoid(z + bias[h * dim + d]) * inv_tau);
         }
         sa[d] = a;
     }

@@ -77,10 +77,6 @@ __global__ void __launch_bounds__(256) gemm_tile_kernel(const T* __restrict__ x,
 // order whatever the tile, so every tile, and the kernel above, give the same bits and the tile may follow the launch's size.
 constexpr int GT_K = 32, GT_LD = GT_K + 4, GT_STAGES = 4;
 
-__device__ __forceinline__ void gt_cp16(float* dst, const float* src, bool there) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
-}
-
 template <int MODE, int BM, int BN, int RM, int RN>
 __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_async_kernel(const float* __restrict__ x, const float* __restrict__ w, void* __restrict__ out,
                                                                            int M, int N, int K, int ldx) {
@@ -99,7 +95,7 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_async_kernel(const
                 const bool isx = r < BM;
                 const int g = isx ? m0 + r : n0 + r - BM;
                 const bool there = k < K && g < (isx ? M : N);
-                gt_cp16(st + r * GT_LD + 4 * (e % (GT_K / 4)), there ? (isx ? x + (size_t)g * ldx + k : w + (size_t)g * K + k) : x, there);
+                copy16_or_zero(st + r * GT_LD + 4 * (e % (GT_K / 4)), there ? (isx ? x + (size_t)g * ldx + k : w + (size_t)g * K + k) : x, there);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");

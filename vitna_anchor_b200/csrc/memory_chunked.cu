@@ -33,8 +33,6 @@ constexpr int CM_Q = 64;                    // tokens of a chunk
 constexpr int CM_LOCAL = 16;                // tokens over which a channel's logarithms are added up (gated linear attention)
 constexpr int CM_T = 64, CM_LD = CM_T + 8;   // the tile of the state that a block of cm_add works out, and a padded row of one of its operands
 
-__device__ __forceinline__ float cm_log_sigmoid(float z) { return fminf(z, 0.0f) - log1pf(expf(-fabsf(z))); }
-
 struct CmArgs {
     const float* proj;              // [tokens][N]: q | k | v | ..
     int N, H, dk, dv, segments, from;       // segments of up to `from` tokens are left alone
@@ -86,7 +84,7 @@ __global__ void __launch_bounds__(MG_THREADS) mlstm_chunk_gates_kernel(const CmA
                 const bool on = t0 + u < end;
                 const float* row = p.proj + (size_t)(on ? t0 + u : first) * p.N;
                 gi[u] = on ? cap * tanhf((row[i_off] + bi) / cap) : -INFINITY;
-                f[u] = on ? (double)cm_log_sigmoid(cap * tanhf((row[f_off] + bf) / cap)) : 0.0;
+                f[u] = on ? (double)log_sigmoid(cap * tanhf((row[f_off] + bf) / cap)) : 0.0;
             }
             double sum = f[0] + f[1];
 #pragma unroll
@@ -168,7 +166,7 @@ __global__ void __launch_bounds__(GD_THREADS) gla_chunk_decays_kernel(const CmAr
     const float b = bias[c];
 #pragma unroll
     for (int t = 0; t < CM_LOCAL; t++)
-        if (t < cnt) p.logs[(size_t)(first + t) * C + c] = cm_log_sigmoid(z[t] + b) * inv_tau * 1.4426950408889634f;
+        if (t < cnt) p.logs[(size_t)(first + t) * C + c] = log_sigmoid(z[t] + b) * inv_tau * 1.4426950408889634f;
 }
 
 // -- the states before the chunks ---------------------------------------------------------------------------------------------------------------
@@ -191,9 +189,9 @@ __global__ void __launch_bounds__(128) cm_add_kernel(const CmArgs p, int col_til
         const int r = e / (CM_T / 4), c = 4 * (e % (CM_T / 4));
         const bool onk = r < rows && d0 + c < dk, onv = r < rows && v0 + c < dv;
         const float* row = p.proj + (size_t)(ch.first + (r < rows ? r : 0)) * p.N;
-        tf_cp16(sk + r * CM_LD + c, onk ? row + H * dk + h * dk + d0 + c : p.proj, onk);
-        tf_cp16(sv + r * CM_LD + c, onv ? row + 2 * H * dk + h * dv + v0 + c : p.proj, onv);
-        if (!MLSTM) tf_cp16(sl + r * CM_LD + c, onk ? p.logs + (size_t)(ch.first + r) * H * dk + h * dk + d0 + c : p.proj, onk);
+        copy16_or_zero(sk + r * CM_LD + c, onk ? row + H * dk + h * dk + d0 + c : p.proj, onk);
+        copy16_or_zero(sv + r * CM_LD + c, onv ? row + 2 * H * dk + h * dv + v0 + c : p.proj, onv);
+        if (!MLSTM) copy16_or_zero(sl + r * CM_LD + c, onk ? p.logs + (size_t)(ch.first + r) * H * dk + h * dk + d0 + c : p.proj, onk);
     }
     tf_commit();
     if (MLSTM && tid < CM_Q) wt[tid] = tid < rows ? p.weight[(size_t)(ch.first + tid) * H + h] : 0.0f;
@@ -392,10 +390,10 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
         const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
         const bool on = r < rows && d < dk;
         const float* src = p.proj + (size_t)(ch.first + (on ? r : 0)) * p.N + h * dk + (on ? d : 0);
-        tf_cp16(sq + r * LDQ + d, src, on);
-        tf_cp16(sk + r * LDQ + d, src + H * dk, on);
+        copy16_or_zero(sq + r * LDQ + d, src, on);
+        copy16_or_zero(sk + r * LDQ + d, src + H * dk, on);
         // the decays' logarithms lie in the first slot until the weights of the chunk are known
-        if (!MLSTM) tf_cp16(ring + r * LDQ + d, p.logs + (size_t)(ch.first + (on ? r : 0)) * H * dk + h * dk + (on ? d : 0), on);
+        if (!MLSTM) copy16_or_zero(ring + r * LDQ + d, p.logs + (size_t)(ch.first + (on ? r : 0)) * H * dk + h * dk + (on ? d : 0), on);
     }
     tf_commit();
     auto issue = [&](int s) {                           // slice s: 32 rows of the state, then of v
@@ -405,7 +403,7 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
                 const int r = e / (DVP / 4), v = 4 * (e % (DVP / 4)), row = (s < KS ? s : s - KS) * 32 + r;
                 const bool on = v < dv && row < (s < KS ? dk : rows);
                 const float* src = s < KS ? p.before + (at * dk + row) * dv + v : p.proj + (size_t)(ch.first + row) * p.N + 2 * H * dk + h * dv + v;
-                tf_cp16(dst + r * LDB + v, on ? src : p.proj, on);
+                copy16_or_zero(dst + r * LDB + v, on ? src : p.proj, on);
             }
         }
         tf_commit();

@@ -29,8 +29,6 @@
 
 namespace vk {
 
-__device__ __forceinline__ float log_sigmoid(float z) { return fminf(z, 0.0f) - log1pf(expf(-fabsf(z))); }
-
 constexpr int ML_THREADS = 128;
 constexpr int ML_COLS = 16;
 constexpr int ML_ROW_GROUPS = 8;

@@ -9,9 +9,6 @@
 
 namespace vk {
 
-__device__ __forceinline__ void tf_cp16(float* dst, const float* src, bool there) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
-}
 __device__ __forceinline__ void tf_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int LEFT> __device__ __forceinline__ void tf_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
