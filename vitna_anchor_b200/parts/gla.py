@@ -44,8 +44,10 @@ class GatedLinearAttention(Mixer):
         self.norm_weight = norm_weight.to(torch.float32).contiguous()
         # Measured, us a mixer, token after token / in chunks, 4 heads of 64 x 256 and 8 of 128 x 256:  one segment of 288: 64 / 72, 86 / 109; of 352: 80 / 72, 96 / 112; of
         # 448: 84 / 73, 119 / 118;  eight of 100: 65 / 78, 160 / 169;  sixteen of 64: 81 / 83, 184 / 184;  eight of 150: 88 / 82, 210 / 188;  one of 512 beside 32
-        # single tokens: 99 / 87, 171 / 212; beside 64: 105 / 108, 198 / 309; of 2,048 beside 64: 426 / 152, 544 / 428, and with the single ones token after token 159, 350.
-        self.chunk_rule = ChunkRule(320 if dim <= 64 else 432, total=1024, a_single=H * vdim // 256, few=max(1, 2621440 // (H * dim * vdim)))
+        # single tokens: 99 / 87, 171 / 212; beside 64: 105 / 108, 198 / 309; of 2,048 beside 64: 426 / 152, 544 / 428.  In chunks
+        # with the single ones / those token after token:  512 beside 8: 75 / 95, 131 / 161; 1,024 beside 32: 101 / 124, 253 / 242; beside 64: 122 / 141, 352 / 294; 2,048
+        # beside 64: 152 / 159, 428 / 351.
+        self.chunk_rule = ChunkRule(320 if dim <= 64 else 432, total=1024, a_single=H * vdim // 256, few=max(1, 4718592 // (H * dim * vdim)))
         self.gate_off = 2 * H * dim + H * vdim
         self.a_off = self.gate_off + H * vdim
 

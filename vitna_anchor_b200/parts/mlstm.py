@@ -41,8 +41,9 @@ class MatrixLSTM(Mixer):
         self.norm_weight = norm_weight.to(torch.float32).contiguous()
         # Measured, us a mixer, token after token / in chunks, 4 heads of 64 x 256 and 8 of 128 x 256:  one segment of 144: 57 / 65, 77 / 85; of 208: 72 / 66, 95 / 85;  four of
         # 100: 55 / 67, 112 / 105;  eight of 150: 90 / 77, 221 / 161;  sixteen of 32: 49 / 71, 113 / 137;  one of 512 beside 32 single tokens: 160 / 82, 208 / 187; beside
-        # 64: 164 / 106, 226 / 284; of 2,048 beside 64: 510 / 147, 712 / 385, and with the single ones token after token 144, 330.
-        self.chunk_rule = ChunkRule(176, total=(1 << 20) // (H * vdim), a_single=H * vdim // 256, few=32)
+        # 64: 164 / 106, 226 / 284; of 2,048 beside 64: 510 / 147, 712 / 385.  In chunks with the single ones / those token after token:  1,024 beside 32: 100 / 111, 224 / 217;
+        # beside 64: 110 / 124, 315 / 279; 2,048 beside 64: 146 / 144, 378 / 328.
+        self.chunk_rule = ChunkRule(176, total=(1 << 20) // (H * vdim), a_single=H * vdim // 256, few=max(32, 4194304 // (H * dim * vdim)))
 
     def tensors(self):
         return [self.w_in, self.gate_bias, self.norm_weight, self.w_out]
