@@ -386,273 +386,273 @@ __global__ void __launch_bounds__(256, 2) cm_out_kernel(const CmArgs p, int gate
     // (a weight of zero times a NaN is one) and an infinity is not made a NaN by its parts.
 #pragma unroll 1
     for (bool careful = false;; careful = true) {
-    for (int e = tid; e < CM_Q * (DKP / 4); e += 256) {
-        const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
-        const bool on = r < rows && d < dk;
-        const float* src = p.proj + (size_t)(ch.first + (on ? r : 0)) * p.N + h * dk + (on ? d : 0);
-        copy16_or_zero(sq + r * LDQ + d, src, on);
-        copy16_or_zero(sk + r * LDQ + d, src + H * dk, on);
-        // the decays' logarithms lie in the first slot until the weights of the chunk are known
-        if (!MLSTM) copy16_or_zero(ring + r * LDQ + d, p.logs + (size_t)(ch.first + (on ? r : 0)) * H * dk + h * dk + (on ? d : 0), on);
-    }
-    tf_commit();
-    auto issue = [&](int s) {                           // slice s: 32 rows of the state, then of v
-        if (s < KS + 2) {
-            float* dst = ring + (s & 1) * L::SLOT;
-            for (int e = tid; e < 32 * (DVP / 4); e += 256) {
-                const int r = e / (DVP / 4), v = 4 * (e % (DVP / 4)), row = (s < KS ? s : s - KS) * 32 + r;
-                const bool on = v < dv && row < (s < KS ? dk : rows);
-                const float* src = s < KS ? p.before + (at * dk + row) * dv + v : p.proj + (size_t)(ch.first + row) * p.N + 2 * H * dk + h * dv + v;
-                copy16_or_zero(dst + r * LDB + v, on ? src : p.proj, on);
-            }
+        for (int e = tid; e < CM_Q * (DKP / 4); e += 256) {
+            const int r = e / (DKP / 4), d = 4 * (e % (DKP / 4));
+            const bool on = r < rows && d < dk;
+            const float* src = p.proj + (size_t)(ch.first + (on ? r : 0)) * p.N + h * dk + (on ? d : 0);
+            copy16_or_zero(sq + r * LDQ + d, src, on);
+            copy16_or_zero(sk + r * LDQ + d, src + H * dk, on);
+            // the decays' logarithms lie in the first slot until the weights of the chunk are known
+            if (!MLSTM) copy16_or_zero(ring + r * LDQ + d, p.logs + (size_t)(ch.first + (on ? r : 0)) * H * dk + h * dk + (on ? d : 0), on);
         }
         tf_commit();
-    };
-    if (MLSTM) {
-        issue(0);
-        if (tid < CM_Q) {
-            const double mb = p.m_before[at];
-            const size_t i = (size_t)(ch.first + (tid < rows ? tid : 0)) * H + h;
-            const double Nt = fmax(mb, p.G[i]);
-            sA[tid] = tid < rows ? p.A[i] : 0.0;
-            sN[tid] = Nt;
-            row_f[tid] = expf((float)(mb - Nt));
-            row_n[tid] = expf(-(float)(p.F[i] + Nt));   // e^-m
-        }
-        for (int d = tid; d < DKP; d += 256) vec[d] = d < dk ? p.n_before[at * dk + d] : 0.0f;
-        tf_wait<1>();
-    } else {
-        tf_wait<0>();
-    }
-    __syncthreads();
-
-    // the chunk's weights, 16 x 16 of them a warp and m: rows 32 wm + 16 m .., columns 16 wn ..
-    float w[2][2][4];
-#pragma unroll
-    for (int m = 0; m < 2; m++)
-#pragma unroll
-        for (int n = 0; n < 2; n++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) w[m][n][e] = 0.0f;
-    if (!MLSTM) {
-        // Pairs inside a piece of 16 tokens by themselves, before q and k are scaled: four threads a row, a quarter of the channels each, walk from the row's
-        // token back to the piece's first with the sum of the logarithms so far.
-        const float* sl = ring;
-        float* sw = misc;                               // [64][17]
-        const int r = tid >> 2, p0 = r & ~15;
-        float pw[CM_LOCAL];
-#pragma unroll
-        for (int i = 0; i < CM_LOCAL; i++) pw[i] = 0.0f;
-        for (int d = tid & 3; d < DKP; d += 4) {
-            float sum = 0.0f;
-            const float qv = sq[r * LDQ + d];
-#pragma unroll
-            for (int j = CM_LOCAL - 1; j >= 0; j--)
-                if (p0 + j <= r) {
-                    pw[j] = fmaf(qv * sk[(p0 + j) * LDQ + d], tf_exp2(sum), pw[j]);
-                    sum += sl[(p0 + j) * LDQ + d];
+        auto issue = [&](int s) {                           // slice s: 32 rows of the state, then of v
+            if (s < KS + 2) {
+                float* dst = ring + (s & 1) * L::SLOT;
+                for (int e = tid; e < 32 * (DVP / 4); e += 256) {
+                    const int r = e / (DVP / 4), v = 4 * (e % (DVP / 4)), row = (s < KS ? s : s - KS) * 32 + r;
+                    const bool on = v < dv && row < (s < KS ? dk : rows);
+                    const float* src = s < KS ? p.before + (at * dk + row) * dv + v : p.proj + (size_t)(ch.first + row) * p.N + 2 * H * dk + h * dv + v;
+                    copy16_or_zero(dst + r * LDB + v, on ? src : p.proj, on);
                 }
-        }
-#pragma unroll
-        for (int j = 0; j < CM_LOCAL; j++) {
-            pw[j] += __shfl_xor_sync(0xffffffffu, pw[j], 1);
-            pw[j] += __shfl_xor_sync(0xffffffffu, pw[j], 2);
-            if ((tid & 3) == (j & 3)) sw[r * 17 + j] = pw[j];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int m = 0; m < 2; m++)
-            if (2 * wm + m == wn) {
-#pragma unroll
-                for (int n = 0; n < 2; n++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) w[m][n][e] = sw[(16 * wn + g + (e >> 1) * 8) * 17 + n * 8 + 2 * t4 + (e & 1)];
             }
-        // q times what its piece leaves up to it, k times what its piece leaves behind it, and what the whole pieces leave: a channel of a piece a thread
-        for (int e = tid; e < 4 * DKP; e += 256) {
-            const int s = e / DKP, d = e % DKP;
-            float before = 0.0f, behind = 0.0f;
-#pragma unroll
-            for (int j = 0; j < CM_LOCAL; j++) {
-                before += sl[(16 * s + j) * LDQ + d];
-                sq[(16 * s + j) * LDQ + d] *= tf_exp2(before);
+            tf_commit();
+        };
+        if (MLSTM) {
+            issue(0);
+            if (tid < CM_Q) {
+                const double mb = p.m_before[at];
+                const size_t i = (size_t)(ch.first + (tid < rows ? tid : 0)) * H + h;
+                const double Nt = fmax(mb, p.G[i]);
+                sA[tid] = tid < rows ? p.A[i] : 0.0;
+                sN[tid] = Nt;
+                row_f[tid] = expf((float)(mb - Nt));
+                row_n[tid] = expf(-(float)(p.F[i] + Nt));   // e^-m
             }
-            vec[e] = tf_exp2(before);
-#pragma unroll
-            for (int j = CM_LOCAL - 1; j >= 0; j--) {
-                sk[(16 * s + j) * LDQ + d] *= tf_exp2(behind);
-                behind += sl[(16 * s + j) * LDQ + d];
-            }
+            for (int d = tid; d < DKP; d += 256) vec[d] = d < dk ? p.n_before[at * dk + d] : 0.0f;
+            tf_wait<1>();
+        } else {
+            tf_wait<0>();
         }
         __syncthreads();
-        issue(0);
-    }
-    // q k^T: MLSTM every pair, else the pairs of different sixteens (q's factor takes what decays between the two)
-#pragma unroll
-    for (int m = 0; m < 2; m++) {
-        const int I = 2 * wm + m;
-        if (MLSTM ? wn > I : wn >= I) continue;
-#pragma unroll 4
-        for (int ks = 0; ks < DKP / 8; ks++) {
-            const int d = ks * 8 + 2 * t4;
-            const float* qa = sq + (16 * I + g) * LDQ + d;
-            float2 x = *reinterpret_cast<const float2*>(qa), y = *reinterpret_cast<const float2*>(qa + 8 * LDQ);
-            if (!MLSTM) {
-                float f0 = 1.0f, f1 = 1.0f;
-                for (int u = wn + 1; u < I; u++) { f0 *= vec[u * DKP + d]; f1 *= vec[u * DKP + d + 1]; }
-                x.x *= f0; x.y *= f1; y.x *= f0; y.y *= f1;
-            }
-            const Tf a[1][4] = {{tf_split(x.x), tf_split(y.x), tf_split(x.y), tf_split(y.y)}};
-            Tf b[2][2];
-#pragma unroll
-            for (int n = 0; n < 2; n++) {
-                const float2 kb = *reinterpret_cast<const float2*>(sk + (16 * wn + n * 8 + g) * LDQ + d);
-                b[n][0] = tf_split(kb.x);
-                b[n][1] = tf_split(kb.y);
-            }
-            float* const d_[1][2] = {{w[m][0], w[m][1]}};
-            tf_mma3(d_, a, b);
-        }
-    }
-    if (MLSTM) {
-        float part[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+
+        // the chunk's weights, 16 x 16 of them a warp and m: rows 32 wm + 16 m .., columns 16 wn ..
+        float w[2][2][4];
 #pragma unroll
         for (int m = 0; m < 2; m++)
 #pragma unroll
             for (int n = 0; n < 2; n++)
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int r = 32 * wm + 16 * m + g + (e >> 1) * 8, i = 16 * wn + n * 8 + 2 * t4 + (e & 1);
-                    w[m][n][e] = (i <= r && i < rows) ? w[m][n][e] * expf((float)(sA[i] - sN[r])) : 0.0f;
-                    part[m][e >> 1] += w[m][n][e];
-                }
+                for (int e = 0; e < 4; e++) w[m][n][e] = 0.0f;
+        if (!MLSTM) {
+            // Pairs inside a piece of 16 tokens by themselves, before q and k are scaled: four threads a row, a quarter of the channels each, walk from the row's
+            // token back to the piece's first with the sum of the logarithms so far.
+            const float* sl = ring;
+            float* sw = misc;                               // [64][17]
+            const int r = tid >> 2, p0 = r & ~15;
+            float pw[CM_LOCAL];
 #pragma unroll
-        for (int m = 0; m < 2; m++)
+            for (int i = 0; i < CM_LOCAL; i++) pw[i] = 0.0f;
+            for (int d = tid & 3; d < DKP; d += 4) {
+                float sum = 0.0f;
+                const float qv = sq[r * LDQ + d];
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                float v = part[m][u];
-                v += __shfl_xor_sync(0xffffffffu, v, 1);
-                v += __shfl_xor_sync(0xffffffffu, v, 2);
-                if (t4 == 0) sums[wn][32 * wm + 16 * m + g + u * 8] = v;
+                for (int j = CM_LOCAL - 1; j >= 0; j--)
+                    if (p0 + j <= r) {
+                        pw[j] = fmaf(qv * sk[(p0 + j) * LDQ + d], tf_exp2(sum), pw[j]);
+                        sum += sl[(p0 + j) * LDQ + d];
+                    }
             }
-        // q . n before the chunk: four threads a row
-        const int r = tid >> 2;
-        float s = 0.0f;
-        for (int d = tid & 3; d < DKP; d += 4) s = fmaf(sq[r * LDQ + d], vec[d], s);
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if ((tid & 3) == 0) squares[0][r] = s;          // (until the squares are needed)
-    }
-    __syncthreads();                                    // nobody reads k any more
-    issue(1);
-    if (MLSTM && tid < CM_Q) {
-        const float nq = fmaf(row_f[tid], squares[0][tid], (sums[0][tid] + sums[1][tid]) + (sums[2][tid] + sums[3][tid])) * qscale;
-        row_n[tid] = 1.0f / (fmaxf(fabsf(nq), row_n[tid]) + 1e-6f);
-    }
 #pragma unroll
-    for (int m = 0; m < 2; m++)
+            for (int j = 0; j < CM_LOCAL; j++) {
+                pw[j] += __shfl_xor_sync(0xffffffffu, pw[j], 1);
+                pw[j] += __shfl_xor_sync(0xffffffffu, pw[j], 2);
+                if ((tid & 3) == (j & 3)) sw[r * 17 + j] = pw[j];
+            }
+            __syncthreads();
 #pragma unroll
-        for (int n = 0; n < NT; n++)
+            for (int m = 0; m < 2; m++)
+                if (2 * wm + m == wn) {
 #pragma unroll
-            for (int e = 0; e < 4; e++) o[m][n][e] = 0.0f;
-#pragma unroll 1
-    for (int s = 0; s < KS + 2; s++) {
-        tf_wait<1>();
-        __syncthreads();                                // slice s is there
-        if (s == KS) {                                  // q with the state is done: the weights take q's place
+                    for (int n = 0; n < 2; n++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) w[m][n][e] = sw[(16 * wn + g + (e >> 1) * 8) * 17 + n * 8 + 2 * t4 + (e & 1)];
+                }
+            // q times what its piece leaves up to it, k times what its piece leaves behind it, and what the whole pieces leave: a channel of a piece a thread
+            for (int e = tid; e < 4 * DKP; e += 256) {
+                const int s = e / DKP, d = e % DKP;
+                float before = 0.0f, behind = 0.0f;
+#pragma unroll
+                for (int j = 0; j < CM_LOCAL; j++) {
+                    before += sl[(16 * s + j) * LDQ + d];
+                    sq[(16 * s + j) * LDQ + d] *= tf_exp2(before);
+                }
+                vec[e] = tf_exp2(before);
+#pragma unroll
+                for (int j = CM_LOCAL - 1; j >= 0; j--) {
+                    sk[(16 * s + j) * LDQ + d] *= tf_exp2(behind);
+                    behind += sl[(16 * s + j) * LDQ + d];
+                }
+            }
+            __syncthreads();
+            issue(0);
+        }
+        // q k^T: MLSTM every pair, else the pairs of different sixteens (q's factor takes what decays between the two)
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            const int I = 2 * wm + m;
+            if (MLSTM ? wn > I : wn >= I) continue;
+#pragma unroll 4
+            for (int ks = 0; ks < DKP / 8; ks++) {
+                const int d = ks * 8 + 2 * t4;
+                const float* qa = sq + (16 * I + g) * LDQ + d;
+                float2 x = *reinterpret_cast<const float2*>(qa), y = *reinterpret_cast<const float2*>(qa + 8 * LDQ);
+                if (!MLSTM) {
+                    float f0 = 1.0f, f1 = 1.0f;
+                    for (int u = wn + 1; u < I; u++) { f0 *= vec[u * DKP + d]; f1 *= vec[u * DKP + d + 1]; }
+                    x.x *= f0; x.y *= f1; y.x *= f0; y.y *= f1;
+                }
+                const Tf a[1][4] = {{tf_split(x.x), tf_split(y.x), tf_split(x.y), tf_split(y.y)}};
+                Tf b[2][2];
+#pragma unroll
+                for (int n = 0; n < 2; n++) {
+                    const float2 kb = *reinterpret_cast<const float2*>(sk + (16 * wn + n * 8 + g) * LDQ + d);
+                    b[n][0] = tf_split(kb.x);
+                    b[n][1] = tf_split(kb.y);
+                }
+                float* const d_[1][2] = {{w[m][0], w[m][1]}};
+                tf_mma3(d_, a, b);
+            }
+        }
+        if (MLSTM) {
+            float part[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
 #pragma unroll
             for (int m = 0; m < 2; m++)
 #pragma unroll
                 for (int n = 0; n < 2; n++)
 #pragma unroll
-                    for (int u = 0; u < 2; u++)
-                        *reinterpret_cast<float2*>(sq + (32 * wm + 16 * m + g + u * 8) * LDP + 16 * wn + n * 8 + 2 * t4) =
-                            make_float2(w[m][n][2 * u], w[m][n][2 * u + 1]);
-            if (MLSTM) {
-#pragma unroll
-                for (int m = 0; m < 2; m++) {
-                    const float fa = row_f[32 * wm + 16 * m + g], fb = row_f[32 * wm + 16 * m + g + 8];
-#pragma unroll
-                    for (int n = 0; n < NT; n++) { o[m][n][0] *= fa; o[m][n][1] *= fa; o[m][n][2] *= fb; o[m][n][3] *= fb; }
-                }
-            }
-            __syncthreads();
-        }
-        const float* sb = ring + (s & 1) * L::SLOT + col0 + g;
-        if (s < KS || 32 * (s - KS) <= 32 * wm + 31) {  // (rows 0..31 do not see tokens 32..63)
-            const int lda = s < KS ? LDQ : LDP;
-            const float* pa = sq + (32 * wm + g) * lda + (s < KS ? 32 * s : 32 * (s - KS));
-            if (careful) {
-#pragma unroll 1
-                for (int i = 0; i < 32; i++)
-#pragma unroll
-                    for (int m = 0; m < 2; m++)
-#pragma unroll
-                        for (int u = 0; u < 2; u++) {
-                            if (s >= KS && 32 * (s - KS) + i > 32 * wm + 16 * m + g + 8 * u) continue;
-                            float x = pa[(16 * m + 8 * u) * lda + i];
-                            if (!MLSTM && s < KS)
-                                for (int z = 0; z < 2 * wm + m; z++) x *= vec[z * DKP + 32 * s + i];
-#pragma unroll
-                            for (int n = 0; n < NT; n++)
-#pragma unroll
-                                for (int e = 0; e < 2; e++) o[m][n][2 * u + e] = fmaf(x, sb[i * LDB + n * 8 + 2 * t4 - g + e], o[m][n][2 * u + e]);
-                        }
-            } else
-#pragma unroll
-            for (int ks = 0; ks < 4; ks++) {
-                Tf a[2][4];
-#pragma unroll
-                for (int m = 0; m < 2; m++) {
-                    const float* q0 = pa + 16 * m * lda + ks * 8 + 2 * t4;
-                    float2 x = *reinterpret_cast<const float2*>(q0), y = *reinterpret_cast<const float2*>(q0 + 8 * lda);
-                    if (!MLSTM && s < KS) {
-                        const int d = 32 * s + ks * 8 + 2 * t4;
-                        float f0 = 1.0f, f1 = 1.0f;
-                        for (int u = 0; u < 2 * wm + m; u++) { f0 *= vec[u * DKP + d]; f1 *= vec[u * DKP + d + 1]; }
-                        x.x *= f0; x.y *= f1; y.x *= f0; y.y *= f1;
+                    for (int e = 0; e < 4; e++) {
+                        const int r = 32 * wm + 16 * m + g + (e >> 1) * 8, i = 16 * wn + n * 8 + 2 * t4 + (e & 1);
+                        w[m][n][e] = (i <= r && i < rows) ? w[m][n][e] * expf((float)(sA[i] - sN[r])) : 0.0f;
+                        part[m][e >> 1] += w[m][n][e];
                     }
-                    a[m][0] = tf_split(x.x); a[m][1] = tf_split(y.x); a[m][2] = tf_split(x.y); a[m][3] = tf_split(y.y);
-                }
 #pragma unroll
-                for (int n = 0; n < NT; n += 2) {
-                    Tf b[2][2];
+            for (int m = 0; m < 2; m++)
 #pragma unroll
-                    for (int u = 0; u < 2; u++) {
-                        const float* vb = sb + (ks * 8 + 2 * t4) * LDB + (n + u) * 8;
-                        b[u][0] = tf_split(vb[0]);
-                        b[u][1] = tf_split(vb[LDB]);
-                    }
-                    float* const d_[2][2] = {{o[0][n], o[0][n + 1]}, {o[1][n], o[1][n + 1]}};
-                    tf_mma3(d_, a, b);
+                for (int u = 0; u < 2; u++) {
+                    float v = part[m][u];
+                    v += __shfl_xor_sync(0xffffffffu, v, 1);
+                    v += __shfl_xor_sync(0xffffffffu, v, 2);
+                    if (t4 == 0) sums[wn][32 * wm + 16 * m + g + u * 8] = v;
                 }
-            }
+            // q . n before the chunk: four threads a row
+            const int r = tid >> 2;
+            float s = 0.0f;
+            for (int d = tid & 3; d < DKP; d += 4) s = fmaf(sq[r * LDQ + d], vec[d], s);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            if ((tid & 3) == 0) squares[0][r] = s;          // (until the squares are needed)
         }
-        __syncthreads();
-        issue(s + 2);
-    }
-    // the heads' norm and gate
-    bool odd = false;
+        __syncthreads();                                    // nobody reads k any more
+        issue(1);
+        if (MLSTM && tid < CM_Q) {
+            const float nq = fmaf(row_f[tid], squares[0][tid], (sums[0][tid] + sums[1][tid]) + (sums[2][tid] + sums[3][tid])) * qscale;
+            row_n[tid] = 1.0f / (fmaxf(fabsf(nq), row_n[tid]) + 1e-6f);
+        }
 #pragma unroll
-    for (int m = 0; m < 2; m++)
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int r = 32 * wm + 16 * m + g + u * 8;
-            const float f = MLSTM ? qscale * row_n[r] : qscale;
-            float ss = 0.0f;
+        for (int m = 0; m < 2; m++)
 #pragma unroll
             for (int n = 0; n < NT; n++)
 #pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    o[m][n][2 * u + e] *= f;
-                    ss = fmaf(o[m][n][2 * u + e], o[m][n][2 * u + e], ss);
+                for (int e = 0; e < 4; e++) o[m][n][e] = 0.0f;
+#pragma unroll 1
+        for (int s = 0; s < KS + 2; s++) {
+            tf_wait<1>();
+            __syncthreads();                                // slice s is there
+            if (s == KS) {                                  // q with the state is done: the weights take q's place
+#pragma unroll
+                for (int m = 0; m < 2; m++)
+#pragma unroll
+                    for (int n = 0; n < 2; n++)
+#pragma unroll
+                        for (int u = 0; u < 2; u++)
+                            *reinterpret_cast<float2*>(sq + (32 * wm + 16 * m + g + u * 8) * LDP + 16 * wn + n * 8 + 2 * t4) =
+                                make_float2(w[m][n][2 * u], w[m][n][2 * u + 1]);
+                if (MLSTM) {
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+                        const float fa = row_f[32 * wm + 16 * m + g], fb = row_f[32 * wm + 16 * m + g + 8];
+#pragma unroll
+                        for (int n = 0; n < NT; n++) { o[m][n][0] *= fa; o[m][n][1] *= fa; o[m][n][2] *= fb; o[m][n][3] *= fb; }
+                    }
                 }
-            ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-            ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-            if (t4 == 0) squares[wn][r] = ss;
-            odd = odd || (r < rows && !tf_finite(ss));
+                __syncthreads();
+            }
+            const float* sb = ring + (s & 1) * L::SLOT + col0 + g;
+            if (s < KS || 32 * (s - KS) <= 32 * wm + 31) {  // (rows 0..31 do not see tokens 32..63)
+                const int lda = s < KS ? LDQ : LDP;
+                const float* pa = sq + (32 * wm + g) * lda + (s < KS ? 32 * s : 32 * (s - KS));
+                if (careful) {
+#pragma unroll 1
+                    for (int i = 0; i < 32; i++)
+#pragma unroll
+                        for (int m = 0; m < 2; m++)
+#pragma unroll
+                            for (int u = 0; u < 2; u++) {
+                                if (s >= KS && 32 * (s - KS) + i > 32 * wm + 16 * m + g + 8 * u) continue;
+                                float x = pa[(16 * m + 8 * u) * lda + i];
+                                if (!MLSTM && s < KS)
+                                    for (int z = 0; z < 2 * wm + m; z++) x *= vec[z * DKP + 32 * s + i];
+#pragma unroll
+                                for (int n = 0; n < NT; n++)
+#pragma unroll
+                                    for (int e = 0; e < 2; e++) o[m][n][2 * u + e] = fmaf(x, sb[i * LDB + n * 8 + 2 * t4 - g + e], o[m][n][2 * u + e]);
+                            }
+                } else
+#pragma unroll
+                for (int ks = 0; ks < 4; ks++) {
+                    Tf a[2][4];
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+                        const float* q0 = pa + 16 * m * lda + ks * 8 + 2 * t4;
+                        float2 x = *reinterpret_cast<const float2*>(q0), y = *reinterpret_cast<const float2*>(q0 + 8 * lda);
+                        if (!MLSTM && s < KS) {
+                            const int d = 32 * s + ks * 8 + 2 * t4;
+                            float f0 = 1.0f, f1 = 1.0f;
+                            for (int u = 0; u < 2 * wm + m; u++) { f0 *= vec[u * DKP + d]; f1 *= vec[u * DKP + d + 1]; }
+                            x.x *= f0; x.y *= f1; y.x *= f0; y.y *= f1;
+                        }
+                        a[m][0] = tf_split(x.x); a[m][1] = tf_split(y.x); a[m][2] = tf_split(x.y); a[m][3] = tf_split(y.y);
+                    }
+#pragma unroll
+                    for (int n = 0; n < NT; n += 2) {
+                        Tf b[2][2];
+#pragma unroll
+                        for (int u = 0; u < 2; u++) {
+                            const float* vb = sb + (ks * 8 + 2 * t4) * LDB + (n + u) * 8;
+                            b[u][0] = tf_split(vb[0]);
+                            b[u][1] = tf_split(vb[LDB]);
+                        }
+                        float* const d_[2][2] = {{o[0][n], o[0][n + 1]}, {o[1][n], o[1][n + 1]}};
+                        tf_mma3(d_, a, b);
+                    }
+                }
+            }
+            __syncthreads();
+            issue(s + 2);
         }
-    if (!__syncthreads_or(odd && !careful)) break;
+        // the heads' norm and gate
+        bool odd = false;
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int r = 32 * wm + 16 * m + g + u * 8;
+                const float f = MLSTM ? qscale * row_n[r] : qscale;
+                float ss = 0.0f;
+#pragma unroll
+                for (int n = 0; n < NT; n++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        o[m][n][2 * u + e] *= f;
+                        ss = fmaf(o[m][n][2 * u + e], o[m][n][2 * u + e], ss);
+                    }
+                ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+                ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+                if (t4 == 0) squares[wn][r] = ss;
+                odd = odd || (r < rows && !tf_finite(ss));
+            }
+        if (!__syncthreads_or(odd && !careful)) break;
     }
 #pragma unroll
     for (int m = 0; m < 2; m++)
