@@ -1,0 +1,357 @@
+// The matrix product of a few dozen rows in bfloat16 on the fifth-generation tensor cores: out[M, N] = x[M, K] * W[N, K]^T, M <= 64, with the weights as
+// the 128-row operand.
+//
+// Decoding a few dozen requests together streams every weight once; what bounds it is how many bytes of weights are on their way.  A tile is 128 rows of the
+// weights (tensor-core rows) by all batch rows (its 16, 32 or 64 columns), so that a stage of the ring is 16 KB of weights and at most 8 KB of x, and a
+// block needs no register and no issue slot for a weight.  Where the tiles are fewer than the multiprocessors, K is split over a cluster's blocks: each
+// leaves its float32 sums in its shared memory, and every block of the cluster adds up a share of the batch rows over all of them, in the order of the
+// splits, and finishes it.  The first four stages' weights are asked for before the wait on the kernel before this one.
+//
+//   warp 0   one lane: TMA copies into a ring of four stages (64 columns of K each)
+//   warp 1   one lane: tcgen05.mma, 128 x NB x 16
+//   warps 2-5  the accumulator out of tensor memory into shared memory, [batch row][weight row]
+//   all      the sums over the cluster, and the epilogue: a thread has four neighbouring output columns of a batch row
+//
+// Measured over weights that are not in the second-level cache, 64 rows, before (mma.sync with the weights through registers, or tiles of 128 batch rows) and
+// now: 6,144 x 2,048 28.9 -> 10.4 us (2.4 TB/s), 2,048 x 8,192 32.7 -> 12.1 (2.8 TB/s), 16,384 x 2,048 gated 23.3 -> 18.4 (3.6 TB/s; 128 tiles are what 128
+// multiprocessors pull), 5,120 x 960 gated 15.4 -> 7.1, 49,152 x 2,048 46.1 -> 43.5 (4.6 TB/s; 34.3 with 8 rows, 5.9 TB/s).  About 3.4 us of a launch are not
+// the stream: set-up, the first copies' way, the cluster's meeting and the epilogue; that is why small matrices stay with linear_skinny_mma.cu.
+//
+// An output does not depend on M or on the other batch rows: the splits of K depend on N and K alone.  Every wait on an mbarrier is bounded (see
+// tcgen05_common.cuh); a block that gave up still meets its cluster.
+#include <cstdlib>
+
+#include "tcgen05_common.cuh"
+
+namespace vk {
+
+constexpr int RT_BM = 128, RT_BK = 64, RT_STAGES = 4, RT_THREADS = 192, RT_MAX_SPLIT = 8;
+enum { RT_SAME = 0, RT_F32 = 1, RT_ACC = 2, RT_SWIGLU = 3, RT_ROPE = 4 };
+
+struct RtArgs {
+    void* out;
+    int M, N, K, splits;
+    int act;                     // RT_SAME: an activation on the float32 sums (activate_dense; 0 none); RT_SWIGLU: the gate's function (0: silu)
+    const int32_t* positions;
+    const float* cos_t;
+    const float* sin_t;
+    const int32_t* slot;
+    __nv_bfloat16* cache;
+    int nh, nkv, hd, page_size;
+};
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+                   "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
+}
+__device__ __forceinline__ float4 ld_peer4(uint32_t local, int rank) {
+    uint32_t at;
+    float4 v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(local), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_meet() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The sums of four neighbouring weight rows for a batch row, over the cluster's blocks in their order.
+__device__ __forceinline__ float4 rt_sum4(const float* red, int m, int c, int splits) {
+    const uint32_t at = smem_u32(red + m * RT_BM + c);
+    if (splits == 1) return *reinterpret_cast<const float4*>(red + m * RT_BM + c);
+    float4 v[RT_MAX_SPLIT];
+#pragma unroll
+    for (int s = 0; s < RT_MAX_SPLIT; s++)
+        if (s < splits) v[s] = ld_peer4(at, s);
+    float4 t = v[0];
+#pragma unroll
+    for (int s = 1; s < RT_MAX_SPLIT; s++)
+        if (s < splits) { t.x += v[s].x; t.y += v[s].y; t.z += v[s].z; t.w += v[s].w; }
+    return t;
+}
+__device__ __forceinline__ uint2 rt_pack4(float a, float b, float c, float d) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
+    return make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
+__device__ __forceinline__ float rt_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+
+// grid (tiles * splits), a cluster of `splits` blocks a tile
+template <int NB, int EPI>
+__global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                                                                         const RtArgs p, const WaitCtl wc) {
+    constexpr uint32_t W_BYTES = RT_BM * RT_BK * 2, X_BYTES = NB * RT_BK * 2, STAGE_BYTES = W_BYTES + X_BYTES;
+    constexpr uint32_t TM_COLS = NB < 32 ? 32 : NB;
+    static_assert(NB * RT_BM * 4 <= RT_STAGES * STAGE_BYTES, "the sums take the stages' place");
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + RT_STAGES * STAGE_BYTES);
+    uint64_t* empty = full + RT_STAGES;
+    uint64_t* acc_full = empty + RT_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+    float* red = reinterpret_cast<float*>(smem);        // [NB][128], once every product has read its stage
+    __shared__ int failed;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int splits = p.splits, tile = blockIdx.x / splits, rank = blockIdx.x % splits;
+    const int n0 = tile * (EPI == RT_SWIGLU ? RT_BM / 2 : RT_BM);
+    const int num_kb = (p.K + RT_BK - 1) / RT_BK, kb0 = rank * num_kb / splits, n_kb = (rank + 1) * num_kb / splits - kb0;      // at least one
+
+    if (threadIdx.x == 0) {
+        failed = 0;
+        for (int s = 0; s < RT_STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(acc_full, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            auto load_w = [&](int kb, int s) {
+                uint8_t* dst = smem + s * STAGE_BYTES;
+                if (EPI == RT_SWIGLU) {                // 64 gate rows and the same 64 up rows: the map's box is 64 rows
+                    tma_load_2d(dst, &map_w, (kb0 + kb) * RT_BK, n0, &full[s]);
+                    tma_load_2d(dst + W_BYTES / 2, &map_w, (kb0 + kb) * RT_BK, p.N / 2 + n0, &full[s]);
+                } else {
+                    tma_load_2d(dst, &map_w, (kb0 + kb) * RT_BK, n0, &full[s]);
+                }
+            };
+            // (a stage named by wc.skip_stage is left unarmed and unfilled: a test of the give-up path)
+            const int early = n_kb < RT_STAGES ? n_kb : RT_STAGES;
+            for (int kb = 0; kb < early; kb++) {
+                if (kb == wc.skip_stage) continue;
+                mbar_expect_tx(&full[kb], STAGE_BYTES);
+                load_w(kb, kb);
+            }
+            dependency_wait();
+            for (int kb = 0; kb < early; kb++)
+                if (kb != wc.skip_stage) tma_load_2d(smem + kb * STAGE_BYTES + W_BYTES, &map_x, (kb0 + kb) * RT_BK, 0, &full[kb]);
+            for (int kb = early; kb < n_kb; kb++) {
+                const int s = kb % RT_STAGES;
+                if (!mbar_wait(&empty[s], ((kb / RT_STAGES) & 1) ^ 1, wc.cycles)) { give_up(wc.error, &failed, 61); break; }
+                if (kb == wc.skip_stage) continue;
+                mbar_expect_tx(&full[s], STAGE_BYTES);
+                load_w(kb, s);
+                tma_load_2d(smem + s * STAGE_BYTES + W_BYTES, &map_x, (kb0 + kb) * RT_BK, 0, &full[s]);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = umma_idesc_bf16(RT_BM, NB);
+            const uint32_t w_lo0 = umma_desc_lo(smem_u32(smem));
+            for (int kb = 0; kb < n_kb; kb++) {
+                const int s = kb % RT_STAGES;
+                if (!mbar_wait(&full[s], (kb / RT_STAGES) & 1, wc.cycles)) { give_up(wc.error, &failed, 62); break; }
+                tc_fence_after();
+                const uint32_t w_lo = w_lo0 + s * (STAGE_BYTES >> 4), x_lo = w_lo + (W_BYTES >> 4);
+#pragma unroll
+                for (int k = 0; k < RT_BK / 16; k++) umma_bf16_lo(tmem, w_lo + 2 * k, x_lo + 2 * k, idesc, (kb | k) != 0);
+                umma_commit(&empty[s]);
+            }
+            umma_commit(acc_full);                     // arrives when every instruction has written the accumulator
+        }
+    } else {
+        if (!mbar_wait(acc_full, 0, wc.cycles)) { if (lane == 0) give_up(wc.error, &failed, 63); }
+        __syncwarp();
+        const int quarter = warp & 3;
+        const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16);
+        // after a failed wait a copy may still be on its way into the stages: the sums are not written, what is added up is not valid
+        const bool ok = *reinterpret_cast<volatile int*>(&failed) == 0;
+        tc_fence_after();
+        if (__all_sync(0xffffffffu, ok)) {
+            float* mine = red + quarter * 32 + lane;
+            if (NB == 16) {
+                uint32_t r[16];
+                tmem_ld16(acc, r);
+#pragma unroll
+                for (int j = 0; j < 16; j++) mine[j * RT_BM] = __uint_as_float(r[j]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < NB; c += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(acc + c, r);
+                    tmem_loaded(r);
+#pragma unroll
+                    for (int j = 0; j < 32; j++) mine[(c + j) * RT_BM] = __uint_as_float(r[j]);
+                }
+            }
+        }
+        tc_fence_before();
+    }
+    __syncwarp();
+    dependency_wait();                                 // what is read and written from here on is after the kernel before this one
+    let_dependents_start();
+    if (splits > 1) cluster_meet();
+    else __syncthreads();
+
+    // the batch rows rank, rank + splits, ..: a thread takes four neighbouring columns of one at a time
+    constexpr int PIECES = EPI == RT_SWIGLU || EPI == RT_ROPE ? RT_BM / 8 : RT_BM / 4;
+    const int my_rows = (p.M - rank + splits - 1) / splits;
+    for (int it = threadIdx.x; it < my_rows * PIECES; it += RT_THREADS) {
+        const int m = rank + (it / PIECES) * splits, piece = it % PIECES;
+        if (EPI == RT_SWIGLU) {
+            const int inter = p.N / 2, col = n0 + 4 * piece;
+            const float4 g = rt_sum4(red, m, 4 * piece, splits), u = rt_sum4(red, m, RT_BM / 2 + 4 * piece, splits);
+            const float gv[4] = {g.x, g.y, g.z, g.w}, uv[4] = {u.x, u.y, u.z, u.w};
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const float a = rt_round(gv[e]), b = rt_round(uv[e]);
+                v[e] = (p.act ? activate_rt(p.act, a) : a / (1.0f + expf(-a))) * b;
+            }
+            if (col < inter) *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)m * inter + col) = rt_pack4(v[0], v[1], v[2], v[3]);
+        } else if (EPI == RT_ROPE) {
+            const int half = p.hd / 2, per_head = half / 4;                // pieces of four pairs a head
+            const int hh = piece / per_head, j = 4 * (piece % per_head), head = n0 / p.hd + hh;
+            if (head >= p.nh + 2 * p.nkv) continue;
+            const float4 a4 = rt_sum4(red, m, hh * p.hd + j, splits), b4 = rt_sum4(red, m, hh * p.hd + half + j, splits);
+            const bool is_q = head < p.nh, is_k = !is_q && head < p.nh + p.nkv;
+            __nv_bfloat16* dst = nullptr;
+            if (is_q) dst = reinterpret_cast<__nv_bfloat16*>(p.out) + ((size_t)m * p.nh + head) * p.hd;
+            else {
+                const int sl = p.slot[m], kvh = is_k ? head - p.nh : head - p.nh - p.nkv;
+                if (sl >= 0)
+                    dst = p.cache + (size_t)(sl / p.page_size) * 2 * p.nkv * p.page_size * p.hd + (is_k ? 0 : (size_t)p.nkv * p.page_size * p.hd) +
+                          ((size_t)kvh * p.page_size + sl % p.page_size) * p.hd;
+            }
+            if (!dst) continue;
+            const float av[4] = {rt_round(a4.x), rt_round(a4.y), rt_round(a4.z), rt_round(a4.w)}, bv[4] = {rt_round(b4.x), rt_round(b4.y), rt_round(b4.z), rt_round(b4.w)};
+            float ra[4], rb[4];
+            if (is_q || is_k) {
+                const int pos = p.positions[m];
+                const float4 c4 = *reinterpret_cast<const float4*>(p.cos_t + (size_t)pos * half + j), s4 = *reinterpret_cast<const float4*>(p.sin_t + (size_t)pos * half + j);
+                const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    ra[e] = av[e] * cs[e] - bv[e] * sn[e];
+                    rb[e] = bv[e] * cs[e] + av[e] * sn[e];
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++) { ra[e] = av[e]; rb[e] = bv[e]; }
+            }
+            *reinterpret_cast<uint2*>(dst + j) = rt_pack4(ra[0], ra[1], ra[2], ra[3]);
+            *reinterpret_cast<uint2*>(dst + half + j) = rt_pack4(rb[0], rb[1], rb[2], rb[3]);
+        } else {
+            const int col = n0 + 4 * piece;
+            if (col >= p.N) continue;                  // (N is a multiple of four)
+            const size_t at = (size_t)m * p.N + col;
+            float4 old = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (EPI == RT_ACC) old = *reinterpret_cast<const float4*>(reinterpret_cast<float*>(p.out) + at);
+            float4 v = rt_sum4(red, m, 4 * piece, splits);
+            if (EPI == RT_SAME) {
+                if (p.act) { v.x = activate_dense(p.act, v.x); v.y = activate_dense(p.act, v.y); v.z = activate_dense(p.act, v.z); v.w = activate_dense(p.act, v.w); }
+                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + at) = rt_pack4(v.x, v.y, v.z, v.w);
+            } else {
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at) = make_float4(old.x + v.x, old.y + v.y, old.z + v.z, old.w + v.w);
+            }
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    if (splits > 1) cluster_meet();                    // the others have read this block's sums
+    else __syncthreads();
+    if (warp == 1) {
+        if (failed) __nanosleep(200000);               // after a failed wait: let copies in flight land
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TM_COLS) : "memory");
+    }
+}
+
+static bool rt_make_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, int box_rows) {
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) return false;
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+    cuuint32_t box[2] = {(cuuint32_t)RT_BK, (cuuint32_t)box_rows};
+    cuuint32_t elem[2] = {1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Blocks that share a tile's K: as many as the multiprocessors have room for, at most eight (a cluster anywhere), at least one step of 64 columns each.
+static int rt_splits(int tiles, int K) {
+    const int num_kb = (K + RT_BK - 1) / RT_BK;
+    int s = 148 / tiles;
+    if (s > RT_MAX_SPLIT) s = RT_MAX_SPLIT;
+    if (s > num_kb) s = num_kb;
+    return s < 1 ? 1 : s;
+}
+
+template <int NB, int EPI>
+static int rt_launch(const CUtensorMap& mx, const CUtensorMap& mw, RtArgs p, int* error, cudaStream_t stream) {
+    const WaitCtl wc = wait_ctl(error, WAIT_FAMILY_LINEAR);
+    const size_t smem = (size_t)RT_STAGES * (RT_BM + NB) * RT_BK * 2 + 1024 + 128;
+    auto kern = linear_rows_tcgen05_kernel<NB, EPI>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    const int per_tile = EPI == RT_SWIGLU ? RT_BM / 2 : RT_BM, cols = EPI == RT_SWIGLU ? p.N / 2 : p.N;
+    const int tiles = (cols + per_tile - 1) / per_tile;
+    p.splits = rt_splits(tiles, p.K);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles * p.splits);
+    cfg.blockDim = dim3(RT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    static const bool plain = getenv("VITNA_NO_DEPENDENT_LAUNCH") != nullptr;      // for measurements: ordinary launches
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = p.splits;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = plain ? 1 : 2;
+    return (int)cudaLaunchKernelEx(&cfg, kern, mx, mw, p, wc);
+}
+
+}  // namespace vk
+
+using namespace vk;
+
+// x [M, K] bfloat16 with row stride ldx, M <= 64; w [N, K] bfloat16; epi 0 out bfloat16 (act: activate_dense's number), 1 float32, 2 float32 +=,
+// 3 [M, N / 2] bfloat16 = f(first half) * second half (act 0 silu, else activate_rt's number), 4 rotated q, with k and v into the cache (hd 64 or 128).
+// K and ldx multiples of 8, N of 4 (3: of 8), x, w, out (and cache, cos, sin) 16-byte aligned.  error: a word the kernel sets if a bounded wait ran out.
+VK_API int vk_linear_rows_tcgen05(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int epi, int act, const int32_t* positions,
+                                  const float* cos_t, const float* sin_t, const int32_t* slot, void* cache, int nh, int nkv, int hd, int page_size, int* error,
+                                  cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return VK_OK;
+    if (M > 64) return VK_TOO_LARGE;
+    if (K <= 0 || ldx < K || K % 8 != 0 || ldx % 8 != 0 || N % 4 != 0 || epi < 0 || epi > 4 || !error || act < 0 || act > 4 ||
+        (act && epi != RT_SAME && (epi != RT_SWIGLU || act > 3)))
+        return VK_BAD_SHAPE;
+    if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)out % 16)) return VK_BAD_ALIGNMENT;
+    if (epi == RT_SWIGLU && N % 8 != 0) return VK_BAD_SHAPE;
+    if (epi == RT_ROPE) {
+        if (nh <= 0 || nkv <= 0 || (hd != 64 && hd != 128) || page_size <= 0 || N != (nh + 2 * nkv) * hd || !positions || !cos_t || !sin_t || !slot || !cache)
+            return VK_BAD_SHAPE;
+        if (((uintptr_t)cache % 16) || ((uintptr_t)cos_t % 16) || ((uintptr_t)sin_t % 16)) return VK_BAD_ALIGNMENT;
+    }
+    const int nb = M <= 16 ? 16 : M <= 32 ? 32 : 64;
+    CUtensorMap mx, mw;
+    if (!rt_make_map(&mx, x, M, K, ldx, nb) || !rt_make_map(&mw, w, N, K, K, epi == RT_SWIGLU ? RT_BM / 2 : RT_BM)) return VK_BAD_SHAPE;
+    RtArgs p{out, M, N, K, 1, act, positions, cos_t, sin_t, slot, (__nv_bfloat16*)cache, nh, nkv, hd, page_size};
+#define GO(NB)                                                              \
+    switch (epi) {                                                          \
+        case RT_SAME: return rt_launch<NB, RT_SAME>(mx, mw, p, error, stream);     \
+        case RT_F32: return rt_launch<NB, RT_F32>(mx, mw, p, error, stream);       \
+        case RT_ACC: return rt_launch<NB, RT_ACC>(mx, mw, p, error, stream);       \
+        case RT_SWIGLU: return rt_launch<NB, RT_SWIGLU>(mx, mw, p, error, stream); \
+        default: return rt_launch<NB, RT_ROPE>(mx, mw, p, error, stream);          \
+    }
+    if (nb == 16) GO(16)
+    if (nb == 32) GO(32)
+    GO(64)
+#undef GO
+}

@@ -480,10 +480,26 @@ def _mma_norm_smem(M: int, K: int, N: int) -> int:
     return rows * (4 * K + 64) + 4 * K + 8 * (rows // 8) * 512
 
 
+def rows_tcgen05_sizes(M: int, N: int, K: int) -> bool:
+    """Sizes at which the few-rows product with the weights as the tensor cores' 128-row operand is the faster one.  Measured over weights that are not in
+    the second-level cache, microseconds, the mma.sync kernels (or the tcgen05 tile product) against this one:
+      16 / 32 / 64 rows  6144 x 2048  12.7 15.6 28.9 against 8.6 8.9 10.4;  2048 x 8192  14.1 22.0 32.7 against 11.0 10.8 12.1
+                         16384 x 2048 gated  29.9 22.1 23.3 against 16.0 16.8 18.4;  5120 x 960 gated  5.5 10.2 15.4 against 5.6 5.8 7.1
+                         960 x 2560  4.7 5.1 6.3 against 4.5 4.9 6.0;  1600 x 960  3.8 4.3 7.9 against 4.8 5.1 5.7 (not taken below 40 rows)
+      up to 8 rows       6144 x 2048  8.3 against 8.6 and the like, and there the other kernel has the norm in front in its own launch
+      any rows           49152 x 576  19.3 to 22.5 against 11.1 to 17.8;  49152 x 960  27.1 to 30.2 against 17.9 to 26.1 (8 rows, 2048 columns: 34.3 and 33.8)
+    Rows of up to 640 columns are normed inside the mma.sync kernel's launch for up to 64 rows, which is worth more than this kernel gains there."""
+    if N * K >= 24_000_000 and K < 2048:
+        return True
+    return M > 8 and K > NORM_IN_REGISTERS_MAX_K and M * N * K >= 60_000_000
+
+
 def fused_norm_takes(dtype: torch.dtype, M: int, K: int, N: int) -> bool:
     """Whether norm and product should be one launch.  Every block norms the rows it stages, so the rows of a
     block must be few (at most 16) and, in float32, small enough that two blocks share a multiprocessor."""
     if not skinny_takes(dtype, M, K, N):
+        return False
+    if dtype == torch.bfloat16 and N % 8 == 0 and rows_tcgen05_sizes(M, N, K):
         return False
     if dtype == torch.float32 or K % 32 != 0:
         return M <= FUSED_NORM_MAX_ROWS
@@ -561,6 +577,46 @@ def linear_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int,
     return out
 
 
+def rows_tcgen05_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether the few-rows tcgen05 product takes these operands (at most 64 rows; what tcgen05_takes asks for, N a multiple of 8)."""
+    return 0 < x.shape[0] <= SKINNY_MAX_ROWS and tcgen05_takes(x, w) and w.shape[0] % 8 == 0 and out.data_ptr() % 16 == 0
+
+
+def rows_tcgen05_pays(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether the few-rows tcgen05 product takes these operands and is the faster kernel for them (rows_tcgen05_sizes)."""
+    return rows_tcgen05_sizes(x.shape[0], w.shape[0], x.shape[1]) and rows_tcgen05_takes(x, w, out)
+
+
+def linear_rows_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, *, act: int = 0, rope: Optional[tuple] = None) -> torch.Tensor:
+    """out = epilogue(x @ w.T) for at most 64 rows in bfloat16 on the tcgen05 tensor cores, the weights as the 128-row operand and K split over a
+    cluster.  epi and rope as in linear_skinny (head sizes 64 and 128); act: the number of an activation (EPI_SAME: DENSE_ACTIVATIONS + 1; EPI_SWIGLU: the
+    gate's, ACTIVATIONS + 1; 0: none, and silu)."""
+    if not rows_tcgen05_takes(x, w, out):
+        raise KernelError("linear_rows_tcgen05: operands must be bfloat16, 16-byte aligned, of at most 64 rows, with N, K and the row stride multiples of 8")
+    _req(w, "w", torch.bfloat16, 2)
+    M, K = x.shape
+    N = w.shape[0]
+    want = {EPI_SAME: ((M, N), w.dtype), EPI_F32: ((M, N), torch.float32), EPI_ACC: ((M, N), torch.float32), EPI_SWIGLU: ((M, N // 2), w.dtype)}
+    pos = cos = sin = slot = cache = None
+    nh = nkv = hd = ps = 0
+    if epi == EPI_ROPE:
+        pos, cos, sin, slot, cache, nh, nkv, hd = rope
+        _req(pos, "positions", torch.int32, 1); _req(cos, "cos", torch.float32, 2); _req(sin, "sin", torch.float32, 2)
+        _req(slot, "slot_mapping", torch.int32, 1); _req(cache, "cache_layer", w.dtype, 5)
+        ps = cache.shape[3]
+        if (cos.shape[1] != hd // 2 or sin.shape != cos.shape or tuple(cache.shape[1:]) != (2, nkv, ps, hd) or pos.shape[0] < M or slot.shape[0] < M
+                or N != (nh + 2 * nkv) * hd):
+            raise KernelError("linear_rows_tcgen05: the rotary epilogue's arrays do not fit the head counts")
+        want[EPI_ROPE] = ((M, nh * hd), w.dtype)
+    _req(out, "out", want[epi][1], 2)
+    if tuple(out.shape) != want[epi][0] or w.shape[1] != K:
+        raise KernelError(f"linear_rows_tcgen05: shapes x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)} do not fit")
+    ldx = x.stride(0) if M > 1 else max(K, x.stride(0))
+    _check(lib().vk_linear_rows_tcgen05(_p(x), _p(w), _p(out), M, N, K, ldx, epi, act, _p(pos), _p(cos), _p(sin), _p(slot), _p(cache), nh, nkv, hd, ps,
+                                        _p(error_word()), _stream()), "linear_rows_tcgen05")
+    return out
+
+
 # ---------------------------------------------------------------------------
 # Dispatch: which kernel a part's call runs, by dtype and size.
 # ---------------------------------------------------------------------------
@@ -568,6 +624,8 @@ def linear_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int,
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int) -> torch.Tensor:
     """out (=, or += in mode LINEAR_ACC_F32) x @ w.T.  float32 runs on CUDA cores in float32 arithmetic
     (no reduced-precision matrix mode); bfloat16 runs the tensor-core kernel where it takes the sizes."""
+    if rows_tcgen05_pays(x, w, out):
+        return linear_rows_tcgen05(x, w, out, mode)
     if skinny_takes(x.dtype, x.shape[0], x.shape[1], w.shape[0]) and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
         return linear_skinny(x, w, out, mode)
     if tcgen05_takes(x, w) and out.data_ptr() % 16 == 0:
@@ -1107,6 +1165,8 @@ def linear_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: str) -
     if x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[1] == K and tuple(out.shape) == (M, N) and out.dtype == x.dtype:
         _req(w, "w", torch.bfloat16, 2); _req(out, "out", torch.bfloat16, 2)
         act = DENSE_ACTIVATIONS[kind] + 1
+        if rows_tcgen05_pays(x, w, out):
+            return linear_rows_tcgen05(x, w, out, EPI_SAME, act=act)
         if (skinny_takes(x.dtype, M, K, N) and K % 32 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
                 and w.data_ptr() % 16 == 0):
             ldx = x.stride(0) if M > 1 else max(K, x.stride(0))
@@ -1300,6 +1360,8 @@ def linear_gated(x: torch.Tensor, w_gate_up: torch.Tensor, gu: torch.Tensor, out
     if (x.dtype == torch.bfloat16 and w_gate_up.dtype == torch.bfloat16 and w_gate_up.shape == (2 * inter, K) and tuple(out.shape) == (M, inter)
             and out.dtype == x.dtype and out.is_contiguous() and w_gate_up.is_contiguous()):
         act = ACTIVATIONS[kind] + 1
+        if rows_tcgen05_pays(x, w_gate_up, out):
+            return linear_rows_tcgen05(x, w_gate_up, out, EPI_SWIGLU, act=act)
         if (skinny_takes(x.dtype, M, K, 2 * inter) and K % 32 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
                 and w_gate_up.data_ptr() % 16 == 0):
             ldx = x.stride(0) if M > 1 else max(K, x.stride(0))

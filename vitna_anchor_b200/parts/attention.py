@@ -115,6 +115,11 @@ class PagedAttention(Mixer):
             nw, eps = norm.as_rms()
             q = ops.linear_skinny(xn, self.wqkv, q_buf, ops.EPI_ROPE, norm_weight=nw, eps=eps,
                                   rope=(ctx.positions, cos, sin, meta.slot_mapping, cache.pages, self.nh, self.nkv, self.hd))
+        elif (norm is None and rot == self.hd and self.hd in (64, 128) and write_cache and ops.rows_tcgen05_pays(xn, self.wqkv, q_buf)
+              and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0):
+            # a few dozen rows and a large matrix: projections, rotation and cache write in one launch of the tcgen05 few-rows kernel
+            q = ops.linear_rows_tcgen05(xn, self.wqkv, q_buf, ops.EPI_ROPE,
+                                        rope=(ctx.positions, cos, sin, meta.slot_mapping, cache.pages, self.nh, self.nkv, self.hd))
         elif (norm is None and rot == self.hd and write_cache and xn.stride(0) % 8 == 0 and xn.data_ptr() % 16 == 0
               and ops.skinny_takes(ctx.dtype, T, self.hidden, self.qd + 2 * self.kvd)):
             # a few dozen rows: the norm ran once for all of them; projections, rotation and cache write in one launch

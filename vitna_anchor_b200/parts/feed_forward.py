@@ -58,6 +58,9 @@ class SwiGLU(FeedForward):
             # few rows: norm, gate and up, and silu(gate) * up in one launch
             nw, eps = norm.as_rms()
             act = ops.linear_skinny(xn, self.w_gate_up, act_buf, ops.EPI_SWIGLU, norm_weight=nw, eps=eps)
+        elif ops.rows_tcgen05_pays(xn, self.w_gate_up, act_buf):
+            # a few dozen rows and large matrices: the same in one launch of the tcgen05 few-rows kernel
+            act = ops.linear_rows_tcgen05(xn, self.w_gate_up, act_buf, ops.EPI_SWIGLU)
         elif (xn.stride(0) % 8 == 0 and xn.data_ptr() % 16 == 0
               and ops.skinny_takes(ctx.dtype, T, self.hidden, 2 * self.intermediate)):
             # a few dozen rows: the norm ran once for all of them; gate, up and silu(gate) * up in one launch
