@@ -1,0 +1,74 @@
+"""The tcgen05 prompt attention's two forms where their hand-overs can go wrong: walks shorter than the groups and the buffers, reference maxima that rise in every
+step, rows that are not there, and parts of a walk."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(params=[0, 1], ids=["two_groups", "four_groups"])
+def form(request):
+    from vitna_anchor_b200 import ops
+    was = ops.set_prefill_streams(request.param)
+    yield request.param
+    ops.set_prefill_streams(was)
+
+
+def _check(segs, window, ps, rise, nh=3, nkv=1, hd=64, seed=0):
+    """segs: (positions before the portion, its tokens).  rise: what a key's score grows by from 64 keys to the next, in units of log2."""
+    from vitna_anchor_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(seed + int(rise))
+    need = [-(-(p + n) // ps) for p, n in segs]
+    pool = torch.full((sum(need) + 1, 2, nkv, ps, hd), math.nan, device="cuda", dtype=torch.bfloat16)      # slots that no key was written to
+    perm = torch.randperm(sum(need) + 1, generator=g, device="cuda").to(torch.int32)
+    bt = torch.full((len(segs), max(need)), int(perm[-1]), device="cuda", dtype=torch.int32)
+    q = torch.randn(sum(n for _, n in segs), nh, hd, generator=g, device="cuda")
+    q[..., 0] = 1.0
+    q = q.to(torch.bfloat16)
+    want, bound, at, page, tiles = torch.empty(q.shape, device="cuda", dtype=torch.float64), torch.empty(q.shape, device="cuda", dtype=torch.float64), 0, 0, []
+    for i, (past, n) in enumerate(segs):
+        bt[i, :need[i]] = perm[page:page + need[i]]
+        page += need[i]
+        k, v = (torch.randn(past + n, nkv, hd, generator=g, device="cuda") for _ in range(2))
+        k[..., 0] = (torch.arange(past + n, device="cuda") // 64)[:, None] * (rise * math.log(2.0) * 8.0)      # the scale is 1/8
+        k, v = k.to(torch.bfloat16), v.to(torch.bfloat16)
+        for j in range(past + n):
+            pool[bt[i, j // ps], 0, :, j % ps], pool[bt[i, j // ps], 1, :, j % ps] = k[j], v[j]
+        qi, kj = torch.arange(past, past + n, device="cuda")[:, None], torch.arange(past + n, device="cuda")[None, :]
+        hidden = (kj > qi) | ((kj <= qi - window) if window else False)
+        for h in range(nh):
+            s = (q[at:at + n, h].double() @ k[:, h // (nh // nkv)].double().T) * 0.125
+            p = torch.softmax(s.masked_fill(hidden, -math.inf), dim=-1)
+            vv = v[:, h // (nh // nkv)].double()
+            want[at:at + n, h], bound[at:at + n, h] = p @ vv, p @ vv.abs()
+        tiles += [(at + o, min(128, n - o), past + o, i) for o in range(0, n, 128)]
+        at += n
+    tiles.sort(key=lambda t: t[2] + t[1])
+    t = torch.tensor(tiles, dtype=torch.int32, device="cuda")
+    out = torch.full((at, nh * hd), 7.0, device="cuda", dtype=torch.bfloat16)
+    ops.attention_prefill_tcgen05(q.reshape(at, -1).contiguous(), pool, bt, t, out, nh, nkv, hd, 0.125, window)
+    ops.check_device_errors()
+    # a probability is off by what float32 scores of up to |s| are off by (64 products of up to 2^-24 of their sum) and its two parts drop (2^-17), the sum over
+    # them and the products likewise; then the result is rounded to bfloat16
+    top = 0.125 * 64 * 16 + rise * max(p + n for p, n in segs) / 64
+    rel = 2.0 * (top * 64 * 2.0 ** -24 + 2.0 ** -17 + 2.0 ** -16)
+    off = (out.view(at, nh, hd).double() - want).abs()
+    assert bool((off <= rel * bound + 2.0 ** -8 * (want.abs() + rel * bound) + 1e-30).all()), float((off / bound).max())
+
+
+@pytest.mark.parametrize("rise", [0.0, 3.0, 12.0])
+@pytest.mark.parametrize("ps", [8, 16, 128])
+def test_short_and_long_walks(form, ps, rise):
+    _check([(0, 1), (0, 64), (0, 65), (3, 130), (0, 257), (190, 3), (0, 321), (64, 128), (400, 77)], 0, ps, rise)
+
+
+@pytest.mark.parametrize("window,rise", [(1, 0.0), (64, 0.0), (65, 9.0), (200, 0.0), (300, 12.0)])
+def test_windows(form, window, rise):
+    _check([(0, 300), (511, 129), (700, 2), (64, 64)], window, 16, rise, nh=4, nkv=2)
+
+
+@pytest.mark.parametrize("rise", [0.0, 9.0])
+def test_parts(form, rise):
+    _check([(2100, 130), (1000, 25), (1023, 2), (0, 200)], 0, 32, rise, nh=2)

@@ -584,7 +584,8 @@ def rows_tcgen05_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> b
 
 def rows_tcgen05_pays(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
     """Whether the few-rows tcgen05 product takes these operands and is the faster kernel for them (rows_tcgen05_sizes)."""
-    return rows_tcgen05_sizes(x.shape[0], w.shape[0], x.shape[1]) and rows_tcgen05_takes(x, w, out)
+    M = x.shape[0]
+    return M <= SKINNY_MAX_ROWS and rows_tcgen05_sizes(M, w.shape[0], w.shape[1]) and rows_tcgen05_takes(x, w, out)
 
 
 def linear_rows_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, *, act: int = 0, rope: Optional[tuple] = None) -> torch.Tensor:
@@ -656,8 +657,8 @@ def attention_prefill(q: torch.Tensor, cache_layer: torch.Tensor, block_tables: 
 
 
 def set_prefill_streams(mode: int) -> int:
-    """Which tcgen05 prompt-attention kernel a launch takes: 0 the kernel with two threads a query row, 1 the kernel with
-    two streams of key steps, 2 by the size of the launch (the default).  Returns the mode that was in force."""
+    """Which form of the tcgen05 prompt attention a launch for heads of 64 takes: 0 two groups of softmax warps and two blocks a
+    multiprocessor, 1 four groups and one block, 2 by the size of the launch (the default).  Returns the mode that was in force."""
     return int(lib().vk_set_prefill_streams(int(mode)))
 
 
