@@ -135,7 +135,8 @@ def _req(t: torch.Tensor, name: str, dtype=None, dims: Optional[int] = None) -> 
 
 
 def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current device's current stream.  (By torch.cuda.current_stream(), which makes a Stream object, 3.3 us of every launch's 8 to 12 on the host; 0.3 so.)"""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 # ---------------------------------------------------------------------------
@@ -412,6 +413,11 @@ def linear_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: in
     """out (=, or += in mode 2) x @ w.T in bfloat16 on the tcgen05 tensor cores, float32 accumulation in tensor memory."""
     if not tcgen05_takes(x, w):
         raise KernelError("linear_tcgen05: operands must be bfloat16, 16-byte aligned, with K and the row stride multiples of 8")
+    return _linear_tcgen05(x, w, out, mode)
+
+
+def _linear_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int) -> torch.Tensor:
+    """The launch, for operands that tcgen05_takes has looked at."""
     _req(w, "w", torch.bfloat16, 2); _req(out, "out", torch.bfloat16 if mode == LINEAR_SAME else torch.float32, 2)
     M, K = x.shape
     N = w.shape[0]
@@ -625,12 +631,14 @@ def linear_rows_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int) -> torch.Tensor:
     """out (=, or += in mode LINEAR_ACC_F32) x @ w.T.  float32 runs on CUDA cores in float32 arithmetic
     (no reduced-precision matrix mode); bfloat16 runs the tensor-core kernel where it takes the sizes."""
-    if rows_tcgen05_pays(x, w, out):
-        return linear_rows_tcgen05(x, w, out, mode)
-    if skinny_takes(x.dtype, x.shape[0], x.shape[1], w.shape[0]) and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
-        return linear_skinny(x, w, out, mode)
+    M = x.shape[0]
+    if M <= SKINNY_MAX_ROWS:
+        if rows_tcgen05_pays(x, w, out):
+            return linear_rows_tcgen05(x, w, out, mode)
+        if skinny_takes(x.dtype, M, x.shape[1], w.shape[0]) and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
+            return linear_skinny(x, w, out, mode)
     if tcgen05_takes(x, w) and out.data_ptr() % 16 == 0:
-        return linear_tcgen05(x, w, out, mode)
+        return _linear_tcgen05(x, w, out, mode)
     if x.dtype == torch.float32 and _float32_exact:
         return linear_simt(x, w, out, mode, few_rows=0)        # the tile kernel for every batch: one order of sums
     return linear_simt(x, w, out, mode)
