@@ -61,3 +61,35 @@ def test_row_groups(N, K, tiles, mode, act):
             off = off + 2.0 ** -8 * (want.abs() + off)                 # rounded to bfloat16
         assert bool(((out[i].double() - want).abs() <= off).all())
     assert bool((room[M * N:] == 5.0).all())
+
+
+# pairs of blocks: row tiles of 256 with an empty half, with rows in both; widths of 160, 192 and 256 whose last tile ends inside a block's half; one round and several
+@pytest.mark.parametrize("M,N,K", [(1297, 2560, 2056), (2176, 2576, 3000), (2048, 5152, 2048), (1100, 6160, 2048), (3000, 4112, 1800), (2049, 2048, 8200)])
+def test_pairs_of_blocks(M, N, K):
+    from vitna_anchor_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    want, off = x.double() @ w.double().T, K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)      # (as above)
+    f32 = torch.full((M * N + 1024,), 5.0, device="cuda")
+    ops.linear_tcgen05(x, w, f32[:M * N].view(M, N), ops.LINEAR_F32)
+    assert bool(((f32[:M * N].view(M, N).double() - want).abs() <= off).all()) and bool((f32[M * N:] == 5.0).all())
+    base = torch.randn(M, N, generator=g, device="cuda")
+    acc = base.clone()
+    ops.linear_tcgen05(x, w, acc, ops.LINEAR_ACC_F32)
+    assert bool(((acc.double() - want - base.double()).abs() <= off + 2.0 ** -23 * (base.double().abs() + want.abs())).all())
+    same = torch.full((M, N), 5.0, device="cuda", dtype=torch.bfloat16)
+    ops.linear_tcgen05(x, w, same, ops.LINEAR_SAME)
+    assert bool(((same.double() - want).abs() <= off + 2.0 ** -8 * (want.abs() + off)).all())
+    gated = torch.full((M, N // 2), 5.0, device="cuda", dtype=torch.bfloat16)
+    ops.linear_tcgen05_swiglu(x, w, gated)
+    ops.check_device_errors()
+    # both halves are rounded to bfloat16 first; silu's slope stays below 1.1, its own error is a few 2^-22
+    a, b, e = want[:, :N // 2], want[:, N // 2:], off + 2.0 ** -8 * (want.abs() + off)
+    ea, eb, f = e[:, :N // 2], e[:, N // 2:], torch.nn.functional.silu(a)
+    bound = 1.1 * ea * b.abs() + (f.abs() + 1.1 * ea) * eb + (2.0 ** -8 + 2.0 ** -18) * (f * b).abs()
+    assert bool(((gated.double() - f * b).abs() <= 1.01 * bound + 1e-6).all())
+    # a row's bits do not hang on the number of rows
+    part = torch.empty(M - 128, N, device="cuda")
+    ops.linear_tcgen05(x[128:], w, part, ops.LINEAR_F32)
+    assert torch.equal(part, f32[128 * N:M * N].view(M - 128, N))

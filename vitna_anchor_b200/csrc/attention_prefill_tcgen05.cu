@@ -61,15 +61,6 @@ struct ApForm {
     static_assert(STAGES >= BUFS && BUFS >= GROUPS, "phases");
 };
 
-// One lane of a converged warp.  The tensor core's instructions are issued under this and not under "lane 0": what the warp computed outside (descriptors, addresses)
-// then stays in uniform registers.  Measured, 128 x 64 x 16 with the first operand in tensor memory: 50.8 cycles an instruction under "lane 0", 32.2 so (the
-// tensor core's rate).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t e;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(e));
-    return e != 0;
-}
-
 // A row's reference maximum and the number of the step that settled it, in one word of shared memory.
 __device__ __forceinline__ void ap_settle(unsigned long long* at, int step, float m) {
     asm volatile("st.volatile.shared.v2.b32 [%0], {%1, %2};" ::"r"(smem_u32(at)), "r"(__float_as_uint(m)), "r"(step) : "memory");

@@ -153,4 +153,24 @@ inline int launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     return (int)cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// The same as clusters of `blocks` neighbouring blocks.
+template <typename... KArgs, typename... Args>
+inline int launch_dependent_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, int blocks, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    static const bool plain = getenv("VITNA_NO_DEPENDENT_LAUNCH") != nullptr;      // for measurements: ordinary launches
+    cfg.attrs = attr;
+    cfg.numAttrs = plain ? 1 : 2;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
 }  // namespace vk

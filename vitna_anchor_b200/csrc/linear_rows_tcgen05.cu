@@ -19,8 +19,6 @@
 //
 // An output does not depend on M or on the other batch rows: the splits of K depend on N and K alone.  Every wait on an mbarrier is bounded (see
 // tcgen05_common.cuh); a block that gave up still meets its cluster.
-#include <cstdlib>
-
 #include "tcgen05_common.cuh"
 
 namespace vk {
@@ -299,21 +297,7 @@ static int rt_launch(const CUtensorMap& mx, const CUtensorMap& mw, RtArgs p, int
     const int per_tile = EPI == RT_SWIGLU ? RT_BM / 2 : RT_BM, cols = EPI == RT_SWIGLU ? p.N / 2 : p.N;
     const int tiles = (cols + per_tile - 1) / per_tile;
     p.splits = rt_splits(tiles, p.K);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(tiles * p.splits);
-    cfg.blockDim = dim3(RT_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    static const bool plain = getenv("VITNA_NO_DEPENDENT_LAUNCH") != nullptr;      // for measurements: ordinary launches
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = p.splits;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = plain ? 1 : 2;
-    return (int)cudaLaunchKernelEx(&cfg, kern, mx, mw, p, wc);
+    return launch_dependent_cluster(kern, dim3(tiles * p.splits), dim3(RT_THREADS), p.splits, smem, stream, mx, mw, p, wc);
 }
 
 }  // namespace vk

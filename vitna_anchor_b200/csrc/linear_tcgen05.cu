@@ -465,47 +465,92 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tcgen05_kernel(const __grid
 // The tiles are walked in bands of row tiles (`band`), so that the tiles being worked on at one time need few different bytes of both matrices.  Down all rows
 // where x stays in the second-level cache; in bands of 24 row tiles where it does not (8,192 x 8,192 of x: 151 -> 142 us for this product and the output
 // projection, each); in bands of eight for row groups, whose neighbours in x share a weight matrix (8,192 rows, 16 groups, 2,048 x 3,072: 109 -> 96 us).
-constexpr int TW_BN = 256, TW_STAGES = 4, TW_THREADS = 320;      // warps 0 and 1 feed and issue; eight warps drain the accumulators
+//
+// PAIR: two neighbouring blocks (a cluster of two, which are the two multiprocessors of a pair) work on 256 x 256 together: tcgen05.mma with cta_group::2, issued by
+// the first block, takes 128 rows of x from either block's shared memory and half of the weight rows from each, and leaves either block its 128 rows of sums.
+// What bounds a tile of one block is its stages' way from the second-level cache: 48 KB for 512 cycles of the tensor core, 94 bytes a cycle where a multiprocessor gets
+// about 64; a block of a pair brings 32 KB for the same 512 cycles
+// (8,192 x 2,048 x 8,192: 229 -> 209 us, 16,384 x 2,048 weights 374 -> 348, at the rate of a library product alone, 1,580 of 1,692 TFLOP/s).
+constexpr int TW_BN = 256, TW_THREADS = 320;                     // warps 0 and 1 feed and issue; eight warps drain the accumulators
+__host__ __device__ constexpr int tw_stages(bool pair) { return pair ? 6 : 4; }
+
+// What the two blocks of a pair say to each other.  All of it without multicast copies: every block loads what it needs.
+__device__ __forceinline__ void tw_pair_meet() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t tw_at_first(const void* p) {          // the place in the first block's shared memory
+    uint32_t at;
+    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at) : "r"(smem_u32(p)));
+    return at;
+}
+__device__ __forceinline__ void tw_arrive_at_first(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tw_at_first(bar)) : "memory");
+}
+__device__ __forceinline__ void tw_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(x), "r"(y)
+        : "memory");
+}
+__device__ __forceinline__ void tw_umma(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(UMMA_DESC_HI_SW128));
+}
+__device__ __forceinline__ void tw_commit(uint64_t* bar) {                // arrives at both blocks' barrier
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
 
 __host__ __device__ constexpr uint32_t wide_boxes(int epi) { return epi == TC_ACC || epi == TC_F32 ? 8 * 4096 : 8 * 2048; }
 
-template <int EPI, int HD = 0, int BNW = TW_BN>
+template <int EPI, int HD = 0, int BNW = TW_BN, bool PAIR = false>
 __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                          const __grid_constant__ CUtensorMap map_w,
                                                                          const __grid_constant__ CUtensorMap map_out, void* __restrict__ out,
                                                                          int M, int N, int K, const WaitCtl wc, const TcExtra ex) {
-    constexpr uint32_t A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BNW * TC_BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+    constexpr int STAGES = tw_stages(PAIR), ROWS = PAIR ? 2 * TC_BM : TC_BM;       // rows of x of a tile
+    constexpr uint32_t A_BYTES = TC_BM * TC_BK * 2, B_BYTES = (PAIR ? BNW / 2 : BNW) * TC_BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+    constexpr int CHUNKS = BNW / 32, SPLIT = (CHUNKS + 1) / 2;       // of 32 columns; the first of a lane quarter's two epilogue warps takes the first SPLIT
     constexpr uint32_t TM_COLS = 2 * BNW <= 256 ? 256 : 512;      // the two accumulators; tensor memory comes in powers of two
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* boxes = smem + TW_STAGES * STAGE_BYTES;             // 4 KB (bfloat16 results: 2 KB) an epilogue warp
+    uint8_t* boxes = smem + STAGES * STAGE_BYTES;             // 4 KB (bfloat16 results: 2 KB) an epilogue warp
     uint64_t* full = reinterpret_cast<uint64_t*>(boxes + wide_boxes(EPI));
-    uint64_t* empty = full + TW_STAGES;
-    uint64_t* acc_full = empty + TW_STAGES;       // [2]
+    uint64_t* empty = full + STAGES;
+    uint64_t* acc_full = empty + STAGES;       // [2]
     uint64_t* acc_empty = acc_full + 2;           // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     __shared__ int failed, used;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = PAIR ? (int)(blockIdx.x & 1) : 0, worker = PAIR ? blockIdx.x >> 1 : blockIdx.x, workers = PAIR ? gridDim.x >> 1 : gridDim.x;
     const int num_kb = (K + TC_BK - 1) / TC_BK;
     const int tile_cols = EPI == TC_SWIGLU ? BNW / 2 : BNW;                // output columns of a tile
     const int out_cols = EPI == TC_SWIGLU ? ex.inter : N;
     const int tiles_n = (out_cols + tile_cols - 1) / tile_cols;
-    int tiles_m = (M + TC_BM - 1) / TC_BM;
+    int tiles_m = (M + ROWS - 1) / ROWS;
 
     if (threadIdx.x == 0) {
         failed = used = 0;
-        for (int s = 0; s < TW_STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+        for (int s = 0; s < STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], PAIR ? 16 : 8); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) tw_pair_meet();                     // the other block's barriers are set up
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // Barriers and tensor memory are set up while the kernel in front ends (its last blocks hold no place that this one's single wave needs): a layer of a
@@ -530,14 +575,23 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
         if (lane == 0) {
             int kc = 0;                            // stages filled so far, over all of this block's tiles
             bool ok = true;
-            for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-                const int m0 = tile_row(t) * TC_BM, g = group_of(t);
+            for (int t = worker; t < num_tiles && ok; t += workers) {
+                const int m0 = tile_row(t) * ROWS + rank * TC_BM, g = group_of(t);
                 if (g < 0) continue;
                 const int n0 = g * ex.group_rows + tile_col(t) * tile_cols;
                 for (int kb = 0; kb < num_kb; kb++, kc++) {
-                    const int s = kc % TW_STAGES;
-                    if (kc >= TW_STAGES && !mbar_wait(&empty[s], ((kc / TW_STAGES) - 1) & 1, wc.cycles)) { give_up(wc.error, &failed, 31); ok = false; break; }
+                    const int s = kc % STAGES;
+                    if (kc >= STAGES && !mbar_wait(&empty[s], ((kc / STAGES) - 1) & 1, wc.cycles)) { give_up(wc.error, &failed, 31); ok = false; break; }
                     if (kc == wc.skip_stage) continue;      // left unarmed and unfilled: a test of the give-up path
+                    if (PAIR) {
+                        // both blocks' copies are counted by the first one's barrier; the maps' boxes are 128 rows (SwiGLU: the first block has the gate rows of the
+                        // tile's columns, the second the up rows)
+                        if (rank == 0) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
+                        const uint32_t bar = tw_at_first(&full[s]);
+                        tw_load_2d(smem + s * STAGE_BYTES, &map_x, kb * TC_BK, m0, bar);
+                        tw_load_2d(smem + s * STAGE_BYTES + A_BYTES, &map_w, kb * TC_BK, n0 + rank * (EPI == TC_SWIGLU ? ex.inter : BNW / 2), bar);
+                        continue;
+                    }
                     mbar_expect_tx(&full[s], STAGE_BYTES);
                     tma_load_2d(smem + s * STAGE_BYTES, &map_x, kb * TC_BK, m0, &full[s]);
                     if (EPI == TC_SWIGLU) {        // the map's box is 128 rows: gate rows, then the same rows of up
@@ -549,20 +603,45 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                 }
             }
         }
+    } else if (PAIR && warp == 1) {
+        if (rank == 0) {                          // the whole warp, one lane of it issuing (descriptors stay in uniform registers)
+            const uint32_t idesc = umma_idesc_bf16(2 * TC_BM, BNW);
+            const uint32_t a_lo0 = umma_desc_lo(smem_u32(smem));
+            int kc = 0, j = 0;
+            bool ok = true;
+            for (int t = worker; t < num_tiles && ok; t += workers, j++) {
+                const int b = j & 1;
+                if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[b], ((j >> 1) - 1) & 1, wc.cycles))) { if (lane == 0) give_up(wc.error, &failed, 32); break; }
+                tc_fence_after();
+                for (int kb = 0; kb < num_kb; kb++, kc++) {
+                    const int s = kc % STAGES;
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (kc / STAGES) & 1, wc.cycles))) { if (lane == 0) give_up(wc.error, &failed, 33); ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t a_lo = a_lo0 + s * (STAGE_BYTES >> 4), b_lo = a_lo + (A_BYTES >> 4);
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < TC_BK / 16; k++) tw_umma(tmem_base + b * BNW, a_lo + 2 * k, b_lo + 2 * k, idesc, (kb | k) != 0);
+                        tw_commit(&empty[s]);
+                        if (kb == num_kb - 1) tw_commit(&acc_full[b]);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
     } else if (warp == 1) {
         if (lane == 0) {
             const uint32_t idesc = umma_idesc_bf16(TC_BM, BNW);
             const uint32_t a_lo0 = umma_desc_lo(smem_u32(smem));      // low words of the descriptors (see umma_bf16_lo)
             int kc = 0, j = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, j++) {
+            for (int t = worker; t < num_tiles && ok; t += workers, j++) {
                 if (group_of(t) < 0) { j--; continue; }
                 const int b = j & 1;
                 if (j >= 2 && !mbar_wait(&acc_empty[b], ((j >> 1) - 1) & 1, wc.cycles)) { give_up(wc.error, &failed, 32); break; }
                 tc_fence_after();
                 for (int kb = 0; kb < num_kb; kb++, kc++) {
-                    const int s = kc % TW_STAGES;
-                    if (!mbar_wait(&full[s], (kc / TW_STAGES) & 1, wc.cycles)) { give_up(wc.error, &failed, 33); ok = false; break; }
+                    const int s = kc % STAGES;
+                    if (!mbar_wait(&full[s], (kc / STAGES) & 1, wc.cycles)) { give_up(wc.error, &failed, 33); ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_lo = a_lo0 + s * (STAGE_BYTES >> 4), b_lo = a_lo + (A_BYTES >> 4);
 #pragma unroll
@@ -579,18 +658,18 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
         const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
         int j = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, j++) {
+        for (int t = worker; t < num_tiles; t += workers, j++) {
             if (group_of(t) < 0) { j--; continue; }
             const int b = j & 1;
-            const int row = tile_row(t) * TC_BM + quarter * 32 + lane, n0 = tile_col(t) * tile_cols;
+            const int row_first = tile_row(t) * ROWS + rank * TC_BM + quarter * 32, row = row_first + lane, n0 = tile_col(t) * tile_cols;
             if (ok && !__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (j >> 1) & 1, wc.cycles))) { if (lane == 0) give_up(wc.error, &failed, 34); ok = false; }
             // A residual sum goes out by TMA reductions from shared memory (see the narrow kernel), a box of 32 rows x 32 columns a warp: from the warp's
             // own box, or, for the block's last tile, whose epilogue hides behind no further tile, from the stages, which are free by now.
             if (ok && EPI == TC_ACC && ex.tma_out) {
                 tc_fence_after();
                 const uint32_t acc = lane_base + b * BNW;
-                const bool last = t + (int)gridDim.x >= num_tiles;
-                const int row0 = tile_row(t) * TC_BM + quarter * 32;
+                const bool last = t + workers >= num_tiles;
+                const int row0 = row_first;
 #pragma unroll 1
                 for (int c = half * (BNW / 2); c < (half + 1) * (BNW / 2); c += 32) {
                     uint32_t r[32];
@@ -620,9 +699,9 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                 if (EPI == TC_SWIGLU) {
                     // the tile's gate columns in chunks of 32: the first of a lane quarter's two warps takes the first half of
                     // them (rounded up), the second the rest
-                    constexpr int CHUNKS = BNW / 2 / 32, SPLIT = (CHUNKS + 1) / 2;
+                    constexpr int GATES = BNW / 2 / 32, GSPLIT = (GATES + 1) / 2;
 #pragma unroll 1
-                    for (int c = (half == 0 ? 0 : SPLIT) * 32; c < (half == 0 ? SPLIT : CHUNKS) * 32; c += 32) {
+                    for (int c = (half == 0 ? 0 : GSPLIT) * 32; c < (half == 0 ? GSPLIT : GATES) * 32; c += 32) {
                         uint32_t gr[32], ur[32];
                         tmem_ld32_nowait(acc + c, gr);
                         tmem_ld32_nowait(acc + BNW / 2 + c, ur);
@@ -689,7 +768,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                     }
                 } else if (EPI == TC_SAME) {
 #pragma unroll 1
-                    for (int c = half * (BNW / 2); c < (half + 1) * (BNW / 2); c += 32) {
+                    for (int c = half * SPLIT * 32; c < (half ? CHUNKS : SPLIT) * 32; c += 32) {
                         uint32_t r[32];
                         tmem_ld32(acc + c, r);
                         tmem_loaded(r);
@@ -708,7 +787,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                     }
                 } else {
 #pragma unroll 1
-                    for (int c = half * (BNW / 2); c < (half + 1) * (BNW / 2); c += 32) {
+                    for (int c = half * SPLIT * 32; c < (half ? CHUNKS : SPLIT) * 32; c += 32) {
                         uint32_t r[32];
                         tmem_ld32(acc + c, r);
                         tmem_loaded(r);
@@ -716,7 +795,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                         if (EPI == TC_F32) {
                             if (col < N)
                                 store_rows_f32(reinterpret_cast<float*>(boxes + (warp - 2) * 4096), r, reinterpret_cast<float*>(out),
-                                               tile_row(t) * TC_BM + quarter * 32, col, M, N, lane);
+                                               row_first, col, M, N, lane);
                             continue;
                         }
                         if (row >= M || col >= N) continue;
@@ -748,11 +827,20 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                 tc_fence_before();
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive_plain(&acc_empty[b]);      // kept even after a failed wait: nobody waits for this warp without a limit
+            if (lane == 0) { if (PAIR) tw_arrive_at_first(&acc_empty[b]); else mbar_arrive_plain(&acc_empty[b]); }      // kept even after a failed wait: nobody waits for this warp without a limit
         }
         if (EPI == TC_ACC && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // the boxes outlive their reductions
     }
+    __syncwarp();
     tc_fence_before();
+    if (PAIR) {
+        if (threadIdx.x == 0 && failed) __nanosleep(200000);      // (as below, before the other block may leave)
+        __syncwarp();
+        tw_pair_meet();                       // what either block sends the other (copies' counts, arrivals) has come; the sums have been read
+        tc_fence_after();
+        if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TM_COLS) : "memory");
+        return;
+    }
     __syncthreads();
     if (warp == 1) {
         if (failed) __nanosleep(200000);      // after a failed wait: let copies in flight land
@@ -830,24 +918,54 @@ static bool wide_takes(int M, int out_cols, int K, int tile_cols = TW_BN) {
     return K >= 2048 || tiles * 4 >= (long long)sm_count() * 5;
 }
 
-template <int EPI, int HD = 0, int BNW = TW_BN>
+template <int EPI, int HD = 0, int BNW = TW_BN, bool PAIR = false>
 static int launch_wide(const CUtensorMap& mx, const CUtensorMap& mw, void* out, int M, int N, int K, int* error, cudaStream_t stream,
                        const TcExtra& ex = TcExtra{}) {
     const WaitCtl wc = wait_ctl(error, WAIT_FAMILY_LINEAR_WIDE);
-    const size_t smem = (size_t)TW_STAGES * (TC_BM * TC_BK * 2 + BNW * TC_BK * 2) + wide_boxes(EPI) + 1024 + 128;
+    const size_t smem = (size_t)tw_stages(PAIR) * (TC_BM * TC_BK * 2 + (PAIR ? BNW / 2 : BNW) * TC_BK * 2) + wide_boxes(EPI) + 1024 + 192;
     TcExtra exx = ex;
     CUtensorMap mo = mx;                               // (a valid map for the epilogues that do not use it)
     exx.tma_out = 0;
     if (EPI == TC_ACC && N % 4 == 0 && ((uintptr_t)out % 16 == 0) && make_out_map(&mo, out, M, N, 32)) exx.tma_out = 1;
     exx.band = exx.tile_group ? 8 : (size_t)M * K * 2 > ((size_t)64 << 20) ? 24 : 1 << 20;
-    auto kern = linear_tcgen05_wide_kernel<EPI, HD, BNW>;
+    auto kern = linear_tcgen05_wide_kernel<EPI, HD, BNW, PAIR>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const int tile_cols = EPI == TC_SWIGLU ? BNW / 2 : BNW;
     const int cols = EPI == TC_SWIGLU ? ex.inter : N;
-    const long long tiles = (long long)((M + TC_BM - 1) / TC_BM) * ((cols + tile_cols - 1) / tile_cols);
-    const int grid = tiles < sm_count() ? (int)tiles : sm_count();
-    return launch_dependent(kern, dim3(grid), dim3(TW_THREADS), smem, stream, mx, mw, mo, out, M, N, K, wc, exx);
+    const int rows = PAIR ? 2 * TC_BM : TC_BM, workers = PAIR ? sm_count() / 2 : sm_count();
+    const long long tiles = (long long)((M + rows - 1) / rows) * ((cols + tile_cols - 1) / tile_cols);
+    if (PAIR) exx.band = (exx.band + 1) / 2;
+    const int grid = (int)(tiles < workers ? tiles : workers) * (PAIR ? 2 : 1);
+    if (!PAIR) return launch_dependent(kern, dim3(grid), dim3(TW_THREADS), smem, stream, mx, mw, mo, out, M, N, K, wc, exx);
+    return launch_dependent_cluster(kern, dim3(grid), dim3(TW_THREADS), 2, smem, stream, mx, mw, mo, out, M, N, K, wc, exx);
+}
+
+// Whether a wide product without row groups is worked out by pairs of blocks: where the multiprocessors have enough columns of K to go through that the shorter
+// way of the operands outweighs the pairs' meetings (about a microsecond a launch), and 256-row tiles need no more rounds.  One block a tile against pairs, us:
+// 8,192 x 16,384 x 2,048 374 / 348, 8,192 x 2,048 x 8,192 229 / 209, 8,192 x 6,144 x 2,048 160 / 142, 2,048 x 16,384 x 2,048 100 / 93, 2,048 x 6,160 x 2,048 46 / 42,
+// 2,048 x 2,560 x 2,048 24.5 / 23.1; but 2,048 x 2,048 x 2,048 17.8 / 19.1, 700 x 2,048 x 8,192 (48 tiles: nothing else wants the second-level cache) 43.6 / 44.9,
+// 1,301 x 5,120 x 960 17.5 / 18.4.
+// VITNA_TCGEN05_PAIR=0 or 1 overrides (for measurements).
+static bool pair_takes(int M, int out_cols, int tile_cols, int K) {
+    static const int forced = [] { const char* e = getenv("VITNA_TCGEN05_PAIR"); return e ? (e[0] == '1' ? 1 : 0) : 2; }();
+    if (forced != 2) return forced == 1;
+    const long long tn = (out_cols + tile_cols - 1) / tile_cols, sms = sm_count(), tiles = (M + 127) / 128 * tn;
+    const long long one = (tiles + sms - 1) / sms, two = ((M + 255) / 256 * tn + sms / 2 - 1) / (sms / 2);
+    return two <= one && tiles >= 100 && tiles * K >= sms * 2800;
+}
+
+// The width in weight rows of a wide tile (256, 192 or 160) that a block's rounds of are the shortest, counting a round's own cost as 32 columns: 2,011 x 2,576 x
+// 1,024 is 176 tiles of 256 columns for 148 multiprocessors (two rounds, and too few for this kernel: 19.8 us in narrow tiles), 272 of 160 (two shorter ones: 15.7).
+static int wide_width(int M, int N) {
+    const long long tiles_m = (M + TC_BM - 1) / TC_BM, sms = sm_count();
+    int best = 256;
+    long long cost = 0;
+    for (int w : {256, 192, 160}) {
+        const long long c = (tiles_m * ((N + w - 1) / w) + sms - 1) / sms * (w + 32);
+        if (w == 256 || c < cost) { best = w; cost = c; }
+    }
+    return best;
 }
 
 }  // namespace vk
@@ -866,20 +984,23 @@ static int linear_tcgen05_impl(const void* x, const void* w, void* out, int M, i
     if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)out % 16)) return VK_BAD_ALIGNMENT;
     const int bn = N >= 2048 ? 128 : 64;
     if ((M + TC_BM - 1) / TC_BM > 65535) return VK_TOO_LARGE;
-    if (wide_takes(M, N, K)) {
+    const int width = mode == 2 ? TW_BN : wide_width(M, N);
+    if (wide_takes(M, N, K, width)) {
         CUtensorMap wx, ww;
-        // tiles of 192 columns where a block's rounds of them are shorter than its rounds of 256 (see the gated form)
-        const long long tiles_m = (M + TC_BM - 1) / TC_BM, sms = sm_count();
-        const long long rounds256 = (tiles_m * ((N + 255) / 256) + sms - 1) / sms, rounds192 = (tiles_m * ((N + 191) / 192) + sms - 1) / sms;
-        if (mode != 2 && rounds192 * 192 < rounds256 * 256) {
-            if (!make_map(&wx, x, M, K, ldx, TC_BM) || !make_map(&ww, w, N, K, K, 192)) return VK_BAD_SHAPE;
-            if (mode == 0) return launch_wide<TC_SAME, 0, 192>(wx, ww, out, M, N, K, error, stream, ex);
-            return launch_wide<TC_F32, 0, 192>(wx, ww, out, M, N, K, error, stream);
+        const bool pair = pair_takes(M, N, width, K);
+        if (!make_map(&wx, x, M, K, ldx, TC_BM) || !make_map(&ww, w, N, K, K, pair ? width / 2 : width)) return VK_BAD_SHAPE;
+#define GO(EPI, W)                                                                                                       \
+    return pair ? launch_wide<EPI, 0, W, true>(wx, ww, out, M, N, K, error, stream, ex) : launch_wide<EPI, 0, W>(wx, ww, out, M, N, K, error, stream, ex)
+        if (mode == 2) GO(TC_ACC, 256);
+        if (mode == 1) {
+            if (width == 160) GO(TC_F32, 160);
+            if (width == 192) GO(TC_F32, 192);
+            GO(TC_F32, 256);
         }
-        if (!make_map(&wx, x, M, K, ldx, TC_BM) || !make_map(&ww, w, N, K, K, TW_BN)) return VK_BAD_SHAPE;
-        if (mode == 0) return launch_wide<TC_SAME>(wx, ww, out, M, N, K, error, stream, ex);
-        if (mode == 1) return launch_wide<TC_F32>(wx, ww, out, M, N, K, error, stream);
-        return launch_wide<TC_ACC>(wx, ww, out, M, N, K, error, stream);
+        if (width == 160) GO(TC_SAME, 160);
+        if (width == 192) GO(TC_SAME, 192);
+        GO(TC_SAME, 256);
+#undef GO
     }
     CUtensorMap mx, mw;
     if (!make_map(&mx, x, M, K, ldx, TC_BM) || !make_map(&mw, w, N, K, K, bn)) return VK_BAD_SHAPE;
@@ -955,11 +1076,12 @@ static int linear_tcgen05_gated_impl(const void* x, const void* w, void* out, in
         // mostly empty (192 tiles on 148 multiprocessors: two rounds of 256 columns against two of 192).
         const long long tiles_m = (M + TC_BM - 1) / TC_BM, sms = sm_count();
         const long long rounds256 = (tiles_m * ((inter + 127) / 128) + sms - 1) / sms, rounds192 = (tiles_m * ((inter + 95) / 96) + sms - 1) / sms;
-        if (rounds192 * 192 < rounds256 * 256) {
-            if (!make_map(&mx, x, M, K, ldx, TC_BM) || !make_map(&mw, w, 2 * inter, K, K, 96)) return VK_BAD_SHAPE;
-            return launch_wide<TC_SWIGLU, 0, 192>(mx, mw, out, M, 2 * inter, K, error, stream, ex);
-        }
-        if (!make_map(&mx, x, M, K, ldx, TC_BM) || !make_map(&mw, w, 2 * inter, K, K, TW_BN / 2)) return VK_BAD_SHAPE;
+        const int half = rounds192 * 192 < rounds256 * 256 ? 96 : 128;
+        const bool pair = pair_takes(M, inter, half, K);
+        if (!make_map(&mx, x, M, K, ldx, TC_BM) || !make_map(&mw, w, 2 * inter, K, K, half)) return VK_BAD_SHAPE;
+        if (half == 96 && pair) return launch_wide<TC_SWIGLU, 0, 192, true>(mx, mw, out, M, 2 * inter, K, error, stream, ex);
+        if (half == 96) return launch_wide<TC_SWIGLU, 0, 192>(mx, mw, out, M, 2 * inter, K, error, stream, ex);
+        if (pair) return launch_wide<TC_SWIGLU, 0, TW_BN, true>(mx, mw, out, M, 2 * inter, K, error, stream, ex);
         return launch_wide<TC_SWIGLU>(mx, mw, out, M, 2 * inter, K, error, stream, ex);
     }
     if (!make_map(&mx, x, M, K, ldx, TC_BM) || !make_map(&mw, w, 2 * inter, K, K, 64)) return VK_BAD_SHAPE;
@@ -1025,7 +1147,10 @@ VK_API int vk_linear_tcgen05_rope(const void* x, const void* w, void* q_out, int
     ex.positions = positions; ex.cos_t = cos_t; ex.sin_t = sin_t; ex.slot = slot; ex.cache = (__nv_bfloat16*)cache;
     ex.nh = nh; ex.nkv = nkv; ex.hd = hd; ex.page_size = page_size;
     if (wide_takes(M, N, K)) {
-        if (!make_map(&mw, w, N, K, K, TW_BN)) return VK_BAD_SHAPE;
+        const bool pair = pair_takes(M, N, TW_BN, K);
+        if (!make_map(&mw, w, N, K, K, pair ? TW_BN / 2 : TW_BN)) return VK_BAD_SHAPE;
+        if (pair && hd == 64) return launch_wide<TC_ROPE, 64, TW_BN, true>(mx, mw, q_out, M, N, K, error, stream, ex);
+        if (pair) return launch_wide<TC_ROPE, 128, TW_BN, true>(mx, mw, q_out, M, N, K, error, stream, ex);
         if (hd == 64) return launch_wide<TC_ROPE, 64>(mx, mw, q_out, M, N, K, error, stream, ex);
         return launch_wide<TC_ROPE, 128>(mx, mw, q_out, M, N, K, error, stream, ex);
     }
