@@ -76,27 +76,31 @@ __global__ void __launch_bounds__(1024) delta_prepare_kernel(
 }
 
 // The same for a prompt's step and convolutions of up to DP_TAPS taps: DP_TOKENS neighbouring tokens a block, so that an input is read once for its taps' tokens and not
-// once for each; the same operations in the same order, so the same bits.  2,048 tokens of 1,152 channels: 23.6 us a block a token, 19.5 here.  smem: act [DP_TOKENS][2 G dk].
-constexpr int DP_TOKENS = 8, DP_TAPS = 4;
+// once for each; the same operations in the same order, so the same bits.  A block has a slice of the channels, about one a thread: whole q or k heads (blockIdx.y up
+// to `head_slices`), or DP_SLICE of v's.  What bounds it are the trips to memory of a thread's channel; a thread with all of a token's channels one after another made
+// four and more of them in a row (2,048 tokens: 19.1 -> 12.7 us with 960 channels, 43.9 -> 21.7 with 3,072).  smem: act [DP_TOKENS][heads of a slice x dk].
+constexpr int DP_TOKENS = 8, DP_TAPS = 4, DP_SLICE = 256;
 
-__global__ void __launch_bounds__(256, 4) delta_prepare_tokens_kernel(
+__global__ void __launch_bounds__(DP_SLICE, 4) delta_prepare_tokens_kernel(
     const float* __restrict__ proj, const float* __restrict__ conv_w, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
     const int32_t* __restrict__ token_seg, const int32_t* __restrict__ seg_starts, const int32_t* __restrict__ seg_slots,
     const float* __restrict__ state, size_t state_stride, size_t conv_off, float* __restrict__ prep, int P, int G, int H, int dk, int dv,
-    int taps, int tokens) {
+    int taps, int tokens, int slice_heads, int head_slices) {
     extern __shared__ float act[];
     __shared__ int place[DP_TOKENS];                         // of the token in this step's portion of its request
     __shared__ const float* olds[DP_TOKENS];                 // [taps-1][C], or null
     const int t0 = blockIdx.x * DP_TOKENS, cnt = min(DP_TOKENS, tokens - t0), tid = threadIdx.x;
     const int QK = 2 * G * dk, C = QK + H * dv, N = C + H * dv + 2 * H;
+    const bool heads = (int)blockIdx.y < head_slices;
+    const int first_head = blockIdx.y * slice_heads, n_heads = heads ? min(slice_heads, 2 * G - first_head) : 0, width = n_heads * dk;
+    const int c_lo = heads ? first_head * dk : QK + ((int)blockIdx.y - head_slices) * DP_SLICE, c_hi = heads ? c_lo + width : min(C, c_lo + DP_SLICE);
     if (tid < cnt) {
         const int seg = token_seg[t0 + tid], slot = seg_slots[seg];
         place[tid] = t0 + tid - seg_starts[seg];
         olds[tid] = slot >= 0 ? state + (size_t)slot * state_stride + conv_off : nullptr;
     }
-    __syncthreads();
-    for (int c = tid; c < C; c += blockDim.x) {
-        float x[DP_TOKENS + DP_TAPS - 1], w[DP_TAPS];        // x[u]: the input of token t0 - (DP_TAPS - 1) + u, whosever it is
+    float x[DP_TOKENS + DP_TAPS - 1], w[DP_TAPS];            // x[u]: the input of token t0 - (DP_TAPS - 1) + u, whosever it is
+    auto fetch = [&](int c) {
 #pragma unroll
         for (int u = 0; u < DP_TOKENS + DP_TAPS - 1; u++) {
             const int t = t0 - (DP_TAPS - 1) + u;
@@ -104,37 +108,56 @@ __global__ void __launch_bounds__(256, 4) delta_prepare_tokens_kernel(
         }
 #pragma unroll
         for (int j = 0; j < DP_TAPS; j++) w[j] = j < taps ? conv_w[(size_t)c * taps + (taps - 1 - j)] : 0.0f;
+    };
+    if (c_lo + tid < c_hi) fetch(c_lo + tid);                // (on their way beside the tokens' places)
+    // most blocks lie inside a request's portion: none of their tokens asks for an input of an earlier step
+    const bool inside = __syncthreads_and(tid >= cnt || place[tid < DP_TOKENS ? tid : 0] >= DP_TAPS - 1) && taps == DP_TAPS && cnt == DP_TOKENS;
+    for (int c = c_lo + tid; c < c_hi; c += DP_SLICE) {
+        if (c != c_lo + tid) fetch(c);
+        float* to = heads ? act + c - c_lo : prep + (size_t)t0 * P + c;
+        const int step = heads ? width : P;
+        if (inside) {
 #pragma unroll
-        for (int q = 0; q < DP_TOKENS; q++) {
+            for (int q = 0; q < DP_TOKENS; q++, to += step) {
+                float acc = 0.0f;
+#pragma unroll
+                for (int j = DP_TAPS - 1; j >= 0; j--) acc = fmaf(w[j], x[q + DP_TAPS - 1 - j], acc);      // oldest input first
+                *to = silu_f(acc);
+            }
+            continue;
+        }
+#pragma unroll
+        for (int q = 0; q < DP_TOKENS; q++, to += step) {
             if (q >= cnt) break;
             const int i = place[q];
             float acc = 0.0f;
 #pragma unroll
-            for (int j = DP_TAPS - 1; j >= 0; j--) {         // oldest input first
+            for (int j = DP_TAPS - 1; j >= 0; j--) {
                 if (j >= taps) continue;
                 float v = x[q + DP_TAPS - 1 - j];
                 if (i < j) v = olds[q] ? olds[q][(size_t)(taps - 1 + i - j) * C + c] : 0.0f;
                 acc = fmaf(w[j], v, acc);
             }
-            const float a = silu_f(acc);
-            if (c < QK) act[q * QK + c] = a;
-            else prep[(size_t)(t0 + q) * P + c] = a;
+            *to = silu_f(acc);
         }
     }
-    __syncthreads();
-    const int warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
-    for (int unit = warp; unit < cnt * 2 * G; unit += nwarps) {      // q heads, then k heads of a token
-        const int q = unit / (2 * G), hq = unit - q * 2 * G;
-        const float* v = act + (size_t)q * QK + (size_t)hq * dk;
-        float ss = 0.0f;
-        for (int d = lane; d < dk; d += 32) ss = fmaf(v[d], v[d], ss);
-        ss = warp_sum(ss);
-        float inv = 1.0f / sqrtf(ss + 1e-6f);
-        if (hq < G) inv *= 1.0f / sqrtf((float)dk);
-        float* out = prep + (size_t)(t0 + q) * P + (size_t)hq * dk;
-        for (int d = lane; d < dk; d += 32) out[d] = v[d] * inv;
+    if (heads) {
+        __syncthreads();
+        const int warp = tid >> 5, lane = tid & 31, nwarps = DP_SLICE / 32;
+        for (int unit = warp; unit < cnt * n_heads; unit += nwarps) {
+            const int q = unit / n_heads, j = unit - q * n_heads, hq = first_head + j;      // q heads, then k heads
+            const float* v = act + (size_t)q * width + (size_t)j * dk;
+            float ss = 0.0f;
+            for (int d = lane; d < dk; d += 32) ss = fmaf(v[d], v[d], ss);
+            ss = warp_sum(ss);
+            float inv = 1.0f / sqrtf(ss + 1e-6f);
+            if (hq < G) inv *= 1.0f / sqrtf((float)dk);
+            float* out = prep + (size_t)(t0 + q) * P + (size_t)hq * dk;
+            for (int d = lane; d < dk; d += 32) out[d] = v[d] * inv;
+        }
     }
-    for (int e = tid; e < cnt * H; e += blockDim.x) {
+    if (blockIdx.y + 1 < gridDim.y) return;
+    for (int e = tid; e < cnt * H; e += DP_SLICE) {          // the last slice: the tokens' gates
         const int q = e / H, h = e - q * H;
         const float* in = proj + (size_t)(t0 + q) * N + C + H * dv;
         float* out = prep + (size_t)(t0 + q) * P + C;
@@ -541,11 +564,14 @@ VK_API int vk_delta_prepare(const float* proj, const float* conv_w, const float*
     if (tokens <= DR_DEPENDENT_TOKENS)
         return launch_dependent(delta_prepare_kernel, dim3(tokens), dim3(threads), smem, stream, proj, conv_w, a_log, dt_bias, token_seg, seg_starts,
                                 seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps);
-    // from 148 blocks on: below, a block a token has the shorter way.  (What a launch may have without asking, 48 KB, counts the kernel's `place` and `olds` too.)
-    const size_t smem8 = (size_t)DP_TOKENS * 2 * G * dk * sizeof(float);
-    if (taps <= DP_TAPS && tokens >= 148 * DP_TOKENS && smem8 + DP_TOKENS * (sizeof(int) + sizeof(float*)) <= 48 * 1024)
-        return launch_plain(delta_prepare_tokens_kernel, dim3((tokens + DP_TOKENS - 1) / DP_TOKENS), dim3(256), smem8, stream, proj, conv_w, a_log, dt_bias, token_seg,
-                            seg_starts, seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps, tokens);
+    // Tokens in eights, the channels in slices, against a block a token, us: 65 / 400 / 2,048 tokens of 960 channels 10.3 / 9.5 / 24.9 against 9.7 / 9.4 / 12.7, of 3,072
+    // channels 12.6 / 16.6 / 55.6 against 6.8 / 8.5 / 21.7.  (What a launch may have without asking, 48 KB, counts the kernel's `place` and `olds` too.)
+    const int slice_heads = dk < DP_SLICE ? (DP_SLICE / dk < 2 * G ? DP_SLICE / dk : 2 * G) : 1, head_slices = (2 * G + slice_heads - 1) / slice_heads;
+    const int slices = head_slices + (H * dv + DP_SLICE - 1) / DP_SLICE;
+    const size_t smem8 = (size_t)DP_TOKENS * slice_heads * dk * sizeof(float);
+    if (taps <= DP_TAPS && slices <= 65535 && smem8 + DP_TOKENS * (sizeof(int) + sizeof(float*)) <= 48 * 1024)
+        return launch_plain(delta_prepare_tokens_kernel, dim3((tokens + DP_TOKENS - 1) / DP_TOKENS, slices), dim3(DP_SLICE), smem8, stream, proj, conv_w, a_log, dt_bias, token_seg,
+                            seg_starts, seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps, tokens, slice_heads, head_slices);
     return launch_plain(delta_prepare_kernel, dim3(tokens), dim3(256), smem, stream, proj, conv_w, a_log, dt_bias, token_seg, seg_starts,
                         seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps);
 }
