@@ -93,3 +93,47 @@ def test_pairs_of_blocks(M, N, K):
     part = torch.empty(M - 128, N, device="cuda")
     ops.linear_tcgen05(x[128:], w, part, ops.LINEAR_F32)
     assert torch.equal(part, f32[128 * N:M * N].view(M - 128, N))
+
+
+# the edge of a round of narrow tiles (296 of 64 rows, 333 go to wide ones; 148 of 128 rows, 152), wide tiles of a short K and of few columns, sums in tiles of 160
+# and 192 columns with and without whole rows of 16 bytes
+@pytest.mark.parametrize("shape", [(4736, 512, 72), (4700, 520, 72), (4736, 2048, 768), (500, 4736, 768), (1000, 2426, 776), (8190, 576, 64), (8190, 570, 136),
+                                   (2999, 2046, 264), (2999, 2052, 128), (20000, 100, 72)])
+def test_products_at_the_edge_of_a_round(shape):
+    test_float32_results_and_sums(shape)
+
+
+# the fused turn in wide tiles where the last tile holds one, two and three heads of four (64 columns) and one of two (128)
+@pytest.mark.parametrize("nh,nkv,hd,K", [(9, 3, 64, 576), (3, 1, 64, 264), (6, 2, 64, 64), (5, 3, 128, 136)])
+def test_turned_heads_at_the_edge_of_a_round(nh, nkv, hd, K):
+    from vitna_anchor_b200 import ops
+    M, ps, N = 8100, 16, (nh + 2 * nkv) * hd
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    pos = torch.randint(0, 500, (M,), generator=g, device="cuda", dtype=torch.int32)
+    slot = torch.randperm(M + 60, generator=g, device="cuda")[:M].to(torch.int32)
+    slot[::7] = -1
+    pages = (M + 60 + ps - 1) // ps
+    ang = torch.rand(500, hd // 2, generator=g, device="cuda") * 6.0
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    cache = torch.full((pages, 2, nkv, ps, hd), 7.0, device="cuda", dtype=torch.bfloat16)
+    q = torch.full((M, nh * hd), 7.0, device="cuda", dtype=torch.bfloat16)
+    ops.linear_tcgen05_rope(x, w, q, pos, cos, sin, slot, cache, nh, nkv, hd)
+    ops.check_device_errors()
+    p, off = x.double() @ w.double().T, K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)
+    p, off = p.view(M, nh + 2 * nkv, hd), (off + 2.0 ** -8 * (p.abs() + off)).view(M, nh + 2 * nkv, hd)      # the projections are rounded to bfloat16 first
+    c, s = cos.double()[pos.long()][:, None], sin.double()[pos.long()][:, None]
+    t, o = p[:, :nh + nkv], off[:, :nh + nkv]
+    a, b, oa, ob = t[..., :hd // 2], t[..., hd // 2:], o[..., :hd // 2], o[..., hd // 2:]
+    turned = torch.cat([a * c - b * s, b * c + a * s], -1)
+    slack = torch.cat([oa * c.abs() + ob * s.abs(), ob * c.abs() + oa * s.abs()], -1) + 2.0 ** -22 * (torch.cat([a, a], -1).abs() + torch.cat([b, b], -1).abs())
+    slack = slack + 2.0 ** -8 * (turned.abs() + slack)                       # rounded to bfloat16
+    assert bool(((q.view(M, nh, hd).double() - turned[:, :nh]).abs() <= slack[:, :nh]).all())
+    held = torch.full((pages * ps, 2, nkv, hd), 7.0, device="cuda", dtype=torch.float64)
+    room = torch.zeros_like(held)
+    on = slot >= 0
+    held[slot[on].long(), 0], room[slot[on].long(), 0] = turned[on, nh:], slack[on, nh:]
+    held[slot[on].long(), 1], room[slot[on].long(), 1] = p[on, nh + nkv:], off[on, nh + nkv:]
+    got = cache.permute(0, 3, 1, 2, 4).reshape(pages * ps, 2, nkv, hd).double()
+    assert bool(((got - held).abs() <= room).all())

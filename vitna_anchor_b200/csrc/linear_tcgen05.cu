@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                 const bool last = t + workers >= num_tiles;
                 const int row0 = row_first;
 #pragma unroll 1
-                for (int c = half * (BNW / 2); c < (half + 1) * (BNW / 2); c += 32) {
+                for (int c = half * SPLIT * 32; c < (half ? CHUNKS : SPLIT) * 32; c += 32) {
                     uint32_t r[32];
                     tmem_ld32(acc + c, r);
                     tmem_loaded(r);
@@ -901,21 +901,27 @@ static int sm_count() {
     return n;
 }
 
-// Whether the wide variant takes a product.  Measured at M = 2,048 (bench.py --only-gemm, replayed from a graph): it wins
-// where a block gets more than one tile (the epilogue of one hides behind the main loop of the next; with eight epilogue
-// warps also at K = 576, where a tile's main loop is only nine stages long) or where K is long enough that the main loop
-// is nearly all of a tile's time; with one short tile a block the narrow kernel's two blocks a multiprocessor do better.
-// tile_cols: output columns of a wide tile.  VITNA_TCGEN05_WIDE=0 or 1 overrides (for measurements).
-static bool wide_takes(int M, int out_cols, int K, int tile_cols = TW_BN) {
-    static int forced = -1;
-    if (forced < 0) {
-        const char* e = getenv("VITNA_TCGEN05_WIDE");
-        forced = e ? (e[0] == '1' ? 1 : 0) : 2;
-    }
+// Whether the wide variant takes a product that the narrow one would cut into tiles of `rows` weight rows (64 or 128), `cols` output columns each.  The narrow
+// kernel's blocks each take one tile, two 64-row or one 128-row tile a multiprocessor at its full rate, and what does not fit beside each other costs another
+// round, whole; the wide one walks its tiles one after another, so that an epilogue hides behind the next main loop, and asks the second-level cache for
+// half the bytes an output.  Until a second round the narrow kernel starts and ends sooner.  Narrow / wide, us (weights in the second-level cache):
+//   64 rows, a round is 296 tiles:  2,048 x 960 x 576 (240) 5.4 / 6.3, 2,048 x 1,024 x 1,024 (256) 7.8 / 10.3, 1,301 x 1,746 x 576 (308) 12.0 / 8.0,
+//     2,048 x 1,746 x 576 (448) 13.1 / 9.8, 3,000 x 960 x 576 (360) 9.5 / 6.5, 8,192 x 320 x 4,096 (320) 40.7 / 21.2, 16,384 x 1,536 x 64 37 / 21
+//   128 rows, a round is 148 tiles:  1,000 x 2,048 x 1,536 (128) 9.4 / 9.9, 1,301 x 2,048 x 1,536 (176) 13.3 / 10.1; two to a multiprocessor share its way to
+//     the operands, so that with a short K, the epilogue most of it, the line is the second pair: 2,048 x 2,048 x 576 (256) 8.0 / 8.5;
+//     gate and up 1,024 x 1,536 (192 tiles) K 576 8.2 / 8.4, K 960 10.9 / 9.9, K 2,048 17.9 / 14.3
+// and with few tiles and a K that is nearly all of a tile's time (8,192) the deeper pipeline of the wide kernel wins, except under a residual sum, whose
+// epilogue it repeats in wider boxes: 200 x 8,192 x 8,192 54 / 40, but 200 x 2,048 x 8,192 into a sum 33.8 / 41.8.  From K = 2,048 with three quarters of a
+// round the two are level (1,024 x 2,048 x 2,048 11.8 / 12.2).  A sum over K < 128 is all epilogue:
+// 16,384 x 4,096 x 64 103 / 124.  Over 1,500 sizes (M 96 to 16,384, N 64 to 49,152, K 64 to 8,192) the rule is 0.8 % behind the better of the two.
+// VITNA_TCGEN05_WIDE=0 or 1 overrides (for measurements).
+static bool wide_takes(int M, int out_cols, int K, int rows, int cols, bool sum = false) {
+    static const int forced = [] { const char* e = getenv("VITNA_TCGEN05_WIDE"); return e ? (e[0] == '1' ? 1 : 0) : 2; }();
     if (forced != 2) return forced == 1;
-    if (M < 512 || out_cols < 1024 || K < 512) return false;
-    const long long tiles = (long long)((M + TC_BM - 1) / TC_BM) * ((out_cols + tile_cols - 1) / tile_cols);
-    return K >= 2048 || tiles * 4 >= (long long)sm_count() * 5;
+    const long long tiles = (long long)((M + TC_BM - 1) / TC_BM) * ((out_cols + cols - 1) / cols), sms = sm_count();
+    if (rows == 64) return tiles > 2 * sms;
+    if (tiles > 2 * sms || (tiles > sms && K >= 768)) return !sum || K >= 128;
+    return !sum && (K >= 8192 || (K >= 2048 && M >= 512 && tiles * 4 >= sms * 3));
 }
 
 template <int EPI, int HD = 0, int BNW = TW_BN, bool PAIR = false>
@@ -955,14 +961,15 @@ static bool pair_takes(int M, int out_cols, int tile_cols, int K) {
     return two <= one && tiles >= 100 && tiles * K >= sms * 2800;
 }
 
-// The width in weight rows of a wide tile (256, 192 or 160) that a block's rounds of are the shortest, counting a round's own cost as 32 columns: 2,011 x 2,576 x
-// 1,024 is 176 tiles of 256 columns for 148 multiprocessors (two rounds, and too few for this kernel: 19.8 us in narrow tiles), 272 of 160 (two shorter ones: 15.7).
+// The width in weight rows of a wide tile (256, 192 or 160) that a block's rounds of are the shortest, counting a round's own cost as 80 columns (over 140 sizes, 1,024 to
+// 16,384 rows, 576 to 4,096 columns and as much K, within 0.1 % of the best width of each; 32 columns 0.5 %): 2,011 x 2,576 x
+// 1,024 is 176 tiles of 256 columns for 148 multiprocessors (two rounds), 272 of 160 (two shorter ones: 15.7 us, 18.0 before).
 static int wide_width(int M, int N) {
     const long long tiles_m = (M + TC_BM - 1) / TC_BM, sms = sm_count();
     int best = 256;
     long long cost = 0;
     for (int w : {256, 192, 160}) {
-        const long long c = (tiles_m * ((N + w - 1) / w) + sms - 1) / sms * (w + 32);
+        const long long c = (tiles_m * ((N + w - 1) / w) + sms - 1) / sms * (w + 80);
         if (w == 256 || c < cost) { best = w; cost = c; }
     }
     return best;
@@ -984,14 +991,18 @@ static int linear_tcgen05_impl(const void* x, const void* w, void* out, int M, i
     if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)out % 16)) return VK_BAD_ALIGNMENT;
     const int bn = N >= 2048 ? 128 : 64;
     if ((M + TC_BM - 1) / TC_BM > 65535) return VK_TOO_LARGE;
-    const int width = mode == 2 ? TW_BN : wide_width(M, N);
-    if (wide_takes(M, N, K, width)) {
+    if (wide_takes(M, N, K, bn, bn, mode == 2)) {
+        const int width = wide_width(M, N);
         CUtensorMap wx, ww;
         const bool pair = pair_takes(M, N, width, K);
         if (!make_map(&wx, x, M, K, ldx, TC_BM) || !make_map(&ww, w, N, K, K, pair ? width / 2 : width)) return VK_BAD_SHAPE;
 #define GO(EPI, W)                                                                                                       \
     return pair ? launch_wide<EPI, 0, W, true>(wx, ww, out, M, N, K, error, stream, ex) : launch_wide<EPI, 0, W>(wx, ww, out, M, N, K, error, stream, ex)
-        if (mode == 2) GO(TC_ACC, 256);
+        if (mode == 2) {
+            if (width == 160) GO(TC_ACC, 160);
+            if (width == 192) GO(TC_ACC, 192);
+            GO(TC_ACC, 256);
+        }
         if (mode == 1) {
             if (width == 160) GO(TC_F32, 160);
             if (width == 192) GO(TC_F32, 192);
@@ -1070,7 +1081,7 @@ static int linear_tcgen05_gated_impl(const void* x, const void* w, void* out, in
     TcExtra ex{};
     ex.inter = inter;
     ex.act = act;
-    if (wide_takes(M, inter, K, TW_BN / 2)) {
+    if (wide_takes(M, inter, K, 128, 64)) {
         // Tiles of 128 x 96 output columns (192 weight rows) where they come out sooner than tiles of 128 x 128: a block
         // walks through ceil(tiles / blocks) tiles, and at the 135M and 360M sizes the last round of the wider tile is
         // mostly empty (192 tiles on 148 multiprocessors: two rounds of 256 columns against two of 192).
@@ -1146,7 +1157,7 @@ VK_API int vk_linear_tcgen05_rope(const void* x, const void* w, void* q_out, int
     TcExtra ex{};
     ex.positions = positions; ex.cos_t = cos_t; ex.sin_t = sin_t; ex.slot = slot; ex.cache = (__nv_bfloat16*)cache;
     ex.nh = nh; ex.nkv = nkv; ex.hd = hd; ex.page_size = page_size;
-    if (wide_takes(M, N, K)) {
+    if (wide_takes(M, N, K, hd, hd)) {
         const bool pair = pair_takes(M, N, TW_BN, K);
         if (!make_map(&mw, w, N, K, K, pair ? TW_BN / 2 : TW_BN)) return VK_BAD_SHAPE;
         if (pair && hd == 64) return launch_wide<TC_ROPE, 64, TW_BN, true>(mx, mw, q_out, M, N, K, error, stream, ex);
