@@ -525,7 +525,10 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
     __shared__ int failed, used;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rank = PAIR ? (int)(blockIdx.x & 1) : 0, worker = PAIR ? blockIdx.x >> 1 : blockIdx.x, workers = PAIR ? gridDim.x >> 1 : gridDim.x;
+    const int rank = PAIR ? (int)(blockIdx.x & 1) : 0;
+    // (read where they are used: held as two numbers they cost the grouped products 1.5 %)
+    auto worker = [] { return PAIR ? blockIdx.x >> 1 : blockIdx.x; };
+    auto workers = [] { return PAIR ? gridDim.x >> 1 : gridDim.x; };
     const int num_kb = (K + TC_BK - 1) / TC_BK;
     const int tile_cols = EPI == TC_SWIGLU ? BNW / 2 : BNW;                // output columns of a tile
     const int out_cols = EPI == TC_SWIGLU ? ex.inter : N;
@@ -575,7 +578,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
         if (lane == 0) {
             int kc = 0;                            // stages filled so far, over all of this block's tiles
             bool ok = true;
-            for (int t = worker; t < num_tiles && ok; t += workers) {
+            for (int t = worker(); t < num_tiles && ok; t += workers()) {
                 const int m0 = tile_row(t) * ROWS + rank * TC_BM, g = group_of(t);
                 if (g < 0) continue;
                 const int n0 = g * ex.group_rows + tile_col(t) * tile_cols;
@@ -609,7 +612,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
             const uint32_t a_lo0 = umma_desc_lo(smem_u32(smem));
             int kc = 0, j = 0;
             bool ok = true;
-            for (int t = worker; t < num_tiles && ok; t += workers, j++) {
+            for (int t = worker(); t < num_tiles && ok; t += workers(), j++) {
                 const int b = j & 1;
                 if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[b], ((j >> 1) - 1) & 1, wc.cycles))) { if (lane == 0) give_up(wc.error, &failed, 32); break; }
                 tc_fence_after();
@@ -634,7 +637,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
             const uint32_t a_lo0 = umma_desc_lo(smem_u32(smem));      // low words of the descriptors (see umma_bf16_lo)
             int kc = 0, j = 0;
             bool ok = true;
-            for (int t = worker; t < num_tiles && ok; t += workers, j++) {
+            for (int t = worker(); t < num_tiles && ok; t += workers(), j++) {
                 if (group_of(t) < 0) { j--; continue; }
                 const int b = j & 1;
                 if (j >= 2 && !mbar_wait(&acc_empty[b], ((j >> 1) - 1) & 1, wc.cycles)) { give_up(wc.error, &failed, 32); break; }
@@ -658,20 +661,20 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
         const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
         int j = 0;
         bool ok = true;
-        for (int t = worker; t < num_tiles; t += workers, j++) {
+        for (int t = worker(); t < num_tiles; t += workers(), j++) {
             if (group_of(t) < 0) { j--; continue; }
             const int b = j & 1;
-            const int row_first = tile_row(t) * ROWS + rank * TC_BM + quarter * 32, row = row_first + lane, n0 = tile_col(t) * tile_cols;
+            const int row = tile_row(t) * ROWS + rank * TC_BM + quarter * 32 + lane, n0 = tile_col(t) * tile_cols;
             if (ok && !__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (j >> 1) & 1, wc.cycles))) { if (lane == 0) give_up(wc.error, &failed, 34); ok = false; }
             // A residual sum goes out by TMA reductions from shared memory (see the narrow kernel), a box of 32 rows x 32 columns a warp: from the warp's
             // own box, or, for the block's last tile, whose epilogue hides behind no further tile, from the stages, which are free by now.
             if (ok && EPI == TC_ACC && ex.tma_out) {
                 tc_fence_after();
                 const uint32_t acc = lane_base + b * BNW;
-                const bool last = t + workers >= num_tiles;
-                const int row0 = row_first;
+                const bool last = t + (int)workers() >= num_tiles;
+                const int row0 = tile_row(t) * ROWS + rank * TC_BM + quarter * 32;
 #pragma unroll 1
-                for (int c = half * SPLIT * 32; c < (half ? CHUNKS : SPLIT) * 32; c += 32) {
+                for (int c = CHUNKS % 2 ? half * SPLIT * 32 : half * (BNW / 2); c < (CHUNKS % 2 ? (half ? CHUNKS : SPLIT) * 32 : (half + 1) * (BNW / 2)); c += 32) {
                     uint32_t r[32];
                     tmem_ld32(acc + c, r);
                     tmem_loaded(r);
@@ -768,7 +771,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                     }
                 } else if (EPI == TC_SAME) {
 #pragma unroll 1
-                    for (int c = half * SPLIT * 32; c < (half ? CHUNKS : SPLIT) * 32; c += 32) {
+                    for (int c = CHUNKS % 2 ? half * SPLIT * 32 : half * (BNW / 2); c < (CHUNKS % 2 ? (half ? CHUNKS : SPLIT) * 32 : (half + 1) * (BNW / 2)); c += 32) {
                         uint32_t r[32];
                         tmem_ld32(acc + c, r);
                         tmem_loaded(r);
@@ -787,7 +790,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                     }
                 } else {
 #pragma unroll 1
-                    for (int c = half * SPLIT * 32; c < (half ? CHUNKS : SPLIT) * 32; c += 32) {
+                    for (int c = CHUNKS % 2 ? half * SPLIT * 32 : half * (BNW / 2); c < (CHUNKS % 2 ? (half ? CHUNKS : SPLIT) * 32 : (half + 1) * (BNW / 2)); c += 32) {
                         uint32_t r[32];
                         tmem_ld32(acc + c, r);
                         tmem_loaded(r);
@@ -795,7 +798,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                         if (EPI == TC_F32) {
                             if (col < N)
                                 store_rows_f32(reinterpret_cast<float*>(boxes + (warp - 2) * 4096), r, reinterpret_cast<float*>(out),
-                                               row_first, col, M, N, lane);
+                                               tile_row(t) * ROWS + rank * TC_BM + quarter * 32, col, M, N, lane);
                             continue;
                         }
                         if (row >= M || col >= N) continue;
@@ -831,7 +834,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
         }
         if (EPI == TC_ACC && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // the boxes outlive their reductions
     }
-    __syncwarp();
+    if (PAIR) __syncwarp();
     tc_fence_before();
     if (PAIR) {
         if (threadIdx.x == 0 && failed) __nanosleep(200000);      // (as below, before the other block may leave)
@@ -928,7 +931,7 @@ template <int EPI, int HD = 0, int BNW = TW_BN, bool PAIR = false>
 static int launch_wide(const CUtensorMap& mx, const CUtensorMap& mw, void* out, int M, int N, int K, int* error, cudaStream_t stream,
                        const TcExtra& ex = TcExtra{}) {
     const WaitCtl wc = wait_ctl(error, WAIT_FAMILY_LINEAR_WIDE);
-    const size_t smem = (size_t)tw_stages(PAIR) * (TC_BM * TC_BK * 2 + (PAIR ? BNW / 2 : BNW) * TC_BK * 2) + wide_boxes(EPI) + 1024 + 192;
+    const size_t smem = (size_t)tw_stages(PAIR) * (TC_BM * TC_BK * 2 + (PAIR ? BNW / 2 : BNW) * TC_BK * 2) + wide_boxes(EPI) + 1024 + (PAIR ? 192 : 128);
     TcExtra exx = ex;
     CUtensorMap mo = mx;                               // (a valid map for the epilogues that do not use it)
     exx.tma_out = 0;
