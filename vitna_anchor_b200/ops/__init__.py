@@ -404,8 +404,8 @@ def skip_stage_once(family: str, stage: int) -> None:
 
 
 def tcgen05_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether the tcgen05 product takes these operands (bfloat16, K and the row stride multiples of 8, aligned)."""
-    return (x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
+    """Whether the tcgen05 product takes these operands (on the device, bfloat16, K and the row stride multiples of 8, aligned)."""
+    return (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
@@ -591,7 +591,7 @@ def rows_tcgen05_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> b
 def rows_tcgen05_pays(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
     """Whether the few-rows tcgen05 product takes these operands and is the faster kernel for them (rows_tcgen05_sizes)."""
     M = x.shape[0]
-    return M <= SKINNY_MAX_ROWS and rows_tcgen05_sizes(M, w.shape[0], w.shape[1]) and rows_tcgen05_takes(x, w, out)
+    return M <= SKINNY_MAX_ROWS and w.dim() == 2 and rows_tcgen05_sizes(M, w.shape[0], w.shape[1]) and rows_tcgen05_takes(x, w, out)
 
 
 def linear_rows_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, *, act: int = 0, rope: Optional[tuple] = None) -> torch.Tensor:
@@ -1171,7 +1171,7 @@ def linear_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: str) -
         raise KernelError(f"linear_act: {kind!r} is not one of {sorted(DENSE_ACTIVATIONS)}")
     M, K = x.shape
     N = w.shape[0]
-    if x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[1] == K and tuple(out.shape) == (M, N) and out.dtype == x.dtype:
+    if x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[1] == K and tuple(out.shape) == (M, N) and out.dtype == x.dtype:
         _req(w, "w", torch.bfloat16, 2); _req(out, "out", torch.bfloat16, 2)
         act = DENSE_ACTIVATIONS[kind] + 1
         if rows_tcgen05_pays(x, w, out):
@@ -1366,7 +1366,7 @@ def linear_gated(x: torch.Tensor, w_gate_up: torch.Tensor, gu: torch.Tensor, out
         raise KernelError(f"linear_gated: {kind!r} is not one of {sorted(ACTIVATIONS)}")
     M, K = x.shape
     inter = w_gate_up.shape[0] // 2
-    if (x.dtype == torch.bfloat16 and w_gate_up.dtype == torch.bfloat16 and w_gate_up.shape == (2 * inter, K) and tuple(out.shape) == (M, inter)
+    if (x.is_cuda and x.dtype == torch.bfloat16 and w_gate_up.dtype == torch.bfloat16 and w_gate_up.shape == (2 * inter, K) and tuple(out.shape) == (M, inter)
             and out.dtype == x.dtype and out.is_contiguous() and w_gate_up.is_contiguous()):
         act = ACTIVATIONS[kind] + 1
         if rows_tcgen05_pays(x, w_gate_up, out):
