@@ -61,16 +61,17 @@ struct ApForm {
     static_assert(STAGES >= BUFS && BUFS >= GROUPS, "phases");
 };
 
-// A row's reference maximum and the number of the step that settled it, in one word of shared memory.
+// A row's reference maximum (the low half) and the number of the step that settled it, in one 64-bit word of shared memory, stored and loaded as one scalar: nothing
+// else orders the two halves (to the memory model a vector access is an access for each component).
 __device__ __forceinline__ void ap_settle(unsigned long long* at, int step, float m) {
-    asm volatile("st.volatile.shared.v2.b32 [%0], {%1, %2};" ::"r"(smem_u32(at)), "r"(__float_as_uint(m)), "r"(step) : "memory");
+    asm volatile("{\n\t.reg .b64 w;\n\tmov.b64 w, {%1, %2};\n\tst.volatile.shared.b64 [%0], w;\n\t}" ::"r"(smem_u32(at)), "r"(__float_as_uint(m)), "r"(step) : "memory");
 }
 __device__ __forceinline__ bool ap_settled(const unsigned long long* at, int step, float& m, unsigned long long limit) {
     const uint32_t addr = smem_u32(at);
     long long start = 0;
     for (int tries = 0;; tries++) {
         uint32_t v, s;
-        asm volatile("ld.volatile.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v), "=r"(s) : "r"(addr) : "memory");
+        asm volatile("{\n\t.reg .b64 w;\n\tld.volatile.shared.b64 w, [%2];\n\tmov.b64 {%0, %1}, w;\n\t}" : "=r"(v), "=r"(s) : "r"(addr) : "memory");
         if ((int)s == step) { m = __uint_as_float(v); return true; }
         if (tries == 0) start = clock64();
         else if ((tries & 15) == 0 && (unsigned long long)(clock64() - start) > limit) return false;
