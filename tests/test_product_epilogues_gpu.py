@@ -137,3 +137,27 @@ def test_turned_heads_at_the_edge_of_a_round(nh, nkv, hd, K):
     held[slot[on].long(), 1], room[slot[on].long(), 1] = p[on, nh + nkv:], off[on, nh + nkv:]
     got = cache.permute(0, 3, 1, 2, 4).reshape(pages * ps, 2, nkv, hd).double()
     assert bool(((got - held).abs() <= room).all())
+
+
+@pytest.mark.parametrize("stage", [0, 7, 90])        # of the first tile and of a later one: the first block's tensor warp, then both blocks' copying and adding-up warps give up
+def test_pairs_of_blocks_give_up_a_wait_and_say_so(stage):
+    """Neither block leaves before both know of it and their copies have had time to land; the next launch is right."""
+    from vitna_anchor_b200 import ops
+    M, N, K = 2048, 6160, 2048
+    g = torch.Generator(device="cuda").manual_seed(stage)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    out = torch.zeros(M, N, device="cuda")
+    ops.set_wait_limit_ms(5.0)
+    try:
+        ops.skip_stage_once("linear_tcgen05_wide", stage)
+        ops.linear_tcgen05(x, w, out, ops.LINEAR_F32)
+        torch.cuda.synchronize()
+        with pytest.raises(ops.KernelGaveUp):
+            ops.check_device_errors()
+    finally:
+        ops.set_wait_limit_ms(0)
+    ops.linear_tcgen05(x, w, out, ops.LINEAR_F32)
+    ops.check_device_errors()
+    want, off = x.double() @ w.double().T, K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)      # (as above)
+    assert bool(((out.double() - want).abs() <= off).all())

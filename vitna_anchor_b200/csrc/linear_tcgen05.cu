@@ -484,6 +484,15 @@ __device__ __forceinline__ uint32_t tw_at_first(const void* p) {          // the
     asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at) : "r"(smem_u32(p)));
     return at;
 }
+// A wait ran out (see give_up): the other block of a pair is told as well.  It is there: neither leaves before both have met.
+__device__ __forceinline__ void tw_give_up(bool pair, int rank, int* error, int* failed, int code) {
+    give_up(error, failed, code);
+    if (pair) {
+        uint32_t at;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(failed)), "r"(rank ^ 1));
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(1) : "memory");
+    }
+}
 __device__ __forceinline__ void tw_arrive_at_first(uint64_t* bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tw_at_first(bar)) : "memory");
 }
@@ -584,7 +593,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
                 const int n0 = g * ex.group_rows + tile_col(t) * tile_cols;
                 for (int kb = 0; kb < num_kb; kb++, kc++) {
                     const int s = kc % STAGES;
-                    if (kc >= STAGES && !mbar_wait(&empty[s], ((kc / STAGES) - 1) & 1, wc.cycles)) { give_up(wc.error, &failed, 31); ok = false; break; }
+                    if (kc >= STAGES && !mbar_wait(&empty[s], ((kc / STAGES) - 1) & 1, wc.cycles)) { tw_give_up(PAIR, rank, wc.error, &failed, 31); ok = false; break; }
                     if (kc == wc.skip_stage) continue;      // left unarmed and unfilled: a test of the give-up path
                     if (PAIR) {
                         // both blocks' copies are counted by the first one's barrier; the maps' boxes are 128 rows (SwiGLU: the first block has the gate rows of the
@@ -614,11 +623,11 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
             bool ok = true;
             for (int t = worker(); t < num_tiles && ok; t += workers(), j++) {
                 const int b = j & 1;
-                if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[b], ((j >> 1) - 1) & 1, wc.cycles))) { if (lane == 0) give_up(wc.error, &failed, 32); break; }
+                if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[b], ((j >> 1) - 1) & 1, wc.cycles))) { if (lane == 0) tw_give_up(PAIR, rank, wc.error, &failed, 32); break; }
                 tc_fence_after();
                 for (int kb = 0; kb < num_kb; kb++, kc++) {
                     const int s = kc % STAGES;
-                    if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (kc / STAGES) & 1, wc.cycles))) { if (lane == 0) give_up(wc.error, &failed, 33); ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (kc / STAGES) & 1, wc.cycles))) { if (lane == 0) tw_give_up(PAIR, rank, wc.error, &failed, 33); ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_lo = a_lo0 + s * (STAGE_BYTES >> 4), b_lo = a_lo + (A_BYTES >> 4);
                     if (elect_one()) {
@@ -640,11 +649,11 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
             for (int t = worker(); t < num_tiles && ok; t += workers(), j++) {
                 if (group_of(t) < 0) { j--; continue; }
                 const int b = j & 1;
-                if (j >= 2 && !mbar_wait(&acc_empty[b], ((j >> 1) - 1) & 1, wc.cycles)) { give_up(wc.error, &failed, 32); break; }
+                if (j >= 2 && !mbar_wait(&acc_empty[b], ((j >> 1) - 1) & 1, wc.cycles)) { tw_give_up(PAIR, rank, wc.error, &failed, 32); break; }
                 tc_fence_after();
                 for (int kb = 0; kb < num_kb; kb++, kc++) {
                     const int s = kc % STAGES;
-                    if (!mbar_wait(&full[s], (kc / STAGES) & 1, wc.cycles)) { give_up(wc.error, &failed, 33); ok = false; break; }
+                    if (!mbar_wait(&full[s], (kc / STAGES) & 1, wc.cycles)) { tw_give_up(PAIR, rank, wc.error, &failed, 33); ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_lo = a_lo0 + s * (STAGE_BYTES >> 4), b_lo = a_lo + (A_BYTES >> 4);
 #pragma unroll
@@ -665,7 +674,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
             if (group_of(t) < 0) { j--; continue; }
             const int b = j & 1;
             const int row = tile_row(t) * ROWS + rank * TC_BM + quarter * 32 + lane, n0 = tile_col(t) * tile_cols;
-            if (ok && !__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (j >> 1) & 1, wc.cycles))) { if (lane == 0) give_up(wc.error, &failed, 34); ok = false; }
+            if (ok && !__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (j >> 1) & 1, wc.cycles))) { if (lane == 0) tw_give_up(PAIR, rank, wc.error, &failed, 34); ok = false; }
             // A residual sum goes out by TMA reductions from shared memory (see the narrow kernel), a box of 32 rows x 32 columns a warp: from the warp's
             // own box, or, for the block's last tile, whose epilogue hides behind no further tile, from the stages, which are free by now.
             if (ok && EPI == TC_ACC && ex.tma_out) {
@@ -837,9 +846,12 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
     if (PAIR) __syncwarp();
     tc_fence_before();
     if (PAIR) {
-        if (threadIdx.x == 0 && failed) __nanosleep(200000);      // (as below, before the other block may leave)
-        __syncwarp();
         tw_pair_meet();                       // what either block sends the other (copies' counts, arrivals) has come; the sums have been read
+        if (failed) {                         // (the same in both blocks: a thread that gave up has said so to both before it met the others)
+            if (lane == 0) __nanosleep(200000);      // after a failed wait: let copies in flight land, in both blocks, before either leaves
+            __syncwarp();
+            tw_pair_meet();
+        }
         tc_fence_after();
         if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TM_COLS) : "memory");
         return;
