@@ -74,54 +74,48 @@ def test_a_wait_that_runs_out_is_reported():
         ops.set_wait_limit_ms(0)
 
 
-def test_neighbouring_tokens_are_prepared_as_single_ones():
-    """A step long enough for eight tokens a block gives the bits of the same tokens in short steps: across segments' borders, carried memories and odd lengths."""
+def _prepare(lens, G, H, dk, dv, taps, first=0, count=None):
+    """Rows first .. first + count of the prepared inputs of a step of segments `lens`, by a step that holds these rows alone (their first segment's memory is
+    then the inputs before them)."""
+    import ctypes
     from vitna_anchor_b200 import ops
-    G, H, dk, dv = 2, 2, 20, 12
-    for taps in (1, 3, 4):
-        g = torch.Generator(device="cuda").manual_seed(taps)
-        r = lambda *s: torch.randn(*s, generator=g, device="cuda")
-        C, N = 2 * G * dk + H * dv, 2 * G * dk + 2 * H * dv + 2 * H
-        lens = [1, 2, 3, 700, 4, 487, 1, 1]
-        T, S = sum(lens), len(lens)
-        proj, conv, a_log, bias = r(T, N), r(C, taps), r(H), r(H)
-        state = r(S, ops.delta_state_floats(G, H, dk, dv, taps))
-        i32 = lambda a: torch.tensor(np.asarray(a), dtype=torch.int32, device="cuda")
-        run = lambda lo, hi, st, starts, tseg, slots: (lambda prep: (ops.delta_rule(
-            proj[lo:hi].contiguous(), conv, a_log, bias, torch.ones(dv, device="cuda"), 1e-5, tseg, starts, slots, st, prep, torch.empty(hi - lo, H * dv, device="cuda"),
-            torch.empty(hi - lo, H * dv, device="cuda"), G, H, dk, dv, taps), prep)[1])(torch.zeros(hi - lo, ops.delta_prep_width(G, H, dk, dv), device="cuda"))
-        whole = run(0, T, state.clone(), i32(np.concatenate([[0], np.cumsum(lens)])), i32(np.repeat(np.arange(S), lens)), i32(np.arange(S)))
-        st, at = state.clone(), 0
-        for s, n in enumerate(lens):
-            for lo in range(at, at + n, 100):
-                hi = min(at + n, lo + 100)
-                part = run(lo, hi, st, i32([0, hi - lo]), i32([0] * (hi - lo)), i32([s]))
-                assert torch.equal(part[:, :C + 2 * H], whole[lo:hi, :C + 2 * H]), (taps, s, lo)
-            at += n
-
-
-@pytest.mark.parametrize("G,dk", [(191, 4), (12, 64), (193, 4)])         # 1,528, 1,536 and 1,544 values of q and k: 47.75, 48 and 48.25 KB for eight tokens
-def test_neighbouring_tokens_at_the_limit_of_shared_memory(G, dk):
-    """Around the largest key heads that eight tokens a block have room for: a long step gives the bits of short ones, whichever kernel prepares it."""
-    from vitna_anchor_b200 import ops
-    H, dv, taps, T = G, 4, 4, 1184
-    g = torch.Generator(device="cuda").manual_seed(G)
+    C = 2 * G * dk + H * dv
+    N, T = C + H * dv + 2 * H, sum(lens)
+    g = torch.Generator(device="cuda").manual_seed(taps)
     r = lambda *s: torch.randn(*s, generator=g, device="cuda")
-    C, N = 2 * G * dk + H * dv, 2 * G * dk + 2 * H * dv + 2 * H
-    proj, conv, a_log, bias = r(T, N), r(C, taps), r(H), r(H)
-    state = r(1, ops.delta_state_floats(G, H, dk, dv, taps))
-    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    proj, conv, a_log, bias, state = r(T, N), r(C, taps), r(H), r(H), r(len(lens), ops.delta_state_floats(G, H, dk, dv, taps))
+    count = T - first if count is None else count
+    ids, at = np.unique(np.repeat(np.arange(len(lens)), lens)[first:first + count], return_index=True)
+    seg, start = np.repeat(np.arange(len(lens)), lens)[first:first + count] - ids[0], np.concatenate([[0], np.cumsum(lens)])
+    if taps > 1 and start[ids[0]] < first:
+        memory = state[ids[0], H * dv * dk:H * dv * dk + (taps - 1) * C].view(taps - 1, C)        # oldest input first
+        memory.copy_(torch.cat([memory, proj[start[ids[0]]:first, :C]])[-(taps - 1):].clone())
+    i32 = lambda a: torch.tensor(np.asarray(a), dtype=torch.int32, device="cuda")
+    rows, out = proj[first:first + count].contiguous(), torch.zeros(count, ops.delta_prep_width(G, H, dk, dv), device="cuda")
+    tseg, starts, slots = i32(seg), i32(np.append(at, count)), i32(ids)
+    assert ops.lib().vk_delta_prepare(ops._p(rows), ops._p(conv), ops._p(a_log), ops._p(bias), ops._p(tseg), ops._p(starts), ops._p(slots), ops._p(state),
+                                      ctypes.c_size_t(state.shape[1]), ops._p(out), count, G, H, dk, dv, taps, ops._stream()) == 0
+    return out[:, :C + 2 * H]
 
-    def run(lo, hi, st):
-        n = hi - lo
-        prep = torch.zeros(n, ops.delta_prep_width(G, H, dk, dv), device="cuda")
-        ops.delta_rule(proj[lo:hi].contiguous(), conv, a_log, bias, torch.ones(dv, device="cuda"), 1e-5, i32([0] * n), i32([0, n]), i32([0]), st, prep,
-                       torch.empty(n, H * dv, device="cuda"), torch.empty(n, H * dv, device="cuda"), G, H, dk, dv, taps)
-        return prep[:, :C + 2 * H]
 
-    whole, st = run(0, T, state.clone()), state.clone()
-    for lo in range(0, T, 100):
-        assert torch.equal(run(lo, min(T, lo + 100), st), whole[lo:lo + 100]), lo
+# one slice of q and k heads and several, a last one that is not full, heads of one channel, of a slice and of more; one slice of v and several, full and not; the longest
+# head that eight tokens have room for, 1,533 channels, and the next, which a block a token takes
+@pytest.mark.parametrize("taps", [1, 3, 4])
+@pytest.mark.parametrize("G,H,dk,dv,sliced", [(2, 2, 20, 12, True), (3, 9, 64, 64, True), (5, 5, 60, 52, True), (3, 6, 100, 43, True), (1, 1, 256, 256, True), (2, 2, 300, 130, True),
+                                              (130, 130, 1, 2, True), (1, 1, 1533, 8, True), (1, 1, 1534, 8, False), (12, 12, 64, 4, True)])
+def test_neighbouring_tokens_are_prepared_as_single_ones(G, H, dk, dv, sliced, taps):
+    """A step whose tokens are prepared eight a block, a slice of the channels each, gives the bits of the same tokens in steps that a block a token prepares: across
+    segments' borders, carried memories and odd lengths."""
+    from vitna_anchor_b200 import ops
+    lens = [1, 2, 3, 700, 4, 487, 1, 1]
+    T = sum(lens)
+    slices = ops.lib().vk_delta_prepare_slices
+    assert (slices(T, G, H, dk, dv, taps) > 0) == sliced
+    whole = _prepare(lens, G, H, dk, dv, taps)
+    for lo in range(0, T, 61):
+        n = min(61, T - lo)
+        assert slices(n, G, H, dk, dv, taps) == 0
+        assert torch.equal(_prepare(lens, G, H, dk, dv, taps, lo, n), whole[lo:lo + n]), lo
 
 
 @pytest.mark.parametrize("strong", [3.0, 200.0, 1e30, float("inf")])       # sums to -100, -6,400, and beyond what any sum holds

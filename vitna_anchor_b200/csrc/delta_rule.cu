@@ -545,6 +545,26 @@ VK_API size_t vk_delta_state_floats(int G, int H, int dk, int dv, int taps) {
 // Floats of a row of prep: q | k | v | log decay | beta, padded to a multiple of four.
 VK_API int vk_delta_prep_width(int G, int H, int dk, int dv) { return (2 * G * dk + H * dv + 2 * H + 3) / 4 * 4; }
 
+// Heads of q and k that a block of delta_prepare_tokens_kernel takes, and its shared memory.
+static int dp_slice_heads(int G, int dk) { return dk < DP_SLICE ? (DP_SLICE / dk < 2 * G ? DP_SLICE / dk : 2 * G) : 1; }
+static size_t dp_smem(int slice_heads, int dk) { return (size_t)DP_TOKENS * slice_heads * dk * sizeof(float); }
+
+// Into how many slices a step's channels are cut for delta_prepare_tokens_kernel (eight tokens a block), or 0: a block a token (delta_prepare_kernel).  A block a token /
+// slices, us, C channels in all:
+//   C   960  65 tokens 5.5 / 6.3, 200 5.9 / 6.3, 300 6.6 / 6.5, 400 6.8 / 6.6, 600 10.3 / 6.9; 2,048 in a prompt 24.9 / 12.7
+//   C 3,072  65 tokens 11.2 / 5.5, 400 14.7 / 6.6, 600 23.1 / 8.6; 2,048 in a prompt 55.6 / 21.7;  C 768 (heads of 256) 200 5.0 / 5.0, 400 5.8 / 5.0
+//   C   384  65 tokens 3.9 / 6.2, 400 4.4 / 6.1, 600 7.0 / 6.3;  C 64 and 104  400 tokens 3.4 / 5.1 and 3.4 / 6.1, 900 5.5 / 5.2 and 5.8 / 6.3
+//   C 2,112 (one head of 1,024)  65 tokens 9.1 / 12.9, 400 11.3 / 13.1, 600 17.8 / 13.9
+// A block a token has the shorter way until its blocks, four to a multiprocessor, need a second round, or until a thread has several channels one after another; a
+// slice of one long head has several itself.  (What a launch may have without asking, 48 KB, counts the kernel's `place` and `olds` too.)
+VK_API int vk_delta_prepare_slices(int tokens, int G, int H, int dk, int dv, int taps) {
+    const int C = 2 * G * dk + H * dv, slice_heads = dp_slice_heads(G, dk);
+    const int slices = (2 * G + slice_heads - 1) / slice_heads + (H * dv + DP_SLICE - 1) / DP_SLICE;
+    if (tokens <= DR_DEPENDENT_TOKENS || taps > DP_TAPS || slices > 65535 || dp_smem(slice_heads, dk) + DP_TOKENS * (sizeof(int) + sizeof(float*)) > 48 * 1024) return 0;
+    const bool pays = tokens > 8 * 148 || (tokens > 4 * 148 && C >= 128) || (C >= 1536 && C >= 8 * dk) || (tokens >= 300 && C >= 768 && dk <= DP_SLICE);
+    return pays ? slices : 0;
+}
+
 // proj [tokens][C + H*dv + 2H] float32; conv_w [C][taps]; state [slots][state_stride] float32; prep [tokens][vk_delta_prep_width].
 VK_API int vk_delta_prepare(const float* proj, const float* conv_w, const float* a_log, const float* dt_bias, const int32_t* token_seg,
                             const int32_t* seg_starts, const int32_t* seg_slots, const float* state, size_t state_stride, float* prep, int tokens,
@@ -564,14 +584,13 @@ VK_API int vk_delta_prepare(const float* proj, const float* conv_w, const float*
     if (tokens <= DR_DEPENDENT_TOKENS)
         return launch_dependent(delta_prepare_kernel, dim3(tokens), dim3(threads), smem, stream, proj, conv_w, a_log, dt_bias, token_seg, seg_starts,
                                 seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps);
-    // Tokens in eights, the channels in slices, against a block a token, us: 65 / 400 / 2,048 tokens of 960 channels 10.3 / 9.5 / 24.9 against 9.7 / 9.4 / 12.7, of 3,072
-    // channels 12.6 / 16.6 / 55.6 against 6.8 / 8.5 / 21.7.  (What a launch may have without asking, 48 KB, counts the kernel's `place` and `olds` too.)
-    const int slice_heads = dk < DP_SLICE ? (DP_SLICE / dk < 2 * G ? DP_SLICE / dk : 2 * G) : 1, head_slices = (2 * G + slice_heads - 1) / slice_heads;
-    const int slices = head_slices + (H * dv + DP_SLICE - 1) / DP_SLICE;
-    const size_t smem8 = (size_t)DP_TOKENS * slice_heads * dk * sizeof(float);
-    if (taps <= DP_TAPS && slices <= 65535 && smem8 + DP_TOKENS * (sizeof(int) + sizeof(float*)) <= 48 * 1024)
-        return launch_plain(delta_prepare_tokens_kernel, dim3((tokens + DP_TOKENS - 1) / DP_TOKENS, slices), dim3(DP_SLICE), smem8, stream, proj, conv_w, a_log, dt_bias, token_seg,
-                            seg_starts, seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps, tokens, slice_heads, head_slices);
+    const int slices = vk_delta_prepare_slices(tokens, G, H, dk, dv, taps);
+    if (slices) {
+        const int slice_heads = dp_slice_heads(G, dk);
+        return launch_plain(delta_prepare_tokens_kernel, dim3((tokens + DP_TOKENS - 1) / DP_TOKENS, slices), dim3(DP_SLICE), dp_smem(slice_heads, dk), stream, proj, conv_w,
+                            a_log, dt_bias, token_seg, seg_starts, seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps, tokens, slice_heads,
+                            (2 * G + slice_heads - 1) / slice_heads);
+    }
     return launch_plain(delta_prepare_kernel, dim3(tokens), dim3(256), smem, stream, proj, conv_w, a_log, dt_bias, token_seg, seg_starts,
                         seg_slots, state, state_stride, (size_t)H * dv * dk, prep, P, G, H, dk, dv, taps);
 }
