@@ -41,6 +41,22 @@ def test_results_and_sums(M, N, K):
         assert torch.equal(part, out[lo:lo + n])
 
 
+# one block a tile, two, three, seven and eight; 16, 32 and 64 columns of batch rows
+@pytest.mark.parametrize("M,N,K", [(1, 49152, 576), (8, 32000, 1024), (24, 49152, 960), (16, 8192, 2048), (40, 5120, 960), (64, 16384, 2048), (64, 6144, 2048), (32, 2560, 2560),
+                                   (64, 2048, 8192)])
+def test_sums_are_as_exact_as_the_kernel_it_stands_in_for(M, N, K):
+    """What is cut off of a sum in tensor memory grows with the products added one after another: no more of them than the mma.sync kernel's warps add."""
+    from vitna_anchor_b200 import ops
+    _, x, w, want, _ = _operands(M, N, K, M + N + K)
+    out, other = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    ops.linear_rows_tcgen05(x, w, out, ops.EPI_F32)
+    ops.linear_skinny(x, w, other, ops.EPI_F32)
+    ops.check_device_errors()
+    mine, theirs = float((out.double() - want).norm()), float((other.double() - want).norm())
+    # both are norms over thousands of sums' rounding errors, which depend on their order: measured within 7 % of each other where the chains are as long
+    assert mine <= 1.15 * theirs, (mine / float(want.norm()), theirs / float(want.norm()))
+
+
 @pytest.mark.parametrize("M,inter,K,kind", [(9, 4, 64, 0), (17, 68, 200, 0), (64, 2560, 960, 0), (33, 1000, 1096, 2), (64, 8192, 256, 0)])
 def test_gated(M, inter, K, kind):
     from vitna_anchor_b200 import ops

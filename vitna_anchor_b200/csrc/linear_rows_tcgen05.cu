@@ -8,8 +8,8 @@
 // splits, and finishes it.  The first four stages' weights are asked for before the wait on the kernel before this one.
 //
 //   warp 0   one lane: TMA copies into a ring of four stages (64 columns of K each)
-//   warp 1   one lane: tcgen05.mma, 128 x NB x 16
-//   warps 2-5  the accumulator out of tensor memory into shared memory, [batch row][weight row]
+//   warp 1   one lane: tcgen05.mma, 128 x NB x 16, to the tile's accumulators in turn
+//   warps 2-5  the accumulators out of tensor memory, added up in float32, into shared memory, [batch row][weight row]
 //   all      the sums over the cluster, and the epilogue: a thread has four neighbouring output columns of a batch row
 //
 // Measured over weights that are not in the second-level cache, 64 rows, before (mma.sync with the weights through registers, or tiles of 128 batch rows) and
@@ -17,18 +17,24 @@
 // multiprocessors pull), 5,120 x 960 gated 15.4 -> 7.1, 49,152 x 2,048 46.1 -> 43.5 (4.6 TB/s; 34.3 with 8 rows, 5.9 TB/s).  About 3.4 us of a launch are not
 // the stream: set-up, the first copies' way, the cluster's meeting and the epilogue; that is why small matrices stay with linear_skinny_mma.cu.
 //
-// An output does not depend on M or on the other batch rows: the splits of K depend on N and K alone.  Every wait on an mbarrier is bounded (see
+// The tensor core cuts off what a sum in tensor memory has no bits for, every time that it adds to it, so that an error grows with the products that are added to
+// one accumulator one after another.  The mma.sync kernels split K over a block's eight warps; here the blocks of a cluster and the accumulators that a block's
+// products go to in turn (`accs`) make as many such chains of an output.  Error against 64 bits over the result's size (2-norms, random operands), the mma.sync kernel / one
+// accumulator a block / as here: 49,152 x 576 1.09e-7 / 5.5e-7 / 0.96e-7,
+// 5,120 x 960 1.53 / 2.9 / 1.12, 6,144 x 2,048 2.36 / 6.5 / 2.11, 16,384 x 2,048 2.35 / 20 / 2.34, 2,048 x 8,192 9.96 / 9.95 / 9.95 (there eight blocks share K).
+//
+// An output does not depend on M or on the other batch rows: the splits of K and the accumulators depend on N and K alone.  Every wait on an mbarrier is bounded (see
 // tcgen05_common.cuh); a block that gave up still meets its cluster.
 #include "tcgen05_common.cuh"
 
 namespace vk {
 
-constexpr int RT_BM = 128, RT_BK = 64, RT_STAGES = 4, RT_THREADS = 192, RT_MAX_SPLIT = 8;
+constexpr int RT_BM = 128, RT_BK = 64, RT_STAGES = 4, RT_THREADS = 192, RT_MAX_SPLIT = 8, RT_CHAINS = 8;
 enum { RT_SAME = 0, RT_F32 = 1, RT_ACC = 2, RT_SWIGLU = 3, RT_ROPE = 4 };
 
 struct RtArgs {
     void* out;
-    int M, N, K, splits;
+    int M, N, K, splits, accs;   // accs: accumulators that a block's products go to in turn
     int act;                     // RT_SAME: an activation on the float32 sums (activate_dense; 0 none); RT_SWIGLU: the gate's function (0: silu)
     const int32_t* positions;
     const float* cos_t;
@@ -77,12 +83,18 @@ __device__ __forceinline__ uint2 rt_pack4(float a, float b, float c, float d) {
 }
 __device__ __forceinline__ float rt_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
+// Columns of tensor memory for `accs` accumulators of nb columns: a power of two, at least 32.
+__host__ __device__ __forceinline__ uint32_t rt_tmem_columns(int nb, int accs) {
+    uint32_t c = 32;
+    while (c < (uint32_t)(nb * accs)) c *= 2;
+    return c;
+}
+
 // grid (tiles * splits), a cluster of `splits` blocks a tile
 template <int NB, int EPI>
 __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                                                                          const RtArgs p, const WaitCtl wc) {
     constexpr uint32_t W_BYTES = RT_BM * RT_BK * 2, X_BYTES = NB * RT_BK * 2, STAGE_BYTES = W_BYTES + X_BYTES;
-    constexpr uint32_t TM_COLS = NB < 32 ? 32 : NB;
     static_assert(NB * RT_BM * 4 <= RT_STAGES * STAGE_BYTES, "the sums take the stages' place");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -96,6 +108,7 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int splits = p.splits, tile = blockIdx.x / splits, rank = blockIdx.x % splits;
     const int n0 = tile * (EPI == RT_SWIGLU ? RT_BM / 2 : RT_BM);
+    const uint32_t tm_cols = rt_tmem_columns(NB, p.accs);
     const int num_kb = (p.K + RT_BK - 1) / RT_BK, kb0 = rank * num_kb / splits, n_kb = (rank + 1) * num_kb / splits - kb0;      // at least one
 
     if (threadIdx.x == 0) {
@@ -106,7 +119,7 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TM_COLS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tm_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
@@ -147,14 +160,19 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
     } else if (warp == 1) {
         if (lane == 0) {
             const uint32_t idesc = umma_idesc_bf16(RT_BM, NB);
-            const uint32_t w_lo0 = umma_desc_lo(smem_u32(smem));
+            const uint32_t w_lo0 = umma_desc_lo(smem_u32(smem)), acc_end = tmem + NB * p.accs;
+            uint32_t acc = tmem, add = 0;              // the first product of an accumulator writes it
             for (int kb = 0; kb < n_kb; kb++) {
                 const int s = kb % RT_STAGES;
                 if (!mbar_wait(&full[s], (kb / RT_STAGES) & 1, wc.cycles)) { give_up(wc.error, &failed, 62); break; }
                 tc_fence_after();
                 const uint32_t w_lo = w_lo0 + s * (STAGE_BYTES >> 4), x_lo = w_lo + (W_BYTES >> 4);
 #pragma unroll
-                for (int k = 0; k < RT_BK / 16; k++) umma_bf16_lo(tmem, w_lo + 2 * k, x_lo + 2 * k, idesc, (kb | k) != 0);
+                for (int k = 0; k < RT_BK / 16; k++) {
+                    umma_bf16_lo(acc, w_lo + 2 * k, x_lo + 2 * k, idesc, add);
+                    acc += NB;
+                    if (acc == acc_end) { acc = tmem; add = 1; }
+                }
                 umma_commit(&empty[s]);
             }
             umma_commit(acc_full);                     // arrives when every instruction has written the accumulator
@@ -169,20 +187,27 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
         tc_fence_after();
         if (__all_sync(0xffffffffu, ok)) {
             float* mine = red + quarter * 32 + lane;
-            if (NB == 16) {
-                uint32_t r[16];
-                tmem_ld16(acc, r);
+            const int used = min(p.accs, n_kb * (RT_BK / 16));
+            constexpr int COLS = NB < 32 ? NB : 32;
+#pragma unroll 1
+            for (int c = 0; c < NB; c += COLS) {
+                float sum[COLS];
 #pragma unroll
-                for (int j = 0; j < 16; j++) mine[j * RT_BM] = __uint_as_float(r[j]);
-            } else {
+                for (int j = 0; j < COLS; j++) sum[j] = 0.0f;
+#pragma unroll 1
+                for (int a = 0; a < used; a++) {
+                    uint32_t r[COLS];
+                    if constexpr (NB == 16) {
+                        tmem_ld16(acc + a * NB, r);
+                    } else {
+                        tmem_ld32(acc + a * NB + c, r);
+                        tmem_loaded(r);
+                    }
 #pragma unroll
-                for (int c = 0; c < NB; c += 32) {
-                    uint32_t r[32];
-                    tmem_ld32(acc + c, r);
-                    tmem_loaded(r);
-#pragma unroll
-                    for (int j = 0; j < 32; j++) mine[(c + j) * RT_BM] = __uint_as_float(r[j]);
+                    for (int j = 0; j < COLS; j++) sum[j] += __uint_as_float(r[j]);
                 }
+#pragma unroll
+                for (int j = 0; j < COLS; j++) mine[(c + j) * RT_BM] = sum[j];
             }
         }
         tc_fence_before();
@@ -263,7 +288,7 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
     if (warp == 1) {
         if (failed) __nanosleep(200000);               // after a failed wait: let copies in flight land
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tm_cols) : "memory");
     }
 }
 
@@ -287,6 +312,9 @@ static int rt_splits(int tiles, int K) {
     return s < 1 ? 1 : s;
 }
 
+// Accumulators of a block: with the splits of K, at least RT_CHAINS chains of an output's products.  (Eight of 64 columns are all of the tensor memory.)
+static int rt_accs(int splits) { return (RT_CHAINS + splits - 1) / splits; }
+
 template <int NB, int EPI>
 static int rt_launch(const CUtensorMap& mx, const CUtensorMap& mw, RtArgs p, int* error, cudaStream_t stream) {
     const WaitCtl wc = wait_ctl(error, WAIT_FAMILY_LINEAR);
@@ -297,6 +325,7 @@ static int rt_launch(const CUtensorMap& mx, const CUtensorMap& mw, RtArgs p, int
     const int per_tile = EPI == RT_SWIGLU ? RT_BM / 2 : RT_BM, cols = EPI == RT_SWIGLU ? p.N / 2 : p.N;
     const int tiles = (cols + per_tile - 1) / per_tile;
     p.splits = rt_splits(tiles, p.K);
+    p.accs = rt_accs(p.splits);
     return launch_dependent_cluster(kern, dim3(tiles * p.splits), dim3(RT_THREADS), p.splits, smem, stream, mx, mw, p, wc);
 }
 
@@ -325,7 +354,7 @@ VK_API int vk_linear_rows_tcgen05(const void* x, const void* w, void* out, int M
     const int nb = M <= 16 ? 16 : M <= 32 ? 32 : 64;
     CUtensorMap mx, mw;
     if (!rt_make_map(&mx, x, M, K, ldx, nb) || !rt_make_map(&mw, w, N, K, K, epi == RT_SWIGLU ? RT_BM / 2 : RT_BM)) return VK_BAD_SHAPE;
-    RtArgs p{out, M, N, K, 1, act, positions, cos_t, sin_t, slot, (__nv_bfloat16*)cache, nh, nkv, hd, page_size};
+    RtArgs p{out, M, N, K, 1, 1, act, positions, cos_t, sin_t, slot, (__nv_bfloat16*)cache, nh, nkv, hd, page_size};
 #define GO(NB)                                                              \
     switch (epi) {                                                          \
         case RT_SAME: return rt_launch<NB, RT_SAME>(mx, mw, p, error, stream);     \
