@@ -486,18 +486,36 @@ def _mma_norm_smem(M: int, K: int, N: int) -> int:
     return rows * (4 * K + 64) + 4 * K + 8 * (rows // 8) * 512
 
 
-def rows_tcgen05_sizes(M: int, N: int, K: int) -> bool:
-    """Sizes at which the few-rows product with the weights as the tensor cores' 128-row operand is the faster one.  Measured over weights that are not in
-    the second-level cache, microseconds, the mma.sync kernels (or the tcgen05 tile product) against this one:
-      16 / 32 / 64 rows  6144 x 2048  12.7 15.6 28.9 against 8.6 8.9 10.4;  2048 x 8192  14.1 22.0 32.7 against 11.0 10.8 12.1
-                         16384 x 2048 gated  29.9 22.1 23.3 against 16.0 16.8 18.4;  5120 x 960 gated  5.5 10.2 15.4 against 5.6 5.8 7.1
-                         960 x 2560  4.7 5.1 6.3 against 4.5 4.9 6.0;  1600 x 960  3.8 4.3 7.9 against 4.8 5.1 5.7 (not taken below 40 rows)
-      up to 8 rows       6144 x 2048  8.3 against 8.6 and the like, and there the other kernel has the norm in front in its own launch
-      any rows           49152 x 576  19.3 to 22.5 against 11.1 to 17.8;  49152 x 960  27.1 to 30.2 against 17.9 to 26.1 (8 rows, 2048 columns: 34.3 and 33.8)
-    Rows of up to 640 columns are normed inside the mma.sync kernel's launch for up to 64 rows, which is worth more than this kernel gains there."""
-    if N * K >= 24_000_000 and K < 2048:
+def rows_tcgen05_sizes(M: int, N: int, K: int, acc: bool = False) -> bool:
+    """Sizes at which the few-rows product with the weights as the tensor cores' 128-row operand is the faster one; acc: it is added into its result.  Measured over
+    weights that are not in the second-level cache, microseconds, what stands in otherwise (up to 8 rows, and up to 8,192 columns: the mma.sync kernels; else
+    128-row tiles) against this one:
+      up to 8 rows, norm in front   49152 x 576 18.4 / 13.4, 32000 x 1024 16.0 / 15.8;  16384 x 1536 12.3 / 13.0, 6144 x 2048 8.3 / 8.6 (not taken)
+      9 to 16 rows   6144 x 2048 12.7 / 8.6, 2048 x 8192 14.1 / 11.0;  2048 x 2048 4.8 / 5.8, 4096 x 1024 4.5 / 5.7, 5120 x 960 5.3 / 6.5, 7680 x 1536 7.8 / 8.8 (not taken:
+                     the mma.sync kernels' blocks norm and stage so few rows once)
+      17 to 64 rows, up to 8,192 columns   64: 6144 x 2048 28.9 / 10.4, 2048 x 8192 32.7 / 12.1, 1600 x 960 6.2 / 5.3;  K a multiple of 256, which the warps of the
+                     other kernel share evenly: 33 x 2048 x 2048 8.6 / 6.2, but 32 x 2048 x 2048 5.8 / 6.2, 64 x 1024 x 2048 5.3 / 5.7, 48 x 1536 x 1536 4.7 / 5.7
+      more columns   16: 49152 x 2048 57.6 / 33.4, 65536 x 512 16.9 / 15.0;  24: 42000 x 576 16.4 / 14.6;  32: 49152 x 960 25.3 / 22.4;  48: 16384 x 2048 18.7 / 16.5,
+                     32000 x 1024 17.4 / 20.4 (not taken);  64: 16384 x 2048 18.4 / 16.9 and gated 22.1 / 18.8, into a sum 18.4 / 20.0 (not taken)
+    A K that is no multiple of 32 stays with the other kernel's float32 multiply-adds, whose sums are the more exact (0.7 against 1.3e-7 of the result's size at K = 1,000),
+    and rows of up to 640 columns with the mma.sync kernel, which norms them in its own launch for up to 64 rows."""
+    if K < 512 or (N <= 8192 and (K % 32 != 0 or K <= NORM_IN_REGISTERS_MAX_K)):
+        return False
+    if M <= 8:
+        return N > 16384 and K < 2048 and K % 32 == 0 and N * K >= 24_000_000
+    if N <= 8192:
+        if M <= 16:
+            return N >= 512 and K >= 2048 and N * K >= 5_000_000
+        return N >= 512 and M * N * K >= (136_000_000 if K % 256 == 0 or N < 1536 else 60_000_000 if M > 32 else 80_000_000)
+    if not (N * K >= 24_000_000 and K < 2048 or K > NORM_IN_REGISTERS_MAX_K and M * N * K >= 60_000_000):
+        return False
+    if M <= 16:
         return True
-    return M > 8 and K > NORM_IN_REGISTERS_MAX_K and M * N * K >= 60_000_000
+    if acc:
+        return False
+    if M <= 32:
+        return N <= 18944 or M <= 24 or NORM_IN_REGISTERS_MAX_K < K < 2048
+    return N <= 18944 if M <= 48 else N <= 16384 and K >= 2048
 
 
 def fused_norm_takes(dtype: torch.dtype, M: int, K: int, N: int) -> bool:
@@ -588,10 +606,10 @@ def rows_tcgen05_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> b
     return 0 < x.shape[0] <= SKINNY_MAX_ROWS and tcgen05_takes(x, w) and w.shape[0] % 8 == 0 and out.data_ptr() % 16 == 0
 
 
-def rows_tcgen05_pays(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+def rows_tcgen05_pays(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, acc: bool = False) -> bool:
     """Whether the few-rows tcgen05 product takes these operands and is the faster kernel for them (rows_tcgen05_sizes)."""
     M = x.shape[0]
-    return M <= SKINNY_MAX_ROWS and w.dim() == 2 and rows_tcgen05_sizes(M, w.shape[0], w.shape[1]) and rows_tcgen05_takes(x, w, out)
+    return M <= SKINNY_MAX_ROWS and w.dim() == 2 and rows_tcgen05_sizes(M, w.shape[0], w.shape[1], acc) and rows_tcgen05_takes(x, w, out)
 
 
 def linear_rows_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, *, act: int = 0, rope: Optional[tuple] = None) -> torch.Tensor:
@@ -633,7 +651,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int) -> to
     (no reduced-precision matrix mode); bfloat16 runs the tensor-core kernel where it takes the sizes."""
     M = x.shape[0]
     if M <= SKINNY_MAX_ROWS:
-        if rows_tcgen05_pays(x, w, out):
+        if rows_tcgen05_pays(x, w, out, mode == LINEAR_ACC_F32):
             return linear_rows_tcgen05(x, w, out, mode)
         if skinny_takes(x.dtype, M, x.shape[1], w.shape[0]) and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
             return linear_skinny(x, w, out, mode)
