@@ -23,3 +23,13 @@ def test_delta_rule_preparation(sizes, sliced):
     ((64, 2048, 8192), True, True), ((64, 2048, 2048), True, True), ((64, 16384, 2048), False, True), ((64, 1600, 960), False, True), ((32, 49152, 960), False, True)])
 def test_few_rows_products(sizes, acc, taken):
     assert ops.rows_tcgen05_sizes(*sizes, acc) == taken
+
+
+# (kind, rows, columns, K) as vk_linear_tcgen05_route has them: where the wide tiles, or pairs of blocks, were measured to be slower, and where they are the faster ones
+@pytest.mark.parametrize("sizes,route", [
+    ((0, 8192, 790, 272), 0), ((0, 1301, 1746, 576), 0), ((0, 16384, 14678, 112), 0), ((2, 8192, 790, 272), 160), ((2, 16384, 1746, 576), 160), ((2, 16384, 6104, 256), 0),
+    ((3, 8192, 1536, 576), 192), ((3, 16384, 3072, 768), 256), ((1, 16384, 1746, 576), 256), ((1, 1000, 4096, 4096), 256), ((2, 1301, 2560, 4096), 256), ((2, 4096, 674, 3536), 192),
+    ((0, 8192, 6144, 2048), 257), ((3, 8192, 8192, 2048), 257), ((2, 8192, 2048, 8192), 257), ((2, 2048, 2048, 8192), 257), ((0, 3000, 1001, 1000), 192),
+    ((4, 8192, 6144, 2048), 257), ((5, 8192, 2560, 2048), 257), ((1, 3000, 960, 4096), 161)])
+def test_wide_products(sizes, route):
+    assert ops.lib().vk_linear_tcgen05_route(*sizes) == route

@@ -657,10 +657,12 @@ def test_linear_tcgen05_swiglu_matches_the_separate_kernels(ops, M, I, K):
 
 
 @pytest.mark.parametrize("nh,nkv,hd,ps,M,K", [(9, 3, 64, 16, 200, 576), (2, 1, 128, 8, 130, 96), (32, 32, 64, 16, 70, 2048),
-                                              (15, 5, 64, 16, 600, 960), (6, 3, 128, 32, 520, 512)])   # the last two: 128 x 256 tiles
+                                              (15, 5, 64, 16, 600, 960), (6, 3, 128, 32, 520, 512),
+                                              (15, 5, 64, 16, 1601, 960), (6, 3, 128, 32, 3201, 512)])   # the last two: 128 x 256 tiles
 def test_linear_tcgen05_rope_matches_the_separate_kernels(ops, nh, nkv, hd, ps, M, K):
     torch.manual_seed(nh + M)
     N = (nh + 2 * nkv) * hd
+    assert ops.lib().vk_linear_tcgen05_route(4 if hd == 64 else 5, M, N, K) == (256 if M > 1600 else 0)
     pages = -(-M // ps) + 3
     x = torch.randn(M, K).to(torch.bfloat16).cuda()
     w = (torch.randn(N, K) / math.sqrt(K) * 2).to(torch.bfloat16).cuda()

@@ -63,10 +63,18 @@ def test_row_groups(N, K, tiles, mode, act):
     assert bool((room[M * N:] == 5.0).all())
 
 
-# pairs of blocks: row tiles of 256 with an empty half, with rows in both; widths of 160, 192 and 256 whose last tile ends inside a block's half; one round and several
-@pytest.mark.parametrize("M,N,K", [(1297, 2560, 2056), (2176, 2576, 3000), (2048, 5152, 2048), (1100, 6160, 2048), (3000, 4112, 1800), (2049, 2048, 8200)])
-def test_pairs_of_blocks(M, N, K):
+def _route(kind, M, N, K):
+    """The wide tiles' weight rows, one more with pairs of blocks; 0 for the narrow kernel."""
     from vitna_anchor_b200 import ops
+    return ops.lib().vk_linear_tcgen05_route(kind, M, N, K)
+
+
+# pairs of blocks: row tiles of 256 with an empty half, with rows in both; widths of 160, 192 and 256 whose last tile ends inside a block's half; one round and several
+@pytest.mark.parametrize("M,N,K,route", [(2048, 2576, 3000, 161), (1900, 2576, 3000, 161), (2048, 5152, 2048, 193), (2048, 6160, 2048, 257), (3000, 4112, 1800, 257),
+                                         (2049, 2048, 8200, 257)])
+def test_pairs_of_blocks(M, N, K, route):
+    from vitna_anchor_b200 import ops
+    assert [_route(kind, M, N, K) for kind in (0, 1, 2)] == [route] * 3
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
     w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
@@ -80,19 +88,48 @@ def test_pairs_of_blocks(M, N, K):
     assert bool(((acc.double() - want - base.double()).abs() <= off + 2.0 ** -23 * (base.double().abs() + want.abs())).all())
     same = torch.full((M, N), 5.0, device="cuda", dtype=torch.bfloat16)
     ops.linear_tcgen05(x, w, same, ops.LINEAR_SAME)
-    assert bool(((same.double() - want).abs() <= off + 2.0 ** -8 * (want.abs() + off)).all())
-    gated = torch.full((M, N // 2), 5.0, device="cuda", dtype=torch.bfloat16)
-    ops.linear_tcgen05_swiglu(x, w, gated)
     ops.check_device_errors()
-    # both halves are rounded to bfloat16 first; silu's slope stays below 1.1, its own error is a few 2^-22
-    a, b, e = want[:, :N // 2], want[:, N // 2:], off + 2.0 ** -8 * (want.abs() + off)
-    ea, eb, f = e[:, :N // 2], e[:, N // 2:], torch.nn.functional.silu(a)
-    bound = 1.1 * ea * b.abs() + (f.abs() + 1.1 * ea) * eb + (2.0 ** -8 + 2.0 ** -18) * (f * b).abs()
-    assert bool(((gated.double() - f * b).abs() <= 1.01 * bound + 1e-6).all())
+    assert bool(((same.double() - want).abs() <= off + 2.0 ** -8 * (want.abs() + off)).all())
     # a row's bits do not hang on the number of rows
     part = torch.empty(M - 128, N, device="cuda")
     ops.linear_tcgen05(x[128:], w, part, ops.LINEAR_F32)
     assert torch.equal(part, f32[128 * N:M * N].view(M - 128, N))
+
+
+@pytest.mark.parametrize("M,inter,K,route", [(2048, 2584, 2048, 193), (2000, 8192, 2048, 257), (1100, 3080, 2048, 257), (8192, 1536, 576, 192)])
+def test_gated_pairs_of_blocks(M, inter, K, route):
+    from vitna_anchor_b200 import ops
+    assert _route(3, M, inter, K) == route
+    g = torch.Generator(device="cuda").manual_seed(M + inter + K)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(2 * inter, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    gated = torch.full((M, inter), 5.0, device="cuda", dtype=torch.bfloat16)
+    ops.linear_tcgen05_swiglu(x, w, gated)
+    ops.check_device_errors()
+    want, off = x.double() @ w.double().T, K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)      # (as above)
+    # both halves are rounded to bfloat16 first; silu's slope stays below 1.1, its own error is a few 2^-22
+    a, b, e = want[:, :inter], want[:, inter:], off + 2.0 ** -8 * (want.abs() + off)
+    ea, eb, f = e[:, :inter], e[:, inter:], torch.nn.functional.silu(a)
+    bound = 1.1 * ea * b.abs() + (f.abs() + 1.1 * ea) * eb + (2.0 ** -8 + 2.0 ** -18) * (f * b).abs()
+    assert bool(((gated.double() - f * b).abs() <= 1.01 * bound + 1e-6).all())
+
+
+# rows that do not begin on 16 bytes, written value by value: bfloat16 in narrow tiles up to K = 600 and in wide ones, sums in tiles of 160 and 192 columns, never by pairs
+@pytest.mark.parametrize("shape,routes", [((4100, 1093, 520), (0, 160)), ((3000, 1001, 1000), (192, 192)), ((4096, 1178, 4472), (160, 160)), ((2048, 1249, 376), (0, 160)),
+                                          ((16384, 142, 112), (0, 0))])
+def test_rows_off_16_bytes(shape, routes):
+    from vitna_anchor_b200 import ops
+    M, N, K = shape
+    assert (_route(0, M, N, K), _route(2, M, N, K)) == routes
+    test_float32_results_and_sums(shape)
+    g = torch.Generator(device="cuda").manual_seed(M * N + K)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    same = torch.full((M, N), 5.0, device="cuda", dtype=torch.bfloat16)
+    ops.linear_tcgen05(x, w, same, ops.LINEAR_SAME)
+    ops.check_device_errors()
+    want, off = x.double() @ w.double().T, K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)      # (as above)
+    assert bool(((same.double() - want).abs() <= off + 2.0 ** -8 * (want.abs() + off)).all())
 
 
 # the edge of a round of narrow tiles (296 of 64 rows, 333 go to wide ones; 148 of 128 rows, 152), wide tiles of a short K and of few columns, sums in tiles of 160
@@ -105,9 +142,10 @@ def test_products_at_the_edge_of_a_round(shape):
 
 # the fused turn in wide tiles where the last tile holds one, two and three heads of four (64 columns) and one of two (128)
 @pytest.mark.parametrize("nh,nkv,hd,K", [(9, 3, 64, 576), (3, 1, 64, 264), (6, 2, 64, 64), (5, 3, 128, 136)])
-def test_turned_heads_at_the_edge_of_a_round(nh, nkv, hd, K):
+def test_turned_heads_at_the_edge_of_a_round(nh, nkv, hd, K, M=8100, route=256):
     from vitna_anchor_b200 import ops
-    M, ps, N = 8100, 16, (nh + 2 * nkv) * hd
+    ps, N = 16, (nh + 2 * nkv) * hd
+    assert _route(4 if hd == 64 else 5, M, N, K) == route
     g = torch.Generator(device="cuda").manual_seed(N + K)
     x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
     w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
@@ -139,11 +177,18 @@ def test_turned_heads_at_the_edge_of_a_round(nh, nkv, hd, K):
     assert bool(((got - held).abs() <= room).all())
 
 
+# by pairs of blocks: row tiles with rows in both halves and with an empty one, a last tile of one head of four and of one of two
+@pytest.mark.parametrize("nh,nkv,hd,K,M", [(29, 16, 64, 2048, 2100), (17, 2, 128, 4096, 2049)])
+def test_turned_heads_by_pairs(nh, nkv, hd, K, M):
+    test_turned_heads_at_the_edge_of_a_round(nh, nkv, hd, K, M, 257)
+
+
 @pytest.mark.parametrize("stage", [0, 7, 90])        # of the first tile and of a later one: the first block's tensor warp, then both blocks' copying and adding-up warps give up
 def test_pairs_of_blocks_give_up_a_wait_and_say_so(stage):
     """Neither block leaves before both know of it and their copies have had time to land; the next launch is right."""
     from vitna_anchor_b200 import ops
     M, N, K = 2048, 6160, 2048
+    assert _route(1, M, N, K) == 257
     g = torch.Generator(device="cuda").manual_seed(stage)
     x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
     w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)

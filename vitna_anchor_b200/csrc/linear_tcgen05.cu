@@ -927,15 +927,15 @@ static int sm_count() {
 //     gate and up 1,024 x 1,536 (192 tiles) K 576 8.2 / 8.4, K 960 10.9 / 9.9, K 2,048 17.9 / 14.3
 // and with few tiles and a K that is nearly all of a tile's time (8,192) the deeper pipeline of the wide kernel wins, except under a residual sum, whose
 // epilogue it repeats in wider boxes: 200 x 8,192 x 8,192 54 / 40, but 200 x 2,048 x 8,192 into a sum 33.8 / 41.8.  From K = 2,048 with three quarters of a
-// round the two are level (1,024 x 2,048 x 2,048 11.8 / 12.2).  A sum over K < 128 is all epilogue:
-// 16,384 x 4,096 x 64 103 / 124.  Over 1,500 sizes (M 96 to 16,384, N 64 to 49,152, K 64 to 8,192) the rule is 0.8 % behind the better of the two.
+// round the two are level (1,024 x 2,048 x 2,048 11.8 / 12.2).  A sum over a short K is all epilogue: 16,384 x 4,096 x 64 103 / 124, 16,384 x 6,104 x 256 173 / 195,
+// 16,384 x 8,216 x 296 261 / 288.  Over 1,500 sizes (M 96 to 16,384, N 64 to 49,152, K 64 to 8,192) the rule is 0.8 % behind the better of the two.
 // VITNA_TCGEN05_WIDE=0 or 1 overrides (for measurements).
 static bool wide_takes(int M, int out_cols, int K, int rows, int cols, bool sum = false) {
     static const int forced = [] { const char* e = getenv("VITNA_TCGEN05_WIDE"); return e ? (e[0] == '1' ? 1 : 0) : 2; }();
     if (forced != 2) return forced == 1;
     const long long tiles = (long long)((M + TC_BM - 1) / TC_BM) * ((out_cols + cols - 1) / cols), sms = sm_count();
     if (rows == 64) return tiles > 2 * sms;
-    if (tiles > 2 * sms || (tiles > sms && K >= 768)) return !sum || K >= 128;
+    if (tiles > 2 * sms || (tiles > sms && K >= 768)) return !sum || K >= 320;
     return !sum && (K >= 8192 || (K >= 2048 && M >= 512 && tiles * 4 >= sms * 3));
 }
 
@@ -966,33 +966,73 @@ static int launch_wide(const CUtensorMap& mx, const CUtensorMap& mw, void* out, 
 // way of the operands outweighs the pairs' meetings (about a microsecond a launch), and 256-row tiles need no more rounds.  One block a tile against pairs, us:
 // 8,192 x 16,384 x 2,048 374 / 348, 8,192 x 2,048 x 8,192 229 / 209, 8,192 x 6,144 x 2,048 160 / 142, 2,048 x 16,384 x 2,048 100 / 93, 2,048 x 6,160 x 2,048 46 / 42,
 // 2,048 x 2,560 x 2,048 24.5 / 23.1; but 2,048 x 2,048 x 2,048 17.8 / 19.1, 700 x 2,048 x 8,192 (48 tiles: nothing else wants the second-level cache) 43.6 / 44.9,
-// 1,301 x 5,120 x 960 17.5 / 18.4.
+// 1,301 x 5,120 x 960 17.5 / 18.4.  A short K leaves a pair's epilogues, which wait for both blocks, in the open: gate and up 8,192 x 1,536 x 576 28.2 / 33.0 and
+// x 768 5 to 41 % behind, 16,384 x 1,746 x 576 52.8 / 60.6; level from K = 800 on (`least`, 1,000 for the gated and the rotated epilogue, which do more).  A single round of
+// 256-column tiles has nothing to hide the meetings behind either: 1,000 x 4,096 x 4,096 25.8 / 27.3, 1,301 x 2,560 x 4,096 25.2 / 26.8, but 2,048 x 2,048 x 8,192 0.93.
 // VITNA_TCGEN05_PAIR=0 or 1 overrides (for measurements).
-static bool pair_takes(int M, int out_cols, int tile_cols, int K) {
+static bool pair_takes(int M, int out_cols, int tile_cols, int K, int least) {
     static const int forced = [] { const char* e = getenv("VITNA_TCGEN05_PAIR"); return e ? (e[0] == '1' ? 1 : 0) : 2; }();
     if (forced != 2) return forced == 1;
     const long long tn = (out_cols + tile_cols - 1) / tile_cols, sms = sm_count(), tiles = (M + 127) / 128 * tn;
     const long long one = (tiles + sms - 1) / sms, two = ((M + 255) / 256 * tn + sms / 2 - 1) / (sms / 2);
-    return two <= one && tiles >= 100 && tiles * K >= sms * 2800;
+    return K >= least && two <= one && tiles >= 100 && tiles * K >= sms * (one == 1 && tile_cols == 256 ? 3600 : 2800);
 }
 
 // The width in weight rows of a wide tile (256, 192 or 160) that a block's rounds of are the shortest, counting a round's own cost as 80 columns (over 140 sizes, 1,024 to
 // 16,384 rows, 576 to 4,096 columns and as much K, within 0.1 % of the best width of each; 32 columns 0.5 %): 2,011 x 2,576 x
-// 1,024 is 176 tiles of 256 columns for 148 multiprocessors (two rounds), 272 of 160 (two shorter ones: 15.7 us, 18.0 before).
-static int wide_width(int M, int N) {
+// 1,024 is 176 tiles of 256 columns for 148 multiprocessors (two rounds), 272 of 160 (two shorter ones: 15.7 us, 18.0 before).  `most` 192: without 256.
+static int wide_width(int M, int N, int most = 256) {
     const long long tiles_m = (M + TC_BM - 1) / TC_BM, sms = sm_count();
     int best = 256;
     long long cost = 0;
     for (int w : {256, 192, 160}) {
         const long long c = (tiles_m * ((N + w - 1) / w) + sms - 1) / sms * (w + 80);
-        if (w == 256 || c < cost) { best = w; cost = c; }
+        if (w <= most && (w == most || c < cost)) { best = w; cost = c; }
     }
     return best;
+}
+
+// How a product without row groups is worked out: by the narrow kernel (width 0), or by the wide one in tiles of `width` weight rows, with pairs of blocks or without.
+struct TcRoute {
+    int width;
+    bool pair;
+};
+static TcRoute route_plain(int M, int N, int K, int mode) {
+    const int bn = N >= 2048 ? 128 : 64;
+    // Rows that do not begin on 16 bytes are written value by value.  As bfloat16 that costs the wide kernel's eight warps more than the narrow one's blocks, until K hides
+    // it: 8,192 x 790 x 272 65 / 80, 1,301 x 1,746 x 576 29 / 33, 3,000 x 1,001 x 1,000 0.81.  A sum reads and writes each value where it lies, and wants a
+    // first-level cache beside the stages: none is left with tiles of 256 columns or with pairs (8,192 x 790 x 272 144 narrow, 169 so; at 160 and 192 columns half of the narrow time).
+    const bool apart = mode == 0 ? N % 8 != 0 : mode == 2 && N % 4 != 0;
+    if (!wide_takes(M, N, K, bn, bn, mode == 2 && !apart) || (apart && K < (mode == 0 ? 600 : 128))) return {0, false};
+    if (apart && mode == 2) return {wide_width(M, N, 192), false};
+    const int width = wide_width(M, N);
+    return {width, (!apart || width == 256) && pair_takes(M, N, width, K, 800)};
+}
+static TcRoute route_gated(int M, int inter, int K) {
+    if (!wide_takes(M, inter, K, 128, 64)) return {0, false};
+    // Tiles of 128 x 96 output columns (192 weight rows) where they come out sooner than tiles of 128 x 128: a block
+    // walks through ceil(tiles / blocks) tiles, and at the 135M and 360M sizes the last round of the wider tile is
+    // mostly empty (192 tiles on 148 multiprocessors: two rounds of 256 columns against two of 192).
+    const long long tiles_m = (M + TC_BM - 1) / TC_BM, sms = sm_count();
+    const long long rounds256 = (tiles_m * ((inter + 127) / 128) + sms - 1) / sms, rounds192 = (tiles_m * ((inter + 95) / 96) + sms - 1) / sms;
+    const int half = rounds192 * 192 < rounds256 * 256 ? 96 : 128;
+    return {2 * half, pair_takes(M, inter, half, K, 1000)};
+}
+static TcRoute route_rope(int M, int N, int K, int hd) {
+    if (!wide_takes(M, N, K, hd, hd)) return {0, false};
+    return {TW_BN, pair_takes(M, N, TW_BN, K, 1000)};
 }
 
 }  // namespace vk
 
 using namespace vk;
+
+// For tests: the route of a product.  kind 0, 1, 2: linear_tcgen05's modes; 3: the gated product (N columns of the result); 4, 5: the rotated one, heads of 64 and 128.
+// The wide tiles' weight rows, one more with pairs of blocks; 0 for the narrow kernel.
+VK_API int vk_linear_tcgen05_route(int kind, int M, int N, int K) {
+    const TcRoute r = kind < 3 ? route_plain(M, N, K, kind) : kind == 3 ? route_gated(M, N, K) : route_rope(M, N, K, kind == 4 ? 64 : 128);
+    return r.width + (r.pair ? 1 : 0);
+}
 
 // x [M, K] bfloat16 with row stride ldx, w [N, K] bfloat16, out [M, N]: mode 0 bfloat16, 1 float32, 2 float32 +=.
 // K and ldx multiples of 8, pointers 16-byte aligned.  error: a word the kernel sets (non-zero) if a bounded wait ran out.
@@ -1006,10 +1046,11 @@ static int linear_tcgen05_impl(const void* x, const void* w, void* out, int M, i
     if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)out % 16)) return VK_BAD_ALIGNMENT;
     const int bn = N >= 2048 ? 128 : 64;
     if ((M + TC_BM - 1) / TC_BM > 65535) return VK_TOO_LARGE;
-    if (wide_takes(M, N, K, bn, bn, mode == 2)) {
-        const int width = wide_width(M, N);
+    const TcRoute route = route_plain(M, N, K, mode);
+    if (route.width) {
+        const int width = route.width;
+        const bool pair = route.pair;
         CUtensorMap wx, ww;
-        const bool pair = pair_takes(M, N, width, K);
         if (!make_map(&wx, x, M, K, ldx, TC_BM) || !make_map(&ww, w, N, K, K, pair ? width / 2 : width)) return VK_BAD_SHAPE;
 #define GO(EPI, W)                                                                                                       \
     return pair ? launch_wide<EPI, 0, W, true>(wx, ww, out, M, N, K, error, stream, ex) : launch_wide<EPI, 0, W>(wx, ww, out, M, N, K, error, stream, ex)
@@ -1096,14 +1137,10 @@ static int linear_tcgen05_gated_impl(const void* x, const void* w, void* out, in
     TcExtra ex{};
     ex.inter = inter;
     ex.act = act;
-    if (wide_takes(M, inter, K, 128, 64)) {
-        // Tiles of 128 x 96 output columns (192 weight rows) where they come out sooner than tiles of 128 x 128: a block
-        // walks through ceil(tiles / blocks) tiles, and at the 135M and 360M sizes the last round of the wider tile is
-        // mostly empty (192 tiles on 148 multiprocessors: two rounds of 256 columns against two of 192).
-        const long long tiles_m = (M + TC_BM - 1) / TC_BM, sms = sm_count();
-        const long long rounds256 = (tiles_m * ((inter + 127) / 128) + sms - 1) / sms, rounds192 = (tiles_m * ((inter + 95) / 96) + sms - 1) / sms;
-        const int half = rounds192 * 192 < rounds256 * 256 ? 96 : 128;
-        const bool pair = pair_takes(M, inter, half, K);
+    const TcRoute route = route_gated(M, inter, K);
+    if (route.width) {
+        const int half = route.width / 2;
+        const bool pair = route.pair;
         if (!make_map(&mx, x, M, K, ldx, TC_BM) || !make_map(&mw, w, 2 * inter, K, K, half)) return VK_BAD_SHAPE;
         if (half == 96 && pair) return launch_wide<TC_SWIGLU, 0, 192, true>(mx, mw, out, M, 2 * inter, K, error, stream, ex);
         if (half == 96) return launch_wide<TC_SWIGLU, 0, 192>(mx, mw, out, M, 2 * inter, K, error, stream, ex);
@@ -1172,8 +1209,9 @@ VK_API int vk_linear_tcgen05_rope(const void* x, const void* w, void* q_out, int
     TcExtra ex{};
     ex.positions = positions; ex.cos_t = cos_t; ex.sin_t = sin_t; ex.slot = slot; ex.cache = (__nv_bfloat16*)cache;
     ex.nh = nh; ex.nkv = nkv; ex.hd = hd; ex.page_size = page_size;
-    if (wide_takes(M, N, K, hd, hd)) {
-        const bool pair = pair_takes(M, N, TW_BN, K);
+    const TcRoute route = route_rope(M, N, K, hd);
+    if (route.width) {
+        const bool pair = route.pair;
         if (!make_map(&mw, w, N, K, K, pair ? TW_BN / 2 : TW_BN)) return VK_BAD_SHAPE;
         if (pair && hd == 64) return launch_wide<TC_ROPE, 64, TW_BN, true>(mx, mw, q_out, M, N, K, error, stream, ex);
         if (pair) return launch_wide<TC_ROPE, 128, TW_BN, true>(mx, mw, q_out, M, N, K, error, stream, ex);
