@@ -33,3 +33,12 @@ def test_few_rows_products(sizes, acc, taken):
     ((4, 8192, 6144, 2048), 257), ((5, 8192, 2560, 2048), 257), ((1, 3000, 960, 4096), 161)])
 def test_wide_products(sizes, route):
     assert ops.lib().vk_linear_tcgen05_route(*sizes) == route
+
+
+# (rows, columns, type of the result: 0 float32, 1 bfloat16): where a warp a row was measured to be slower than eight rows a block, and where it is the faster one
+@pytest.mark.parametrize("sizes,warps", [
+    ((3000, 64, 1), False), ((4096, 256, 0), False), ((3000, 576, 1), False), ((3552, 640, 1), False), ((7000, 640, 1), False), ((16384, 644, 1), False), ((16384, 768, 1), False),
+    ((16384, 576, 0), False), ((16, 2052, 1), False),
+    ((64, 2048, 1), True), ((1, 576, 1), True), ((2048, 576, 1), True), ((3000, 576, 0), True), ((4096, 576, 1), True), ((2048, 960, 1), True), ((8192, 2048, 1), True), ((16384, 960, 1), True)])
+def test_norms(sizes, warps):
+    assert bool(ops.lib().vk_rmsnorm_warp_blocks(*sizes)) == warps

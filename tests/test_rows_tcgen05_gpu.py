@@ -115,18 +115,21 @@ def test_gives_up_a_wait_and_says_so(stage):
     assert bool(((out.double() - want).abs() <= off).all())
 
 
-# a warp a row (up to 4,096 rows of up to 640 values, every number of longer ones) and eight rows a block
-@pytest.mark.parametrize("n", [4, 576, 640, 644, 1024, 1028, 2048])
+# a warp a row (`rows` in all and 77 of them) and eight rows a block
+@pytest.mark.parametrize("n,rows,warps", [(4, 2048, True), (4, 2500, False), (512, 2048, True), (576, 5000, True), (576, 3000, None), (640, 5001, False), (644, 5000, True), (700, 7001, False),
+                                          (1024, 5000, True), (1028, 5000, True), (2048, 5000, True), (2052, 200, False)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-def test_norm_rows(n, dtype):
+def test_norm_rows(n, rows, warps, dtype):
     from vitna_anchor_b200 import ops
+    warps = dtype == torch.float32 if warps is None else warps         # (None: it is the result's type that decides)
+    assert bool(ops.lib().vk_rmsnorm_warp_blocks(rows, n, 0 if dtype == torch.float32 else 1)) == warps
     g = torch.Generator(device="cuda").manual_seed(n)
-    x = torch.randn(5000, n, generator=g, device="cuda") * 3
+    x = torch.randn(rows, n, generator=g, device="cuda") * 3
     w = torch.randn(n, generator=g, device="cuda")
-    rows = torch.randperm(5000, generator=g, device="cuda")[:77].to(torch.int32)
-    out, some = torch.empty(5000, n, device="cuda", dtype=dtype), torch.empty(77, n, device="cuda", dtype=dtype)
+    picked = torch.randperm(rows, generator=g, device="cuda")[:77].to(torch.int32)
+    out, some = torch.empty(rows, n, device="cuda", dtype=dtype), torch.empty(77, n, device="cuda", dtype=dtype)
     ops.rmsnorm_rows(x, w, 1e-5, out)
-    ops.rmsnorm_rows(x, w, 1e-5, some, rows)
-    assert torch.equal(some, out[rows.long()])
+    ops.rmsnorm_rows(x, w, 1e-5, some, picked)
+    assert torch.equal(some, out[picked.long()])                       # the same order of sums in both forms
     want = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5) * w.double()
     assert bool(((out.double() - want).abs() <= ((n / 32 + 8) * 2.0 ** -24 + (2.0 ** -8 if dtype == torch.bfloat16 else 0)) * want.abs() + 1e-9).all())

@@ -284,13 +284,25 @@ VK_API int vk_embed_rows(const void* table, const int32_t* ids, float* x, int to
     return launch_status();
 }
 
+// Whether a norm's rows are a block of one warp each, or eight to a block.  Eight rows a block / a warp a row, us, results in bfloat16:
+//   64 rows of 2,048 4.8 / 1.9 (in a decode step 9.2 / 2.5);  1,024 rows of 64 2.0 / 1.7, of 576 2.8 / 1.9;  2,048 rows of 960 4.1 / 3.1, of 2,048 7.3 / 5.9;  8,192 of 2,048 18.6 / 16.0
+// and, as shares of the time of eight rows a block,
+//   n up to 512    2,048 rows 0.90 to 0.99, 2,400 rows of 64 and 448 1.11 and 1.02, 4,096 rows 1.35 and 1.03, 16,384 1.9 and 1.4
+//   n 576, 640     2,048 rows 0.86, 0.83;  2,800 1.04, 1.03;  3,552 1.13, 1.04;  3,600 0.93, 0.82;  5,000 0.96, 0.94;  7,000 1.13, 1.09
+//   n 704, 768     5,000 rows 0.86, 0.85;  7,000 1.04, 1.01;  8,192 1.01, 0.99;  n 832, 896  10,000 rows 1.01, 0.98;  16,384 1.11, 1.06;  n 960 and more  16,384 rows 1.01 and less
+// Small blocks bring many rows' trips to memory side by side; in great number they cost more to begin than their rows' work.  Eight rows a block come three blocks to
+// a multiprocessor: 3,552 rows are one round of theirs, which they end sooner than the warps from 2,400 rows on where n is up to 640 (bfloat16).
+VK_API int vk_rmsnorm_warp_blocks(int out_rows, int n, int dtype) {
+    if (n > 2048) return 0;
+    const int most = n <= 512 ? 2048 : n < 700 ? 5000 : n < 800 ? 7000 : n < 960 ? 10000 : 0x7fffffff;
+    return out_rows <= most && !(dtype != 0 && n <= 640 && out_rows > 2400 && out_rows <= 3552);
+}
+
 VK_API int vk_rmsnorm_rows(const float* x, const float* w, const int32_t* rows, void* y, int out_rows, int n, float eps,
                            int dtype, cudaStream_t stream) {
     if (out_rows <= 0) return VK_OK;
     if (n <= 0) return VK_BAD_SHAPE;
-    // A block of one warp a row, or eight rows a block: 64 rows of 2,048 in a decode step 9.2 against 2.5 us; 2,048 / 8,192 rows of 2,048 8.2 / 19.5 against 6.1 / 15.9,
-    // 4,096 / 8,192 rows of 576 6.6 / 9.0 against 5.4 / 10.0: short rows in great number are better off with fewer and larger blocks.
-    if (n % 4 == 0 && n <= 2048 && (n > 640 || out_rows <= 4096) && !(((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) % 16)) {
+    if (n % 4 == 0 && vk_rmsnorm_warp_blocks(out_rows, n, dtype) && !(((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) % 16)) {
 #define GO(KEEP)                                                                                                                                          \
     return dtype == 0 ? launch_dependent(rmsnorm_row_kernel<float, KEEP>, dim3(out_rows), dim3(32), 0, stream, x, w, rows, (float*)y, n, eps)         \
                       : launch_dependent(rmsnorm_row_kernel<__nv_bfloat16, KEEP>, dim3(out_rows), dim3(32), 0, stream, x, w, rows, (__nv_bfloat16*)y, n, eps)
