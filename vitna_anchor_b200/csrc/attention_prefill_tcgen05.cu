@@ -12,6 +12,10 @@
 //   one warp   tcgen05.mma, scores: S[128 x 64] = Q K^T into one of BUFS buffers in tensor memory, as soon as the product that read it last is done
 //   one warp   tcgen05.mma, O[128 x VD] += P V in the order of the steps, P from tensor memory, the values as they lie in the cache (N-major)
 //
+// The tensor core cuts off what a sum in tensor memory has no bits for, every time that it adds to it; the form for launches of few blocks and long walks has two
+// outputs, even and odd steps', which halves the products that are added to one.  (9 heads, 4,096 tokens: 8,187 of 2,359,296 results rounded to the wrong
+// bfloat16 with one output, 6,533 with two.)
+//
 // O stays in tensor memory for the whole walk, and all groups share it and a row's reference maximum.  The maximum is only raised when a step's exceeds it by more
 // than 2^8 (then the warp scales its rows of O, once every earlier product has landed); until then the probabilities are taken against the older maximum and may
 // reach 256, which float32 sums and the two bfloat16 parts hold as well as values up to 1.  Every step settles the maximum for the next: a row's thread leaves it for
@@ -31,8 +35,9 @@
 // leaves its unnormalised output, reference maxima and sums in scratch memory, and the part that arrives last (a counter per tile and head, no waiting) adds them in
 // part order and writes the result.
 //
-// A row's result does not depend on what else is in the batch: its keys are walked in 64s from absolute position 0 (or the window's first tile), parts lie at fixed
-// steps of that walk, and every decision above is the row's own.  (It depends on the form only in that a row's sum is added up over the groups.)
+// A row's result does not depend on the other rows: its keys are walked in 64s from absolute position 0 (or the window's first tile), parts lie at fixed
+// steps of that walk, and every decision above is the row's own.  What the launcher chooses by the size of the whole launch, the form (over how many groups a row's
+// sum is added up, over how many outputs its products are) and whether walks are cut, does move its last bits.
 //
 // Every wait is bounded (see tcgen05_common.cuh); a thread that gave up keeps its appointments.
 //
@@ -47,16 +52,16 @@ constexpr int AP_BM = 128, AP_BN = 64;
 constexpr int AP_PART = 16;          // steps of 64 keys a block walks at most, where walks are cut
 
 // A form of the kernel: keys of HD and values of VD values (64 or 128), GROUPS groups of four softmax warps, BUFS buffers of scores and probabilities in tensor
-// memory, STAGES of keys and of values in shared memory, BLOCKS a multiprocessor.
-template <int HD_, int VD_, int GROUPS_, int BUFS_, int STAGES_, int BLOCKS_>
+// memory, STAGES of keys and of values in shared memory, BLOCKS a multiprocessor, OUTS outputs in tensor memory that the steps' products go to in turn.
+template <int HD_, int VD_, int GROUPS_, int BUFS_, int STAGES_, int BLOCKS_, int OUTS_ = 1>
 struct ApForm {
-    static constexpr int HD = HD_, VD = VD_, GROUPS = GROUPS_, BUFS = BUFS_, STAGES = STAGES_, BLOCKS = BLOCKS_;
+    static constexpr int HD = HD_, VD = VD_, GROUPS = GROUPS_, BUFS = BUFS_, STAGES = STAGES_, BLOCKS = BLOCKS_, OUTS = OUTS_;
     static constexpr int KP = HD / 64, VP = VD / 64;            // panels of 64 columns: rows of 128 bytes each
     static constexpr int SOFT = 4 * GROUPS, THREADS = 32 * (SOFT + 4);
     static constexpr uint32_t PANEL = AP_BN * 128, Q_PANEL = AP_BM * 128, Q_BYTES = KP * Q_PANEL, K_BYTES = KP * PANEL, V_BYTES = VP * PANEL;
     static constexpr uint32_t K_OFF = Q_BYTES, V_OFF = K_OFF + STAGES * K_BYTES, BAR_OFF = V_OFF + STAGES * V_BYTES, SMEM = BAR_OFF + 512 + 1024;
-    static constexpr uint32_t O_COL = BUFS * AP_BN, TMEM = O_COL + VD <= 256 ? 256 : 512;
-    static_assert((HD == 64 || HD == 128) && (VD == 64 || VD == 128) && O_COL + VD <= 512 && TMEM * BLOCKS <= 512, "tensor memory");
+    static constexpr uint32_t O_COL = BUFS * AP_BN, O_END = O_COL + OUTS * VD, TMEM = O_END <= 128 ? 128 : O_END <= 256 ? 256 : 512;
+    static_assert((HD == 64 || HD == 128) && (VD == 64 || VD == 128) && O_END <= 512 && TMEM * BLOCKS <= 512, "tensor memory");
     // A thread waits on a barrier's phases by parity, so it must never be two phases behind: a group takes every GROUPS-th step, a buffer every BUFS-th.
     static_assert(STAGES >= BUFS && BUFS >= GROUPS, "phases");
 };
@@ -182,7 +187,7 @@ __global__ void __launch_bounds__(F::THREADS, F::BLOCKS) attention_prefill_tcgen
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
     const int32_t* __restrict__ block_tables, const int32_t* __restrict__ tiles, __nv_bfloat16* __restrict__ out, int nh, int nkv, int page_size, int max_blocks,
     float scale, int window, int out_ld, const float* __restrict__ gate, int gate_ld, const WaitCtl wc, const ApScratch sc) {
-    constexpr int HD = F::HD, VD = F::VD, GROUPS = F::GROUPS, BUFS = F::BUFS, STAGES = F::STAGES, SOFT = F::SOFT, OUT = VD / GROUPS;
+    constexpr int HD = F::HD, VD = F::VD, GROUPS = F::GROUPS, BUFS = F::BUFS, STAGES = F::STAGES, SOFT = F::SOFT, OUTS = F::OUTS, OUT = VD / GROUPS;
     constexpr float RAISE = 8.0f;                    // the reference maximum follows when a maximum exceeds it by 2^8
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -322,11 +327,11 @@ __global__ void __launch_bounds__(F::THREADS, F::BLOCKS) attention_prefill_tcgen
             tc_fence_after();
             if (elect_one()) {
                 // 16 keys an instruction: two groups of eight 128-byte rows of the values; 32 columns hold 32 keys' high parts, then their low parts
-                const uint32_t v_lo = v_lo0 + s * (F::V_BYTES >> 4), p_at = tmem + b * AP_BN;
+                const uint32_t v_lo = v_lo0 + s * (F::V_BYTES >> 4), p_at = tmem + b * AP_BN, o_at = tmem + F::O_COL + i % OUTS * VD;
 #pragma unroll
-                for (int k = 0; k < AP_BN / 16; k++) ap_umma_ts(tmem + F::O_COL, p_at + 32 * (k / 2) + 8 * (k % 2), v_lo + k * (2048 >> 4), idesc, (i | k) != 0);
+                for (int k = 0; k < AP_BN / 16; k++) ap_umma_ts(o_at, p_at + 32 * (k / 2) + 8 * (k % 2), v_lo + k * (2048 >> 4), idesc, i >= OUTS || k != 0);
 #pragma unroll
-                for (int k = 0; k < AP_BN / 16; k++) ap_umma_ts(tmem + F::O_COL, p_at + 32 * (k / 2) + 16 + 8 * (k % 2), v_lo + k * (2048 >> 4), idesc, 1);
+                for (int k = 0; k < AP_BN / 16; k++) ap_umma_ts(o_at, p_at + 32 * (k / 2) + 16 + 8 * (k % 2), v_lo + k * (2048 >> 4), idesc, 1);
                 umma_commit(&pv_done[b]);
                 umma_commit(&v_empty[s]);
             }
@@ -397,7 +402,7 @@ __global__ void __launch_bounds__(F::THREADS, F::BLOCKS) attention_prefill_tcgen
                 tc_fence_after();
                 const float alpha = raise ? ap_ex2(had - mx) : 1.0f;
 #pragma unroll 1
-                for (int c = 0; c < VD; c += 16) {
+                for (int c = 0; c < OUTS * VD; c += 16) {       // (an output that no product has been added to yet is written whole by its first)
                     uint32_t orr[16];
                     ap_tmem_ld16(my_o + c, orr);
 #pragma unroll
@@ -494,6 +499,13 @@ __global__ void __launch_bounds__(F::THREADS, F::BLOCKS) attention_prefill_tcgen
                 ap_tmem_ld16(my_o + c + d0, o);
 #pragma unroll
                 for (int d = 0; d < 16; d++) acc[d] = __uint_as_float(o[d]);
+#pragma unroll
+                for (int u = 1; u < OUTS; u++) {
+                    if (u >= n_it) break;
+                    ap_tmem_ld16(my_o + u * VD + c + d0, o);
+#pragma unroll
+                    for (int d = 0; d < 16; d++) acc[d] += __uint_as_float(o[d]);
+                }
                 if (valid && n_parts == 1) write(d0, acc, inv);
                 if (valid && n_parts > 1) {
                     // this part's unnormalised output, reference maximum and sum; a row without a counted key in this part (its keys all lie in earlier
@@ -660,21 +672,22 @@ VK_API int vk_attention_prefill_tcgen05(const void* q, const void* cache, const 
     sc.parts = cut ? ((grid_context - 1) / AP_BN) / sc.part_steps + 1 : 1;
     sc.n_tiles = n_tiles;
     if ((long long)n_tiles * sc.parts * nh > 0x7fffffffll) return VK_TOO_LARGE;
-    // Which form.  Two groups and two blocks a multiprocessor where there are blocks for it: 32 heads and 8,192 / 2,048 / 1,024 / 700 tokens (2,048 to 192 blocks) 442 /
-    // 47 / 20.4 / 15.8 us against 529 / 56 / 23.1 / 18.0 with four groups in one block.  Four groups where a block has a multiprocessor to itself, or two share
-    // one for a long walk: 9 heads and 2,048 tokens (144 blocks) 25.3 against 27.3, 2,600 (189) 30.7 against 34.2, 4,096 (288) 49.1 against 53.3, 100 tokens
-    // 6,000 into a context (nine blocks, cut) 25.2 against 29.1.
+    // Which form.  Two groups and two blocks a multiprocessor where there are blocks for it: 32 heads and 8,192 / 2,048 tokens (2,048 and 512 blocks) 442 / 47 us against
+    // 529 / 56 with four groups in one block.  Four groups, and two outputs, where a block has a multiprocessor to itself, or two or three share one for a long walk:
+    // 9 heads and 2,048 tokens (144 blocks) 25.3 against 27.3, 2,600 (189) 30.7 against 34.2, 4,096 (288) 49.1 against 53.3; 100 tokens 6,000 into a context (nine blocks, cut)
+    // 25.2 against 29.1.  From 297 to 369 blocks two groups are 13 % the faster and their one output rounds 25 % more results to the wrong bfloat16: the two outputs' sums
+    // are worth that.
     // VITNA_ATT_STREAMS=0 / 1 in the environment, or vk_set_prefill_streams, forces one or the other (tests, measurements).
     const int forced_form = prefill_streams_mode();
     const long long blocks = (long long)n_tiles * sc.parts * nh;
-    const bool four = forced_form == 2 ? blocks <= 148 || (blocks <= 296 && grid_context > 1024) : forced_form == 1;
+    const bool four = forced_form == 2 ? blocks <= 148 || (blocks < 370 && grid_context > 512) : forced_form == 1;
     CUtensorMap mk, mv;
     const long long page_elems = 2ll * nkv * page_size * hd;
     if (!ap_make_page_map(&mk, cache, hd, nkv * page_size, pages, page_elems, box_rows) ||
         !ap_make_page_map(&mv, (const __nv_bfloat16*)cache + (size_t)nkv * page_size * hd, hd, nkv * page_size, pages, page_elems, box_rows))
         return VK_BAD_SHAPE;
     if (four)
-        return launch_ap<ApForm<64, 64, 4, 5, 5, 1>>(mq, mk, mv, block_tables, tiles, out, nh, nkv, page_size, max_blocks, scale, window, nh * hd, nullptr, 0, error, sc, stream);
+        return launch_ap<ApForm<64, 64, 4, 5, 5, 1, 2>>(mq, mk, mv, block_tables, tiles, out, nh, nkv, page_size, max_blocks, scale, window, nh * hd, nullptr, 0, error, sc, stream);
     return launch_ap<ApForm<64, 64, 2, 3, 4, 2>>(mq, mk, mv, block_tables, tiles, out, nh, nkv, page_size, max_blocks, scale, window, nh * hd, nullptr, 0, error, sc, stream);
 }
 
