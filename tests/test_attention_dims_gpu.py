@@ -7,7 +7,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dims", [(128, 128), (64, 128), (128, 64)])
-@pytest.mark.parametrize("form", [(4, 2, 16, 0, False), (3, 1, 8, 100, False), (2, 2, 32, 64, True), (2, 1, 64, 1, False), (6, 3, 128, 65, True), (1, 1, 16, 1000, False)])
+# (the last four: more than 148 blocks, which come two to a multiprocessor)
+@pytest.mark.parametrize("form", [(4, 2, 16, 0, False), (3, 1, 8, 100, False), (2, 2, 32, 64, True), (2, 1, 64, 1, False), (6, 3, 128, 65, True), (1, 1, 16, 1000, False), (32, 4, 16, 0, False), (24, 8, 8, 65, True), (20, 4, 128, 300, False),
+                                  (17, 17, 64, 1, True)])
 def test_dims_against_the_general_kernel(dims, form):
     from vitna_anchor_b200 import ops
     hd, vd = dims

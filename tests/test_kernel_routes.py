@@ -42,3 +42,11 @@ def test_wide_products(sizes, route):
     ((64, 2048, 1), True), ((1, 576, 1), True), ((2048, 576, 1), True), ((3000, 576, 0), True), ((4096, 576, 1), True), ((2048, 960, 1), True), ((8192, 2048, 1), True), ((16384, 960, 1), True)])
 def test_norms(sizes, warps):
     assert bool(ops.lib().vk_rmsnorm_warp_blocks(*sizes)) == warps
+
+
+# (tiles, heads, window, context): the groups of the prompt attention's form for heads of 64, and the parts that a walk may be cut into
+@pytest.mark.parametrize("sizes,groups,parts", [
+    ((16, 32, 0, 2048), 2, 1), ((64, 32, 0, 8192), 2, 1), ((41, 9, 0, 5200), 4, 1), ((42, 9, 0, 5300), 2, 1), ((16, 9, 0, 2048), 4, 1), ((1, 9, 0, 6100), 4, 6), ((8, 32, 0, 1024), 4, 1),
+    ((32, 32, 0, 16), 1, 1), ((8, 20, 0, 128), 2, 1), ((32, 32, 64, 4096), 1, 1), ((3, 9, 64, 300), 2, 1), ((4, 20, 256, 3128), 2, 1), ((12, 9, 256, 1536), 2, 1), ((4, 20, 2000, 3128), 4, 3)])
+def test_prompt_attention(sizes, groups, parts):
+    assert ops.lib().vk_attention_prefill_plan(*sizes) == groups + 16 * parts

@@ -522,9 +522,9 @@ def test_attention_prefill_tiles(ops, nh, nkv, hd, ps, window):
     _prefill_case(ops, ops.attention_prefill, 64, nh, nkv, hd, ps, window, [150, 140, 601, 128 + 70], [150, 37, 2, 70])
 
 
-@pytest.fixture(params=[0, 1], ids=["two_threads_a_row", "two_streams"])
+@pytest.fixture(params=[0, 1], ids=["two_groups", "four_groups"])
 def prefill_kernel(ops, request):
-    """Both tcgen05 prompt-attention kernels, whatever the launcher's size rule would take."""
+    """Two forms of the tcgen05 prompt attention, whatever the launcher's size rule would take."""
     was = ops.set_prefill_streams(request.param)
     yield request.param
     ops.set_prefill_streams(was)
@@ -533,7 +533,7 @@ def prefill_kernel(ops, request):
 @pytest.mark.parametrize("nh,nkv,ps,window", [(9, 3, 16, 0), (4, 4, 8, 0), (2, 1, 32, 0), (6, 2, 64, 0), (3, 1, 128, 0),
                                               (3, 3, 16, 70), (2, 1, 8, 200)])
 def test_attention_prefill_tcgen05(ops, prefill_kernel, nh, nkv, ps, window):
-    """The same on the fifth-generation tensor cores (head size 64, tiles of up to 128 tokens), both kernels: a whole
+    """The same on the fifth-generation tensor cores (head size 64, tiles of up to 128 tokens), both forms: a whole
     prompt of 300 tokens, portions in mid-request across boundaries of 64 and 128, two tokens far into a context, a
     portion that ends exactly at a multiple of 64, and pages of many sizes.  Unused slots of the pages hold 1000."""
     _prefill_case(ops, ops.attention_prefill_tcgen05, 128, nh, nkv, 64, ps, window, [300, 140, 601, 128 + 70, 448], [300, 37, 2, 70, 200])
@@ -544,14 +544,14 @@ def test_attention_prefill_tcgen05_cuts_long_walks_into_parts(ops, prefill_kerne
     """Tiles whose walk over the keys is longer than 16 steps of 64 are cut into parts that different blocks take and the
     last to arrive adds up: portions at the end of contexts of 2,300 and 4,000 positions (three and four parts), a whole
     prompt of 1,025 tokens (its last tile has one row, whose second part is a single key), a walk of exactly 16 steps, and
-    a window that shortens the walk.  Run twice over the same scratch (the counters return to zero).  Both kernels."""
+    a window that shortens the walk.  Run twice over the same scratch (the counters return to zero).  Both forms."""
     for _ in range(2):
         _prefill_case(ops, ops.attention_prefill_tcgen05, 128, nh, nkv, 64, ps, window, [2300, 1100, 1025, 4000, 1024], [300, 70, 1025, 2, 128])
 
 
 def test_attention_prefill_tcgen05_takes_the_kernel_by_the_size_of_the_launch(ops):
-    """A launch of 32 heads and 13 tiles (416 blocks: the first kernel) and one of 8 heads (104 blocks: two streams) give
-    the same result as each kernel forced on the same operands, to rounding: the size rule only chooses."""
+    """A launch of 32 heads and 13 tiles (416 blocks: two groups) and one of 8 heads (104 blocks: four) give
+    the same result as each form forced on the same operands, to rounding: the size rule only chooses."""
     torch.manual_seed(5)
     hd, ps, T = 64, 16, 13 * 128
     pages = T // ps + 3
@@ -573,7 +573,7 @@ def test_attention_prefill_tcgen05_takes_the_kernel_by_the_size_of_the_launch(op
                 ops.set_prefill_streams(was)
         scale = float(outs[0].abs().max())
         assert (outs[0] - outs[1]).abs().max() <= 2e-2 * scale and (outs[0] - outs[2]).abs().max() <= 2e-2 * scale
-        assert torch.equal(outs[0], outs[1] if nh == 32 else outs[2])        # the rule took the kernel this size stands for
+        assert torch.equal(outs[0], outs[1] if nh == 32 else outs[2])        # the rule took the form this size stands for
 
 
 def test_attention_prefill_tcgen05_refuses_what_it_does_not_take(ops):
@@ -714,7 +714,7 @@ def test_linear_tcgen05_gives_up_a_wait_and_says_so(ops, family, M, N, K, stage)
 
 @pytest.mark.parametrize("stage", [0, 2])
 def test_attention_prefill_tcgen05_gives_up_a_wait_and_says_so(ops, prefill_kernel, stage):
-    """The same for the prompt attention, both kernels: one step's keys never arrive; the tensor-core lanes, the softmax
+    """The same for the prompt attention, both forms: one step's keys never arrive; the tensor-core lanes, the softmax
     warps and the copying warps each give up within the limit, keep their appointments, and the block returns."""
     ops.set_wait_limit_ms(5.0)
     try:

@@ -1,4 +1,4 @@
-"""The tcgen05 prompt attention's two forms where their hand-overs can go wrong: walks shorter than the groups and the buffers, reference maxima that rise in every
+"""The tcgen05 prompt attention's three forms where their hand-overs can go wrong: walks shorter than the groups and the buffers, reference maxima that rise in every
 step, rows that are not there, and parts of a walk."""
 import math
 
@@ -8,7 +8,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(params=[0, 1], ids=["two_groups", "four_groups"])
+@pytest.fixture(params=[0, 1, 3], ids=["two_groups", "four_groups", "one_group"])
 def form(request):
     from vitna_anchor_b200 import ops
     was = ops.set_prefill_streams(request.param)
@@ -72,6 +72,22 @@ def test_windows(form, window, rise):
 @pytest.mark.parametrize("rise", [0.0, 9.0])
 def test_parts(form, rise):
     _check([(2100, 130), (1000, 25), (1023, 2), (0, 200)], 0, 32, rise, nh=2)
+
+
+def test_cut_walks_under_windows(form):
+    """A window's walks have fewer parts than the context would have: as many as the longest of them needs, whatever its place."""
+    from vitna_anchor_b200 import ops
+    assert ops.lib().vk_attention_prefill_plan(4, 2, 1100, 3100) // 16 == 2 and ops.lib().vk_attention_prefill_plan(4, 2, 0, 3100) // 16 == 4
+    _check([(2900, 128), (2945, 130), (0, 60)], 1100, 16, 0.0, nh=2)
+    assert ops.lib().vk_attention_prefill_plan(4, 2, 1026, 3100) // 16 == 2 and ops.lib().vk_attention_prefill_plan(4, 2, 834, 3100) // 16 == 1
+    _check([(2945, 128), (3000, 100)], 1026, 16, 0.0, nh=2)
+    _check([(2945, 128), (2950, 128)], 834, 8, 9.0, nh=2)
+
+
+def test_long_windows_over_large_pages(form):
+    """A walk that begins in the middle of a page of 128 slots or more, and goes over more pages than are fetched at a time."""
+    _check([(5000, 129), (4700, 40)], 4480, 128, 0.0, nh=2)
+    _check([(5000, 70)], 4300, 192, 0.0, nh=2)
 
 
 def test_two_outputs_are_the_more_exact():

@@ -552,9 +552,7 @@ __global__ void __launch_bounds__(F::THREADS, F::BLOCKS) attention_prefill_tcgen
                         }
                         mm = cm;
                     }
-                    float inv = 1.0f / ll;
-                    if (gate) inv = gated(inv, gate, gate_ld, tok0 + r, h);
-                    write(d0, acc, inv);
+                    write(d0, acc, 1.0f / ll);      // (no gate: the launches that have one do not cut their walks)
                 }
             }
         }
@@ -609,20 +607,58 @@ static int launch_ap(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
 
 using namespace vk;
 
-// Which form a launch for heads of 64 takes: 0 two groups and two blocks a multiprocessor, 1 four groups and one block, 2 (default) by the size of the launch.
+// Which form a launch for heads of 64 takes: 0 two groups and two blocks a multiprocessor, 1 four groups and one block, 2 (default) by the size of the launch, 3 one
+// group and three blocks.
 static int g_prefill_streams_mode = -1;
 static int prefill_streams_mode() {
     if (g_prefill_streams_mode < 0) {
         const char* e = getenv("VITNA_ATT_STREAMS");
-        g_prefill_streams_mode = e ? (atoi(e) ? 1 : 0) : 2;
+        g_prefill_streams_mode = e ? (atoi(e) == 3 ? 3 : atoi(e) ? 1 : 0) : 2;
     }
     return g_prefill_streams_mode;
 }
 // Returns the mode that was in force.
 VK_API int vk_set_prefill_streams(int mode) {
     const int was = prefill_streams_mode();
-    if (mode >= 0 && mode <= 2) g_prefill_streams_mode = mode;
+    if (mode >= 0 && mode <= 3) g_prefill_streams_mode = mode;
     return was;
+}
+
+// How a launch for heads of 64 is worked out: the steps of a part, the parts that a tile can have, and the softmax groups of the form (1, 2 or 4).
+struct ApPlan {
+    int part_steps, parts, groups;
+};
+static ApPlan ap_plan(int n_tiles, int nh, int window, int grid_context) {
+    // Walks are cut only when the launch has fewer blocks than three quarters of the multiprocessors (a portion of a few
+    // hundred tokens far into a context): measured, a part costs about five key steps of set-up, meeting and adding
+    // up, which a whole prompt's launch (a block or more a multiprocessor already) does not win back.
+    // VITNA_ATT_PART=n (n >= 16) cuts every launch into parts of n steps, for measurements.
+    static const int forced = [] { const char* e = getenv("VITNA_ATT_PART"); const int v = e ? atoi(e) : 0; return v >= AP_PART ? v : 0; }();
+    const bool cut = forced || (long long)n_tiles * nh * 4 <= (long long)148 * 3;
+    const int part_steps = forced ? forced : cut ? AP_PART : (1 << 24);      // never below AP_PART: the scratch is laid out for that
+    // The steps of the longest walk that a tile can have.  Under a window its rows' keys lie within window + 126 positions of each other: without that bound a window's cut
+    // launch had blocks for parts that no tile reaches, and real ones came to lie two on a multiprocessor (20 heads, 4 portions of 128 behind 3,000 tokens, window 256: 14.1 -> 17.0 us).
+    const int steps = (grid_context - 1) / AP_BN + 1;
+    const int walk = window > 0 ? (int)min((long long)steps, ((long long)window + AP_BM - 2) / AP_BN + 2) : steps;
+    const int parts = cut ? (walk - 1) / part_steps + 1 : 1;
+    // Which form.
+    //   Two groups and two blocks a multiprocessor where there are blocks for it: 32 heads and 8,192 / 2,048 tokens (2,048 and 512 blocks) 442 / 47 us against 529 / 56 with
+    //     four groups in one block; and for short walks in few blocks, which end before four groups have begun (a window of 64, 300 tokens of 9 heads 9.9 against 10.4).
+    //   Four groups, and two outputs, where a block has a multiprocessor to itself, or two or three share one for a long walk: 9 heads and 2,048 tokens (144 blocks) 25.3
+    //     against 27.3, 2,600 (189) 30.7 against 34.2, 4,096 (288) 49.1 against 53.3; 100 tokens 6,000 into a context (nine blocks, cut) 25.2 against 29.1.  From 297 to 369
+    //     blocks two groups are 13 % the faster and their one output rounds 25 % more results to the wrong bfloat16: the two outputs' sums are worth that.
+    //   One group and three blocks for many blocks of walks that have nothing to overlap inside a block: 32 heads and 32 portions of 16 tokens 20.9 us with the kernel
+    //     before, 24.1 with two groups, 18.6 with one; three and four steps in more than 600 blocks 1.06 and 0.91 of that kernel's time.
+    // VITNA_ATT_STREAMS=0 / 1 / 3 in the environment, or vk_set_prefill_streams, forces one (tests, measurements).
+    const int mode = prefill_streams_mode();
+    const long long blocks = (long long)n_tiles * parts * nh;
+    const int groups = mode != 2 ? (mode == 3 ? 1 : mode == 1 ? 4 : 2) : walk <= 4 && blocks > 296 ? 1 : walk > 8 && blocks < 370 ? 4 : 2;
+    return {part_steps, parts, groups};
+}
+// For tests: the groups of the form that such a launch takes, and 16 times the parts that a tile can have.
+VK_API int vk_attention_prefill_plan(int n_tiles, int nh, int window, int grid_context) {
+    const ApPlan p = ap_plan(n_tiles, nh, window, grid_context);
+    return p.groups + 16 * p.parts;
 }
 
 // Bytes of scratch for launches of up to cap_tiles tiles whose contexts reach max_context positions: the parts' outputs,
@@ -662,39 +698,30 @@ VK_API int vk_attention_prefill_tcgen05(const void* q, const void* cache, const 
     sc.part_o = (float*)scratch;
     sc.part_ml = (float*)((char*)scratch + up((size_t)cap_tiles * nh * max_parts * AP_BM * 64 * 4));
     sc.counters = (int*)((char*)sc.part_ml + up((size_t)cap_tiles * nh * max_parts * AP_BM * 2 * 4));
-    // Walks are cut only when the launch has fewer blocks than three quarters of the multiprocessors (a portion of a few
-    // hundred tokens far into a context): measured, a part costs about five key steps of set-up, meeting and adding
-    // up, which a whole prompt's launch (a block or more a multiprocessor already) does not win back.
-    // VITNA_ATT_PART=n (n >= 16) cuts every launch into parts of n steps, for measurements.
-    static const int forced = [] { const char* e = getenv("VITNA_ATT_PART"); const int v = e ? atoi(e) : 0; return v >= AP_PART ? v : 0; }();
-    const bool cut = forced || (long long)n_tiles * nh * 4 <= (long long)148 * 3;
-    sc.part_steps = forced ? forced : cut ? AP_PART : (1 << 24);      // never below AP_PART: the scratch is laid out for that
-    sc.parts = cut ? ((grid_context - 1) / AP_BN) / sc.part_steps + 1 : 1;
+    const ApPlan plan = ap_plan(n_tiles, nh, window, grid_context);
+    sc.part_steps = plan.part_steps;
+    sc.parts = plan.parts;
     sc.n_tiles = n_tiles;
     if ((long long)n_tiles * sc.parts * nh > 0x7fffffffll) return VK_TOO_LARGE;
-    // Which form.  Two groups and two blocks a multiprocessor where there are blocks for it: 32 heads and 8,192 / 2,048 tokens (2,048 and 512 blocks) 442 / 47 us against
-    // 529 / 56 with four groups in one block.  Four groups, and two outputs, where a block has a multiprocessor to itself, or two or three share one for a long walk:
-    // 9 heads and 2,048 tokens (144 blocks) 25.3 against 27.3, 2,600 (189) 30.7 against 34.2, 4,096 (288) 49.1 against 53.3; 100 tokens 6,000 into a context (nine blocks, cut)
-    // 25.2 against 29.1.  From 297 to 369 blocks two groups are 13 % the faster and their one output rounds 25 % more results to the wrong bfloat16: the two outputs' sums
-    // are worth that.
-    // VITNA_ATT_STREAMS=0 / 1 in the environment, or vk_set_prefill_streams, forces one or the other (tests, measurements).
-    const int forced_form = prefill_streams_mode();
-    const long long blocks = (long long)n_tiles * sc.parts * nh;
-    const bool four = forced_form == 2 ? blocks <= 148 || (blocks < 370 && grid_context > 512) : forced_form == 1;
     CUtensorMap mk, mv;
     const long long page_elems = 2ll * nkv * page_size * hd;
     if (!ap_make_page_map(&mk, cache, hd, nkv * page_size, pages, page_elems, box_rows) ||
         !ap_make_page_map(&mv, (const __nv_bfloat16*)cache + (size_t)nkv * page_size * hd, hd, nkv * page_size, pages, page_elems, box_rows))
         return VK_BAD_SHAPE;
-    if (four)
-        return launch_ap<ApForm<64, 64, 4, 5, 5, 1, 2>>(mq, mk, mv, block_tables, tiles, out, nh, nkv, page_size, max_blocks, scale, window, nh * hd, nullptr, 0, error, sc, stream);
-    return launch_ap<ApForm<64, 64, 2, 3, 4, 2>>(mq, mk, mv, block_tables, tiles, out, nh, nkv, page_size, max_blocks, scale, window, nh * hd, nullptr, 0, error, sc, stream);
+#define GO(...) \
+    return launch_ap<ApForm<__VA_ARGS__>>(mq, mk, mv, block_tables, tiles, out, nh, nkv, page_size, max_blocks, scale, window, nh * hd, nullptr, 0, error, sc, stream)
+    if (plan.groups == 4) GO(64, 64, 4, 5, 5, 1, 2);
+    if (plan.groups == 1) GO(64, 64, 1, 1, 2, 3);
+    GO(64, 64, 2, 3, 4, 2);
+#undef GO
 }
 
 // The same for keys of hd and values of vd values, one of them 128 and the other 64 or 128 (a page holds its keys [nkv][page_size][hd], then its values
 // [nkv][page_size][vd]); rows of out are out_ld elements apart; gate float32 [n_tokens][gate_ld] or null: head h of token t times sigmoid(gate[t][h]).  Walks are not
-// cut and there is no scratch.  Four groups and a block a multiprocessor (97 to 193 KB of shared memory); with two groups and two blocks, where tensor memory and
-// shared memory allow it (64 x 128 and 128 x 64), 16 heads and 2,048 tokens under a window of 1,024 took 30 and 27 us against 35, but whole prompts 39 to 69 against 35 to 57.
+// cut and there is no scratch.  Up to 148 blocks have a multiprocessor each: four groups (97 to 193 KB of shared memory).  More than that share them: two groups and two
+// blocks.  Four groups / two, of the time that the kernel before them took: 149 to 296 blocks, walks of 5 and 6 steps (windows of up to 256) 1.09 / 0.81 (64 x 128), 1.04 / 0.76
+// (128 x 64), 1.07 / 0.82 (128 x 128), of 41 steps and more 0.68 / 0.72, 0.73 / 0.67, 0.64 / 0.67; above 600 blocks 1.20 / 0.81, - and 1.09 / 0.75, 0.83 / 0.73 and 0.64 / 0.63.  In up to
+// 148 blocks walks of up to 6 steps are at 0.90 to 1.12 with four groups (0.92 to 1.15 with two), longer ones at 0.56 to 0.92 (0.64 to 1.09).
 VK_API int vk_attention_prefill_tcgen05_dims(const void* q, const void* cache, const int32_t* block_tables, const int32_t* tiles, void* out, int n_tokens, int n_tiles,
                                              int pages, int nh, int nkv, int hd, int vd, int page_size, int max_blocks, float scale, int window, int out_ld,
                                              const float* gate, int gate_ld, int* error, cudaStream_t stream) {
@@ -713,11 +740,12 @@ VK_API int vk_attention_prefill_tcgen05_dims(const void* q, const void* cache, c
     sc.parts = 1;
     sc.part_steps = 1 << 24;
     sc.n_tiles = n_tiles;
-#define GO(HD, VD) \
-    return launch_ap<ApForm<HD, VD, 4, 5, 5, 1>>(mq, mk, mv, block_tables, tiles, out, nh, nkv, page_size, max_blocks, scale, window, out_ld, gate, gate_ld, error, sc, stream)
-    if (hd == 128 && vd == 128) GO(128, 128);
-    if (hd == 64 && vd == 128) GO(64, 128);
-    if (hd == 128 && vd == 64) GO(128, 64);
+    const bool two = (long long)n_tiles * nh > 148;
+#define GO(...) \
+    return launch_ap<ApForm<__VA_ARGS__>>(mq, mk, mv, block_tables, tiles, out, nh, nkv, page_size, max_blocks, scale, window, out_ld, gate, gate_ld, error, sc, stream)
+    if (hd == 128 && vd == 128) { if (two) GO(128, 128, 2, 2, 2, 2); GO(128, 128, 4, 5, 5, 1); }
+    if (hd == 64 && vd == 128) { if (two) GO(64, 128, 2, 2, 3, 2); GO(64, 128, 4, 5, 5, 1); }
+    if (hd == 128 && vd == 64) { if (two) GO(128, 64, 2, 3, 3, 2); GO(128, 64, 4, 5, 5, 1); }
 #undef GO
     return VK_BAD_SHAPE;
 }

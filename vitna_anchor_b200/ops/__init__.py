@@ -684,7 +684,7 @@ def attention_prefill(q: torch.Tensor, cache_layer: torch.Tensor, block_tables: 
 
 def set_prefill_streams(mode: int) -> int:
     """Which form of the tcgen05 prompt attention a launch for heads of 64 takes: 0 two groups of softmax warps and two blocks a
-    multiprocessor, 1 four groups and one block, 2 by the size of the launch (the default).  Returns the mode that was in force."""
+    multiprocessor, 1 four groups and one block, 2 by the size of the launch (the default), 3 one group and three blocks.  Returns the mode that was in force."""
     return int(lib().vk_set_prefill_streams(int(mode)))
 
 
