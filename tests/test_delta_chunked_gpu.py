@@ -64,7 +64,7 @@ def test_a_wait_that_runs_out_is_reported():
         ops.skip_stage_once("delta_chunked", 1)
         go()
         torch.cuda.synchronize()
-        with pytest.raises(ops.KernelGaveUp):
+        with pytest.raises(ops.KernelGaveUp, match=r"code 61\)"):
             ops.check_device_errors()
         out = go()
         torch.cuda.synchronize()

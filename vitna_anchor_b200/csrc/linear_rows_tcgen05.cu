@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
                 if (kb != wc.skip_stage) tma_load_2d(smem + kb * STAGE_BYTES + W_BYTES, &map_x, (kb0 + kb) * RT_BK, 0, &full[kb]);
             for (int kb = early; kb < n_kb; kb++) {
                 const int s = kb % RT_STAGES;
-                if (!mbar_wait(&empty[s], ((kb / RT_STAGES) & 1) ^ 1, wc.cycles)) { give_up(wc.error, &failed, 61); break; }
+                if (!mbar_wait(&empty[s], ((kb / RT_STAGES) & 1) ^ 1, wc.cycles)) { give_up(wc.error, &failed, 71); break; }
                 if (kb == wc.skip_stage) continue;
                 mbar_expect_tx(&full[s], STAGE_BYTES);
                 load_w(kb, s);
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
             uint32_t acc = tmem, add = 0;              // the first product of an accumulator writes it
             for (int kb = 0; kb < n_kb; kb++) {
                 const int s = kb % RT_STAGES;
-                if (!mbar_wait(&full[s], (kb / RT_STAGES) & 1, wc.cycles)) { give_up(wc.error, &failed, 62); break; }
+                if (!mbar_wait(&full[s], (kb / RT_STAGES) & 1, wc.cycles)) { give_up(wc.error, &failed, 72); break; }
                 tc_fence_after();
                 const uint32_t w_lo = w_lo0 + s * (STAGE_BYTES >> 4), x_lo = w_lo + (W_BYTES >> 4);
 #pragma unroll
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
             umma_commit(acc_full);                     // arrives when every instruction has written the accumulator
         }
     } else {
-        if (!mbar_wait(acc_full, 0, wc.cycles)) { if (lane == 0) give_up(wc.error, &failed, 63); }
+        if (!mbar_wait(acc_full, 0, wc.cycles)) { if (lane == 0) give_up(wc.error, &failed, 73); }
         __syncwarp();
         const int quarter = warp & 3;
         const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16);

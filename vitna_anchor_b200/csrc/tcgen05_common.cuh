@@ -157,7 +157,8 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// A bounded wait ran out: tell the block and the host (error may be a mapped host word: a plain store).
+// A bounded wait ran out: tell the block and the host (error may be a mapped host word: a plain store).  The codes say whose: 1 to 3 narrow products, 11 to 23 prompt
+// attention, 31 to 34 wide products, 41 decoding attention, 61 the delta rule's scan, 71 to 73 few-rows products.
 __device__ __forceinline__ void give_up(int* error, int* failed, int code) {
     *reinterpret_cast<volatile int*>(failed) = 1;
     *reinterpret_cast<volatile int*>(error) = code;
