@@ -152,13 +152,6 @@ __device__ __forceinline__ float ap_largest32(const uint32_t* s) {
         for (int u = 0; u < 4; u++) m[u] = ap_max3(m[u], __uint_as_float(s[j + 2 * u]), __uint_as_float(s[j + 2 * u + 1]));
     return fmaxf(ap_max3(m[0], m[1], m[2]), m[3]);
 }
-__device__ __forceinline__ void ap_tmem_ld16(uint32_t taddr, uint32_t* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-                   "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr)
-                 : "memory");
-}
 __device__ __forceinline__ void ap_tmem_st16(uint32_t taddr, const uint32_t* r) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
@@ -404,7 +397,7 @@ __global__ void __launch_bounds__(F::THREADS, F::BLOCKS) attention_prefill_tcgen
 #pragma unroll 1
                 for (int c = 0; c < OUTS * VD; c += 16) {       // (an output that no product has been added to yet is written whole by its first)
                     uint32_t orr[16];
-                    ap_tmem_ld16(my_o + c, orr);
+                    tmem_ld16(my_o + c, orr);
 #pragma unroll
                     for (int j = 0; j < 16; j++) orr[j] = __float_as_uint(__uint_as_float(orr[j]) * alpha);
                     ap_tmem_st16(my_o + c, orr);
@@ -496,13 +489,13 @@ __global__ void __launch_bounds__(F::THREADS, F::BLOCKS) attention_prefill_tcgen
                 uint32_t o[16];
                 float acc[16];
                 __syncwarp();
-                ap_tmem_ld16(my_o + c + d0, o);
+                tmem_ld16(my_o + c + d0, o);
 #pragma unroll
                 for (int d = 0; d < 16; d++) acc[d] = __uint_as_float(o[d]);
 #pragma unroll
                 for (int u = 1; u < OUTS; u++) {
                     if (u >= n_it) break;
-                    ap_tmem_ld16(my_o + u * VD + c + d0, o);
+                    tmem_ld16(my_o + u * VD + c + d0, o);
 #pragma unroll
                     for (int d = 0; d < 16; d++) acc[d] += __uint_as_float(o[d]);
                 }

@@ -44,24 +44,12 @@ struct RtArgs {
     int nh, nkv, hd, page_size;
 };
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-                   "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
-                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
-}
 __device__ __forceinline__ float4 ld_peer4(uint32_t local, int rank) {
     uint32_t at;
     float4 v;
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(local), "r"(rank));
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
     return v;
-}
-__device__ __forceinline__ void cluster_meet() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // The sums of four neighbouring weight rows for a batch row, over the cluster's blocks in their order.
 __device__ __forceinline__ float4 rt_sum4(const float* red, int m, int c, int splits) {
@@ -306,7 +294,7 @@ static bool rt_make_map(CUtensorMap* map, const void* base, int rows, int cols, 
 // Blocks that share a tile's K: as many as the multiprocessors have room for, at most eight (a cluster anywhere), at least one step of 64 columns each.
 static int rt_splits(int tiles, int K) {
     const int num_kb = (K + RT_BK - 1) / RT_BK;
-    int s = 148 / tiles;
+    int s = sm_count() / tiles;
     if (s > RT_MAX_SPLIT) s = RT_MAX_SPLIT;
     if (s > num_kb) s = num_kb;
     return s < 1 ? 1 : s;

@@ -475,10 +475,6 @@ constexpr int TW_BN = 256, TW_THREADS = 320;                     // warps 0 and 
 __host__ __device__ constexpr int tw_stages(bool pair) { return pair ? 6 : 4; }
 
 // What the two blocks of a pair say to each other.  All of it without multicast copies: every block loads what it needs.
-__device__ __forceinline__ void tw_pair_meet() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ uint32_t tw_at_first(const void* p) {          // the place in the first block's shared memory
     uint32_t at;
     asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at) : "r"(smem_u32(p)));
@@ -562,7 +558,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
     }
     tc_fence_before();
     __syncthreads();
-    if (PAIR) tw_pair_meet();                     // the other block's barriers are set up
+    if (PAIR) cluster_meet();                     // the other block's barriers are set up
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // Barriers and tensor memory are set up while the kernel in front ends (its last blocks hold no place that this one's single wave needs): a layer of a
@@ -846,11 +842,11 @@ __global__ void __launch_bounds__(TW_THREADS, 1) linear_tcgen05_wide_kernel(cons
     if (PAIR) __syncwarp();
     tc_fence_before();
     if (PAIR) {
-        tw_pair_meet();                       // what either block sends the other (copies' counts, arrivals) has come; the sums have been read
+        cluster_meet();                       // what either block sends the other (copies' counts, arrivals) has come; the sums have been read
         if (failed) {                         // (the same in both blocks: a thread that gave up has said so to both before it met the others)
             if (lane == 0) __nanosleep(200000);      // after a failed wait: let copies in flight land, in both blocks, before either leaves
             __syncwarp();
-            tw_pair_meet();
+            cluster_meet();
         }
         tc_fence_after();
         if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TM_COLS) : "memory");
@@ -904,16 +900,6 @@ static int launch_tc(const CUtensorMap& mx, const CUtensorMap& mw, void* out, in
     const int cols = EPI == TC_SWIGLU ? ex.inter : N;
     dim3 grid((cols + tile_cols - 1) / tile_cols, (M + TC_BM - 1) / TC_BM);
     return launch_dependent(kern, grid, dim3(TC_THREADS), smem, stream, mx, mw, mo, out, M, N, K, wc, exx);
-}
-
-static int sm_count() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    }
-    return n;
 }
 
 // Whether the wide variant takes a product that the narrow one would cut into tiles of `rows` weight rows (64 or 128), `cols` output columns each.  The narrow
