@@ -908,6 +908,7 @@ static int launch_tc(const CUtensorMap& mx, const CUtensorMap& mw, void* out, in
 // half the bytes an output.  Until a second round the narrow kernel starts and ends sooner.  Narrow / wide, us (weights in the second-level cache):
 //   64 rows, a round is 296 tiles:  2,048 x 960 x 576 (240) 5.4 / 6.3, 2,048 x 1,024 x 1,024 (256) 7.8 / 10.3, 1,301 x 1,746 x 576 (308) 12.0 / 8.0,
 //     2,048 x 1,746 x 576 (448) 13.1 / 9.8, 3,000 x 960 x 576 (360) 9.5 / 6.5, 8,192 x 320 x 4,096 (320) 40.7 / 21.2, 16,384 x 1,536 x 64 37 / 21
+//     two of them on a multiprocessor share its way to the operands, which a long K feels before that: 1,301 x 1,352 x 4,656 (242) 31.1 / 26.3, 1,301 x 960 x 2,560 (165) level
 //   128 rows, a round is 148 tiles:  1,000 x 2,048 x 1,536 (128) 9.4 / 9.9, 1,301 x 2,048 x 1,536 (176) 13.3 / 10.1; two to a multiprocessor share its way to
 //     the operands, so that with a short K, the epilogue most of it, the line is the second pair: 2,048 x 2,048 x 576 (256) 8.0 / 8.5;
 //     gate and up 1,024 x 1,536 (192 tiles) K 576 8.2 / 8.4, K 960 10.9 / 9.9, K 2,048 17.9 / 14.3
@@ -920,7 +921,7 @@ static bool wide_takes(int M, int out_cols, int K, int rows, int cols, bool sum 
     static const int forced = [] { const char* e = getenv("VITNA_TCGEN05_WIDE"); return e ? (e[0] == '1' ? 1 : 0) : 2; }();
     if (forced != 2) return forced == 1;
     const long long tiles = (long long)((M + TC_BM - 1) / TC_BM) * ((out_cols + cols - 1) / cols), sms = sm_count();
-    if (rows == 64) return tiles > 2 * sms;
+    if (rows == 64) return tiles > 2 * sms || (tiles > sms && K >= 4200);
     if (tiles > 2 * sms || (tiles > sms && K >= 768)) return !sum || K >= 320;
     return !sum && (K >= 8192 || (K >= 2048 && M >= 512 && tiles * 4 >= sms * 3));
 }
