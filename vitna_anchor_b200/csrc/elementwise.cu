@@ -291,11 +291,11 @@ VK_API int vk_embed_rows(const void* table, const int32_t* ids, float* x, int to
 //   n 576, 640     2,048 rows 0.86, 0.83;  2,800 1.04, 1.03;  3,552 1.13, 1.04;  3,600 0.93, 0.82;  5,000 0.96, 0.94;  7,000 1.13, 1.09
 //   n 704, 768     5,000 rows 0.86, 0.85;  7,000 1.04, 1.01;  8,192 1.01, 0.99;  n 832, 896  10,000 rows 1.01, 0.98;  16,384 1.11, 1.06;  n 960 and more  16,384 rows 1.01 and less
 // Small blocks bring many rows' trips to memory side by side; in great number they cost more to begin than their rows' work.  Eight rows a block come three blocks to
-// a multiprocessor: 3,552 rows are one round of theirs, which they end sooner than the warps from 2,400 rows on where n is up to 640 (bfloat16).
+// a multiprocessor: 3,552 rows are one round of theirs, which they end sooner than the warps from 2,700 rows on where n is below 700 (bfloat16).
 VK_API int vk_rmsnorm_warp_blocks(int out_rows, int n, int dtype) {
     if (n > 2048) return 0;
     const int most = n <= 512 ? 2048 : n < 700 ? 5000 : n < 800 ? 7000 : n < 960 ? 10000 : 0x7fffffff;
-    return out_rows <= most && !(dtype != 0 && n <= 640 && out_rows > 2400 && out_rows <= 3552);
+    return out_rows <= most && !(dtype != 0 && n < 700 && out_rows > 2700 && out_rows <= 3552);
 }
 
 VK_API int vk_rmsnorm_rows(const float* x, const float* w, const int32_t* rows, void* y, int out_rows, int n, float eps,
