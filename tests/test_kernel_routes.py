@@ -29,7 +29,7 @@ def test_few_rows_products(sizes, acc, taken):
 @pytest.mark.parametrize("sizes,route", [
     ((0, 8192, 790, 272), 0), ((0, 1301, 1746, 576), 0), ((0, 16384, 14678, 112), 0), ((2, 8192, 790, 272), 160), ((2, 16384, 1746, 576), 160), ((2, 16384, 6104, 256), 0),
     ((3, 8192, 1536, 576), 192), ((3, 16384, 3072, 768), 256), ((1, 16384, 1746, 576), 256), ((1, 1000, 4096, 4096), 256), ((2, 1301, 2560, 4096), 256), ((2, 4096, 674, 3536), 192),
-    ((0, 8192, 6144, 2048), 257), ((3, 8192, 8192, 2048), 257), ((2, 8192, 2048, 8192), 257), ((2, 2048, 2048, 8192), 257), ((0, 3000, 1001, 1000), 192),
+    ((0, 8192, 6144, 2048), 257), ((3, 8192, 8192, 2048), 257), ((2, 8192, 2048, 8192), 257), ((2, 2048, 2048, 8192), 257), ((0, 3000, 1001, 1000), 192), ((0, 1301, 1352, 4656), 160), ((1, 1000, 1178, 4472), 160), ((0, 1301, 960, 2560), 0),
     ((4, 8192, 6144, 2048), 257), ((5, 8192, 2560, 2048), 257), ((1, 3000, 960, 4096), 161)])
 def test_wide_products(sizes, route):
     assert ops.lib().vk_linear_tcgen05_route(*sizes) == route
@@ -37,7 +37,7 @@ def test_wide_products(sizes, route):
 
 # (rows, columns, type of the result: 0 float32, 1 bfloat16): where a warp a row was measured to be slower than eight rows a block, and where it is the faster one
 @pytest.mark.parametrize("sizes,warps", [
-    ((3000, 64, 1), False), ((4096, 256, 0), False), ((3000, 576, 1), False), ((3552, 640, 1), False), ((7000, 640, 1), False), ((16384, 644, 1), False), ((16384, 768, 1), False),
+    ((3000, 64, 1), False), ((4096, 256, 0), False), ((3000, 576, 1), False), ((3552, 640, 1), False), ((3200, 644, 1), False), ((7000, 640, 1), False), ((16384, 644, 1), False), ((16384, 768, 1), False),
     ((16384, 576, 0), False), ((16, 2052, 1), False),
     ((64, 2048, 1), True), ((1, 576, 1), True), ((2048, 576, 1), True), ((3000, 576, 0), True), ((4096, 576, 1), True), ((2048, 960, 1), True), ((8192, 2048, 1), True), ((16384, 960, 1), True)])
 def test_norms(sizes, warps):

@@ -79,9 +79,9 @@ def test_cut_walks_under_windows(form):
     from vitna_anchor_b200 import ops
     assert ops.lib().vk_attention_prefill_plan(4, 2, 1100, 3100) // 16 == 2 and ops.lib().vk_attention_prefill_plan(4, 2, 0, 3100) // 16 == 4
     _check([(2900, 128), (2945, 130), (0, 60)], 1100, 16, 0.0, nh=2)
-    assert ops.lib().vk_attention_prefill_plan(4, 2, 1026, 3100) // 16 == 2 and ops.lib().vk_attention_prefill_plan(4, 2, 834, 3100) // 16 == 1
+    assert ops.lib().vk_attention_prefill_plan(4, 2, 1026, 3100) // 16 == 2 and ops.lib().vk_attention_prefill_plan(4, 2, 833, 3100) // 16 == 1
     _check([(2945, 128), (3000, 100)], 1026, 16, 0.0, nh=2)
-    _check([(2945, 128), (2950, 128)], 834, 8, 9.0, nh=2)
+    _check([(2945, 128), (2950, 128)], 833, 8, 9.0, nh=2)
 
 
 def test_long_windows_over_large_pages(form):
