@@ -98,12 +98,29 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
     const uint32_t tm_cols = rt_tmem_columns(NB, p.accs);
     const int num_kb = (p.K + RT_BK - 1) / RT_BK, kb0 = rank * num_kb / splits, n_kb = (rank + 1) * num_kb / splits - kb0;      // at least one
 
+    auto load_w = [&](int kb, int s) {
+        uint8_t* dst = smem + s * STAGE_BYTES;
+        if (EPI == RT_SWIGLU) {                // 64 gate rows and the same 64 up rows: the map's box is 64 rows
+            tma_load_2d(dst, &map_w, (kb0 + kb) * RT_BK, n0, &full[s]);
+            tma_load_2d(dst + W_BYTES / 2, &map_w, (kb0 + kb) * RT_BK, p.N / 2 + n0, &full[s]);
+        } else {
+            tma_load_2d(dst, &map_w, (kb0 + kb) * RT_BK, n0, &full[s]);
+        }
+    };
+    // (a stage named by wc.skip_stage is left unarmed and unfilled: a test of the give-up path)
+    const int early = n_kb < RT_STAGES ? n_kb : RT_STAGES;
     if (threadIdx.x == 0) {
         failed = 0;
         for (int s = 0; s < RT_STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         mbar_init(acc_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        // the first weights, before the block has its tensor memory: under the end of a kernel whose blocks hold the multiprocessor's, that is a long wait
+        for (int kb = 0; kb < early; kb++) {
+            if (kb == wc.skip_stage) continue;
+            mbar_expect_tx(&full[kb], STAGE_BYTES);
+            load_w(kb, kb);
+        }
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tm_cols) : "memory");
@@ -116,22 +133,6 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
 
     if (warp == 0) {
         if (lane == 0) {
-            auto load_w = [&](int kb, int s) {
-                uint8_t* dst = smem + s * STAGE_BYTES;
-                if (EPI == RT_SWIGLU) {                // 64 gate rows and the same 64 up rows: the map's box is 64 rows
-                    tma_load_2d(dst, &map_w, (kb0 + kb) * RT_BK, n0, &full[s]);
-                    tma_load_2d(dst + W_BYTES / 2, &map_w, (kb0 + kb) * RT_BK, p.N / 2 + n0, &full[s]);
-                } else {
-                    tma_load_2d(dst, &map_w, (kb0 + kb) * RT_BK, n0, &full[s]);
-                }
-            };
-            // (a stage named by wc.skip_stage is left unarmed and unfilled: a test of the give-up path)
-            const int early = n_kb < RT_STAGES ? n_kb : RT_STAGES;
-            for (int kb = 0; kb < early; kb++) {
-                if (kb == wc.skip_stage) continue;
-                mbar_expect_tx(&full[kb], STAGE_BYTES);
-                load_w(kb, kb);
-            }
             dependency_wait();
             for (int kb = 0; kb < early; kb++)
                 if (kb != wc.skip_stage) tma_load_2d(smem + kb * STAGE_BYTES + W_BYTES, &map_x, (kb0 + kb) * RT_BK, 0, &full[kb]);
