@@ -491,10 +491,11 @@ def rows_tcgen05_sizes(M: int, N: int, K: int, acc: bool = False) -> bool:
     weights that are not in the second-level cache, microseconds, what stands in otherwise (up to 8 rows, and up to 8,192 columns: the mma.sync kernels; else
     128-row tiles) against this one:
       up to 8 rows, norm in front   49152 x 576 18.4 / 13.4, 32000 x 1024 16.0 / 15.8;  16384 x 1536 12.3 / 13.0, 6144 x 2048 8.3 / 8.6 (not taken)
-      9 to 16 rows   6144 x 2048 12.7 / 8.6, 2048 x 8192 14.1 / 11.0;  2048 x 2048 4.8 / 5.8, 4096 x 1024 4.5 / 5.7, 5120 x 960 5.3 / 6.5, 7680 x 1536 7.8 / 8.8 (not taken:
-                     the mma.sync kernels' blocks norm and stage so few rows once)
+      9 to 16 rows   6144 x 2048 12.7 / 8.6, 2048 x 8192 14.1 / 11.0;  2048 x 2048 4.8 / 5.8, 4096 x 1024 4.5 / 5.7, 7680 x 1536 7.8 / 8.8 (not taken:
+                     the mma.sync kernels' blocks norm and stage so few rows once);  16: a layer of the 360M sizes with 5120 x 960 gated 33.1 / 31.6
       17 to 64 rows, up to 8,192 columns   64: 6144 x 2048 28.9 / 10.4, 2048 x 8192 32.7 / 12.1, 1600 x 960 6.2 / 5.3;  K a multiple of 256, which the warps of the
-                     other kernel share evenly: 33 x 2048 x 2048 8.6 / 6.2, but 32 x 2048 x 2048 5.8 / 6.2, 64 x 1024 x 2048 5.3 / 5.7, 48 x 1536 x 1536 4.7 / 5.7
+                     other kernel share evenly: 33 x 2048 x 2048 8.6 / 6.2, but 32 x 2048 x 2048 5.8 / 6.2, 64 x 1024 x 2048 5.3 / 5.7, 48 x 1536 x 1536 4.7 / 5.7;
+                     more weights than that (a layer with them): 17 x 2560 x 2560 110.1 / 105.1, 17 x 1536 x 4096 42.9 / 38.9
       more columns   16: 49152 x 2048 57.6 / 33.4, 65536 x 512 16.9 / 15.0;  24: 42000 x 576 16.4 / 14.6;  32: 49152 x 960 25.3 / 22.4;  48: 16384 x 2048 18.7 / 16.5,
                      32000 x 1024 17.4 / 20.4 (not taken);  64: 16384 x 2048 18.4 / 16.9 and gated 22.1 / 18.8, into a sum 18.4 / 20.0 (not taken)
     A K that is no multiple of 32 stays with the other kernel's float32 multiply-adds, whose sums are the more exact (0.7 against 1.3e-7 of the result's size at K = 1,000),
@@ -505,8 +506,9 @@ def rows_tcgen05_sizes(M: int, N: int, K: int, acc: bool = False) -> bool:
         return N > 16384 and K < 2048 and K % 32 == 0 and N * K >= 24_000_000
     if N <= 8192:
         if M <= 16:
-            return N >= 512 and K >= 2048 and N * K >= 5_000_000
-        return N >= 512 and M * N * K >= (136_000_000 if K % 256 == 0 or N < 1536 else 60_000_000 if M > 32 else 80_000_000)
+            return N >= 512 and (K >= 2048 and N * K >= 5_000_000 or N >= 5000 and K % 256 != 0 and M * N * K >= 75_000_000)
+        shared = (K % 256 == 0 and N * K < 6_000_000) or N < 1536
+        return N >= 512 and M * N * K >= (136_000_000 if shared else 60_000_000 if M > 32 else 80_000_000)
     if not (N * K >= 24_000_000 and K < 2048 or K > NORM_IN_REGISTERS_MAX_K and M * N * K >= 60_000_000):
         return False
     if M <= 16:
@@ -514,7 +516,7 @@ def rows_tcgen05_sizes(M: int, N: int, K: int, acc: bool = False) -> bool:
     if acc:
         return False
     if M <= 32:
-        return N <= 18944 or M <= 24 or NORM_IN_REGISTERS_MAX_K < K < 2048
+        return M <= 24 or K > NORM_IN_REGISTERS_MAX_K
     return N <= 18944 if M <= 48 else N <= 16384 and K >= 2048
 
 
