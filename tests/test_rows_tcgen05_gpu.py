@@ -42,15 +42,19 @@ def test_results_and_sums(M, N, K):
 
 
 # one block a tile, two, three, seven and eight; 16, 32 and 64 columns of batch rows
-@pytest.mark.parametrize("M,N,K", [(1, 49152, 576), (8, 32000, 1024), (24, 49152, 960), (16, 8192, 2048), (40, 5120, 960), (64, 16384, 2048), (64, 6144, 2048), (32, 2560, 2560),
+@pytest.mark.parametrize("M,N,K", [(1, 49152, 576), (8, 32000, 1024), (8, 32768, 768), (24, 49152, 960), (16, 8192, 2048), (40, 5120, 960), (64, 16384, 2048), (64, 6144, 2048), (32, 2560, 2560),
                                    (64, 2048, 8192)])
 def test_sums_are_as_exact_as_the_kernel_it_stands_in_for(M, N, K):
-    """What is cut off of a sum in tensor memory grows with the products added one after another: no more of them than the mma.sync kernel's warps add."""
+    """What is cut off of a sum in tensor memory grows with the products added one after another: no more of them than the mma.sync kernel's warps add, or, for many
+    columns and more than eight rows, the tile kernel."""
     from vitna_anchor_b200 import ops
     _, x, w, want, _ = _operands(M, N, K, M + N + K)
     out, other = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
     ops.linear_rows_tcgen05(x, w, out, ops.EPI_F32)
-    ops.linear_skinny(x, w, other, ops.EPI_F32)
+    if M > 8 and N > 8192:
+        ops.linear_tcgen05(x, w, other, ops.LINEAR_F32)
+    else:
+        ops.linear_skinny(x, w, other, ops.EPI_F32)
     ops.check_device_errors()
     mine, theirs = float((out.double() - want).norm()), float((other.double() - want).norm())
     # both are norms over thousands of sums' rounding errors, which depend on their order: measured within 7 % of each other where the chains are as long

@@ -20,7 +20,8 @@
 // The tensor core cuts off what a sum in tensor memory has no bits for, every time that it adds to it, so that an error grows with the products that are added to
 // one accumulator one after another.  The mma.sync kernels split K over a block's eight warps; here the blocks of a cluster and the accumulators that a block's
 // products go to in turn (`accs`) make as many such chains of an output.  Error against 64 bits over the result's size (2-norms, random operands), the mma.sync kernel / one
-// accumulator a block / as here, in 1e-7: 49,152 x 576 1.09 / 5.5 / 0.96, 5,120 x 960 1.53 / 2.9 / 1.12, 6,144 x 2,048 2.36 / 6.5 / 2.11, 16,384 x 2,048 2.35 / 20 / 2.34, 2,048 x 8,192 9.96 / 9.95 / 9.95 (there eight blocks share K).
+// accumulator a block / as here, in 1e-7: 49,152 x 576 1.09 / 5.5 / 0.97, 5,120 x 960 1.53 / 2.9 / 1.13, 6,144 x 2,048 2.36 / 6.5 / 2.1, 2,048 x 8,192 9.96 / 9.95 / 9.95 (eight blocks
+// share K there); 16,384 x 2,048, in tiles of 128 rows otherwise, 21 / 21 / 4.7.
 //
 // An output does not depend on M or on the other batch rows: the splits of K and the accumulators depend on N and K alone.  Every wait on an mbarrier is bounded (see
 // tcgen05_common.cuh); a block that gave up still meets its cluster.
@@ -69,6 +70,17 @@ __device__ __forceinline__ uint2 rt_pack4(float a, float b, float c, float d) {
     return make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
 }
 __device__ __forceinline__ float rt_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+
+// 16 or 32 columns of this thread's lane of tensor memory.
+template <int COLS>
+__device__ __forceinline__ void rt_load(uint32_t taddr, uint32_t* r) {
+    if constexpr (COLS == 16) {
+        tmem_ld16(taddr, r);
+    } else {
+        tmem_ld32(taddr, r);
+        tmem_loaded(r);
+    }
+}
 
 // Columns of tensor memory for `accs` accumulators of nb columns: a power of two, at least 32.
 __host__ __device__ __forceinline__ uint32_t rt_tmem_columns(int nb, int accs) {
@@ -149,15 +161,16 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
         if (lane == 0) {
             const uint32_t idesc = umma_idesc_bf16(RT_BM, NB);
             const uint32_t w_lo0 = umma_desc_lo(smem_u32(smem)), acc_end = tmem + NB * p.accs;
-            uint32_t acc = tmem, add = 0;              // the first product of an accumulator writes it
+            uint32_t acc = tmem, add = 0;              // the first product of an accumulator writes it; half a stage's products go to one
             for (int kb = 0; kb < n_kb; kb++) {
                 const int s = kb % RT_STAGES;
                 if (!mbar_wait(&full[s], (kb / RT_STAGES) & 1, wc.cycles)) { give_up(wc.error, &failed, 72); break; }
                 tc_fence_after();
                 const uint32_t w_lo = w_lo0 + s * (STAGE_BYTES >> 4), x_lo = w_lo + (W_BYTES >> 4);
 #pragma unroll
-                for (int k = 0; k < RT_BK / 16; k++) {
+                for (int k = 0; k < RT_BK / 16; k += 2) {
                     umma_bf16_lo(acc, w_lo + 2 * k, x_lo + 2 * k, idesc, add);
+                    umma_bf16_lo(acc, w_lo + 2 * k + 2, x_lo + 2 * k + 2, idesc, 1);
                     acc += NB;
                     if (acc == acc_end) { acc = tmem; add = 1; }
                 }
@@ -175,27 +188,21 @@ __global__ void __launch_bounds__(RT_THREADS) linear_rows_tcgen05_kernel(const _
         tc_fence_after();
         if (__all_sync(0xffffffffu, ok)) {
             float* mine = red + quarter * 32 + lane;
-            const int used = min(p.accs, n_kb * (RT_BK / 16));
+            const int used = min(p.accs, n_kb * (RT_BK / 32));
             constexpr int COLS = NB < 32 ? NB : 32;
-#pragma unroll 1
+#pragma unroll
             for (int c = 0; c < NB; c += COLS) {
-                float sum[COLS];
-#pragma unroll
-                for (int j = 0; j < COLS; j++) sum[j] = 0.0f;
+                uint32_t sum[COLS];
+                rt_load<COLS>(acc + c, sum);
 #pragma unroll 1
-                for (int a = 0; a < used; a++) {
+                for (int a = 1; a < used; a++) {
                     uint32_t r[COLS];
-                    if constexpr (NB == 16) {
-                        tmem_ld16(acc + a * NB, r);
-                    } else {
-                        tmem_ld32(acc + a * NB + c, r);
-                        tmem_loaded(r);
-                    }
+                    rt_load<COLS>(acc + a * NB + c, r);
 #pragma unroll
-                    for (int j = 0; j < COLS; j++) sum[j] += __uint_as_float(r[j]);
+                    for (int j = 0; j < COLS; j++) sum[j] = __float_as_uint(__uint_as_float(sum[j]) + __uint_as_float(r[j]));
                 }
 #pragma unroll
-                for (int j = 0; j < COLS; j++) mine[(c + j) * RT_BM] = sum[j];
+                for (int j = 0; j < COLS; j++) mine[(c + j) * RT_BM] = __uint_as_float(sum[j]);
             }
         }
         tc_fence_before();
@@ -300,8 +307,13 @@ static int rt_splits(int tiles, int K) {
     return s < 1 ? 1 : s;
 }
 
-// Accumulators of a block: with the splits of K, at least RT_CHAINS chains of an output's products.  (Eight of 64 columns are all of the tensor memory.)
-static int rt_accs(int splits) { return (RT_CHAINS + splits - 1) / splits; }
+// Accumulators of a block: with the splits of K, RT_CHAINS chains of an output's products; but four where K is long and not split (matrices of more than 8,192 columns,
+// which tiles of 128 rows with one accumulator have otherwise): eight of 64 columns are all of a multiprocessor's tensor memory, and the next launch's blocks
+// cannot begin beside them (a layer of 1.7B with 64 decoding requests 224.8 us with four for gate and up, 233.5 with eight).
+static int rt_accs(int splits, int K) {
+    const int a = (RT_CHAINS + splits - 1) / splits;
+    return K >= 2048 && a > 4 ? 4 : a;
+}
 
 template <int NB, int EPI>
 static int rt_launch(const CUtensorMap& mx, const CUtensorMap& mw, RtArgs p, int* error, cudaStream_t stream) {
@@ -313,7 +325,7 @@ static int rt_launch(const CUtensorMap& mx, const CUtensorMap& mw, RtArgs p, int
     const int per_tile = EPI == RT_SWIGLU ? RT_BM / 2 : RT_BM, cols = EPI == RT_SWIGLU ? p.N / 2 : p.N;
     const int tiles = (cols + per_tile - 1) / per_tile;
     p.splits = rt_splits(tiles, p.K);
-    p.accs = rt_accs(p.splits);
+    p.accs = rt_accs(p.splits, p.K);
     return launch_dependent_cluster(kern, dim3(tiles * p.splits), dim3(RT_THREADS), p.splits, smem, stream, mx, mw, p, wc);
 }
 
