@@ -16,12 +16,12 @@ def test_delta_rule_preparation(sizes, sliced):
 # (rows, columns, K), into a sum or not: where the few-rows tcgen05 product was measured to be slower, or less exact, than what stands in, and where it is the faster one
 @pytest.mark.parametrize("sizes,acc,taken", [
     ((8, 16384, 1536), False, False), ((4, 12800, 1920), False, False), ((8, 6144, 2048), False, False), ((16, 2048, 2048), False, False), ((16, 4096, 1024), False, False),
-    ((12, 5120, 960), False, False), ((32, 2112, 1024), False, False), ((28, 2048, 2048), True, False), ((40, 16384, 1536), False, False), ((64, 1024, 1056), False, False), ((48, 1536, 1536), False, False),
+    ((12, 5120, 960), False, False), ((32, 2112, 1024), False, False), ((28, 2048, 2048), True, False), ((40, 16384, 1536), False, False), ((64, 1024, 1056), False, False), ((33, 1536, 1536), False, False), ((32, 1600, 960), False, False), ((64, 768, 2048), True, False),
     ((64, 49152, 576), False, False), ((40, 49152, 960), False, False), ((64, 131072, 192), False, False), ((8, 131072, 192), False, False), ((64, 16384, 2048), True, False),
     ((64, 2048, 1000), False, False), ((64, 6144, 2056), False, False), ((64, 576, 576), False, False),
     ((1, 49152, 576), False, True), ((8, 49152, 960), False, True), ((16, 49152, 2048), False, True), ((16, 2048, 8192), True, True), ((64, 6144, 2048), False, True),
     ((64, 2048, 8192), True, True), ((64, 2048, 2048), True, True), ((64, 16384, 2048), False, True), ((64, 1600, 960), False, True), ((32, 49152, 960), False, True), ((16, 5120, 960), False, True), ((17, 2560, 2560), True, True),
-    ((17, 1536, 4096), True, True), ((32, 22016, 4096), False, True)])
+    ((17, 1536, 4096), True, True), ((33, 1600, 960), False, True), ((33, 960, 2560), True, True), ((32, 22016, 4096), False, True)])
 def test_few_rows_products(sizes, acc, taken):
     assert ops.rows_tcgen05_sizes(*sizes, acc) == taken
 

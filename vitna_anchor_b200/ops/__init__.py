@@ -494,8 +494,9 @@ def rows_tcgen05_sizes(M: int, N: int, K: int, acc: bool = False) -> bool:
       9 to 16 rows   6144 x 2048 12.7 / 8.6, 2048 x 8192 14.1 / 11.0;  2048 x 2048 4.8 / 5.8, 4096 x 1024 4.5 / 5.7, 7680 x 1536 7.8 / 8.8 (not taken:
                      the mma.sync kernels' blocks norm and stage so few rows once);  16: a layer of the 360M sizes with 5120 x 960 gated 33.1 / 31.6
       17 to 64 rows, up to 8,192 columns   64: 6144 x 2048 28.9 / 10.4, 2048 x 8192 32.7 / 12.1, 1600 x 960 6.2 / 5.3;  K a multiple of 256, which the warps of the
-                     other kernel share evenly: 33 x 2048 x 2048 8.6 / 6.2, but 24 x 2048 x 2048 5.7 / 6.0, 64 x 1024 x 2048 5.3 / 5.7, 48 x 1536 x 1536 4.7 / 5.7;
-                     more weights than that (a layer with them): 17 x 2560 x 2560 110.1 / 105.1, 17 x 1536 x 4096 42.9 / 38.9
+                     other kernel share evenly: 33 x 2048 x 2048 8.6 / 6.2, but 24 x 2048 x 2048 5.7 / 6.0, 64 x 1024 x 2048 5.3 / 5.7, 33 x 1536 x 1536 4.7 / 5.4;
+                     more weights than that (a layer with them): 17 x 2560 x 2560 110.1 / 105.1, 17 x 1536 x 4096 42.9 / 38.9;  a whole step of the 360M sizes, 33: 1600 x 960
+                     1096 / 1060 and 960 x 2560 with it 1040, 48: 1164 / 1144 and 1126, but 32: 998 / 1032 and 994 / 1023
       more columns   16: 49152 x 2048 57.6 / 33.4, 65536 x 512 16.9 / 15.0;  24: 42000 x 576 16.4 / 14.6;  32: 49152 x 960 25.3 / 22.4;  48: 16384 x 2048 18.7 / 16.5,
                      32000 x 1024 17.4 / 20.4 (not taken: eight accumulators of 64 columns leave no tensor memory for a second block);  64: 16384 x 2048 18.4 / 16.9 and gated 22.1 / 18.8, into a sum 18.4 / 20.0 (not taken)
     A K that is no multiple of 32 stays with the other kernel's float32 multiply-adds, whose sums are the more exact (0.7 against 1.3e-7 of the result's size at K = 1,000),
@@ -508,7 +509,9 @@ def rows_tcgen05_sizes(M: int, N: int, K: int, acc: bool = False) -> bool:
         if M <= 16:
             return N >= 512 and (K >= 2048 and N * K >= 5_000_000 or N >= 5000 and K % 256 != 0 and M * N * K >= 75_000_000)
         shared = K % 256 == 0 and N * K < 6_000_000
-        return N >= 512 and M * N * K >= (136_000_000 if N < 1536 else 128_000_000 if shared else 60_000_000 if M > 32 else 80_000_000)
+        if M <= 32:
+            return N >= 512 and M * N * K >= (136_000_000 if N < 1536 else 128_000_000 if shared else 80_000_000)
+        return N >= 512 and M * N * K >= (136_000_000 if N < 900 else 80_000_000 if shared or N < 1536 else 50_000_000)
     if not (N * K >= 24_000_000 and K < 2048 or K > NORM_IN_REGISTERS_MAX_K and M * N * K >= 60_000_000):
         return False
     if M <= 16:
