@@ -13,14 +13,14 @@
 //   all      the sums over the cluster, and the epilogue: a thread has four neighbouring output columns of a batch row
 //
 // Measured over weights that are not in the second-level cache, 64 rows, what stands in otherwise (mma.sync with the weights through registers up to 8,192 columns, else
-// tiles of 128 batch rows) / this: 6,144 x 2,048 26.8 / 10.9 us (2.3 TB/s), 2,048 x 8,192 into a sum 33.2 / 12.8 (2.6 TB/s), 16,384 x 2,048 gated 22.1 / 18.8 (3.6 TB/s; 128 tiles
-// are what 128 multiprocessors pull), 5,120 x 960 gated 15.5 / 8.6; 16 rows of 49,152 x 2,048 57.6 / 33.4 (6.0 TB/s), one of 49,152 x 576 18.8 / 10.9 (5.2 TB/s).  About 3.4 us of
+// tiles of 128 batch rows) / this: 6,144 x 2,048 26.8 / 10.4 us (2.4 TB/s), 2,048 x 8,192 into a sum 33.2 / 12.8 (2.6 TB/s), 16,384 x 2,048 gated 22.1 / 18.6 (3.6 TB/s; 128 tiles
+// are what 128 multiprocessors pull), 5,120 x 960 gated 15.5 / 8.5; 16 rows of 49,152 x 2,048 57.6 / 33.4 (6.0 TB/s), one of 49,152 x 576 18.8 / 10.9 (5.2 TB/s).  About 3.4 us of
 // a launch are not the stream: set-up, the first copies' way, the cluster's meeting and the epilogue; that is why small matrices stay with linear_skinny_mma.cu.
 //
 // The tensor core cuts off what a sum in tensor memory has no bits for, every time that it adds to it, so that an error grows with the products that are added to
 // one accumulator one after another.  The mma.sync kernels split K over a block's eight warps; here the blocks of a cluster and the accumulators that a block's
 // products go to in turn (`accs`) make as many such chains of an output.  Error against 64 bits over the result's size (2-norms, random operands), the mma.sync kernel / one
-// accumulator a block / as here, in 1e-7: 49,152 x 576 1.09 / 5.5 / 0.97, 5,120 x 960 1.53 / 2.9 / 1.13, 6,144 x 2,048 2.36 / 6.5 / 2.1, 2,048 x 8,192 9.96 / 9.95 / 9.95 (eight blocks
+// accumulator a block / as here, in 1e-7: 49,152 x 576 1.09 / 5.5 / 1.00, 5,120 x 960 1.53 / 2.9 / 1.14, 6,144 x 2,048 2.36 / 6.5 / 2.1, 2,048 x 8,192 9.96 / 9.95 / 9.95 (eight blocks
 // share K there); 16,384 x 2,048, in tiles of 128 rows otherwise, 21 / 21 / 4.7.
 //
 // An output does not depend on M or on the other batch rows: the splits of K and the accumulators depend on N and K alone.  Every wait on an mbarrier is bounded (see
